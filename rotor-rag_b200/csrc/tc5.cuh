@@ -50,6 +50,16 @@ __device__ __forceinline__ void t5_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         : "r"(taddr));
 }
 
+// The first 16 columns alone (the rest of v is left as it was).
+__device__ __forceinline__ void t5_ld16(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+
 // Read-back store of a warp's 32 tokens x 32 values (lane = token after tcgen05.ld) as whole 128-byte
 // rows: through a per-warp shared-memory block (32 rows of 144 bytes: conflict-free both ways) so that
 // one store instruction covers four tokens' rows (four lines) instead of one 16-byte piece of 32
@@ -187,6 +197,17 @@ __device__ __forceinline__ void t5_bar_expect(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void t5_tma_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+// The same for what is read once: its lines leave L2 first.
+__device__ __forceinline__ void t5_tma_2d_once(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "{\n\t"
+        ".reg .b64 pol;\n\t"
+        "createpolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], pol;\n\t"
+        "}\n" ::"r"(dst),
         "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
