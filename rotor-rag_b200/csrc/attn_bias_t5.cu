@@ -254,7 +254,7 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             }
         }
     } else if (warp == 8) {
-        if (lane == 0) {
+        if (elect_lane()) {
             for (int j = 0; j < ntiles; ++j) {
                 const int s = j & 1;
                 if (!t5_wait(smem_u32(&s_kempty[s]), ((uint32_t)(j >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x79000003u)) break;
@@ -268,7 +268,7 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             }
         }
     } else if (warp == 9) {
-        if (lane == 0) {
+        if (elect_lane()) {
             for (int j = 0; j < ntiles; ++j) {
                 const int s = j & 1;
                 if (!t5_wait(smem_u32(&s_vempty[s]), ((uint32_t)(j >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x79000009u)) break;
@@ -280,7 +280,7 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             }
         }
     } else {
-        if (lane == 0) {
+        if (elect_lane()) {
             constexpr uint32_t idesc_s = t5_idesc_bf16(128, B5_BN), idesc_o = t5_idesc_bf16(128, DV, true);
             const uint64_t dq = t5_desc(qbase);
             auto issue_s = [&](int j) {

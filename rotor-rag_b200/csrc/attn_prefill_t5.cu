@@ -470,7 +470,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
         }
     } else if (warp == 8) {
         // ---------------- K tiles by TMA
-        if (lane == 0) {
+        if (elect_lane()) {
             const int krow0 = ((b * p.n_kv_heads + hk) * p.split_seq);
             for (int j = 0; j < ntiles; ++j) {
                 const int s = j & 1;
@@ -496,7 +496,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
         }
     } else if (warp == 9) {
         // ---------------- V^T tiles by TMA
-        if (lane == 0) {
+        if (elect_lane()) {
             const int vrow0 = ((b * p.n_kv_heads + hk) * (p.split_seq / A5_BN)) * A5_D;
             for (int j = 0; j < ntiles; ++j) {
                 const int s = j & 1;
@@ -518,7 +518,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
         }
     } else {
         // ---------------- MMA issue
-        if (lane == 0) {
+        if (elect_lane()) {
             // kind::f16: float32 accumulate (bit 4), A and B bf16 (bits 7, 10), both K-major, N >> 3 at 17, M >> 4 at 24
             const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(A5_BN >> 3) << 17) | ((128u >> 4) << 24);
             const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(A5_D >> 3) << 17) | ((128u >> 4) << 24);

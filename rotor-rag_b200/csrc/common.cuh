@@ -127,6 +127,15 @@ __device__ __forceinline__ float block_max_alt(float v, float* scratch, int& k) 
     return warp_max(r);
 }
 
+// One lane of a whole, converged warp.  The compiler knows that exactly one lane runs the guarded code and keeps the
+// operands of tcgen05 and TMA instructions in uniform registers; behind `lane == 0` every operand is moved there one by
+// one (an MMA then took about 60 cycles to issue, here 16).
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t e;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(e));
+    return e != 0;
+}
+
 // L2 prefetch of the 128-byte line that holds `p` (constants a kernel will need after its
 // programmatic-launch wait).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }

@@ -132,7 +132,7 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_lane()) {
             int it = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
@@ -152,7 +152,7 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_lane()) {
             constexpr uint32_t idesc = t5_idesc_bf16(128, BN);
             int it = 0, lt = 0;
             bool ok = true;

@@ -375,7 +375,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
 #endif
     } else if (warp == NDW) {
         // ---------------- token operand by TMA
-        if (lane == 0) {
+        if (elect_lane()) {
             for (int kt = 0; kt < nk; ++kt) {
                 const int s = kt % T5_STAGES;
                 if (!t5_wait(smem_u32(&s_empty[s]), ((kt / T5_STAGES) & 1) ^ 1, abort_flag, p.status, 0x7c000003u)) break;
@@ -395,7 +395,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
         }
     } else {
         // ---------------- MMA issue
-        if (lane == 0) {
+        if (elect_lane()) {
             // kind::i8, S32 accumulate, signed tokens (A) x unsigned weight codes (B), both K-major, N = ROWS, M = 128
             const uint32_t idesc = (2u << 4) | (1u << 7) | (0u << 10) | ((uint32_t)(T5_ROWS >> 3) << 17) | ((128u >> 4) << 24);
             bool ok = true;

@@ -119,7 +119,7 @@ lmhead_t5_kernel(const __grid_constant__ CUtensorMap tm_e, const __grid_constant
     const uint32_t tmem = s_tmem;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_lane()) {
             // a stage's table rows (only those of the CTA's share: the tile's other rows keep what was there, in
             // accumulator lanes nobody reads) and the hi and lo token tiles
             auto table = [&](int it, int vt, int kt) {
@@ -151,7 +151,7 @@ lmhead_t5_kernel(const __grid_constant__ CUtensorMap tm_e, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_lane()) {
             constexpr uint32_t idesc = t5_idesc_bf16(128, NT);
             int it = 0, lt = 0;
             bool ok = true;
