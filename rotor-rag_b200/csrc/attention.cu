@@ -96,6 +96,8 @@ __device__ __forceinline__ float4 qf_deq4(const QkvFinishParams& p, const float 
 }
 
 __global__ void __launch_bounds__(256) qkv_finish_vec_kernel(const __grid_constant__ QkvFinishParams p) {
+    pdl_wait();
+    pdl_trigger();
     const int m = blockIdx.x;
     const int b = m / p.seq, s = m % p.seq;
     const int pos = p.past_len[b] + s;
@@ -136,9 +138,29 @@ __global__ void __launch_bounds__(256) qkv_finish_vec_kernel(const __grid_consta
     }
 }
 
+// A launch that may start while the kernel before it ends (the kernel calls pdl_wait()).
+template <typename P>
+static int launch_dependent(void (*kernel)(P), dim3 grid, int threads, size_t smem, const P& p, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) {
+        ++g_launch_count;
+        return ROTOR_B200_ERR_CUDA;
+    }
+    return launch_status();
+}
+
 int launch_qkv_finish(const QkvFinishParams& p, int rows, cudaStream_t st) {
     if (rows >= 5 && p.acc.planes == 1 && p.acc.out % 4 == 0 && p.head_dim % 8 == 0 && p.terms >= 1 && p.terms <= 3)
-        qkv_finish_vec_kernel<<<rows, 256, 0, st>>>(p);
+        return launch_dependent(qkv_finish_vec_kernel, dim3(rows), 256, 0, p, st);
     else
         qkv_finish_kernel<<<rows, 256, 0, st>>>(p);
     return launch_status();
@@ -768,7 +790,12 @@ __global__ void __launch_bounds__(32 * AC_MAX_GROUP) attn_decode_stream_kernel(c
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (nchunk > 0) fetch(0, 0);
+    // rows behind the new one are older than the kernel before this one (see the rule in common.cuh)
+    const bool early = nchunk > 0 && min(k0 + AS_KEYS, k1) < T;
+    if (early) fetch(0, 0);
+    pdl_wait();
+    pdl_trigger();
+    if (nchunk > 0 && !early) fetch(0, 0);
     {  // this warp's q rows, pre-scaled (read back by the same warp only, after the first CTA barrier)
         const float* qh = p.q + (size_t)b * dq + (size_t)(hk * G + warp * H) * D;
         const float scale = 1.0f / sqrtf((float)D);
@@ -850,18 +877,9 @@ static int launch_attn_decode_stream(const AttnParams& p, int rows, cudaStream_t
     const size_t smem = ((size_t)G * D + (size_t)G * 32 + (size_t)4 * AS_KEYS * (D + AC_PAD)) * sizeof(float);
     dim3 grid(p.n_kv_heads, rows, p.nsplit > 1 ? p.nsplit : 1);
     // two heads per warp when the group is even and leaves at least two warps
-    if (G % 2 == 0 && G >= 4) {
-        if (D == 64)
-            attn_decode_stream_kernel<64, 2><<<grid, 16 * G, smem, st>>>(p);
-        else
-            attn_decode_stream_kernel<128, 2><<<grid, 16 * G, smem, st>>>(p);
-    } else {
-        if (D == 64)
-            attn_decode_stream_kernel<64, 1><<<grid, 32 * G, smem, st>>>(p);
-        else
-            attn_decode_stream_kernel<128, 1><<<grid, 32 * G, smem, st>>>(p);
-    }
-    return launch_status();
+    if (G % 2 == 0 && G >= 4)
+        return launch_dependent(D == 64 ? attn_decode_stream_kernel<64, 2> : attn_decode_stream_kernel<128, 2>, grid, 16 * G, smem, p, st);
+    return launch_dependent(D == 64 ? attn_decode_stream_kernel<64, 1> : attn_decode_stream_kernel<128, 1>, grid, 32 * G, smem, p, st);
 }
 
 static size_t attn_cluster_smem(int G, int D, int lcmax, int ns) {

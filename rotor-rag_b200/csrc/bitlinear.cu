@@ -278,13 +278,19 @@ GemvPlan plan_gemv(size_t out, size_t in, int ncols) {
     return g;
 }
 
+bool gemv_adds(size_t out, size_t in, int ncols, const void* xq, int variant) {
+    if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO)
+        return gemm_tcgen05_supported(out, in, ncols, xq) && gemm_tcgen05_splits(out, in, ncols) >= 2;
+    return plan_gemv(out, in, ncols).ksplit > 1;
+}
+
 int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
-                       int32_t* acc, size_t plane_stride, const GemvPlan& plan, int variant, cudaStream_t st) {
+                       int32_t* acc, size_t plane_stride, const GemvPlan& plan, int variant, cudaStream_t st, bool zeroed) {
     int rc = (library_status_word() ? ROTOR_B200_OK : ROTOR_B200_ERR_CUDA);
     if (rc) return rc;
     if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO) {
         // compute-bound regime: the tiled GEMM writes complete sums into plane 0 (callers use one plane)
-        if (gemm_tcgen05_supported(out, in, ncols, xq)) return launch_gemm_tcgen05(tiles, out, in, xq, xsum, ncols, acc, st);
+        if (gemm_tcgen05_supported(out, in, ncols, xq)) return launch_gemm_tcgen05(tiles, out, in, xq, xsum, ncols, acc, st, zeroed);
         return launch_gemm_mma(tiles, out, in, xq, xsum, ncols, acc, st);
     }
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
@@ -305,7 +311,7 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
         // plane_stride 0 with a split K range: the splits add into one zeroed plane (exact in any order)
         p.atomic = plane_stride == 0 && plan.ksplit > 1;
         p.plane_stride = plane_stride;
-        if (p.atomic) RB_CUDA(cudaMemsetAsync(p.acc, 0, (size_t)p.ncols * out * sizeof(int32_t), st));
+        if (p.atomic && !zeroed) RB_CUDA(cudaMemsetAsync(p.acc, 0, (size_t)p.ncols * out * sizeof(int32_t), st));
         rc = dispatch_acc(p, nrt, plan.ksplit, variant, st);
         if (rc) return rc;
     }

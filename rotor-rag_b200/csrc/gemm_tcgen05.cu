@@ -497,8 +497,21 @@ int configure_gemm_tcgen05() {
     return ROTOR_B200_OK;
 }
 
+// fewer 256-row tiles than SMs: split the K range so that the grid covers the GPU (a K step of a
+// 256-row tile costs a decoder less per weight than four steps of 64-row tiles); at least four K
+// steps per CTA, partial sums added into the zeroed accumulators
+int gemm_tcgen05_splits(size_t out, size_t in, int ncols) {
+    const int nkt = (int)(kpad_of(in) / TILE_K), rows = (int)opad_of(out);
+    const int tiles256 = (ncols + 255) / 256 * ((rows + 255) / 256), sms = fused_sm_count();
+    int splits = tiles256 < sms ? sms / tiles256 : 1;
+    if (splits > nkt / 4) splits = nkt / 4;
+    if (splits < 2) return 1;
+    const int per = (nkt + splits - 1) / splits;
+    return (nkt + per - 1) / per;
+}
+
 int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
-                        int32_t* acc, cudaStream_t st) {
+                        int32_t* acc, cudaStream_t st, bool zeroed) {
     int rc = configure_gemm_tcgen05();
     if (rc) return rc;
     Tc5Params p = {};
@@ -522,22 +535,11 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return ROTOR_B200_ERR_CUDA;
     const int tok_tiles = (ncols + 255) / 256, rows = p.nrt * TILE_ROWS;
-    static PerDevice<int> sm_counts;
-    int& sms = sm_counts.here();
-    if (!sms) {
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current_device()) != cudaSuccess || sms <= 0)
-            sms = 148;
-    }
-    const int tiles256 = tok_tiles * ((rows + 255) / 256);
-    // fewer 256-row tiles than SMs: split the K range so that the grid covers the GPU (a K step of a
-    // 256-row tile costs a decoder less per weight than four steps of 64-row tiles); at least four K
-    // steps per CTA, partial sums added into the zeroed accumulators
-    int splits = tiles256 < sms ? sms / tiles256 : 1;
-    if (splits > p.nkt / 4) splits = p.nkt / 4;
+    const int sms = fused_sm_count(), tiles256 = tok_tiles * ((rows + 255) / 256);
+    int splits = gemm_tcgen05_splits(out, in, ncols);
     if (splits >= 2) {
         p.kt_per_split = (p.nkt + splits - 1) / splits;
-        splits = (p.nkt + p.kt_per_split - 1) / p.kt_per_split;
-        RB_CUDA(cudaMemsetAsync(acc, 0, (size_t)ncols * out * sizeof(int32_t), st));
+        if (!zeroed) RB_CUDA(cudaMemsetAsync(acc, 0, (size_t)ncols * out * sizeof(int32_t), st));
         dim3 grid(tok_tiles, (rows + 255) / 256, splits);
         gemm_tcgen05_kernel<256><<<grid, T5Cfg<256>::THREADS, T5Cfg<256>::SMEM, st>>>(tmap, p);
     } else if (tiles256 < sms) {  // 256-row tiles would leave SMs idle

@@ -164,7 +164,42 @@ static int gemv(Ctx& c, const void* tiles, size_t out, size_t in, int ncols, int
     // (many columns go to the tiled GEMM, which leaves complete sums in the first plane)
     view->planes = one_plane ? 1 : plan.ksplit;
     view->out = (int)out;
-    return launch_gemv_planes(tiles, out, in, c.xq, c.xsum[xs], ncols, acc, plane_stride, plan, c.variant, st);
+    const bool zeroed = one_plane && c.zeroed == acc;
+    c.zeroed = nullptr;
+    return launch_gemv_planes(tiles, out, in, c.xq, c.xsum[xs], ncols, acc, plane_stride, plan, c.variant, st, zeroed);
+}
+
+// The stage `p` clears the accumulators of the product that follows it, if that product adds to them (see gemv()).
+static void clear_for(Ctx& c, VecStageParams& p, size_t out, size_t in, int ncols, int32_t* acc) {
+    c.zeroed = nullptr;
+    if (ncols < 5 || !gemv_adds(out, in, ncols, c.xq, c.variant)) return;
+    p.zero = acc;
+    p.zero_n = (size_t)ncols * out;
+    c.zeroed = acc;
+}
+// ... the q/k/v product of a block, where it is not the one that finishes its rows itself
+static bool qkv_finishes(const Ctx& c, int seq, int cols) {
+    // prompt-sized row counts, one activation term, head_dim 128: the q/k/v product dequantises, rotates and
+    // appends to the cache in its read-back (no int32 accumulators, no separate finish kernel)
+    return c.terms == 1 && c.variant == ROTOR_B200_VARIANT_AUTO && seq >= 16 &&
+           gemm_tcgen05_qkv_supported((size_t)c.dq, (size_t)c.dkv, c.d, c.head_dim, cols, c.xq);
+}
+static void clear_for_qkv(Ctx& c, VecStageParams& p, int seq, int cols) {
+    if (qkv_finishes(c, seq, cols))
+        c.zeroed = nullptr;
+    else
+        clear_for(c, p, (size_t)c.dq + 2 * c.dkv, c.d, cols, c.accA);
+}
+// ... the gate/up product, where its read-back does not gate
+static bool gate_up_gates(const Ctx& c, int cols) {
+    return c.terms == 1 && c.tp_size <= 1 && c.variant == ROTOR_B200_VARIANT_AUTO &&
+           gemm_tcgen05_gated_supported((size_t)c.ff, c.d, cols, c.xq);
+}
+static void clear_for_gate_up(Ctx& c, VecStageParams& p, int cols) {
+    if (gate_up_gates(c, cols))
+        c.zeroed = nullptr;
+    else
+        clear_for(c, p, 2 * (size_t)c.ff, c.d, cols, c.accA);
 }
 
 static void quant_sink(const Ctx& c, VecStageParams& p, int slot, int n) {
@@ -181,10 +216,7 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
                           cudaStream_t st) {
     const int rows = batch * seq, cols = rows * c.terms;
     const size_t qkv_out = (size_t)c.dq + 2 * c.dkv;
-    // prompt-sized row counts, one activation term, head_dim 128: the q/k/v product dequantises, rotates and
-    // appends to the cache in its read-back (no int32 accumulators, no separate finish kernel)
-    const bool fuse_qkv = c.terms == 1 && c.variant == ROTOR_B200_VARIANT_AUTO && seq >= 16 &&
-                          gemm_tcgen05_qkv_supported((size_t)c.dq, (size_t)c.dkv, c.d, c.head_dim, cols, c.xq);
+    const bool fuse_qkv = qkv_finishes(c, seq, cols);
     AccView va = {};
     if (!fuse_qkv) RB_TRY(gemv(c, L.qkv_tiles, qkv_out, c.d, cols, 0, c.accA, &va, st));
     // (sixteen and more sequences: the tiled attention kernel streams each sequence's cache once per
@@ -277,6 +309,7 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
     qa.head_dim = c.head_dim;
     qa.eps = c.eps;
     quant_sink(c, qa, 1, c.dq);
+    clear_for(c, qa, c.d, c.dq, cols, c.accB);
     RB_TRY(launch_vec_stage(qa, rows, st));
     return gemv(c, L.o_tiles, c.d, c.dq, cols, 1, c.accB, vo, st);
 }
@@ -285,8 +318,7 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
 // Out: accumulators of the down projection (view *vd), activation scales in sx[1].
 static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView* vd, cudaStream_t st) {
     const int cols = rows * c.terms;
-    if (c.terms == 1 && c.tp_size <= 1 && c.variant == ROTOR_B200_VARIANT_AUTO &&
-        gemm_tcgen05_gated_supported((size_t)c.ff, c.d, cols, c.xq)) {
+    if (gate_up_gates(c, cols)) {
         // prompt-sized row counts, one activation term: the gate/up product applies the gating in its epilogue and
         // writes float32 gated rows (into the accumulator area: a quarter of the bytes of the two int32 halves);
         // the stage that follows only has to sub-norm and quantise them
@@ -300,6 +332,7 @@ static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView
         gp.norm1 = L.ffn_sub_norm;
         gp.eps = c.eps;
         quant_sink(c, gp, 1, c.ff);
+        clear_for(c, gp, c.d, c.ff, cols, c.accB);
         RB_TRY(launch_vec_stage(gp, rows, st));
         return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
     }
@@ -317,6 +350,7 @@ static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView
     fp.norm1 = L.ffn_sub_norm;
     fp.eps = c.eps;
     quant_sink(c, fp, 1, c.ff);
+    clear_for(c, fp, c.d, c.ff, cols, c.accB);
     RB_TRY(launch_vec_stage(fp, rows, st));
     return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
 }
@@ -327,7 +361,7 @@ static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView
 // of the quantiser.
 static int run_blocks(Ctx& c, const rotor_b200_layer_weights* layers, int l0, int l1, const float* next_norm,
                       bool to_float, int batch, int seq, cudaStream_t st) {
-    const int rows = batch * seq;
+    const int rows = batch * seq, cols = rows * c.terms;
     for (int l = l0; l < l1; ++l) {
         const rotor_b200_layer_weights& L = layers[l];
         AccView vo, vd;
@@ -344,6 +378,7 @@ static int run_blocks(Ctx& c, const rotor_b200_layer_weights* layers, int l0, in
         op.norm1 = L.post_attn_norm;
         op.eps = c.eps;
         quant_sink(c, op, 0, c.d);
+        clear_for_gate_up(c, op, cols);
         RB_TRY(launch_vec_stage(op, rows, st));
         RB_TRY(ffn_part(c, L, rows, &vd, st));
         VecStageParams dn = {};
@@ -357,10 +392,12 @@ static int run_blocks(Ctx& c, const rotor_b200_layer_weights* layers, int l0, in
         dn.eps = c.eps;
         const bool last = l + 1 == l1;
         dn.norm1 = last ? next_norm : layers[l + 1].input_norm;
+        c.zeroed = nullptr;
         if (last && to_float)
             dn.y_out = c.hn;
         else
             quant_sink(c, dn, 0, c.d);
+        if (!last) clear_for_qkv(c, dn, seq, cols);
         RB_TRY(launch_vec_stage(dn, rows, st));
     }
     return ROTOR_B200_OK;
@@ -911,6 +948,7 @@ static int run_layers(Model& m, const long long* ids, int batch, int seq, int lo
     e.norm1 = m.layers[0].input_norm;
     e.eps = c.eps;
     quant_sink(c, e, 0, d);
+    clear_for_qkv(c, e, seq, rows * c.terms);
     RB_TRY(launch_vec_stage(e, rows, st));
     RB_TRY(run_blocks(c, m.layers, 0, m.cfg.n_layers, m.final_norm, true, batch, seq, st));
     if (logits_mode == ROTOR_B200_LOGITS_NONE && !next_ids) return ROTOR_B200_OK;
@@ -1056,6 +1094,7 @@ int rotor_b200_model_forward_hidden(void* handle, const float* hidden_in, int ba
     e.norm1 = m->layers[layer_begin].input_norm;
     e.eps = c.eps;
     quant_sink(c, e, 0, c.d);
+    if (c.tp_size <= 1) clear_for_qkv(c, e, seq, rows * c.terms);
     RB_TRY(launch_vec_stage(e, rows, st));
     const float* next_norm = layer_end < m->cfg.n_layers ? m->layers[layer_end].input_norm : m->final_norm;
     if (c.tp_size > 1) {
@@ -1159,6 +1198,7 @@ int rotor_b200_ffn_forward(const rotor_b200_model_config* cfg, const rotor_b200_
     e.norm1 = pre_norm;
     e.eps = c.eps;
     quant_sink(c, e, 0, c.d);
+    clear_for_gate_up(c, e, rows * c.terms);
     RB_TRY(launch_vec_stage(e, rows, st));
     AccView vd;
     RB_TRY(ffn_part(c, *layer, rows, &vd, st));
@@ -1197,6 +1237,7 @@ int rotor_b200_attention_forward(const rotor_b200_model_config* cfg, const rotor
     e.src = x;
     e.eps = c.eps;
     quant_sink(c, e, 0, c.d);
+    clear_for_qkv(c, e, seq, rows * c.terms);
     RB_TRY(launch_vec_stage(e, rows, st));
     AccView vo;
     RB_TRY(attention_part(c, *layer, batch, seq, &vo, st));

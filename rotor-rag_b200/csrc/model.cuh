@@ -53,6 +53,9 @@ struct VecStageParams {
     const float* ext_absmax;     // [rows] max|.| of the whole row, used by the quantiser
     float* out_sumsq;            // [rows] optional: local sum of squares of the built row (before norm1)
     float* out_absmax;           // [rows] optional: local max|.| of the row after norm1
+    // accumulators that the product behind this stage adds to: the stage clears them (no memset node between the two)
+    int32_t* zero;
+    size_t zero_n;               // a multiple of 4
 };
 
 int launch_vec_stage(const VecStageParams& p, int rows, cudaStream_t st);
@@ -68,15 +71,19 @@ struct GemvPlan {
     int kt_per_split;
 };
 GemvPlan plan_gemv(size_t out, size_t in, int ncols);
+// Whether launch_gemv_planes with plane_stride 0 adds to acc (which it clears first, unless it is told `zeroed`).
+bool gemv_adds(size_t out, size_t in, int ncols, const void* xq, int variant);
 int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
-                       int32_t* acc, size_t plane_stride, const GemvPlan& plan, int variant, cudaStream_t st);
+                       int32_t* acc, size_t plane_stride, const GemvPlan& plan, int variant, cudaStream_t st,
+                       bool zeroed = false);
 int gemv_cols_per_launch(int variant, int ncols);
 
 // Many-column product (gemm_mma.cu): complete int32 sums into acc[ncols][out].
 constexpr int GEMM_MIN_COLS = 32;
 bool gemm_tcgen05_supported(size_t out, size_t in, int ncols, const void* xq);
 int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
-                        int32_t* acc, cudaStream_t st);
+                        int32_t* acc, cudaStream_t st, bool zeroed = false);
+int gemm_tcgen05_splits(size_t out, size_t in, int ncols);
 int configure_gemm_tcgen05();
 // gate/up product with the gating in its epilogue (float32 gated rows out, one activation term per token)
 bool gemm_tcgen05_gated_supported(size_t ff, size_t in, int ncols, const void* xq);

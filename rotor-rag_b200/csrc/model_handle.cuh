@@ -42,6 +42,7 @@ struct Ctx {
     int32_t* xsum[2];
     int32_t* accA;  // q/k/v and gate/up accumulators
     int32_t* accB;  // o and down accumulators
+    const int32_t* zeroed;  // accumulators the stage launched last has cleared for the product that follows (host state of one call)
     int* d_pos;
     float2* rope;        // cos/sin table, or null
     float2* rope_buf;    // storage for it

@@ -13,6 +13,7 @@
 // association follow vec_stage_row, which this kernel replaces from RS_MIN_ROWS rows on.
 #include <cstdlib>
 
+#include "vecstage.cuh"
 #include "leanstage.cuh"
 #include "model.cuh"
 
@@ -21,9 +22,15 @@ namespace rb {
 constexpr int RS_THREADS = 128;
 constexpr int RS_MIN_ROWS = 5;         // (fewer rows: the generation-step kernels or the shared-memory stage)
 constexpr int RS_WIDE_THREADS = 512;
-// With fewer rows than SMs every CTA runs its code once, from a cold instruction cache: the duration is
-// the length of the unrolled code, so the widest rows take 1024 threads with half the groups each.
+// With fewer rows than two per SM every CTA runs its code once, from a cold instruction cache, and waits once for
+// each load: the duration is the length of that chain, so a row takes as many threads as leave one or two groups to
+// each (512, or 1024 above 4096 elements) and the widest rows 1024 with seven.  These stages are launched as dependent
+// kernels and clear the accumulators of the product behind them, so that no memset stands between two kernels of a
+// generation step.  One step of 8 sequences of the 2B model: 2.71 -> 1.62 ms (with the partial rows of the decode
+// attention merged here, RS_RUN_BATCH loads at a time, instead of in the shared-memory stage: 16.5 -> 6 us a layer).
 constexpr int RS_FEW_ROWS = 296;
+constexpr int RS_MAX_RUNS = 32;        // VS_ATTN: runs of a sequence, one per lane
+constexpr int RS_RUN_BATCH = 8;        // ... whose partial rows a thread requests together
 
 __device__ __forceinline__ float4 rs_deq(const VecStageParams& p, size_t col0, int off, int g, const float (&sxv)[3],
                                          float wscale) {
@@ -85,8 +92,9 @@ __device__ __forceinline__ float4 rs_deq_staged(const int4* stage, int n4, int h
 // one.  Every thread stages exactly the 16-byte pieces it will read itself, so the staging area
 // needs no barrier: cp.async.wait_group by the owner is enough, and the next fetch may start
 // as soon as the owner has the pieces in registers.  Accumulator modes only.
-template <int V, bool RESID, int TH, bool PF>
-__global__ void __launch_bounds__(TH, TH > 128 ? (V <= 4 ? 2 : 1) : (V > 8 ? 4 : 5))
+// MERGE: VS_ATTN, the row is merged from the partial results of the decode attention's runs.
+template <int V, bool RESID, int TH, bool PF, bool MERGE = false>
+__global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 128 ? (V <= 4 ? 2 : 1) : (V > 8 ? 4 : 5))
     row_stage_kernel(const __grid_constant__ VecStageParams p, int rows) {
     __shared__ float scratch[64];
     extern __shared__ __align__(16) int4 rs_stage[];
@@ -95,6 +103,14 @@ __global__ void __launch_bounds__(TH, TH > 128 ? (V <= 4 ? 2 : 1) : (V > 8 ? 4 :
     const int halves = p.mode == VS_FFN ? 2 : 1;
     float* hdst = p.h_out ? p.h_out : p.h;
     float sxn[3] = {0.f, 0.f, 0.f};
+    if (!PF && (tid & 7) == 0)  // constants: requested while the kernel before this one ends
+        for (int i = 4 * tid; i < n; i += 4 * TH) {
+            if (p.norm0) prefetch_l2(p.norm0 + i);
+            if (p.norm1) prefetch_l2(p.norm1 + i);
+        }
+    pdl_wait();
+    pdl_trigger();
+    clear_sums(p);
 
     // PF: start the fetch of `row` (pieces into the staging area, scales into registers)
     auto fetch = [&](int row) {
@@ -142,6 +158,42 @@ __global__ void __launch_bounds__(TH, TH > 128 ? (V <= 4 ? 2 : 1) : (V > 8 ? 4 :
 
     // ---- build the row: every load of the stage in flight together
     float4 v[V], aux[RESID ? V : 1];
+    if constexpr (MERGE) {
+        // weights exp(m_s - M) / L of every (head, run) into shared memory, one warp per head, lane = run
+        const int D = p.head_dim, ns = p.nsplit, lane = tid & 31;
+        float* wf = reinterpret_cast<float*>(rs_stage);
+        const size_t hb = (size_t)m * p.n_heads * ns;
+        for (int h = tid >> 5; h < p.n_heads; h += TH / 32) {
+            const float ms = lane < ns ? __ldcg(p.part_m + hb + h * ns + lane) : -INFINITY;
+            const float ls = lane < ns ? __ldcg(p.part_l + hb + h * ns + lane) : 0.f;
+            const float M = warp_max(ms), f = ms == -INFINITY ? 0.f : __expf(ms - M), L = warp_sum(ls * f);
+            if (lane < ns) wf[h * ns + lane] = f * (1.0f / L);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            const int g = tid + j * TH;
+            v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (g >= n4) continue;
+            const int h = 4 * g / D;
+            const float* po = p.part_o + (hb + (size_t)h * ns) * D + (4 * g - h * D);
+            for (int s0 = 0; s0 < ns; s0 += RS_RUN_BATCH) {
+                float4 pv[RS_RUN_BATCH];
+#pragma unroll
+                for (int u = 0; u < RS_RUN_BATCH; ++u)
+                    pv[u] = s0 + u < ns ? ldcg4(po + (size_t)(s0 + u) * D) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int u = 0; u < RS_RUN_BATCH; ++u) {
+                    const float f = s0 + u < ns ? wf[h * ns + s0 + u] : 0.f;
+                    v[j].x += pv[u].x * f;
+                    v[j].y += pv[u].y * f;
+                    v[j].z += pv[u].z * f;
+                    v[j].w += pv[u].w * f;
+                }
+            }
+        }
+    }
+    if constexpr (!MERGE) {
 #pragma unroll
     for (int j = 0; j < V; ++j) {
         const int g = tid + j * TH;
@@ -180,6 +232,7 @@ __global__ void __launch_bounds__(TH, TH > 128 ? (V <= 4 ? 2 : 1) : (V > 8 ? 4 :
             v[j] = a;
             if (RESID) aux[RESID ? j : 0] = ldcg4(p.h + ro + 4 * g);
         }
+    }
     }
     if (PF && m + (int)gridDim.x < rows) fetch(m + gridDim.x);  // the staged pieces are in registers now
     if constexpr (RESID) {
@@ -278,7 +331,10 @@ bool row_stage_supported(const VecStageParams& p, int rows) {
     static const bool off = getenv("ROTOR_B200_NO_ROWSTAGE") != nullptr;  // comparison aid
     if (off || rows < RS_MIN_ROWS) return false;
     if (p.mode != VS_EMBED && p.mode != VS_PLAIN && p.mode != VS_OPROJ && p.mode != VS_FFN && p.mode != VS_DOWN &&
-        p.mode != VS_DEQ)
+        p.mode != VS_DEQ && p.mode != VS_ATTN)
+        return false;
+    if (p.mode == VS_ATTN && (rows > RS_FEW_ROWS || p.nsplit > RS_MAX_RUNS || p.head_dim % 4 ||
+                              (size_t)p.n_heads * p.nsplit * sizeof(float) > 40 * 1024))
         return false;
     const bool from_acc = p.mode == VS_OPROJ || p.mode == VS_FFN || p.mode == VS_DOWN || p.mode == VS_DEQ;
     if (from_acc && (p.acc.planes != 1 || p.acc.out % 4 || p.terms < 1 || p.terms > 3)) return false;
@@ -324,6 +380,26 @@ static int launch_one(const VecStageParams& p, int rows, cudaStream_t st) {
     return launch_status();
 }
 
+// One CTA per row (a single wave).
+template <int V, bool RESID, int TH, bool MERGE = false>
+static int launch_few(const VecStageParams& p, int rows, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows);
+    cfg.blockDim = dim3(TH);
+    cfg.dynamicSmemBytes = MERGE ? (size_t)p.n_heads * p.nsplit * sizeof(float) : 0;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, row_stage_kernel<V, RESID, TH, false, MERGE>, p, rows) != cudaSuccess) {
+        ++g_launch_count;
+        return ROTOR_B200_ERR_CUDA;
+    }
+    return launch_status();
+}
+
 template <bool RESID>
 static int launch_row_stage_v(const VecStageParams& p, int rows, int v, cudaStream_t st) {
     if (v <= 5) return launch_one<5, RESID, RS_THREADS>(p, rows, st);
@@ -337,8 +413,17 @@ static int launch_row_stage_v(const VecStageParams& p, int rows, int v, cudaStre
 
 int launch_row_stage(const VecStageParams& p, int rows, cudaStream_t st) {
     const int width = p.xq && p.kpad > p.n ? p.kpad : p.n;   // the quantiser also writes the zero padding
+    if (rows <= RS_FEW_ROWS) {
+        const bool resid = p.mode == VS_OPROJ || p.mode == VS_DOWN;
+        if (p.mode == VS_ATTN)
+            return width <= 4096 ? launch_few<2, false, 512, true>(p, rows, st) : width <= 8192 ? launch_few<2, false, 1024, true>(p, rows, st)
+                                                                                : launch_few<7, false, 1024, true>(p, rows, st);
+        if (width <= 2048) return resid ? launch_few<1, true, 512>(p, rows, st) : launch_few<1, false, 512>(p, rows, st);
+        if (width <= 4096) return resid ? launch_few<2, true, 512>(p, rows, st) : launch_few<2, false, 512>(p, rows, st);
+        if (width <= 8192) return resid ? launch_few<2, true, 1024>(p, rows, st) : launch_few<2, false, 1024>(p, rows, st);
+        return launch_few<7, false, 1024>(p, rows, st);
+    }
     if (width > 4 * 16 * RS_THREADS) {  // wide rows without a residual: 512 threads, up to 14 groups each
-        if (rows <= RS_FEW_ROWS) return launch_one<7, false, 1024>(p, rows, st);  // see RS_FEW_ROWS
         return launch_one<14, false, RS_WIDE_THREADS>(p, rows, st);
     }
     const int v = (width / 4 + RS_THREADS - 1) / RS_THREADS;

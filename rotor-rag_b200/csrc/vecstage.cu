@@ -17,6 +17,8 @@ __global__ void __launch_bounds__(1024) vec_stage_kernel(VecStageParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* scratch = reinterpret_cast<float*>(smem_raw);
     pdl_wait();
+    pdl_trigger();
+    clear_sums(p);
     vec_stage_row(p, blockIdx.x, scratch + 64, scratch);
 }
 

@@ -6,6 +6,12 @@
 
 namespace rb {
 
+// Clears the accumulators of the product that follows, a share per CTA.
+__device__ __forceinline__ void clear_sums(const VecStageParams& p) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.zero_n / 4; i += (size_t)gridDim.x * blockDim.x)
+        reinterpret_cast<int4*>(p.zero)[i] = make_int4(0, 0, 0, 0);
+}
+
 constexpr int VS_U = 8;  // elements per thread whose global loads are in flight together
 
 // y[i] = row[i] / sqrt(mean(row^2) + eps) * w[i], in place.  The first batch of norm
