@@ -14,6 +14,7 @@
 //          per pass at the cost of one, which also carries the residual terms of the
 //          multi-term activation quantiser.
 #include "gemv_core.cuh"
+#include "leanstage.cuh"
 #include "model.cuh"
 
 namespace rb {
@@ -60,6 +61,8 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar) {
     }
     return ok != 0;
 }
+
+constexpr size_t LINEAR_FUSED_ROWS = 4;  // rows of a stand-alone layer call that are quantised in the product's prologue
 
 struct AccParams {
     const uint4* tiles;
@@ -174,6 +177,7 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
 __global__ void dequant_kernel(const int32_t* __restrict__ acc, const float* __restrict__ sx, int m, int terms,
                                int out, float wscale, const float* __restrict__ wscale_vec,
                                float* __restrict__ y) {
+    pdl_wait();
     const size_t total = (size_t)m * out;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int r = (int)(i / out), o = (int)(i % out);
@@ -322,22 +326,19 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
 
 using namespace rb;
 
-extern "C" {
-
-int rotor_b200_bitlinear_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum,
-                             size_t ncols, int32_t* acc, int variant, void* stream) {
+static int run_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, size_t ncols,
+                   int32_t* acc, int variant, cudaStream_t st, bool zeroed) {
     RB_REQUIRE(tiles && xq && xsum && acc && out > 0 && in > 0 && ncols > 0);
     RB_REQUIRE(out < (1u << 30) && in < (1u << 30));
     RB_REQUIRE(((uintptr_t)tiles & 15) == 0 && ((uintptr_t)xq & 15) == 0);
     RB_REQUIRE(variant >= ROTOR_B200_VARIANT_AUTO && variant <= ROTOR_B200_VARIANT_MMA);
     int rc = (library_status_word() ? ROTOR_B200_OK : ROTOR_B200_ERR_CUDA);
     if (rc) return rc;
-    cudaStream_t st = as_stream(stream);
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
     const size_t kpad = kpad_of(in);
     if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO) {
         if (gemm_tcgen05_supported(out, in, (int)ncols, xq))
-            return launch_gemm_tcgen05(tiles, out, in, xq, xsum, (int)ncols, acc, st);
+            return launch_gemm_tcgen05(tiles, out, in, xq, xsum, (int)ncols, acc, st, zeroed);
         return launch_gemm_mma(tiles, out, in, xq, xsum, (int)ncols, acc, st);
     }
     // small matrices, up to eight columns: the staged kernel (every CTA's share of the tiles sits in shared
@@ -362,11 +363,28 @@ int rotor_b200_bitlinear_acc(const void* tiles, size_t out, size_t in, const int
         const int ksplit_eff = (nkt + p.kt_per_split - 1) / p.kt_per_split;
         p.atomic = ksplit_eff > 1;
         p.plane_stride = 0;
-        if (p.atomic) RB_CUDA(cudaMemsetAsync(p.acc, 0, (size_t)nc * out * sizeof(int32_t), st));
+        if (p.atomic && !zeroed) RB_CUDA(cudaMemsetAsync(p.acc, 0, (size_t)nc * out * sizeof(int32_t), st));
         rc = dispatch_acc(p, nrt, ksplit_eff, variant, st);
         if (rc) return rc;
     }
     return ROTOR_B200_OK;
+}
+
+// Whether run_acc adds to acc for any of its column chunks (it then clears acc first unless it is told `zeroed`).
+static bool acc_adds(size_t out, size_t in, size_t ncols, const int8_t* xq, int variant) {
+    if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO)
+        return gemm_tcgen05_supported(out, in, (int)ncols, xq) && gemm_tcgen05_splits(out, in, (int)ncols) >= 2;
+    if (ncols <= 8 && staged_acc_supported(out, in, (int)ncols, variant)) return false;
+    const size_t chunk = pick_variant(variant, (int)(ncols < 8 ? ncols : 8)) == ROTOR_B200_VARIANT_MMA ? 8 : 4;
+    const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS), rest = (int)(ncols % chunk);
+    return (ncols >= chunk && choose_ksplit(nrt, nkt, (int)chunk, 4) > 1) || (rest && choose_ksplit(nrt, nkt, rest, 4) > 1);
+}
+
+extern "C" {
+
+int rotor_b200_bitlinear_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum,
+                             size_t ncols, int32_t* acc, int variant, void* stream) {
+    return run_acc(tiles, out, in, xq, xsum, ncols, acc, variant, as_stream(stream), false);
 }
 
 int rotor_b200_bitlinear_dequant(const int32_t* acc, const float* sx, size_t m, int terms, size_t out,
@@ -375,7 +393,19 @@ int rotor_b200_bitlinear_dequant(const int32_t* acc, const float* sx, size_t m, 
     const size_t total = m * out;
     unsigned grid = (unsigned)((total + 255) / 256);
     if (grid > 148 * 16) grid = 148 * 16;
-    dequant_kernel<<<grid, 256, 0, as_stream(stream)>>>(acc, sx, (int)m, terms, (int)out, wscale, wscale_vec, y);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = as_stream(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, dequant_kernel, acc, sx, (int)m, terms, (int)out, wscale, wscale_vec, y) != cudaSuccess) {
+        ++g_launch_count;
+        return ROTOR_B200_ERR_CUDA;
+    }
     return launch_status();
 }
 
@@ -393,6 +423,23 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
     RB_REQUIRE(((uintptr_t)workspace & 255) == 0);
     if (workspace_bytes < rotor_b200_bitlinear_workspace_bytes(out, in, m, terms)) return ROTOR_B200_ERR_WORKSPACE;
     const size_t nc = m * (size_t)terms;
+    // A few rows: one launch, the rows are quantised in the product's prologue by every CTA (a row costs each about a
+    // microsecond, the two launches saved cost five) and leave it as floats.  Every CTA reads x, so y must not lie on it.
+    // One row of 2560 -> 6912: 9.7 -> 5.1 us on the GPU, 25.8 -> 19.4 us a call.
+    const uintptr_t x0 = (uintptr_t)x, x1 = x0 + m * in * sizeof(float), y0 = (uintptr_t)y, y1 = y0 + m * out * sizeof(float);
+    if (variant == ROTOR_B200_VARIANT_AUTO && !wscale_vec && m <= LINEAR_FUSED_ROWS && nc <= 8 && (x0 & 15) == 0 &&
+        ((uintptr_t)tiles & 15) == 0 && out < (1u << 30) && in <= 49152 && (y1 <= x0 || x1 <= y0) &&
+        fused_gemv_supported(out, in, (int)m, terms, 1, 0)) {
+        LeanStage stage = {};
+        stage.mode = LM_PLAIN;
+        stage.n = (int)in;
+        stage.y = x;
+        stage.terms = terms;
+        stage.kpad = (int)kpad_of(in);
+        stage.clamp = 1;
+        const float scale[3] = {wscale, wscale, wscale};
+        return launch_fused_gemv(tiles, out, in, 1, (int)m, stage, y, scale, (int)out, (int)out, 0, as_stream(stream), nullptr, true);
+    }
     unsigned char* w = (unsigned char*)workspace;
     int8_t* xq = (int8_t*)w;
     w += al256(nc * kpad_of(in));
@@ -401,9 +448,11 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
     int32_t* xsum = (int32_t*)w;
     w += al256(nc * 4);
     int32_t* acc = (int32_t*)w;
-    int rc = rotor_b200_quantize_rows(x, m, in, terms, xq, sx, xsum, stream);
+    // sums that the product adds to are cleared by the quantiser: no memset node in between
+    const bool adds = out < (1u << 30) && in <= 49152 && acc_adds(out, in, nc, xq, variant);
+    int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, as_stream(stream));
     if (rc) return rc;
-    rc = rotor_b200_bitlinear_acc(tiles, out, in, xq, xsum, nc, acc, variant, stream);
+    rc = run_acc(tiles, out, in, xq, xsum, nc, acc, variant, as_stream(stream), adds);
     if (rc) return rc;
     return rotor_b200_bitlinear_dequant(acc, sx, m, terms, out, wscale, wscale_vec, y, stream);
 }

@@ -70,7 +70,7 @@ static int launch_fused_tp(const FusedGemvParams& p, int grid, cudaStream_t st) 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_use_pdl ? 1 : 0;
+    cfg.numAttrs = g_use_pdl && !p.alone ? 1 : 0;
     if (cudaLaunchKernelEx(&cfg, fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, TP>, p) != cudaSuccess) {
         ++g_launch_count;
         return ROTOR_B200_ERR_CUDA;
@@ -119,11 +119,12 @@ bool fused_gemv_supported(size_t out, size_t in, int rows, int terms, int halves
 }
 
 int launch_fused_gemv(const void* tiles, size_t out, size_t in, int halves, int rows, const LeanStage& stage, float* y,
-                      const float* scale, int seg1, int seg2, int ffn_act, cudaStream_t st, const FusedTpExtra* tp) {
+                      const float* scale, int seg1, int seg2, int ffn_act, cudaStream_t st, const FusedTpExtra* tp, bool alone) {
     FusedGemvParams p;
     int grid = fused_sm_count();
     int rc = make_fused_params(p, tiles, out, in, halves, rows, stage, y, scale, seg1, seg2, ffn_act, grid);
     if (rc) return rc;
+    p.alone = alone;
     if (tp) {
         if (stage.terms != 1 || rows > XS_ROWS || (tp->part && halves != 1)) return ROTOR_B200_ERR_ARG;
         p.xs = tp->xs;

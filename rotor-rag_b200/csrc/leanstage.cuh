@@ -37,6 +37,7 @@ struct LeanStage {
     // quantiser
     int terms;
     int kpad;
+    int clamp;                   // quantise NaN to -128, as the stand-alone quantiser does (the packed conversion gives 0)
     // tensor parallel: the row is this rank's slice of a longer one.  Exchange index + 1 (0 = none)
     // of the sum of squares under norm1 and of the absolute maximum under the quantiser; norm_n is
     // the width of the whole row.
@@ -187,7 +188,7 @@ __device__ __forceinline__ void lean_prefetch(const LeanStage& p) {
 // the saturating pack instruction.  `lsum` gains the four integers (one dp4a).  With RESIDUAL the
 // values are replaced by v - q * s (float32, one rounding per operation) for the next term.
 template <bool RESIDUAL>
-__device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& lsum) {
+__device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& lsum, bool clamp = false) {
     const float r0 = v.x * rs, r1 = v.y * rs, r2 = v.z * rs, r3 = v.w * rs;
     float q0 = rintf(r0), q1 = rintf(r1), q2 = rintf(r2), q3 = rintf(r3);
     const float dm = fmaxf(fmaxf(fabsf(r0 - q0), fabsf(r1 - q1)), fmaxf(fabsf(r2 - q2), fabsf(r3 - q3)));
@@ -197,11 +198,13 @@ __device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& ls
         q2 = rintf(__fdiv_rn(v.z, s));
         q3 = rintf(__fdiv_rn(v.w, s));
     }
-    if (RESIDUAL) {
+    if (RESIDUAL || clamp) {
         q0 = fminf(fmaxf(q0, -128.f), 127.f);
         q1 = fminf(fmaxf(q1, -128.f), 127.f);
         q2 = fminf(fmaxf(q2, -128.f), 127.f);
         q3 = fminf(fmaxf(q3, -128.f), 127.f);
+    }
+    if (RESIDUAL) {
         v.x = __fsub_rn(v.x, __fmul_rn(q0, s));
         v.y = __fsub_rn(v.y, __fmul_rn(q1, s));
         v.z = __fsub_rn(v.z, __fmul_rn(q2, s));
@@ -244,7 +247,7 @@ __device__ __forceinline__ void lean_quantize(const LeanStage& p, float4 (&v)[LE
             if (g < k4) {
                 int packed = 0;
                 if (g < n4) packed = (!ONE_TERM && t + 1 < terms) ? quant4_pack<true>(v[j], s, rs, lsum)
-                                                                  : quant4_pack<false>(v[j], s, rs, lsum);
+                                                                  : quant4_pack<false>(v[j], s, rs, lsum, p.clamp != 0);
                 *reinterpret_cast<int*>(xq + (size_t)t * tstride + (size_t)g * 4) = packed;
             }
         }

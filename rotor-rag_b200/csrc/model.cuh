@@ -98,6 +98,10 @@ int launch_gemm_tcgen05_qkv(const void* tiles, size_t in, const int8_t* xq, cons
 int launch_gemm_mma(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
                     int32_t* acc, cudaStream_t st);
 
+// rotor_b200_quantize_rows that also clears `zero_n` accumulators
+int launch_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* xq, float* sx, int32_t* xsum, int32_t* zero,
+                         size_t zero_n, cudaStream_t st);
+
 // Generation-step product with the consuming vector stage fused in (fused.cu, leanstage.cuh).
 struct LeanStage;
 // Tensor-parallel extras of a product: the scalar exchange ring its prologue uses and, for a
@@ -109,7 +113,7 @@ struct FusedTpExtra {
 };
 int launch_fused_gemv(const void* tiles, size_t out, size_t in, int halves, int rows, const LeanStage& stage, float* y,
                       const float* scale, int seg1, int seg2, int ffn_act, cudaStream_t st,
-                      const FusedTpExtra* tp = nullptr);
+                      const FusedTpExtra* tp = nullptr, bool alone = false);
 bool fused_gemv_supported(size_t out, size_t in, int rows, int terms, int halves, int merge_weights);
 int configure_fused_gemv();
 // Stand-alone int8 x ternary product of a small matrix through the staged generation-step kernel.

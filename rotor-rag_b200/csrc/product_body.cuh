@@ -47,6 +47,7 @@ struct FusedGemvParams {
     const int8_t* xq_in;
     const int32_t* xsum_in;
     int32_t* acc_out;
+    int alone;            // launched as an ordinary kernel: the weights may be the work of the kernel before it
 };
 
 // Input rows wider than the register-resident prologue holds (4 * FG_V * FG_THREADS elements)
@@ -291,7 +292,7 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
                             packed = quant4_pack<true>(v, s, rs, lsum);
                             *rp = v;
                         } else {
-                            packed = quant4_pack<false>(v, s, rs, lsum);
+                            packed = quant4_pack<false>(v, s, rs, lsum, p.st.clamp != 0);
                         }
                     }
                     *reinterpret_cast<int*>(xq + (size_t)t * xs_stride + i) = packed;

@@ -1,11 +1,15 @@
 // Stand-alone activation quantiser (one CTA per token row).
 #include "quant.cuh"
+#include "model.cuh"
 
 namespace rb {
 
 __global__ void __launch_bounds__(1024) quantize_rows_kernel(const float* __restrict__ x, int k, int kpad,
                                                              int terms, int8_t* __restrict__ xq,
-                                                             float* __restrict__ sx, int32_t* __restrict__ xsum) {
+                                                             float* __restrict__ sx, int32_t* __restrict__ xsum,
+                                                             int32_t* __restrict__ zero, size_t zero_n) {
+    pdl_trigger();  // launched as an ordinary kernel: everything before it is complete
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < zero_n; i += (size_t)gridDim.x * blockDim.x) zero[i] = 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* scratch = reinterpret_cast<float*>(smem_raw);
     float* row = scratch + 64;
@@ -16,12 +20,8 @@ __global__ void __launch_bounds__(1024) quantize_rows_kernel(const float* __rest
                            xsum + m * terms, scratch);
 }
 
-}  // namespace rb
-
-using namespace rb;
-
-extern "C" int rotor_b200_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* xq, float* sx,
-                                        int32_t* xsum, void* stream) {
+int launch_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* xq, float* sx, int32_t* xsum, int32_t* zero,
+                         size_t zero_n, cudaStream_t st) {
     RB_REQUIRE(x && xq && sx && xsum && m > 0 && k > 0 && terms >= 1 && terms <= 4);
     RB_REQUIRE(k <= 49152 && m < (1u << 31));
     RB_REQUIRE(((uintptr_t)xq & 3) == 0);
@@ -36,7 +36,15 @@ extern "C" int rotor_b200_quantize_rows(const float* x, size_t m, size_t k, int 
         }
     }
     const int threads = k >= 4096 ? 1024 : (k >= 1024 ? 512 : 128);
-    quantize_rows_kernel<<<(unsigned)m, threads, smem, as_stream(stream)>>>(x, (int)k, (int)kpad_of(k), terms,
-                                                                           xq, sx, xsum);
+    quantize_rows_kernel<<<(unsigned)m, threads, smem, st>>>(x, (int)k, (int)kpad_of(k), terms, xq, sx, xsum, zero, zero_n);
     return launch_status();
+}
+
+}  // namespace rb
+
+using namespace rb;
+
+extern "C" int rotor_b200_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* xq, float* sx,
+                                        int32_t* xsum, void* stream) {
+    return launch_quantize_rows(x, m, k, terms, xq, sx, xsum, nullptr, 0, as_stream(stream));
 }

@@ -101,6 +101,46 @@ def test_many_column_product_bit_exact(ops, abi, shape):
     assert np.array_equal(acc2, want)
 
 
+@pytest.mark.parametrize("terms", [1, 2, 3])
+@pytest.mark.parametrize("shape", [(1, 4), (17, 132), (3001, 1924), (2560, 8192), (640, 9220), (8192, 2048)])
+@pytest.mark.parametrize("rows", [1, 2, 4, 5])
+def test_layer_call_of_few_rows(ops, abi, shape, rows, terms):
+    """One launch up to four rows of eight columns, quantiser, product and dequantiser above: both against the general path
+    (the variant forced), with a row of zeros, NaN and infinities, rows that start off a 16-byte boundary, and y on x."""
+    import torch
+    out, inn = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(out + inn + rows + terms)
+    tiles = ops.int8_to_tiles(torch.randint(-1, 2, (out, inn), generator=g, device="cuda", dtype=torch.int8))
+    buf = torch.randn(rows * inn + 1, generator=g, device="cuda")
+    buf[:2 * inn:2] *= 1e-3
+    for x in (buf[:-1].view(rows, inn), buf[1:].view(rows, inn)):
+        for spoil in (None, 0.0, float("nan"), float("inf")):
+            x = x.clone() if x.data_ptr() % 16 == 0 else x
+            if spoil == 0.0:
+                x[rows - 1] = 0.0
+            elif spoil is not None:
+                x[rows - 1, inn // 2] = spoil
+            got = ops.bitlinear_forward(tiles, out, inn, x, terms, 0.037)
+            want = ops.bitlinear_forward(tiles, out, inn, x, terms, 0.037, variant=abi.VARIANT_MMA)
+            if terms == 1:
+                assert torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0)) and torch.equal(got.isnan(), want.isnan())
+            else:  # the terms' sum may be fused: one rounding of the largest term
+                fin = want.isfinite()
+                assert torch.equal(got.isfinite(), fin)
+                scale = want[fin].abs().max() if fin.any() else torch.ones((), device="cuda")
+                assert (got[fin] - want[fin]).abs().max().nan_to_num(0.0) <= 3e-7 * scale if fin.any() else True
+    if out <= inn:
+        x = torch.randn((rows, inn), generator=g, device="cuda")
+        want = ops.bitlinear_forward(tiles, out, inn, x, terms, 0.5, variant=abi.VARIANT_MMA)
+        ws = torch.empty(abi.lib.rotor_b200_bitlinear_workspace_bytes(out, inn, rows, terms), dtype=torch.uint8, device="cuda")
+        abi.check(abi.lib.rotor_b200_bitlinear_forward(abi.ptr(tiles), out, inn, abi.ptr(x), rows, terms, 0.5, None, abi.ptr(x),
+                                                       abi.ptr(ws), ws.numel(), 0, abi.stream()))
+        got = x.flatten()[:rows * out].view(rows, out)
+        assert (got - want).abs().max() <= 3e-7 * want.abs().max()
+    abi.device_status()
+
+
 def test_tcgen05_extreme_values(ops, abi):
     """-128 x -1 and 127 x +1 over K = 6912 on the tcgen05 path: sums stay exact in int32."""
     out, inn, ncols = 256, 6912, 256

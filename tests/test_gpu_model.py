@@ -533,3 +533,37 @@ def test_batched_greedy_generation_ragged(rb, lens):
     assert np.array_equal(model.generate_greedy_batch(prompts, new, use_graph=False), got)
     with pytest.raises(ValueError):  # without a causal mask a row would attend to its padding
         _tiny(rb, "hd64", rb.sem.REFERENCE, max_batch=batch)[2].generate_greedy_batch(prompts, new)
+
+
+@pytest.mark.parametrize("shape", [(1024, 8, 2, 1536), (2560, 20, 5, 6912), (8192, 64, 8, 9216)])
+@pytest.mark.parametrize("batch,context", [(5, 300), (16, 30), (33, 129)])
+def test_batched_steps_equal_single_sequences(rb, shape, batch, context):
+    """Two steps of several sequences (row stages with few rows, merged runs of the decode attention, sums cleared ahead
+    of split products) against the same steps of each sequence alone: widths of every thread count, contexts with and
+    without several runs per sequence, ragged runs.  Three activation terms: float32 rounding is all that may differ."""
+    import torch
+    d, heads, kv, ff = shape
+    cfg = dict(vocab_size=512, d_model=d, n_layers=2, n_heads=heads, n_kv_heads=kv, d_ff=ff)
+    model = rb.synth.random_model_on_device(cfg, seed=batch + context, semantics=rb.sem.REFERENCE, max_seq=context + 2, max_batch=batch,
+                                            max_rows=batch)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d + batch)
+    held = []
+    for layer in model.layers:
+        held.append([torch.randn((batch, kv, context, d // heads), generator=g, device="cuda") for _ in range(2)])
+    ids = np.random.default_rng(batch).integers(0, 512, size=(2, batch, 1))
+
+    def steps(rows):
+        for layer, (k, v) in zip(model.layers, held):
+            for cache, t in zip(layer.attention.ensure_cache(batch, context + 2), (k, v)):
+                cache[:len(rows), :, :context] = t[rows]
+        caches = [rb.tr.KVCache(layer.attention, context, len(rows)) for layer in model.layers]
+        out = []
+        for i in range(2):
+            logits, caches = model.forward_last_logits_device(ids[i][rows], caches)
+            out.append(logits.clone())
+        return torch.stack(out, 1)
+
+    got = steps(list(range(batch)))
+    for b in (0, batch // 2, batch - 1):
+        assert rel_err(got[b].cpu().numpy(), steps([b])[0].cpu().numpy()) < 2e-4, b   # about 60 float32 sums of up to 9216 in a row
