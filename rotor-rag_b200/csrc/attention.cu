@@ -446,112 +446,6 @@ __device__ __forceinline__ void attn_warp_chunk(const float4 (&q4)[D / 32], cons
     m_run = m_new;
 }
 
-// The same step of the online softmax for the streaming kernel, where many warps per SM make issue
-// slots, not latency, the limit: fewer instructions per key.  K and V rows lie in shared memory with a
-// row stride of D + AC_PAD floats (consecutive rows start four banks apart, so 32 lanes reading the
-// same piece of 32 different rows do not collide).  Scores: lane j multiplies key j's whole row with q
-// (shared memory, pre-scaled; every lane reads the same piece: a broadcast) in four independent
-// chains, no shuffles.  Weighted V: the probabilities go through `ps` (32 floats of this warp) and
-// come back four at a time as broadcasts; lane l accumulates output dimensions (D / 32) l .. in two
-// alternating sets.
-constexpr int AC_PAD = 4;
-
-// H query heads of the group per warp (H = 1 or 2): a K or V piece is read from shared memory once and
-// multiplied for every head of the warp, which halves the shared-memory traffic that bounds this kernel.
-// qs: H rows of D floats, ps: H rows of 32.
-template <int D, int H>
-__device__ __forceinline__ void attn_warp_chunk_rows(const float* qs, const float* Kc, const float* Vc, float* ps, int nk,
-                                                     int lane, float (&m_run)[H], float (&l_run)[H], float4 (&o)[H]) {
-    constexpr int KS = D + AC_PAD, OPL = D / 32, C4 = D / 4;
-    float my_s[H];
-#pragma unroll
-    for (int h = 0; h < H; ++h) my_s[h] = -INFINITY;
-    if (lane < nk) {
-        const float4* kr = reinterpret_cast<const float4*>(Kc + (size_t)lane * KS);
-        const float4* qr = reinterpret_cast<const float4*>(qs);
-        float acc[H][2];
-#pragma unroll
-        for (int h = 0; h < H; ++h) acc[h][0] = acc[h][1] = 0.f;
-#pragma unroll
-        for (int c = 0; c < C4; ++c) {
-            const float4 k4 = kr[c];
-#pragma unroll
-            for (int h = 0; h < H; ++h) {
-                const float4 q4 = qr[h * C4 + c];
-                acc[h][c & 1] += q4.x * k4.x + q4.y * k4.y + q4.z * k4.z + q4.w * k4.w;
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < H; ++h) my_s[h] = acc[h][0] + acc[h][1];
-    }
-    float keep[H];
-    __syncwarp();  // the previous chunk's readers of ps are done
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-        const float m_new = fmaxf(m_run[h], warp_max(my_s[h]));
-        keep[h] = m_run[h] == -INFINITY ? 0.f : __expf(m_run[h] - m_new);
-        const float pr = lane < nk ? __expf(my_s[h] - m_new) : 0.f;
-        l_run[h] = l_run[h] * keep[h] + warp_sum(pr);
-        ps[h * 32 + lane] = pr;
-        m_run[h] = m_new;
-    }
-    __syncwarp();
-    float4 oa[H], ob[H];
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-        oa[h] = make_float4(o[h].x * keep[h], o[h].y * keep[h], o[h].z * keep[h], o[h].w * keep[h]);
-        ob[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    const float* vr = Vc + OPL * lane;
-    auto fma_row = [&](float4 (&acc4)[H], const float (&pj)[H], int j) {
-        if constexpr (OPL == 4) {
-            const float4 v4 = *reinterpret_cast<const float4*>(vr + (size_t)j * KS);
-#pragma unroll
-            for (int h = 0; h < H; ++h) {
-                acc4[h].x += pj[h] * v4.x;
-                acc4[h].y += pj[h] * v4.y;
-                acc4[h].z += pj[h] * v4.z;
-                acc4[h].w += pj[h] * v4.w;
-            }
-        } else {
-            const float2 v2 = *reinterpret_cast<const float2*>(vr + (size_t)j * KS);
-#pragma unroll
-            for (int h = 0; h < H; ++h) {
-                acc4[h].x += pj[h] * v2.x;
-                acc4[h].y += pj[h] * v2.y;
-            }
-        }
-    };
-    int j = 0;
-    for (; j + 4 <= nk; j += 4) {  // rows at and beyond nk are never read: they may hold anything
-        float4 p4[H];
-#pragma unroll
-        for (int h = 0; h < H; ++h) p4[h] = *reinterpret_cast<const float4*>(ps + h * 32 + j);
-        float pj[H];
-#pragma unroll
-        for (int h = 0; h < H; ++h) pj[h] = p4[h].x;
-        fma_row(oa, pj, j);
-#pragma unroll
-        for (int h = 0; h < H; ++h) pj[h] = p4[h].y;
-        fma_row(ob, pj, j + 1);
-#pragma unroll
-        for (int h = 0; h < H; ++h) pj[h] = p4[h].z;
-        fma_row(oa, pj, j + 2);
-#pragma unroll
-        for (int h = 0; h < H; ++h) pj[h] = p4[h].w;
-        fma_row(ob, pj, j + 3);
-    }
-    for (; j < nk; ++j) {
-        float pj[H];
-#pragma unroll
-        for (int h = 0; h < H; ++h) pj[h] = ps[h * 32 + j];
-        fma_row(oa, pj, j);
-    }
-#pragma unroll
-    for (int h = 0; h < H; ++h)
-        o[h] = make_float4(oa[h].x + ob[h].x, oa[h].y + ob[h].y, oa[h].z + ob[h].z, oa[h].w + ob[h].w);
-}
-
 // MAXS: the most slices (cluster size) this instantiation merges: 8 for portable clusters, 16 beyond.
 template <int D, int MAXS>
 __global__ void __launch_bounds__(AC_MAX_THREADS) attn_decode_cluster_kernel(const __grid_constant__ AttnDecodeParams p) {
@@ -753,103 +647,179 @@ __global__ void __launch_bounds__(AC_MAX_THREADS) attn_decode_cluster_kernel(con
 
 // ---------------------------------------------------------------------------------------
 // One-token attention for many sequences at once (batched generation steps): grid
-// (n_kv_heads, batch, runs), H query heads of the group per warp.  q is finished (rotated), the new
-// k / v row is in the cache already.  The CTA streams its run of the sequence's K and V rows through
-// shared memory AS_KEYS keys at a time, double buffered with cp.async, and every warp runs the
-// per-head chunk routine (attn_warp_chunk_rows).  One run (64 sequences and more): whole sequences,
-// finished attention rows, no partials, no merge.  Several runs (fewer sequences, so that about 512
-// CTAs exist): every run writes its un-normalised output with its (max, sum), merged by the stage
-// that quantises the attention rows.
-constexpr int AS_KEYS = 24;  // two stages of 24 keys: four CTAs per SM at head_dim 128, so that 64 sequences x 8 KV heads run as one wave
+// (n_kv_heads, batch, runs), the H query heads of a group together.  q is finished (rotated), the new
+// k / v row is in the cache already.  One run: whole sequences, finished attention rows.  Several runs:
+// every run writes its un-normalised output with its (max, sum), merged by the stage that quantises the
+// attention rows.
+//
+// Bound by the cache's stream as long as issue slots keep up, so the rows go straight to registers (a
+// row of D floats is one load of the warp, read once for all H heads) and a warp takes four keys at a time: 4 H
+// partial dot products per lane are folded over the lanes by halving (a lane hands over half of its values and keeps the
+// sums of the other half: 31 shuffles for 32 products, after which a lane holds one finished score), so that exponentials
+// are one instruction per 32 scores; the weights return through a line of shared memory.  The warps of a CTA take every
+// fourth group of four keys and merge at the end.  The next four keys are requested before the present ones are used.
+// 64 sequences of 1025 positions, 64 / 8 heads of 128: 167 us through shared memory with two heads a warp, 126 us here
+// (4.3 TB/s of cache); 8 sequences of 518, 20 / 5 heads: 11.7 -> 10.7 us with its wait for the kernel before.
+constexpr int AS_WARPS = 4, AS_KEYS = 4;
+
+template <int E>
+__device__ __forceinline__ void as_load(const float* src, bool live, float (&v)[E]) {
+    if constexpr (E == 4) {
+        const float4 r = live ? __ldcg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[0] = r.x, v[1] = r.y, v[2] = r.z, v[3] = r.w;
+    } else {
+        const float2 r = live ? __ldcg(reinterpret_cast<const float2*>(src)) : make_float2(0.f, 0.f);
+        v[0] = r.x, v[1] = r.y;
+    }
+}
 
 template <int D, int H>
-__global__ void __launch_bounds__(32 * AC_MAX_GROUP) attn_decode_stream_kernel(const __grid_constant__ AttnParams p) {
-    extern __shared__ __align__(16) float sm[];
-    constexpr int C4 = D / 4, OPL = D / 32, KS = D + AC_PAD;
-    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    const int G = p.n_heads / p.n_kv_heads;  // blockDim.x == 32 * G / H: warp w takes heads H w .. H w + H - 1 of the group
-    const int hk = blockIdx.x, b = blockIdx.y;
-    const int dq = p.n_heads * D;
+__global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_stream_kernel(const __grid_constant__ AttnParams p) {
+    constexpr int E = D / 32, HP = H > 4 ? 8 : H > 2 ? 4 : H;      // heads, rounded up to a power of two for the folding
+    constexpr int N = HP * AS_KEYS, SH = N == 32 ? 0 : N == 16 ? 1 : N == 8 ? 2 : 3;  // lane >> SH: value 4 h + key
+    __shared__ __align__(16) float s_w[AS_WARPS][2][N];            // weights of a group of keys
+    __shared__ float s_a[AS_WARPS][HP];                            // rescaling factors
+    __shared__ float s_m[AS_WARPS][HP], s_l[AS_WARPS][HP];
+    __shared__ __align__(16) float s_o[AS_WARPS][H][D];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int hk = blockIdx.x, b = blockIdx.y, dq = p.n_heads * D;
     const int T = min(p.past_len[b] + 1, p.max_seq);
-    const float* kc = p.k_cache + ((size_t)b * p.n_kv_heads + hk) * p.max_seq * D;
-    const float* vc = p.v_cache + ((size_t)b * p.n_kv_heads + hk) * p.max_seq * D;
-    float* qs = sm;                         // [G][D]
-    float* ps = qs + G * D;                 // [G][32]
-    float* Ks = ps + G * 32;                // [2][AS_KEYS][KS]
-    float* Vs = Ks + 2 * AS_KEYS * KS;      // [2][AS_KEYS][KS]
+    const size_t head0 = ((size_t)b * p.n_kv_heads + hk) * p.max_seq * D + E * lane;
+    const float *kc = p.k_cache + head0, *vc = p.v_cache + head0;
     // this CTA's run of the sequence: all of it, or one of gridDim.z equal parts
     const int nrun = (int)gridDim.z, run = (int)blockIdx.z;
     const int rlen = (T + nrun - 1) / nrun, k0 = run * rlen, k1 = min(T, k0 + rlen);
-    const int nchunk = k1 > k0 ? (k1 - k0 + AS_KEYS - 1) / AS_KEYS : 0;
-    auto fetch = [&](int chunk, int stage) {
-        const int t0 = k0 + chunk * AS_KEYS, n = min(AS_KEYS, k1 - t0);
-        for (int idx = tid; idx < n * C4; idx += nthr) {
-            const int r = idx / C4, c4 = idx - r * C4;
-            cp_async16(Ks + ((size_t)stage * AS_KEYS + r) * KS + 4 * c4, kc + (size_t)(t0 + r) * D + 4 * c4);
-            cp_async16(Vs + ((size_t)stage * AS_KEYS + r) * KS + 4 * c4, vc + (size_t)(t0 + r) * D + 4 * c4);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+
+    float ka[AS_KEYS][E], va[AS_KEYS][E], kb[AS_KEYS][E], vb[AS_KEYS][E];
+    auto fetch = [&](int t, float (&k)[AS_KEYS][E], float (&v)[AS_KEYS][E]) {
+#pragma unroll
+        for (int u = 0; u < AS_KEYS; ++u) as_load<E>(kc + (size_t)(t + u) * D, t + u < k1, k[u]);
+#pragma unroll
+        for (int u = 0; u < AS_KEYS; ++u) as_load<E>(vc + (size_t)(t + u) * D, t + u < k1, v[u]);
     };
+    int t = k0 + AS_KEYS * warp;
     // rows behind the new one are older than the kernel before this one (see the rule in common.cuh)
-    const bool early = nchunk > 0 && min(k0 + AS_KEYS, k1) < T;
-    if (early) fetch(0, 0);
+    const bool early = t < k1 && min(t + AS_KEYS, k1) < T;
+    if (early) fetch(t, ka, va);
     pdl_wait();
     pdl_trigger();
-    if (nchunk > 0 && !early) fetch(0, 0);
-    {  // this warp's q rows, pre-scaled (read back by the same warp only, after the first CTA barrier)
-        const float* qh = p.q + (size_t)b * dq + (size_t)(hk * G + warp * H) * D;
-        const float scale = 1.0f / sqrtf((float)D);
-        for (int i = lane; i < H * C4; i += 32) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(qh) + i);
-            reinterpret_cast<float4*>(qs + warp * H * D)[i] = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
-        }
-    }
-    float m_run[H], l_run[H];
-    float4 o[H];
+    if (t < k1 && !early) fetch(t, ka, va);
+    float q[H][E];
+    const float scale = 1.0f / sqrtf((float)D);
 #pragma unroll
     for (int h = 0; h < H; ++h) {
-        m_run[h] = -INFINITY;
-        l_run[h] = 0.f;
-        o[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+        as_load<E>(p.q + (size_t)b * dq + (size_t)(hk * H + h) * D + E * lane, true, q[h]);
+#pragma unroll
+        for (int e = 0; e < E; ++e) q[h][e] *= scale;
     }
-    for (int c = 0; c < nchunk; ++c) {
-        if (c + 1 < nchunk) {
-            fetch(c + 1, (c + 1) & 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float m_run = -INFINITY, l_run = 0.f;  // of this lane's head; l_run: of this lane's keys alone
+    float o[H][E];
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int e = 0; e < E; ++e) o[h][e] = 0.f;
+    const int mine = lane >> SH, my_key = mine & 3, my_head = mine >> 2;
+    int flip = 0;
+    auto step = [&](int t0, const float (&k)[AS_KEYS][E], const float (&v)[AS_KEYS][E]) {
+        float s[N];
+#pragma unroll
+        for (int h = 0; h < HP; ++h)
+#pragma unroll
+            for (int u = 0; u < AS_KEYS; ++u) {
+                float d = 0.f;
+                if (h < H) {
+#pragma unroll
+                    for (int e = 0; e < E; ++e) d += q[h < H ? h : 0][e] * k[u][e];
+                }
+                s[4 * h + u] = d;
+            }
+#pragma unroll
+        for (int w = 16, n = N; w >= 1; w >>= 1) {
+            if (n > 1) {
+                n >>= 1;
+                const bool up = lane & w;
+#pragma unroll
+                for (int i = 0; i < N / 2; ++i)
+                    if (i < n) {
+                        const float give = up ? s[i] : s[i + n], keep = up ? s[i + n] : s[i];
+                        s[i] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+                    }
+            } else {
+                s[0] += __shfl_xor_sync(0xffffffffu, s[0], w);
+            }
         }
-        __syncthreads();  // chunk c has landed for every thread
-        const int st = c & 1;
-        attn_warp_chunk_rows<D, H>(qs + warp * H * D, Ks + (size_t)st * AS_KEYS * KS, Vs + (size_t)st * AS_KEYS * KS,
-                                   ps + warp * H * 32, min(AS_KEYS, k1 - k0 - c * AS_KEYS), lane, m_run, l_run, o);
-        __syncthreads();  // every warp is done with this stage before chunk c + 2 overwrites it
-    }
-    if (nrun > 1) {  // partial results of this run: merged by the stage that follows
+        const bool live = t0 + my_key < k1;
+        float top = live ? s[0] : -INFINITY;
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1 << SH));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2 << SH));
+        const float m_new = fmaxf(m_run, top);
+        const float w = live ? __expf(s[0] - m_new) : 0.f;
+        s_w[warp][flip][mine] = w;
+        if (__any_sync(0xffffffffu, m_new > m_run)) {  // (rare after the first keys)
+            const float a = m_run == -INFINITY ? 0.f : __expf(m_run - m_new);
+            s_a[warp][my_head] = a;
+            __syncwarp();
+            l_run *= a;
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                const float ah = s_a[warp][h];
+#pragma unroll
+                for (int e = 0; e < E; ++e) o[h][e] *= ah;
+            }
+        }
+        m_run = m_new;
+        l_run += w;
+        __syncwarp();  // weights written; the other buffer's readers have passed the previous one
 #pragma unroll
         for (int h = 0; h < H; ++h) {
-            const size_t slot = ((size_t)b * p.n_heads + (hk * G + warp * H + h)) * nrun + run;
-            float* dst = p.part_o + slot * D + OPL * lane;
-            if constexpr (OPL == 4) {
-                *reinterpret_cast<float4*>(dst) = o[h];
-            } else {
-                *reinterpret_cast<float2*>(dst) = make_float2(o[h].x, o[h].y);
-            }
-            if (lane == 0) {
-                p.part_m[slot] = m_run[h];
-                p.part_l[slot] = l_run[h];
-            }
-        }
-        return;
-    }
+            const float4 w4 = *reinterpret_cast<const float4*>(&s_w[warp][flip][4 * h]);
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-        const float inv = 1.0f / l_run[h];
-        float* dst = p.out + (size_t)b * dq + (size_t)(hk * G + warp * H + h) * D + OPL * lane;
-        if constexpr (OPL == 4) {
-            *reinterpret_cast<float4*>(dst) = make_float4(o[h].x * inv, o[h].y * inv, o[h].z * inv, o[h].w * inv);
+            for (int e = 0; e < E; ++e) o[h][e] += w4.x * v[0][e] + w4.y * v[1][e] + w4.z * v[2][e] + w4.w * v[3][e];
+        }
+        flip ^= 1;
+    };
+    constexpr int STRIDE = AS_KEYS * AS_WARPS;
+    while (t < k1) {
+        if (t + STRIDE < k1) fetch(t + STRIDE, kb, vb);
+        step(t, ka, va);
+        t += STRIDE;
+        if (t >= k1) break;
+        if (t + STRIDE < k1) fetch(t + STRIDE, ka, va);
+        step(t, kb, vb);
+        t += STRIDE;
+    }
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 1 << SH);
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 2 << SH);
+    s_m[warp][my_head] = m_run;
+    s_l[warp][my_head] = l_run;
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int e = 0; e < E; ++e) s_o[warp][h][E * lane + e] = o[h][e];
+    __syncthreads();
+    // ---- merge of the warps: thread = output element
+#pragma unroll
+    for (int i = threadIdx.x; i < H * D; i += 32 * AS_WARPS) {
+        const int h = i / D, d = i - h * D;
+        float M = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < AS_WARPS; ++w) M = fmaxf(M, s_m[w][h]);
+        float acc = 0.f, L = 0.f;
+#pragma unroll
+        for (int w = 0; w < AS_WARPS; ++w) {
+            const float f = s_m[w][h] == -INFINITY ? 0.f : __expf(s_m[w][h] - M);
+            acc += f * s_o[w][h][d];
+            L += f * s_l[w][h];
+        }
+        if (nrun > 1) {  // partial results of this run: merged by the stage that follows
+            const size_t slot = ((size_t)b * p.n_heads + (hk * H + h)) * nrun + run;
+            p.part_o[slot * D + d] = acc;
+            if (d == 0) {
+                p.part_m[slot] = M;
+                p.part_l[slot] = L;
+            }
         } else {
-            *reinterpret_cast<float2*>(dst) = make_float2(o[h].x * inv, o[h].y * inv);
+            p.out[(size_t)b * dq + (size_t)(hk * H + h) * D + d] = acc * (1.0f / L);
         }
     }
 }
@@ -861,25 +831,38 @@ static bool attn_decode_stream_ok(const AttnParams& p, int rows) {
     return G >= 1 && G <= AC_MAX_GROUP;
 }
 
-// Fewer sequences than fill the GPU: cut each into runs so that about 512 CTAs exist (a power of two,
-// at most max_nsplit).
-int attn_stream_splits(int rows, int n_heads, int n_kv_heads, int head_dim, int max_nsplit) {
+// Fewer sequences than fill the GPU: cut each into runs (a power of two, at most max_nsplit), about 512 CTAs for any
+// length, so that every SM has work, and up to 2048 while a run keeps 64 of the cache's positions: three CTAs share an SM,
+// and with one CTA too many for a whole round the SMs that end first would idle.
+int attn_stream_splits(int rows, int n_heads, int n_kv_heads, int head_dim, int max_nsplit, int max_seq) {
     if (n_kv_heads < 1 || n_heads % n_kv_heads || (head_dim != 64 && head_dim != 128)) return 0;
     const int G = n_heads / n_kv_heads;
     if (G < 1 || G > AC_MAX_GROUP) return 0;
     int s = 1;
-    while (2 * s <= max_nsplit && (long)rows * n_kv_heads * 2 * s <= 512) s *= 2;
+    while (2 * s <= max_nsplit && ((long)rows * n_kv_heads * 2 * s <= 512 ||
+                                   ((long)rows * n_kv_heads * 2 * s <= 2048 && max_seq / (2 * s) >= 64)))
+        s *= 2;
     return s;
 }
 
+template <int D>
+static int launch_attn_decode_stream_d(const AttnParams& p, int rows, cudaStream_t st) {
+    const dim3 grid(p.n_kv_heads, rows, p.nsplit > 1 ? p.nsplit : 1);
+    switch (p.n_heads / p.n_kv_heads) {
+        case 1: return launch_dependent(attn_decode_stream_kernel<D, 1>, grid, 32 * AS_WARPS, 0, p, st);
+        case 2: return launch_dependent(attn_decode_stream_kernel<D, 2>, grid, 32 * AS_WARPS, 0, p, st);
+        case 3: return launch_dependent(attn_decode_stream_kernel<D, 3>, grid, 32 * AS_WARPS, 0, p, st);
+        case 4: return launch_dependent(attn_decode_stream_kernel<D, 4>, grid, 32 * AS_WARPS, 0, p, st);
+        case 5: return launch_dependent(attn_decode_stream_kernel<D, 5>, grid, 32 * AS_WARPS, 0, p, st);
+        case 6: return launch_dependent(attn_decode_stream_kernel<D, 6>, grid, 32 * AS_WARPS, 0, p, st);
+        case 7: return launch_dependent(attn_decode_stream_kernel<D, 7>, grid, 32 * AS_WARPS, 0, p, st);
+        case 8: return launch_dependent(attn_decode_stream_kernel<D, 8>, grid, 32 * AS_WARPS, 0, p, st);
+    }
+    return ROTOR_B200_ERR_SHAPE;
+}
+
 static int launch_attn_decode_stream(const AttnParams& p, int rows, cudaStream_t st) {
-    const int G = p.n_heads / p.n_kv_heads, D = p.head_dim;
-    const size_t smem = ((size_t)G * D + (size_t)G * 32 + (size_t)4 * AS_KEYS * (D + AC_PAD)) * sizeof(float);
-    dim3 grid(p.n_kv_heads, rows, p.nsplit > 1 ? p.nsplit : 1);
-    // two heads per warp when the group is even and leaves at least two warps
-    if (G % 2 == 0 && G >= 4)
-        return launch_dependent(D == 64 ? attn_decode_stream_kernel<64, 2> : attn_decode_stream_kernel<128, 2>, grid, 16 * G, smem, p, st);
-    return launch_dependent(D == 64 ? attn_decode_stream_kernel<64, 1> : attn_decode_stream_kernel<128, 1>, grid, 32 * G, smem, p, st);
+    return p.head_dim == 64 ? launch_attn_decode_stream_d<64>(p, rows, st) : launch_attn_decode_stream_d<128>(p, rows, st);
 }
 
 static size_t attn_cluster_smem(int G, int D, int lcmax, int ns) {
@@ -1042,14 +1025,6 @@ int configure_attention() {
     RB_CUDA(cudaFuncSetAttribute(attn_decode_cluster_kernel<128, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     RB_CUDA(cudaFuncSetAttribute(attn_decode_cluster_kernel<64, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     RB_CUDA(cudaFuncSetAttribute(attn_decode_cluster_kernel<128, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<128, 1>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared));
-    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<128, 2>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared));
-    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
-    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
-    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
-    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
     RB_CUDA(cudaFuncSetAttribute(attn_decode_cluster_kernel<64, 8>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared));
     RB_CUDA(cudaFuncSetAttribute(attn_decode_cluster_kernel<128, 8>, cudaFuncAttributePreferredSharedMemoryCarveout,

@@ -224,7 +224,7 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
     // 5 to 63 sequences: the streaming kernel over runs of every sequence (about 512 CTAs), partial results
     // merged by the stage that quantises the attention rows
     const int runs = (seq == 1 && batch >= 5 && batch <= c.max_batch)
-                         ? attn_stream_splits(batch, c.n_heads, c.n_kv_heads, c.head_dim, c.nsplit) : 0;
+                         ? attn_stream_splits(batch, c.n_heads, c.n_kv_heads, c.head_dim, c.nsplit, c.max_seq) : 0;
     if (seq == 1 && batch <= c.max_batch && batch < 16 && runs <= 1) {
         // generation step: dequantise, rotate, append to the cache, attend, merge and quantise in one launch
         AttnDecodeParams dp = {};

@@ -194,7 +194,7 @@ struct AttnParams {
 int launch_attention(const AttnParams& p, int rows, cudaStream_t st);
 // Runs for a one-token step of `rows` sequences handled by the streaming kernel (1 = whole sequences,
 // finished rows in `out`); 0 if that kernel does not take the shape.
-int attn_stream_splits(int rows, int n_heads, int n_kv_heads, int head_dim, int max_nsplit);
+int attn_stream_splits(int rows, int n_heads, int n_kv_heads, int head_dim, int max_nsplit, int max_seq);
 bool attn_prefill_supported(const AttnParams& p, int rows);
 int launch_attn_prefill_tc(const AttnParams& p, int rows, cudaStream_t st);
 // head_dim 128 on tcgen05 / tensor memory (attn_prefill_t5.cu); needs the split planes sized for

@@ -535,12 +535,13 @@ def test_batched_greedy_generation_ragged(rb, lens):
         _tiny(rb, "hd64", rb.sem.REFERENCE, max_batch=batch)[2].generate_greedy_batch(prompts, new)
 
 
-@pytest.mark.parametrize("shape", [(1024, 8, 2, 1536), (2560, 20, 5, 6912), (8192, 64, 8, 9216)])
+@pytest.mark.parametrize("shape", [(1024, 8, 2, 1536), (2560, 20, 5, 6912), (8192, 64, 8, 9216), (512, 8, 8, 512), (512, 4, 2, 512),
+                                   (768, 12, 4, 512), (1280, 20, 4, 512), (768, 6, 1, 512), (1792, 14, 2, 512), (1024, 16, 2, 512)])
 @pytest.mark.parametrize("batch,context", [(5, 300), (16, 30), (33, 129)])
 def test_batched_steps_equal_single_sequences(rb, shape, batch, context):
     """Two steps of several sequences (row stages with few rows, merged runs of the decode attention, sums cleared ahead
     of split products) against the same steps of each sequence alone: widths of every thread count, contexts with and
-    without several runs per sequence, ragged runs.  Three activation terms: float32 rounding is all that may differ."""
+    without several runs per sequence, ragged runs, one to eight query heads per key head.  Three activation terms: float32 rounding is all that may differ."""
     import torch
     d, heads, kv, ff = shape
     cfg = dict(vocab_size=512, d_model=d, n_layers=2, n_heads=heads, n_kv_heads=kv, d_ff=ff)
