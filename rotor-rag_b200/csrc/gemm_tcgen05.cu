@@ -33,9 +33,9 @@ RB_TRACE_DEFINE(rotor_b200_trace_read_gemm5)
 
 namespace rb {
 
-// Tokens per CTA is a template argument too: 256 (two MMA M halves, one CTA per SM: all 512
-// tensor-memory columns) or 128 (one half, 256 columns and a two-stage ring, so that TWO CTAs share
-// an SM and the accumulator read-back of one overlaps the MMAs of the other).
+// Tokens per CTA is a template argument too: 256 (two MMA M halves, all 512 tensor-memory columns) or 128 (one
+// half) for at most 128 tokens: the product is then bound by the weight stream, and the halved token operand leaves
+// room for a fourth stage; four K steps of weights are requested ahead instead of two.
 // Decoder warps (they also read the accumulators back), then one TMA + TMEM warp and one MMA warp.
 // Eight decoders for 256-row tiles: a lone warp per scheduler issues about one instruction every
 // four cycles, and at four warps the decode of a K step (about 550 instructions per warp) took
@@ -49,14 +49,15 @@ struct T5Cfg {
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     // ring depth and decoder look-ahead: with 64-row tiles a stage is only four short MMAs, so the
     // copy and weight-load latencies need more stages in flight to stay hidden
-    static constexpr int STAGES = TOK == 128 ? 2 : (ROWS >= 256 ? 3 : 5);
-    static constexpr int PREFETCH = ROWS >= 256 ? 2 : 6;           // K steps of weight tiles requested ahead
+    static constexpr int STAGES = TOK == 128 ? 4 : (ROWS >= 256 ? 3 : 5);
+    static constexpr int PREFETCH = ROWS < 256 ? 6 : TOK == 128 ? 4 : 2;           // K steps of weight tiles requested ahead
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024;       // + slack to align the ring to 1024 bytes
     static constexpr int TMEM_COLS = (TOK / 128) * ROWS < 32 ? 32 : (TOK / 128) * ROWS;  // one accumulator of ROWS columns per token half
     static constexpr int DECODERS = ROWS >= 256 ? 8 : 4;           // decoder warps
     static constexpr int THREADS = (DECODERS + 2) * 32;
     static constexpr int TILES_PER_WARP = ROWS / TILE_ROWS / DECODERS;  // row tiles each decoder warp handles
 };
+constexpr int T5_DEEP_STEPS = 12;  // K steps of a CTA from which the 128-token variant is taken
 struct Tc5Params {
     const uint4* tiles;
     const int32_t* xsum;  // [ncols] sum of each token's int8 activations (removes the +1 of the weight codes)
@@ -192,7 +193,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
                 }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_full[s])) : "memory");
+            t5_bar_arrive(smem_u32(&s_full[s]));
             fetch(kt + PF, wv[par]);
 #ifdef RB_TRACE
             if (tracedd) { const unsigned long long n_ = gtime(); trd.t[1] += n_ - tld; tld = n_; }
@@ -346,12 +347,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
 #pragma unroll
                         for (int q = 0; q < 32; ++q) v[q] -= xs;
                         if (p.kt_per_split) {  // one of several partial sums: exact, in any order
-                            if (token < p.ncols) {
-                                int32_t* dst = p.acc + (size_t)token * p.out + rbase;
+                            // Whole lines at a time; a lane per token touches 32 lines per instruction, which wins only while one
+                            // warp's worth of tokens adds at all (2560 x 2560: 32 tokens 12.0 against 13.9 us, 64 tokens
+                            // 17.4 against 14.0, 903 tokens 56.8 against 25.4).
+                            if (p.ncols <= 32) {
+                                if (token < p.ncols) {
+                                    int32_t* dst = p.acc + (size_t)token * p.out + rbase;
 #pragma unroll
-                                for (int q = 0; q < 32; ++q)
-                                    if (rbase + q < p.out) atomicAdd(dst + q, (int32_t)v[q]);
-                            }
+                                    for (int q = 0; q < 32; ++q)
+                                        if (rbase + q < p.out) atomicAdd(dst + q, (int32_t)v[q]);
+                                }
+                            } else
+                            t5_add_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
+                                        (size_t)p.out, p.out - rbase, tok_base, p.ncols, lane);
                         } else if (rbase + 32 <= p.out && (p.out & 3) == 0) {
                             t5_store_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
                                           (size_t)p.out * sizeof(int32_t), tok_base, p.ncols, lane);
@@ -488,6 +496,7 @@ int configure_gemm_tcgen05() {
     if (!fn || q != cudaDriverEntryPointSuccess) return ROTOR_B200_ERR_CUDA;
     g_encode = (EncodeTiledFn)fn;
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<256>::SMEM));
+    RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<256, 128>::SMEM));
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<64>::SMEM));
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  T5Cfg<256>::SMEM));
@@ -537,17 +546,24 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
     const int tok_tiles = (ncols + 255) / 256, rows = p.nrt * TILE_ROWS;
     const int sms = fused_sm_count(), tiles256 = tok_tiles * ((rows + 255) / 256);
     int splits = gemm_tcgen05_splits(out, in, ncols);
+    auto launch256 = [&](dim3 grid) {
+        // (64 tokens, 57344 x 8192: 78.3 -> 66.9 us, 8192 x 28672: 44.7 -> 38.7; runs of fewer steps end before the
+        // deeper look-ahead is filled and take the variant with less code)
+        if (ncols <= 128 && (p.kt_per_split ? p.kt_per_split : p.nkt) >= T5_DEEP_STEPS)
+            gemm_tcgen05_kernel<256, 128><<<grid, T5Cfg<256, 128>::THREADS, T5Cfg<256, 128>::SMEM, st>>>(tmap, p);
+        else
+            gemm_tcgen05_kernel<256><<<grid, T5Cfg<256>::THREADS, T5Cfg<256>::SMEM, st>>>(tmap, p);
+    };
     if (splits >= 2) {
         p.kt_per_split = (p.nkt + splits - 1) / splits;
         if (!zeroed) RB_CUDA(cudaMemsetAsync(acc, 0, (size_t)ncols * out * sizeof(int32_t), st));
         dim3 grid(tok_tiles, (rows + 255) / 256, splits);
-        gemm_tcgen05_kernel<256><<<grid, T5Cfg<256>::THREADS, T5Cfg<256>::SMEM, st>>>(tmap, p);
+        launch256(grid);
     } else if (tiles256 < sms) {  // 256-row tiles would leave SMs idle
         dim3 grid(tok_tiles, (rows + 63) / 64);
         gemm_tcgen05_kernel<64><<<grid, T5Cfg<64>::THREADS, T5Cfg<64>::SMEM, st>>>(tmap, p);
     } else {
-        dim3 grid(tok_tiles, (rows + 255) / 256);
-        gemm_tcgen05_kernel<256><<<grid, T5Cfg<256>::THREADS, T5Cfg<256>::SMEM, st>>>(tmap, p);
+        launch256(dim3(tok_tiles, (rows + 255) / 256));
     }
     return launch_status();
 }

@@ -86,6 +86,25 @@ __device__ __forceinline__ void t5_store_rows(uint32_t stage, const uint32_t (&v
     __syncwarp();  // the block is rewritten by the warp's next item
 }
 
+// The same block of int32 sums, added to what is there: a token's 32 values are one line per instruction.
+__device__ __forceinline__ void t5_add_rows(uint32_t stage, const uint32_t (&v)[32], int32_t* dst0, size_t row_ints, int n,
+                                            int tok_base, int ntok, int lane) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)lane * 144u + 16u * q),
+                     "r"(v[4 * q]), "r"(v[4 * q + 1]), "r"(v[4 * q + 2]), "r"(v[4 * q + 3])
+                     : "memory");
+    __syncwarp();
+#pragma unroll 8
+    for (int tl = 0; tl < 32; ++tl) {
+        uint32_t w;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(stage + (uint32_t)tl * 144u + 4u * lane));
+        if (tok_base + tl >= ntok) break;  // warp-uniform
+        if (lane < n) atomicAdd(dst0 + (size_t)tl * row_ints + lane, (int32_t)w);
+    }
+    __syncwarp();
+}
+
 // The same with a destination per token: dst_of(tl) is the address of token tok_base + tl's 128 bytes
 // (null = skip).
 template <typename F>
