@@ -82,6 +82,7 @@ __device__ __forceinline__ float4 rs_deq_staged(const int4* stage, int n4, int h
     return make_float4(f.x * wscale, f.y * wscale, f.z * wscale, f.w * wscale);
 }
 
+// Rows of up to five groups with a residual: six CTAs per SM (16384 rows of 2560: 119 us against 129 with five).
 // Wide rows (V > 8) are capped at 128 registers so that four CTAs share an SM: with fewer, the
 // reductions and the quantiser of one row leave the memory pipe idle.
 // RESID: the stage adds to the residual stream (VS_OPROJ, VS_DOWN) and keeps a second register
@@ -94,7 +95,7 @@ __device__ __forceinline__ float4 rs_deq_staged(const int4* stage, int n4, int h
 // as soon as the owner has the pieces in registers.  Accumulator modes only.
 // MERGE: VS_ATTN, the row is merged from the partial results of the decode attention's runs.
 template <int V, bool RESID, int TH, bool PF, bool MERGE = false>
-__global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 128 ? (V <= 4 ? 2 : 1) : (V > 8 ? 4 : 5))
+__global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1) : TH > 128 ? 4 : V > 8 ? 4 : RESID && V <= 5 ? 6 : 5)
     row_stage_kernel(const __grid_constant__ VecStageParams p, int rows) {
     __shared__ float scratch[64];
     extern __shared__ __align__(16) int4 rs_stage[];
@@ -427,10 +428,14 @@ int launch_row_stage(const VecStageParams& p, int rows, cudaStream_t st) {
         return launch_one<14, false, RS_WIDE_THREADS>(p, rows, st);
     }
     const int v = (width / 4 + RS_THREADS - 1) / RS_THREADS;
-    if (v > 8 && p.mode != VS_OPROJ && p.mode != VS_DOWN)
-        // 4097..8192 elements without a residual (the 2B FFN row): four groups per thread at 512 threads
-        // keep more warps per SM busy than fourteen groups at 128
+    if (v > 8 && p.mode != VS_OPROJ && p.mode != VS_DOWN) {
+        // 4097..8192 elements without a residual (the 2B FFN row).  Gated rows are one staged piece: four CTAs of 256
+        // threads with seven groups each share an SM, and one row's reductions hide behind three others' (16384 rows of
+        // 6912: 164 us, two CTAs of 512 threads 191, three 217, fourteen groups at 128 threads 195).  Accumulators are
+        // two to six pieces, which leave room for fewer CTAs: these want the 512 threads.
+        if (p.mode == VS_PLAIN && width <= 4 * 7 * 256) return launch_one<7, false, 256>(p, rows, st);
         return launch_one<4, false, RS_WIDE_THREADS>(p, rows, st);
+    }
     if (p.mode == VS_OPROJ || p.mode == VS_DOWN) {
         // 4097..8192 elements with a residual row: sixteen groups per thread do not fit the registers of a
         // 128-thread CTA, four groups at 512 threads do

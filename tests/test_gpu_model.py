@@ -498,6 +498,23 @@ def test_wide_ffn_many_rows(rb):
     assert rel_err(got, want) < TOL, rel_err(got, want)
 
 
+@pytest.mark.parametrize("ff", [4112, 6912, 7168, 7184, 8192])
+def test_gated_rows_of_a_prompt(rb, ff):
+    """300 rows whose gate/up product gates in its read-back: the stage that norms and quantises the float rows, at the widths
+    where its thread counts change, against the same rows five at a time.  One term: a value on a tie of the quantiser may
+    fall either way (one step of 1/127 of a row's largest value in a row of thousands)."""
+    import torch
+    ffn = rb.tr.GatedFFN(256, ff, semantics=rb.sem.BASELINE)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(ff)
+    for p in (ffn.gate_proj, ffn.up_proj, ffn.down_proj):
+        p.load_from_int8(torch.randint(-1, 2, (p.out_features, p.in_features), generator=g, device="cuda", dtype=torch.int8), 0.02)
+    x = torch.randn((300, 256), generator=g, device="cuda")
+    got, want = ffn.forward_device(x), torch.cat([ffn.forward_device(x[i:i + 5].contiguous()) for i in range(0, 300, 5)])
+    assert (got - want).norm() < 4e-3 * want.norm()
+    assert ((got - want).abs().amax(1) == 0).float().mean() > 0.3   # most rows hold no tie
+
+
 @pytest.mark.parametrize("batch", [3, 6])
 def test_batched_greedy_generation(rb, batch):
     """Equal-length prompts generated together give, sequence by sequence, the oracle's tokens
