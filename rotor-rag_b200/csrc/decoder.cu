@@ -293,6 +293,7 @@ struct DecoderPass {
         p.f32 = f32;
         p.x = x;
         p.ldx = ldx;
+        p.early = rows <= DENSE_EARLY_ROWS;
         return p;
     }
     DenseProduct plain(const void* w, int n, int k, const void* x, int ldx, float* y, int ldy) const {

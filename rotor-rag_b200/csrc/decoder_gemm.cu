@@ -83,6 +83,7 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* abort_flag = &s_abort;
     const int nk = (p.k + 63) >> 6;
+    if (p.table) pdl_wait();  // (the table is the work of the kernel before; without one only the weights are read ahead)
     const int mt = p.table ? __ldg(p.table) : p.mt, per_group = mt * p.nt, ntiles = per_group * p.groups;
 
     if (threadIdx.x == 0) {
@@ -135,19 +136,32 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (elect_lane()) {
             int it = 0;
             bool ok = true;
+            auto weights = [&](const DgTile& at, int kt, int s) {
+                const uint32_t bar = smem_u32(&s_full[s]), st = ring + s * C::STAGE;
+                t5_bar_expect(bar, C::STAGE);
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+                    t5_tma_2d(st + C::A_BYTES + b * BOX * 128, &tm_b, kt * 64,
+                              at.w_row + (EPI == DENSE_GATED ? b * p.n + at.n * TN : at.n * TN + b * BOX), bar);
+            };
+            // the first stages' weights (constants) are requested while the kernel before this one ends; no trigger: what
+            // follows starts when this kernel has ended
+            const int ahead = (int)blockIdx.x < ntiles ? min(ST, nk) : 0;
+            if (ahead) {
+                const DgTile at = place(blockIdx.x);
+                for (int kt = 0; kt < ahead; ++kt) weights(at, kt, kt);
+            }
+            pdl_wait();
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 const DgTile at = place(t);
                 for (int kt = 0; kt < nk; ++kt, ++it) {
                     const int s = it % ST;
-                    ok = t5_wait(smem_u32(&s_empty[s]), ((it / ST) & 1) ^ 1, abort_flag, p.status, 0x7a000001u);
-                    if (!ok) break;
-                    const uint32_t bar = smem_u32(&s_full[s]), st = ring + s * C::STAGE;
-                    t5_bar_expect(bar, C::STAGE);
-                    t5_tma_2d(st, &tm_a, at.x_col + kt * 64, at.x_row, bar);
-#pragma unroll
-                    for (int b = 0; b < NB; ++b)
-                        t5_tma_2d(st + C::A_BYTES + b * BOX * 128, &tm_b, kt * 64,
-                                  at.w_row + (EPI == DENSE_GATED ? b * p.n + at.n * TN : at.n * TN + b * BOX), bar);
+                    if (it >= ahead) {
+                        ok = t5_wait(smem_u32(&s_empty[s]), ((it / ST) & 1) ^ 1, abort_flag, p.status, 0x7a000001u);
+                        if (!ok) break;
+                        weights(at, kt, s);
+                    }
+                    t5_tma_2d(ring + s * C::STAGE, &tm_a, at.x_col + kt * 64, at.x_row, smem_u32(&s_full[s]));
                 }
             }
         }
@@ -180,6 +194,7 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         const int wq = warp & 3;  // the quarter of the tensor-memory lanes this warp reaches
         const uint32_t stage = xpose + (uint32_t)(warp - 2) * T5_XPOSE_BYTES;
         int lt = 0;
+        pdl_wait();  // outputs, cached lengths and gates belong to earlier kernels until here
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
             const DgTile at = place(t);
             const int n = at.n;
@@ -405,7 +420,9 @@ static int dg5_launch(const DenseProduct& p, int rows, cudaStream_t st) {
     if (!t5_map_bf16(&ta, p.x, x_rows, x_cols, p.ldx, 128) || !t5_map_bf16(&tb, p.w, w_rows, p.k, p.ldw, BOX)) return ROTOR_B200_ERR_CUDA;
     const long long tiles = dg5_token_tiles(p, rows) * a.nt;
     const int sms = fused_sm_count();
-    dense_gemm_t5_kernel<BN, EPI><<<(int)(tiles < sms ? tiles : sms), DG5_THREADS, C::SMEM, st>>>(ta, tb, a);
+    const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
+    if (p.early) return launch_chained(dense_gemm_t5_kernel<BN, EPI>, dim3(grid), dim3(DG5_THREADS), C::SMEM, st, 1, ta, tb, a);
+    dense_gemm_t5_kernel<BN, EPI><<<grid, DG5_THREADS, C::SMEM, st>>>(ta, tb, a);
     return launch_status();
 }
 
