@@ -219,10 +219,8 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
     const bool fuse_qkv = qkv_finishes(c, seq, cols);
     AccView va = {};
     if (!fuse_qkv) RB_TRY(gemv(c, L.qkv_tiles, qkv_out, c.d, cols, 0, c.accA, &va, st));
-    // (sixteen and more sequences: the tiled attention kernel streams each sequence's cache once per
-    // group of heads, which beats thousands of small split CTAs; measured on the XL shape, batch 64)
-    // 5 to 63 sequences: the streaming kernel over runs of every sequence (about 512 CTAs), partial results
-    // merged by the stage that quantises the attention rows
+    // five and more sequences: the streaming kernel reads each sequence's cache once per group of heads, cut into runs
+    // (attn_stream_splits) whose partial results the stage that quantises the attention rows merges
     const int runs = (seq == 1 && batch >= 5 && batch <= c.max_batch)
                          ? attn_stream_splits(batch, c.n_heads, c.n_kv_heads, c.head_dim, c.nsplit, c.max_seq) : 0;
     if (seq == 1 && batch <= c.max_batch && batch < 16 && runs <= 1) {

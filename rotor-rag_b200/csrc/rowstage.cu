@@ -2,8 +2,8 @@
 // vecstage.cuh with the row held in registers.
 //
 // With thousands of rows the stages are pure HBM traffic (int32 accumulators or float rows in,
-// residual stream in and out, int8 activations out); what matters is bytes in flight.  A CTA of 128,
-// 512 or 1024 threads per row; a thread owns up to V groups of four consecutive elements and issues
+// residual stream in and out, int8 activations out); what matters is bytes in flight.  A CTA of 128
+// to 1024 threads per row; a thread owns up to V groups of four consecutive elements and issues
 // ALL of its 128-bit loads (accumulators of every term, residual stream, norm weights) before the
 // first use.  In the prefetching variant a grid of resident CTAs walks the rows, and a thread copies
 // its pieces of the next row into a private shared-memory area (cp.async) while the current row is
