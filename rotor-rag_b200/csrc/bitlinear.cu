@@ -419,7 +419,7 @@ size_t rotor_b200_bitlinear_workspace_bytes(size_t out, size_t in, size_t m, int
 int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const float* x, size_t m, int terms,
                                  float wscale, const float* wscale_vec, float* y, void* workspace,
                                  size_t workspace_bytes, int variant, void* stream) {
-    RB_REQUIRE(tiles && x && y && workspace && m > 0 && terms >= 1 && terms <= 4);
+    RB_REQUIRE(tiles && x && y && workspace && m > 0 && out > 0 && in > 0 && terms >= 1 && terms <= 4);
     RB_REQUIRE(((uintptr_t)workspace & 255) == 0);
     if (workspace_bytes < rotor_b200_bitlinear_workspace_bytes(out, in, m, terms)) return ROTOR_B200_ERR_WORKSPACE;
     const size_t nc = m * (size_t)terms;

@@ -103,7 +103,7 @@ int configure_fused_gemv() {
 // activation terms each.
 bool fused_gemv_supported(size_t out, size_t in, int rows, int terms, int halves, int merge_weights) {
     const int cols = rows * terms;
-    if (rows < 1 || cols > 8 || terms > 3 || in % 4) return false;
+    if (!out || !in || rows < 1 || cols > 8 || terms > 3 || in % 4) return false;
     FusedGemvParams p = {};
     p.st.n = (int)in;
     if (fused_wide(p.st) && merge_weights) return false;

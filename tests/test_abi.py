@@ -65,3 +65,21 @@ def test_argument_errors_do_not_need_a_gpu(lib):
     lib.rotor_b200_pack.restype = ctypes.c_int
     lib.rotor_b200_pack.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p]
     assert lib.rotor_b200_pack(None, None, 6, None, None) == 1      # length must be a multiple of 4
+
+
+@pytest.mark.parametrize("out,inn", [(0, 128), (16, 0), (0, 0)])
+@pytest.mark.parametrize("rows,terms,variant", [(1, 1, 0), (4, 2, 0), (5, 3, 0), (1, 1, 2)])
+def test_layer_call_of_no_rows_or_columns_is_an_argument_error(lib, out, inn, rows, terms, variant):
+    """A weight matrix of size zero is refused on the host, before a grid is sized by it and before any CUDA call (the
+    addresses are never read: one call in a process of its own, which a division by zero would end)."""
+    import sys
+    code = """
+import ctypes as C, sys
+f = C.CDLL(sys.argv[1]).rotor_b200_bitlinear_forward
+f.argtypes = [C.c_void_p, C.c_size_t, C.c_size_t, C.c_void_p, C.c_size_t, C.c_int, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p,
+              C.c_size_t, C.c_int, C.c_void_p]
+out, inn, rows, terms, variant = map(int, sys.argv[2:])
+print(f(1 << 20, out, inn, 1 << 21, rows, terms, 1.0, None, 1 << 22, 1 << 23, 1 << 20, variant, None))
+"""
+    r = subprocess.run([sys.executable, "-c", code, LIB] + [str(v) for v in (out, inn, rows, terms, variant)], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.split() == ["1"], (r.returncode, r.stdout, r.stderr)
