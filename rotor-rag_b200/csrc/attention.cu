@@ -753,7 +753,8 @@ __global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_str
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1 << SH));
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2 << SH));
         const float m_new = fmaxf(m_run, top);
-        const float w = live ? __expf(s[0] - m_new) : 0.f;
+        // (no finite score yet: a score of -inf weighs nothing, and NaN stays NaN)
+        const float w = live ? __expf(s[0] - (m_new == -INFINITY ? 0.f : m_new)) : 0.f;
         s_w[warp][flip][mine] = w;
         if (__any_sync(0xffffffffu, m_new > m_run)) {  // (rare after the first keys)
             const float a = m_run == -INFINITY ? 0.f : __expf(m_run - m_new);

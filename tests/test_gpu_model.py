@@ -585,3 +585,30 @@ def test_batched_steps_equal_single_sequences(rb, shape, batch, context):
     got = steps(list(range(batch)))
     for b in (0, batch // 2, batch - 1):
         assert rel_err(got[b].cpu().numpy(), steps([b])[0].cpu().numpy()) < 2e-4, b   # about 60 float32 sums of up to 9216 in a row
+
+
+@pytest.mark.parametrize("heads,kv", [(4, 2), (8, 1), (3, 3)])
+@pytest.mark.parametrize("batch,context,hidden", [(5, 300, 4), (5, 300, 45), (5, 300, 300), (16, 30, 17), (33, 129, 128), (18, 5, 5)])
+def test_infinite_scores_weigh_nothing(rb, heads, kv, batch, context, hidden):
+    """Cached keys whose score is minus infinity, the first `hidden` of a context, in steps of several sequences: a warp's
+    first keys, whole runs, everything but the new key.  The same as keys so far below the others that their weight
+    underflows to zero, to the bit."""
+    import torch
+    d = 64 * heads
+    at = rb.tr.MultiHeadAttention(d, heads, kv, semantics=rb.sem.REFERENCE, max_seq=context + 1, max_batch=batch)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(context + hidden + heads)
+    for p in (at.k_proj, at.v_proj, at.o_proj):
+        p.load_from_int8(torch.randint(-1, 2, (p.out_features, p.in_features), generator=g, device="cuda", dtype=torch.int8), 0.05)
+    at.q_proj.load_from_int8(torch.ones((d, d), device="cuda", dtype=torch.int8), 0.1 / d)   # positive rows: positive queries
+    x = np.random.default_rng(batch).uniform(0.5, 1.5, size=(batch, 1, d)).astype(np.float32)
+    k, v = at.ensure_cache()
+    v[:, :, :context] = torch.randn(v[:, :, :context].shape, generator=g, device="cuda")
+    keys = torch.randn(k[:, :, :context].shape, generator=g, device="cuda")
+    got = []
+    for low in (-np.inf, -1e30):
+        k[:, :, :context] = keys
+        k[:, :, :hidden, 5] = low
+        got.append(at.forward(x, kv_cache=rb.tr.KVCache(at, context, batch))[0])
+    assert np.isfinite(got[1]).all() and np.abs(got[1]).max() > 0
+    assert np.array_equal(*got)
