@@ -93,7 +93,6 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
     int* red = reinterpret_cast<int*>(smem_raw + 16);            // [WARPS][128]
     int8_t* xs = reinterpret_cast<int8_t*>(smem_raw + 16 + WARPS * 128 * 4);
 
-    pdl_trigger();
     stage_init(bar);
 
     const uint4* trow = p.tiles + ((size_t)rt * p.nkt) * 32 + lane;
@@ -114,7 +113,8 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
 #pragma unroll
     for (int u = 0; u < UMAX; ++u)
         if (base + u * WARPS < kt1) wv[u] = ld_stream_v4(trow + (size_t)(base + u * WARPS) * 32);
-    pdl_wait();  // weights above are constants; everything below depends on the producer kernel
+    pdl_wait();     // weights above are constants; everything below depends on the producer kernel
+    pdl_trigger();  // after the wait: see the rule in common.cuh
     stage_issue(bar, xs, xs_stride, p.xq + (size_t)kt0 * TILE_K, (size_t)p.nkt * TILE_K, p.ncols, (uint32_t)ks);
     __syncthreads();  // mbarrier initialised, bulk copies issued
     if (!stage_wait(bar) && threadIdx.x == 0) atomicMax(p.status, (unsigned)ROTOR_B200_ERR_TIMEOUT);

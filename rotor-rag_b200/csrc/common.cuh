@@ -159,7 +159,8 @@ __device__ __forceinline__ uint4 ld_stream_v4(const uint4* p) {
 // predecessor has passed its wait, i.e. once everything launched before the predecessor is
 // complete: that code may read constants (weights) and anything written two or more kernels
 // earlier (the cached length, older KV-cache rows), never the predecessor's outputs, and
-// writes nothing outside its own CTA.
+// writes nothing outside its own CTA.  A kernel that is always launched without the attribute needs no
+// wait and may trigger at once: everything before it is complete when it starts.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

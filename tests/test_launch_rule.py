@@ -1,0 +1,44 @@
+"""CPU: the order of griddepcontrol.wait and .launch_dependents in every kernel of the sources.
+
+A kernel that lets its successor start before it has itself waited gives away what the successor's early reads rely on:
+that everything launched before its predecessor is complete.  Only a kernel that is always an ordinary launch (nothing
+before it is running any more) may trigger without a wait."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "rotor-rag_b200", "csrc")
+
+
+def kernels():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__[^;{]*?\b(\w+)\s*\((?=[^;{]*\)\s*\{)(?:[^()]|\([^()]*\))*\)\s*\{", text):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                i += 1
+            yield os.path.basename(path), re.findall(r"(\w+_kernel)\b", m.group(0))[-1], text[m.end():i], text
+
+
+FOUND = list(kernels())
+
+
+def test_the_kernels_are_found():
+    names = {name for _, name, _, _ in FOUND}
+    assert {"bitlinear_acc_kernel", "row_stage_kernel", "vec_stage_kernel", "fused_gemv_kernel", "attn_decode_stream_kernel",
+            "attn_decode_cluster_kernel", "dequant_kernel", "quantize_rows_kernel", "dense_gemm_t5_kernel"} <= names
+    assert len(FOUND) == sum(len(re.findall(r"__global__", re.sub(r"//[^\n]*", "", open(p).read())))
+                             for p in glob.glob(os.path.join(CSRC, "*.cu")))
+
+
+@pytest.mark.parametrize("file,name", [(f, n) for f, n, b, _ in FOUND if "pdl_trigger()" in b])
+def test_trigger_follows_wait(file, name):
+    body, text = next((b, t) for f, n, b, t in FOUND if (f, n) == (file, name))
+    waits, triggers = ([m.start() for m in re.finditer(w, body)] for w in (r"pdl_wait\(\)", r"pdl_trigger\(\)"))
+    if not waits:
+        assert re.search(name + r"(<[^;()]*>)?<<<", text) and not re.search(r"cudaLaunchKernelEx\([^;]*\b" + name, text), name
+    else:
+        assert len(waits) >= len(triggers) and all(w < t for w, t in zip(waits, triggers)), name
