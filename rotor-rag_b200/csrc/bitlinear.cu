@@ -436,7 +436,6 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
         stage.y = x;
         stage.terms = terms;
         stage.kpad = (int)kpad_of(in);
-        stage.clamp = 1;
         const float scale[3] = {wscale, wscale, wscale};
         return launch_fused_gemv(tiles, out, in, 1, (int)m, stage, y, scale, (int)out, (int)out, 0, as_stream(stream), nullptr, true);
     }

@@ -22,7 +22,7 @@ RB_TRACE_DEFINE(rotor_b200_trace_read_fused)
 
 namespace rb {
 
-template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, bool TP>
+template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, int KIND>
 __global__ void __launch_bounds__(FG_THREADS, DEEP ? 1 : 2) fused_gemv_kernel(const __grid_constant__ FusedGemvParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_sx[8];
@@ -41,21 +41,21 @@ __global__ void __launch_bounds__(FG_THREADS, DEEP ? 1 : 2) fused_gemv_kernel(co
     pdl_wait();     // the weights above are constants; everything below depends on earlier kernels
     pdl_trigger();  // after the wait: see the rule in common.cuh
     RB_STAMP(tr, 2);
-    product_run<USE_MMA, NCOL, WIDE, DEEP, TP>(p, c, wv, s_sx, s_xsum, tr);
+    product_run<USE_MMA, NCOL, WIDE, DEEP, KIND>(p, c, wv, s_sx, s_xsum, tr);
     RB_STAMP(tr, 5);
     RB_TRACE_COMMIT(tr, p.st.mode * 10 + p.halves);
 }
 
-template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, bool TP>
-static int launch_fused_tp(const FusedGemvParams& p, int grid, cudaStream_t st) {
+template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, int KIND>
+static int launch_fused_kind(const FusedGemvParams& p, int grid, cudaStream_t st) {
     static PerDevice<bool> once;  // each variant raises its own shared-memory limit once per device
     bool& configured = once.here();
     if (!configured) {
-        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, TP>,
+        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, KIND>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         // the largest shared-memory split for every variant: kernels of a step share SMs, and a CTA
         // whose request does not fit the split left by its neighbour waits for the SM to drain
-        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, TP>,
+        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, KIND>,
                                      cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         configured = true;
     }
@@ -70,8 +70,8 @@ static int launch_fused_tp(const FusedGemvParams& p, int grid, cudaStream_t st) 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_use_pdl && !p.alone ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, TP>, p) != cudaSuccess) {
+    cfg.numAttrs = g_use_pdl && KIND != FG_ALONE ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, KIND>, p) != cudaSuccess) {
         ++g_launch_count;
         return ROTOR_B200_ERR_CUDA;
     }
@@ -79,22 +79,23 @@ static int launch_fused_tp(const FusedGemvParams& p, int grid, cudaStream_t st) 
 }
 
 template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP>
-static int launch_fused(const FusedGemvParams& p, int grid, cudaStream_t st) {
-    if (p.xs.size || p.part) return launch_fused_tp<USE_MMA, NCOL, WIDE, DEEP, true>(p, grid, st);
-    return launch_fused_tp<USE_MMA, NCOL, WIDE, DEEP, false>(p, grid, st);
+static int launch_fused(const FusedGemvParams& p, int grid, cudaStream_t st, bool alone) {
+    if (alone) return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, FG_ALONE>(p, grid, st);
+    if (p.xs.size || p.part) return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, FG_SHARDED>(p, grid, st);
+    return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, FG_STEP>(p, grid, st);
 }
 
 int configure_fused_gemv() {
     const int big = 200 * 1024;
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, false, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, false, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, false, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, true, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, true, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, true, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     fused_sm_count();
     return ROTOR_B200_OK;
 }
@@ -124,7 +125,6 @@ int launch_fused_gemv(const void* tiles, size_t out, size_t in, int halves, int 
     int grid = fused_sm_count();
     int rc = make_fused_params(p, tiles, out, in, halves, rows, stage, y, scale, seg1, seg2, ffn_act, grid);
     if (rc) return rc;
-    p.alone = alone;
     if (tp) {
         if (stage.terms != 1 || rows > XS_ROWS || (tp->part && halves != 1)) return ROTOR_B200_ERR_ARG;
         p.xs = tp->xs;
@@ -136,18 +136,18 @@ int launch_fused_gemv(const void* tiles, size_t out, size_t in, int halves, int 
     // and so do rows too wide for the shallow variant's register budget
     const long tiles_per_warp = (long)p.units * p.halves * p.nkt / ((long)grid * FG_WARPS);
     if (fused_wide(p.st)) {
-        if (p.cols == 1) return launch_fused<false, 1, true, true>(p, grid, st);
-        if (p.cols == 2) return launch_fused<false, 2, true, true>(p, grid, st);
-        return launch_fused<true, 1, true, true>(p, grid, st);
+        if (p.cols == 1) return launch_fused<false, 1, true, true>(p, grid, st, alone);
+        if (p.cols == 2) return launch_fused<false, 2, true, true>(p, grid, st, alone);
+        return launch_fused<true, 1, true, true>(p, grid, st, alone);
     }
     if (tiles_per_warp >= 16 || !fused_shallow_fits(p.st) || fused_stage_bytes(p) > FG_STAGE_MAX) {
-        if (p.cols == 1) return launch_fused<false, 1, false, true>(p, grid, st);
-        if (p.cols == 2) return launch_fused<false, 2, false, true>(p, grid, st);
-        return launch_fused<true, 1, false, true>(p, grid, st);
+        if (p.cols == 1) return launch_fused<false, 1, false, true>(p, grid, st, alone);
+        if (p.cols == 2) return launch_fused<false, 2, false, true>(p, grid, st, alone);
+        return launch_fused<true, 1, false, true>(p, grid, st, alone);
     }
-    if (p.cols == 1) return launch_fused<false, 1, false, false>(p, grid, st);
-    if (p.cols == 2) return launch_fused<false, 2, false, false>(p, grid, st);
-    return launch_fused<true, 1, false, false>(p, grid, st);
+    if (p.cols == 1) return launch_fused<false, 1, false, false>(p, grid, st, alone);
+    if (p.cols == 2) return launch_fused<false, 2, false, false>(p, grid, st, alone);
+    return launch_fused<true, 1, false, false>(p, grid, st, alone);
 }
 
 // Stand-alone integer product through the staged kernel: the matrix is small enough for every
@@ -186,9 +186,9 @@ int launch_staged_acc(const void* tiles, size_t out, size_t in, const int8_t* xq
     p.acc_out = acc;
     if (grid > p.units) grid = p.units;
     const bool mma = variant == ROTOR_B200_VARIANT_MMA || ncols > 2;
-    if (mma) return launch_fused_tp<true, 1, false, false, false>(p, grid, st);
-    if (ncols == 1) return launch_fused_tp<false, 1, false, false, false>(p, grid, st);
-    return launch_fused_tp<false, 2, false, false, false>(p, grid, st);
+    if (mma) return launch_fused_kind<true, 1, false, false, FG_STEP>(p, grid, st);
+    if (ncols == 1) return launch_fused_kind<false, 1, false, false, FG_STEP>(p, grid, st);
+    return launch_fused_kind<false, 2, false, false, FG_STEP>(p, grid, st);
 }
 
 }  // namespace rb

@@ -37,7 +37,6 @@ struct LeanStage {
     // quantiser
     int terms;
     int kpad;
-    int clamp;                   // quantise NaN to -128, as the stand-alone quantiser does (the packed conversion gives 0)
     // tensor parallel: the row is this rank's slice of a longer one.  Exchange index + 1 (0 = none)
     // of the sum of squares under norm1 and of the absolute maximum under the quantiser; norm_n is
     // the width of the whole row.
@@ -186,9 +185,10 @@ __device__ __forceinline__ void lean_prefetch(const LeanStage& p) {
 // (v * (1/s) is within 2e-5 of v / s for |v / s| <= 127, so the multiply decides unless it lands
 // within 1e-4 of a tie), packed with
 // the saturating pack instruction.  `lsum` gains the four integers (one dp4a).  With RESIDUAL the
-// values are replaced by v - q * s (float32, one rounding per operation) for the next term.
-template <bool RESIDUAL>
-__device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& lsum, bool clamp = false) {
+// values are replaced by v - q * s (float32, one rounding per operation) for the next term.  CLAMP: NaN becomes -128, as in
+// the stand-alone quantiser (the packed conversion gives 0).
+template <bool RESIDUAL, bool CLAMP = false>
+__device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& lsum) {
     const float r0 = v.x * rs, r1 = v.y * rs, r2 = v.z * rs, r3 = v.w * rs;
     float q0 = rintf(r0), q1 = rintf(r1), q2 = rintf(r2), q3 = rintf(r3);
     const float dm = fmaxf(fmaxf(fabsf(r0 - q0), fabsf(r1 - q1)), fmaxf(fabsf(r2 - q2), fabsf(r3 - q3)));
@@ -198,7 +198,7 @@ __device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& ls
         q2 = rintf(__fdiv_rn(v.z, s));
         q3 = rintf(__fdiv_rn(v.w, s));
     }
-    if (RESIDUAL || clamp) {
+    if (RESIDUAL || CLAMP) {
         q0 = fminf(fmaxf(q0, -128.f), 127.f);
         q1 = fminf(fmaxf(q1, -128.f), 127.f);
         q2 = fminf(fmaxf(q2, -128.f), 127.f);
@@ -222,8 +222,8 @@ __device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& ls
 // (shared memory, zero padded to kpad), its scale and sum to sx[t] / xsum[t] (shared).
 // Same results as quantize_row_from_smem.  Requires kpad <= 4 * LEAN_V * blockDim.x; sx / xsum are
 // complete after the next CTA barrier.  ONE_TERM: p.terms is 1 (the loop and the residual drop out).
-// given_absmax: optional max|row| of term 0 supplied by the caller (sharded rows).
-template <int LEAN_V, bool ONE_TERM = false>
+// given_absmax: optional max|row| of term 0 supplied by the caller (sharded rows).  CLAMP: see quant4_pack.
+template <int LEAN_V, bool ONE_TERM = false, bool CLAMP = false>
 __device__ __forceinline__ void lean_quantize(const LeanStage& p, float4 (&v)[LEAN_V], float* scratch, int8_t* xq,
                                               size_t tstride, float* sx, int* xsum, int& rk, int m = 0,
                                               bool writer = false, const XchScalarDev* x = nullptr,
@@ -247,7 +247,7 @@ __device__ __forceinline__ void lean_quantize(const LeanStage& p, float4 (&v)[LE
             if (g < k4) {
                 int packed = 0;
                 if (g < n4) packed = (!ONE_TERM && t + 1 < terms) ? quant4_pack<true>(v[j], s, rs, lsum)
-                                                                  : quant4_pack<false>(v[j], s, rs, lsum, p.clamp != 0);
+                                                                  : quant4_pack<false, CLAMP>(v[j], s, rs, lsum);
                 *reinterpret_cast<int*>(xq + (size_t)t * tstride + (size_t)g * 4) = packed;
             }
         }

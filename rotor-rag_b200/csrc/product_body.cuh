@@ -22,6 +22,10 @@ constexpr int FG_L2_AHEAD = 32;  // deep variant: further tiles per warp pulled 
 constexpr size_t FG_STAGE_MAX = 96 * 1024;  // shallow variant: most tile bytes a CTA stages
 constexpr int FG_V = 4;        // float4 groups per thread in the register prologue: input width <= 8192
 constexpr int FG_V_NARROW = 2; // shallow variant, stages that hold four arrays per group: width <= 4096
+// What the product is part of: a generation step; the same with tensor-parallel hooks (scalar exchanges in the prologue,
+// int32 partial output); a stand-alone layer call (LM_PLAIN; an ordinary launch, because its weights may be the work of the
+// kernel before it).
+enum { FG_STEP = 0, FG_SHARDED = 1, FG_ALONE = 2 };
 
 struct FusedGemvParams {
     const uint4* tiles;   // tiles of the (stacked) matrix
@@ -47,7 +51,6 @@ struct FusedGemvParams {
     const int8_t* xq_in;
     const int32_t* xsum_in;
     int32_t* acc_out;
-    int alone;            // launched as an ordinary kernel: the weights may be the work of the kernel before it
 };
 
 // Input rows wider than the register-resident prologue holds (4 * FG_V * FG_THREADS elements)
@@ -193,10 +196,12 @@ __device__ __forceinline__ void product_prefetch(const FusedGemvParams& p, const
 // (large matrices): the loop requests the following batch of tiles before multiplying the
 // current one and tracks its position by counting; the shallow loop (a few tiles per warp, the
 // latency-bound small matrices) keeps the shortest code path.
-// TP: tensor-parallel hooks compiled in (scalar exchanges in the prologue, int32 partial output).
-template <bool USE_MMA, int NCOL, bool WIDE = false, bool DEEP = false, bool TP = false>
+// KIND: what only one caller needs is compiled for that one alone (a flag that every quantiser tested cost the generation
+// step of one sequence 0.3 %: 2B shape 890.9 against 888.5 us).
+template <bool USE_MMA, int NCOL, bool WIDE = false, bool DEEP = false, int KIND = FG_STEP>
 __device__ __forceinline__ void product_run(const FusedGemvParams& p, const ProductCtx& c, uint4 (&wv)[FG_U],
                                             float* s_sx, int* s_xsum, TraceRec& tr) {
+    constexpr bool TP = KIND == FG_SHARDED, ALONE = KIND == FG_ALONE;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     int8_t* xs = c.xs;
     int* merge = c.merge;
@@ -206,7 +211,7 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
 
     // ---- prologue: activation rows -> int8 in shared memory
     const bool writer = blockIdx.x == 0;
-    if (!WIDE && !TP && p.xq_in) {
+    if (!WIDE && !TP && !ALONE && p.xq_in) {
         // already quantised: the columns are copied as they are
         const int k16 = p.nkt * (TILE_K / 16);  // 16-byte pieces per column
         for (int i = threadIdx.x; i < p.cols * k16; i += blockDim.x) {
@@ -292,7 +297,7 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
                             packed = quant4_pack<true>(v, s, rs, lsum);
                             *rp = v;
                         } else {
-                            packed = quant4_pack<false>(v, s, rs, lsum, p.st.clamp != 0);
+                            packed = quant4_pack<false, ALONE>(v, s, rs, lsum);
                         }
                     }
                     *reinterpret_cast<int*>(xq + (size_t)t * xs_stride + i) = packed;
@@ -315,12 +320,12 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
                 float4 v[V];
                 lean_row<V, PLAIN>(p.st, m, v, scratch, aux, writer, rk, x);
                 RB_STAMP(tr, 6);
-                lean_quantize<V, ONE>(p.st, v, scratch, xs + (size_t)m * terms * xs_stride, (size_t)xs_stride,
+                lean_quantize<V, ONE, ALONE>(p.st, v, scratch, xs + (size_t)m * terms * xs_stride, (size_t)xs_stride,
                                       s_sx + m * terms, s_xsum + m * terms, rk, m, writer, x);
             }
         };
-        if constexpr (DEEP) {
-            rows(std::integral_constant<int, FG_V>(), std::false_type());
+        if constexpr (DEEP || ALONE) {
+            rows(std::integral_constant<int, FG_V>(), std::bool_constant<ALONE>());
         } else {
             if (p.st.mode == LM_PLAIN)
                 rows(std::integral_constant<int, FG_V>(), std::true_type());
@@ -471,7 +476,7 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
     RB_STAMP(tr, 4);
 
     // ---- epilogue: the CTA's rows are complete: remove the +1 code offset, dequantise, write
-    if (!WIDE && !TP && p.acc_out) {  // stand-alone product: exact integer sums, column major
+    if (!WIDE && !TP && !ALONE && p.acc_out) {  // stand-alone product: exact integer sums, column major
         for (int e = threadIdx.x; e < (u1 - u0) * 16 * p.cols; e += blockDim.x) {
             const int q = e / p.cols, col = e - q * p.cols;
             const int rl = q & 15, lu = q >> 4;
