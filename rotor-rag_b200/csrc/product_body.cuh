@@ -506,7 +506,10 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
             const int slot = DEEP ? lu * p.halves + half : half * (u1 - u0) + lu;
             const int* src = merge + slot * 128 + rl * 8 + m * T;
             float f = 0.f;
-            for (int tt = 0; tt < T; ++tt) f += (float)(src[tt] - s_xsum[m * T + tt]) * s_sx[m * T + tt];
+            for (int tt = 0; tt < T; ++tt) {
+                const float q = (float)(src[tt] - s_xsum[m * T + tt]), sc = s_sx[m * T + tt];
+                f = ALONE ? __fadd_rn(f, __fmul_rn(q, sc)) : f + q * sc;  // (as dequant_kernel rounds: one result for any row count)
+            }
             return f;
         };
         const float val0 = deq(0), val1 = p.halves == 2 ? deq(1) : 0.f;

@@ -141,6 +141,28 @@ def test_layer_call_of_few_rows(ops, abi, shape, rows, terms):
     abi.device_status()
 
 
+@pytest.mark.parametrize("terms", [1, 2, 3])
+@pytest.mark.parametrize("shape", [(17, 132), (640, 2560), (6912, 2560), (640, 9220), (2560, 8192)])
+def test_row_alone_equals_row_among_others(ops, abi, shape, terms):
+    """A row's result is the same to the bit whatever rows come with it, wherever it starts in memory and whether its scale
+    is one number or one per output."""
+    import torch
+    out, inn = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(out + inn + terms)
+    tiles = ops.int8_to_tiles(torch.randint(-1, 2, (out, inn), generator=g, device="cuda", dtype=torch.int8))
+    buf = torch.randn(5 * inn + 1, generator=g, device="cuda")
+    x = buf[1:].view(5, inn)                                   # (off a 16-byte boundary)
+    want = ops.bitlinear_forward(tiles, out, inn, x, terms, 0.037)
+    vec = torch.full((out,), 0.037, device="cuda")
+    for n in (1, 2, 3, 4):
+        rows = x[:n].clone()
+        assert torch.equal(ops.bitlinear_forward(tiles, out, inn, rows, terms, 0.037), want[:n]), n
+        assert torch.equal(ops.bitlinear_forward(tiles, out, inn, rows, terms, wscale_vec=vec), want[:n]), n
+        assert torch.equal(ops.bitlinear_forward(tiles, out, inn, x[:n], terms, 0.037), want[:n]), n
+    abi.device_status()
+
+
 def test_tcgen05_extreme_values(ops, abi):
     """-128 x -1 and 127 x +1 over K = 6912 on the tcgen05 path: sums stay exact in int32."""
     out, inn, ncols = 256, 6912, 256
