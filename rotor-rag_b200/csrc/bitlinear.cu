@@ -62,7 +62,7 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar) {
     return ok != 0;
 }
 
-constexpr size_t LINEAR_FUSED_ROWS = 4;  // rows of a stand-alone layer call that are quantised in the product's prologue
+constexpr size_t LINEAR_FUSED_ROWS = 4, LINEAR_FUSED_COLS = 6;  // a stand-alone layer call in one launch: see its rule
 
 struct AccParams {
     const uint4* tiles;
@@ -423,11 +423,13 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
     RB_REQUIRE(((uintptr_t)workspace & 255) == 0);
     if (workspace_bytes < rotor_b200_bitlinear_workspace_bytes(out, in, m, terms)) return ROTOR_B200_ERR_WORKSPACE;
     const size_t nc = m * (size_t)terms;
-    // A few rows: one launch, the rows are quantised in the product's prologue by every CTA (a row costs each about a
-    // microsecond, the two launches saved cost five) and leave it as floats.  Every CTA reads x, so y must not lie on it.
-    // One row of 2560 -> 6912: 9.7 -> 5.1 us on the GPU, 25.8 -> 19.4 us a call.
+    // A few rows: one launch, the rows are quantised in the product's prologue by every CTA (a row and term costs each about
+    // a microsecond, the two launches saved cost four) and leave it as floats.  Every CTA reads x, so y must not lie on it.
+    // On the GPU, one launch against three: 1 row of 2560 -> 6912 4.5 / 8.3 us, 4 rows 8.5 / 8.5, 2 rows of three terms
+    // 9.9 / 12.2, 3 of two 9.9 / 9.9, 4 of two 12.6 / 11.3; 8192 -> 8192 8.0 / 12.2, 14.4 / 13.7, 16.6 / 19.3, 16.7 / 16.7,
+    // 19.8 / 17.6.  Up to six columns the two are within 5 % at worst and the host saves two launches (25.8 -> 19.4 us a call).
     const uintptr_t x0 = (uintptr_t)x, x1 = x0 + m * in * sizeof(float), y0 = (uintptr_t)y, y1 = y0 + m * out * sizeof(float);
-    if (variant == ROTOR_B200_VARIANT_AUTO && !wscale_vec && m <= LINEAR_FUSED_ROWS && nc <= 8 && (x0 & 15) == 0 &&
+    if (variant == ROTOR_B200_VARIANT_AUTO && !wscale_vec && m <= LINEAR_FUSED_ROWS && nc <= LINEAR_FUSED_COLS && (x0 & 15) == 0 &&
         ((uintptr_t)tiles & 15) == 0 && out < (1u << 30) && in <= 49152 && (y1 <= x0 || x1 <= y0) &&
         fused_gemv_supported(out, in, (int)m, terms, 1, 0)) {
         LeanStage stage = {};

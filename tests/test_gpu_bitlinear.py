@@ -105,7 +105,7 @@ def test_many_column_product_bit_exact(ops, abi, shape):
 @pytest.mark.parametrize("shape", [(1, 4), (17, 132), (3001, 1924), (2560, 8192), (640, 9220), (8192, 2048)])
 @pytest.mark.parametrize("rows", [1, 2, 4, 5])
 def test_layer_call_of_few_rows(ops, abi, shape, rows, terms):
-    """One launch up to four rows of eight columns, quantiser, product and dequantiser above: both against the general path
+    """One launch up to four rows of six columns, quantiser, product and dequantiser above: both against the general path
     (the variant forced), with a row of zeros, NaN and infinities, rows that start off a 16-byte boundary, and y on x."""
     import torch
     out, inn = shape
