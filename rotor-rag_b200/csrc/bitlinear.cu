@@ -62,6 +62,11 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar) {
     return ok != 0;
 }
 
+// Sums that the product adds to are cleared by the quantiser, a share per row, so that no memset stands between the two, up to
+// this many bytes a row: 8192 -> 28672, 8 rows (115 KB) 27.1 / 27.5 us, 5 rows of two terms (229 KB) 43.4 / 41.9, of three
+// (344 KB) 56.8 / 53.1.  The product starts early where it is one launch (4096 -> 11008, 8 rows: 10.6 against 12.6 us); several
+// launches of eight columns get in each other's way then (2560 -> 6912: 16 rows 12.4 / 11.4, 31 rows 19.9 / 17.6).
+constexpr size_t LINEAR_CLEAR_MAX = 128 * 1024;
 constexpr size_t LINEAR_FUSED_ROWS = 4, LINEAR_FUSED_COLS = 6;  // a stand-alone layer call in one launch: see its rule
 
 struct AccParams {
@@ -449,9 +454,8 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
     int32_t* xsum = (int32_t*)w;
     w += al256(nc * 4);
     int32_t* acc = (int32_t*)w;
-    // sums that the product adds to are cleared by the quantiser: no memset node in between
-    const bool adds = out < (1u << 30) && in <= 49152 && acc_adds(out, in, nc, xq, variant);
-    int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, as_stream(stream));
+    const bool adds = out < (1u << 30) && in <= 49152 && nc * out * sizeof(int32_t) <= m * LINEAR_CLEAR_MAX && acc_adds(out, in, nc, xq, variant);
+    int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, nc <= 8, as_stream(stream));
     if (rc) return rc;
     rc = run_acc(tiles, out, in, xq, xsum, nc, acc, variant, as_stream(stream), adds);
     if (rc) return rc;

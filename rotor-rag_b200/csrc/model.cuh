@@ -98,9 +98,10 @@ int launch_gemm_tcgen05_qkv(const void* tiles, size_t in, const int8_t* xq, cons
 int launch_gemm_mma(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
                     int32_t* acc, cudaStream_t st);
 
-// rotor_b200_quantize_rows that also clears `zero_n` accumulators
+// rotor_b200_quantize_rows that also clears `zero_n` accumulators.  early: what follows may start, and request its weights,
+// while the rows are quantised, else when they are
 int launch_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* xq, float* sx, int32_t* xsum, int32_t* zero,
-                         size_t zero_n, cudaStream_t st);
+                         size_t zero_n, bool early, cudaStream_t st);
 
 // Generation-step product with the consuming vector stage fused in (fused.cu, leanstage.cuh).
 struct LeanStage;

@@ -7,8 +7,8 @@ namespace rb {
 __global__ void __launch_bounds__(1024) quantize_rows_kernel(const float* __restrict__ x, int k, int kpad,
                                                              int terms, int8_t* __restrict__ xq,
                                                              float* __restrict__ sx, int32_t* __restrict__ xsum,
-                                                             int32_t* __restrict__ zero, size_t zero_n) {
-    pdl_trigger();  // launched as an ordinary kernel: everything before it is complete
+                                                             int32_t* __restrict__ zero, size_t zero_n, int early) {
+    if (early) pdl_trigger();  // launched as an ordinary kernel: everything before it is complete
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < zero_n; i += (size_t)gridDim.x * blockDim.x) zero[i] = 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* scratch = reinterpret_cast<float*>(smem_raw);
@@ -18,10 +18,11 @@ __global__ void __launch_bounds__(1024) quantize_rows_kernel(const float* __rest
     __syncthreads();
     quantize_row_from_smem(row, k, kpad, terms, xq + m * terms * (size_t)kpad, sx + m * terms,
                            xsum + m * terms, scratch);
+    if (!early) pdl_trigger();
 }
 
 int launch_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* xq, float* sx, int32_t* xsum, int32_t* zero,
-                         size_t zero_n, cudaStream_t st) {
+                         size_t zero_n, bool early, cudaStream_t st) {
     RB_REQUIRE(x && xq && sx && xsum && m > 0 && k > 0 && terms >= 1 && terms <= 4);
     RB_REQUIRE(k <= 49152 && m < (1u << 31));
     RB_REQUIRE(((uintptr_t)xq & 3) == 0);
@@ -36,7 +37,7 @@ int launch_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* 
         }
     }
     const int threads = k >= 4096 ? 1024 : (k >= 1024 ? 512 : 128);
-    quantize_rows_kernel<<<(unsigned)m, threads, smem, st>>>(x, (int)k, (int)kpad_of(k), terms, xq, sx, xsum, zero, zero_n);
+    quantize_rows_kernel<<<(unsigned)m, threads, smem, st>>>(x, (int)k, (int)kpad_of(k), terms, xq, sx, xsum, zero, zero_n, early);
     return launch_status();
 }
 
@@ -46,5 +47,5 @@ using namespace rb;
 
 extern "C" int rotor_b200_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* xq, float* sx,
                                         int32_t* xsum, void* stream) {
-    return launch_quantize_rows(x, m, k, terms, xq, sx, xsum, nullptr, 0, as_stream(stream));
+    return launch_quantize_rows(x, m, k, terms, xq, sx, xsum, nullptr, 0, true, as_stream(stream));
 }

@@ -163,6 +163,27 @@ def test_row_alone_equals_row_among_others(ops, abi, shape, terms):
     abi.device_status()
 
 
+@pytest.mark.parametrize("out,inn,rows,terms", [(12001, 8192, 5, 3), (3001, 1923, 13, 3), (640, 9000, 9, 1), (33001, 2048, 5, 1), (6912, 2560, 16, 1),
+                                                (512, 8192, 8, 1), (1001, 4000, 7, 4), (600, 3000, 40, 1)])
+def test_layer_call_equals_its_three_parts(ops, abi, out, inn, rows, terms):
+    """Sums cleared by the quantiser or by a memset, products of one and of several launches, early and late starts: the call
+    against quantiser, product and dequantiser called one by one, to the bit, twice over the same workspace."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(out + inn + rows)
+    tiles = ops.int8_to_tiles(torch.randint(-1, 2, (out, inn), generator=g, device="cuda", dtype=torch.int8))
+    ws = torch.full((abi.lib.rotor_b200_bitlinear_workspace_bytes(out, inn, rows, terms),), 0x5A, dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        x = torch.randn((rows, inn), generator=g, device="cuda")
+        got = ops.bitlinear_forward(tiles, out, inn, x, terms, 0.037, workspace=ws)
+        xq, sx, xsum = ops.quantize_rows(x, terms)
+        acc = ops.bitlinear_acc(tiles, out, inn, xq, xsum, abi.VARIANT_AUTO)
+        want = torch.empty_like(got)
+        abi.check(abi.lib.rotor_b200_bitlinear_dequant(abi.ptr(acc), abi.ptr(sx), rows, terms, out, 0.037, None, abi.ptr(want), abi.stream()))
+        assert torch.equal(got, want)
+    abi.device_status()
+
+
 def test_tcgen05_extreme_values(ops, abi):
     """-128 x -1 and 127 x +1 over K = 6912 on the tcgen05 path: sums stay exact in int32."""
     out, inn, ncols = 256, 6912, 256
