@@ -57,6 +57,7 @@ struct T5Cfg {
     static constexpr int THREADS = (DECODERS + 2) * 32;
     static constexpr int TILES_PER_WARP = ROWS / TILE_ROWS / DECODERS;  // row tiles each decoder warp handles
 };
+constexpr int T5_SCATTER_COLS = 48;  // columns up to which a split product's sums are added by a lane per token
 constexpr int T5_DEEP_STEPS = 12;  // K steps of a CTA from which the 128-token variant is taken
 struct Tc5Params {
     const uint4* tiles;
@@ -347,19 +348,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
 #pragma unroll
                         for (int q = 0; q < 32; ++q) v[q] -= xs;
                         if (p.kt_per_split) {  // one of several partial sums: exact, in any order
-                            // Whole lines at a time; a lane per token touches 32 lines per instruction, which wins only while one
-                            // warp's worth of tokens adds at all (2560 x 2560: 32 tokens 12.0 against 13.9 us, 64 tokens
-                            // 17.4 against 14.0, 903 tokens 56.8 against 25.4).
-                            if (p.ncols <= 32) {
+                            // A lane per token adds to 32 lines an instruction and takes longer with every token; whole lines at a
+                            // time take the same time for any number.  us at 36 / 48 / 64 columns: 2560 x 2560 12.5 / 14.5 / 16.7
+                            // against 14.5 / 14.7 / 14.5, 8192 x 8192 18.4 / 20.5 / 23.0 against 21.6 / 21.9 / 21.8, 1000 x 1000
+                            // 12.1 / 13.7 / 15.7 against 14.7, 13824 x 2560 17.9 / 20.2 / 21.9 against 18.5 / 18.7 / 18.7 (903
+                            // columns of 2560 x 2560: 56.8 against 25.4).
+                            if (p.ncols <= T5_SCATTER_COLS) {
                                 if (token < p.ncols) {
                                     int32_t* dst = p.acc + (size_t)token * p.out + rbase;
 #pragma unroll
                                     for (int q = 0; q < 32; ++q)
                                         if (rbase + q < p.out) atomicAdd(dst + q, (int32_t)v[q]);
                                 }
-                            } else
-                            t5_add_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
-                                        (size_t)p.out, p.out - rbase, tok_base, p.ncols, lane);
+                            } else {
+                                t5_add_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
+                                            (size_t)p.out, p.out - rbase, tok_base, p.ncols, lane);
+                            }
                         } else if (rbase + 32 <= p.out && (p.out & 3) == 0) {
                             t5_store_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
                                           (size_t)p.out * sizeof(int32_t), tok_base, p.ncols, lane);

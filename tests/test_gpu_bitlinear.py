@@ -313,3 +313,21 @@ print("ok")
     env = dict(os.environ, ROTOR_B200_NO_TCGEN05="1")
     r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("shape", [(2560, 2560, 48), (2560, 2560, 49), (3001, 1923, 33), (8192, 9216, 33), (18432, 8192, 100), (8192, 9216, 128),
+                                   (8192, 9216, 129), (38000, 1700, 127), (38000, 1700, 128), (600, 1536, 64), (600, 1408, 64)])
+def test_products_of_up_to_128_columns_bit_exact(ops, abi, shape):
+    """Both ways of adding the sums of a split product, and the 128-token variant split and whole, on either side of the
+    column counts and K steps where they are chosen: the integers against a float64 product, in which they are exact."""
+    import torch
+    out, inn, ncols = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(sum(shape))
+    w = torch.randint(-1, 2, (out, inn), generator=g, device="cuda", dtype=torch.int8)
+    kpad = abi.lib.rotor_b200_in_padded(inn)
+    q = torch.zeros((ncols, kpad), dtype=torch.int8, device="cuda")
+    q[:, :inn] = torch.randint(-128, 128, (ncols, inn), generator=g, device="cuda", dtype=torch.int8)
+    acc = ops.bitlinear_acc(ops.int8_to_tiles(w), out, inn, q, q.sum(1, dtype=torch.int32), abi.VARIANT_AUTO)
+    assert torch.equal(acc, (q[:, :inn].double() @ w.double().T).to(torch.int32))
+    abi.device_status()
