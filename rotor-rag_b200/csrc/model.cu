@@ -169,10 +169,12 @@ static int gemv(Ctx& c, const void* tiles, size_t out, size_t in, int ncols, int
     return launch_gemv_planes(tiles, out, in, c.xq, c.xsum[xs], ncols, acc, plane_stride, plan, c.variant, st, zeroed);
 }
 
-// The stage `p` clears the accumulators of the product that follows it, if that product adds to them (see gemv()).
+// The stage `p` clears the accumulators of the product that follows it, if that product adds to them (see gemv()); one
+// CTA a row clears its share, and beyond CLEAR_ROW_MAX a memset is faster.
+constexpr size_t CLEAR_ROW_MAX = 256 * 1024;
 static void clear_for(Ctx& c, VecStageParams& p, size_t out, size_t in, int ncols, int32_t* acc) {
     c.zeroed = nullptr;
-    if (ncols < 5 || !gemv_adds(out, in, ncols, c.xq, c.variant)) return;
+    if (ncols < 5 || (size_t)c.terms * out * sizeof(int32_t) > CLEAR_ROW_MAX || !gemv_adds(out, in, ncols, c.xq, c.variant)) return;
     p.zero = acc;
     p.zero_n = (size_t)ncols * out;
     c.zeroed = acc;

@@ -612,3 +612,19 @@ def test_infinite_scores_weigh_nothing(rb, heads, kv, batch, context, hidden):
         got.append(at.forward(x, kv_cache=rb.tr.KVCache(at, context, batch))[0])
     assert np.isfinite(got[1]).all() and np.abs(got[1]).max() > 0
     assert np.array_equal(*got)
+
+
+@pytest.mark.parametrize("rows", [2, 4, 5, 9])
+@pytest.mark.parametrize("ff", [10880, 10944])
+def test_ffn_sums_cleared_by_stage_or_memset(rb, ff, rows):
+    """Three terms, at the width where a row's gate and up sums pass the size that a stage clears itself, in the stages of few
+    and of more rows, against the rows one at a time (float32 rounding is all that may differ)."""
+    import torch
+    ffn = rb.tr.GatedFFN(512, ff, semantics=rb.sem.REFERENCE)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(ff + rows)
+    for p in (ffn.gate_proj, ffn.up_proj, ffn.down_proj):
+        p.load_from_int8(torch.randint(-1, 2, (p.out_features, p.in_features), generator=g, device="cuda", dtype=torch.int8), 0.02)
+    x = torch.randn((rows, 512), generator=g, device="cuda")
+    got, want = ffn.forward_device(x), torch.cat([ffn.forward_device(x[i:i + 1].contiguous()) for i in range(rows)])
+    assert (got - want).norm() < 2e-5 * want.norm()
