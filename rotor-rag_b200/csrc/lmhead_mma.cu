@@ -322,9 +322,15 @@ int launch_lmhead_mma(const __nv_bfloat16* embed, const float* x, __nv_bfloat16*
     p.logits = logits;
     p.part_val = part_val;
     p.part_idx = part_idx;
-    if (rows <= 16) return lm5_launch<16>(embed, xsplit, p, st);
-    if (rows <= 32) return lm5_launch<32>(embed, xsplit, p, st);
-    if (rows <= 64) return lm5_launch<64>(embed, xsplit, p, st);
+    // The token tile: all rows up to 128 in one pass over the table; a vocabulary of fewer shares than SMs takes narrower
+    // tiles while the grid still fits one CTA to an SM (its table is small and comes from L2).
+    int nt = rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128;
+    while (nt > 16 && lmhead_mma_parts(vocab) * ((rows + nt / 2 - 1) / (nt / 2)) <= fused_sm_count()) nt /= 2;
+    switch (nt) {
+        case 16: return lm5_launch<16>(embed, xsplit, p, st);
+        case 32: return lm5_launch<32>(embed, xsplit, p, st);
+        case 64: return lm5_launch<64>(embed, xsplit, p, st);
+    }
     return lm5_launch<128>(embed, xsplit, p, st);
 }
 

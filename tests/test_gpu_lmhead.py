@@ -36,3 +36,49 @@ def test_pick(model, batch):
     first = model.generate_greedy_batch(ids, 1)[:, 0]
     assert np.array_equal(first, logits[:, 0].argmax(-1))
     assert (first < model.vocab_size // 2).any()
+
+
+@pytest.fixture(scope="module")
+def tall():
+    """A vocabulary of several 256-row tiles per CTA, the last ragged, and a table of several rings of stages per tile."""
+    from rotor_b200.synth import random_model_on_device
+    return random_model_on_device(dict(vocab_size=148 * 600 + 5, d_model=512, n_layers=1, n_heads=4, n_kv_heads=1, d_ff=512), seed=5,
+                                  max_seq=300, max_batch=129, max_rows=390)
+
+
+@pytest.mark.parametrize("rows", [5, 16, 17, 33, 65, 129])
+def test_logits_of_several_tiles(tall, rows):
+    import torch
+    ids = np.random.default_rng(rows).integers(0, tall.vocab_size, size=(1, rows))
+    hidden, _ = tall.forward(ids, return_logits=False)
+    logits, _ = tall.forward(ids)
+    want = (torch.from_numpy(hidden[0]).cuda().double() @ tall._embed.double().T).cpu().numpy()
+    err = np.linalg.norm(logits[0] - want) / np.linalg.norm(want)
+    assert err < 2.0 ** -16, err
+    assert np.abs(logits[0] - want).max() < 2.0 ** -12 * np.abs(want).max()     # (no tile missing: one wrong row would show)
+
+
+@pytest.mark.parametrize("batch", [5, 17, 33, 65, 129])
+def test_pick_of_equal_rows(tall, batch):
+    """Every sequence's best vocabulary row twice, the second in the next lane, another half of the tile, the next tile, the
+    ragged last tile, another CTA: the lower index is picked."""
+    import torch
+    ids = np.stack(divmod(np.random.default_rng(batch).permutation(10000)[:batch], 100), 1)     # (no two alike)
+    hidden, _ = tall.forward(ids, return_logits=False)
+    h = torch.from_numpy(hidden[:, -1]).cuda()
+    units, parts = (tall.vocab_size + 15) // 16, min((tall.vocab_size + 127) // 128, torch.cuda.get_device_properties(0).multi_processor_count)
+    kept, first = tall._embed.clone(), []
+    try:
+        for b in range(batch):
+            cta = 1 + (b * 37) % (parts - 9)
+            at = units * cta // parts * 16 + b // 5
+            far = [1, 130, 256, 520, (units * (cta + 7) // parts - units * cta // parts) * 16 + 3][b % 5]
+            first.append(at)
+            tall._embed[at] = tall._embed[at + far] = (4 * h[b]).to(torch.bfloat16)
+        assert len(set(first)) == batch
+        got = tall.generate_greedy_batch(ids, 1)[:, 0]
+        logits, _ = tall.forward(ids, logits_positions="last")
+    finally:
+        tall._embed.copy_(kept)
+    assert np.array_equal(logits[:, 0].argmax(-1), first)
+    assert np.array_equal(got, first)
