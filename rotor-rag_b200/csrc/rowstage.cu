@@ -29,6 +29,11 @@ constexpr int RS_WIDE_THREADS = 512;
 // generation step.  One step of 8 sequences of the 2B model: 2.71 -> 1.62 ms (with the partial rows of the decode
 // attention merged here, RS_RUN_BATCH loads at a time, instead of in the shared-memory stage: 16.5 -> 6 us a layer).
 constexpr int RS_FEW_ROWS = 296;
+// Six CTAs an SM leave a thread 80 registers instead of 96: a row takes longer, so they are taken where the rows then need
+// fewer rounds over the SMs, while the shared memory of six fits.  Rows of 2560, one term, five / six: 1200 rows (two rounds
+// either way) 12.6 / 12.8 us, 1500 (three, two) 17.8 / 14.0, 2700 (four) 25.9 / 26.6, 4096 37.1 / 34.0, 16384 132.6 / 123.1;
+// three terms (40 KB: five fit) 1500 32.0 / 35.8.
+constexpr size_t RS_SIX_BYTES = 36 * 1024;
 constexpr int RS_MAX_RUNS = 32;        // VS_ATTN: runs of a sequence, one per lane
 constexpr int RS_RUN_BATCH = 8;        // ... whose partial rows a thread requests together
 
@@ -82,7 +87,7 @@ __device__ __forceinline__ float4 rs_deq_staged(const int4* stage, int n4, int h
     return make_float4(f.x * wscale, f.y * wscale, f.z * wscale, f.w * wscale);
 }
 
-// Rows of up to five groups with a residual: six CTAs per SM (16384 rows of 2560: 119 us against 129 with five).
+// SIX: rows of up to five groups with a residual, six CTAs per SM instead of five (see RS_SIX_BYTES).
 // Wide rows (V > 8) are capped at 128 registers so that four CTAs share an SM: with fewer, the
 // reductions and the quantiser of one row leave the memory pipe idle.
 // RESID: the stage adds to the residual stream (VS_OPROJ, VS_DOWN) and keeps a second register
@@ -94,8 +99,8 @@ __device__ __forceinline__ float4 rs_deq_staged(const int4* stage, int n4, int h
 // needs no barrier: cp.async.wait_group by the owner is enough, and the next fetch may start
 // as soon as the owner has the pieces in registers.  Accumulator modes only.
 // MERGE: VS_ATTN, the row is merged from the partial results of the decode attention's runs.
-template <int V, bool RESID, int TH, bool PF, bool MERGE = false>
-__global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1) : TH > 128 ? 4 : V > 8 ? 4 : RESID && V <= 5 ? 6 : 5)
+template <int V, bool RESID, int TH, bool PF, bool MERGE = false, bool SIX = false>
+__global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1) : TH > 128 ? 4 : V > 8 ? 4 : SIX ? 6 : 5)
     row_stage_kernel(const __grid_constant__ VecStageParams p, int rows) {
     __shared__ float scratch[64];
     extern __shared__ __align__(16) int4 rs_stage[];
@@ -104,13 +109,15 @@ __global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1)
     const int halves = p.mode == VS_FFN ? 2 : 1;
     float* hdst = p.h_out ? p.h_out : p.h;
     float sxn[3] = {0.f, 0.f, 0.f};
-    if (!PF && (tid & 7) == 0)  // constants: requested while the kernel before this one ends
-        for (int i = 4 * tid; i < n; i += 4 * TH) {
-            if (p.norm0) prefetch_l2(p.norm0 + i);
-            if (p.norm1) prefetch_l2(p.norm1 + i);
-        }
-    pdl_wait();
-    pdl_trigger();
+    if constexpr (!PF) {  // (the prefetching variant is always an ordinary launch, and so is this one with more rows)
+        if ((tid & 7) == 0 && gridDim.x <= RS_FEW_ROWS)  // constants: requested while the kernel before this one ends
+            for (int i = 4 * tid; i < n; i += 4 * TH) {
+                if (p.norm0) prefetch_l2(p.norm0 + i);
+                if (p.norm1) prefetch_l2(p.norm1 + i);
+            }
+        pdl_wait();
+        pdl_trigger();
+    }
     clear_sums(p);
 
     // PF: start the fetch of `row` (pieces into the staging area, scales into registers)
@@ -348,14 +355,14 @@ bool row_stage_supported(const VecStageParams& p, int rows) {
 
 // Launches one instantiation.  Accumulator modes whose staging area fits run the prefetching
 // variant on a grid of resident CTAs; everything else runs one CTA per row.
-template <int V, bool RESID, int TH>
+template <int V, bool RESID, int TH, bool SIX = false>
 static int launch_one(const VecStageParams& p, int rows, cudaStream_t st) {
     const bool from_acc = p.mode == VS_OPROJ || p.mode == VS_FFN || p.mode == VS_DOWN || p.mode == VS_DEQ;
     const bool plain = p.mode == VS_PLAIN && !RESID;  // float rows in: one staged piece
     const size_t pieces = plain ? 1 : (size_t)p.terms * (p.mode == VS_FFN ? 2 : 1) + (RESID ? 1 : 0);
     const size_t smem = pieces * (size_t)p.n * sizeof(int);
     if ((from_acc || plain) && smem <= 200 * 1024) {
-        auto* k = row_stage_kernel<V, RESID, TH, true>;
+        auto* k = row_stage_kernel<V, RESID, TH, true, false, SIX>;
         static PerDevice<size_t> once;  // per instantiation and device
         static PerDevice<int> sm_counts;
         size_t& configured = once.here();
@@ -403,6 +410,12 @@ static int launch_few(const VecStageParams& p, int rows, cudaStream_t st) {
 
 template <bool RESID>
 static int launch_row_stage_v(const VecStageParams& p, int rows, int v, cudaStream_t st) {
+    if constexpr (RESID) {
+        const size_t staged = ((size_t)p.terms + 1) * p.n * sizeof(int);
+        const int five = 5 * fused_sm_count(), six = 6 * fused_sm_count();
+        if (v <= 5 && staged <= RS_SIX_BYTES && (rows + six - 1) / six < (rows + five - 1) / five)
+            return launch_one<5, true, RS_THREADS, true>(p, rows, st);
+    }
     if (v <= 5) return launch_one<5, RESID, RS_THREADS>(p, rows, st);
     if (v <= 8) return launch_one<8, RESID, RS_THREADS>(p, rows, st);
     if constexpr (!RESID) {

@@ -628,3 +628,17 @@ def test_ffn_sums_cleared_by_stage_or_memset(rb, ff, rows):
     x = torch.randn((rows, 512), generator=g, device="cuda")
     got, want = ffn.forward_device(x), torch.cat([ffn.forward_device(x[i:i + 1].contiguous()) for i in range(rows)])
     assert (got - want).norm() < 2e-5 * want.norm()
+
+
+@pytest.mark.parametrize("d", [512, 1536, 2560])
+def test_prompt_rows_of_many_equal_few(rb, d):
+    """2300 rows of a prompt of two sequences (three rounds of six CTAs an SM in the residual stages, four of five) against the
+    1150 of each sequence alone (two rounds either way: five CTAs; rows of 2560 with three terms: always five).  The integer sums are the same and the stages add in the same order."""
+    import torch
+    model = rb.synth.random_model_on_device(dict(vocab_size=512, d_model=d, n_layers=2, n_heads=d // 128, n_kv_heads=1, d_ff=512), seed=d,
+                                            semantics=rb.sem.REFERENCE, max_seq=1150, max_batch=2, max_rows=2300)
+    ids = np.random.default_rng(d).integers(0, 512, size=(2, 1150))
+    got = model.forward_last_logits_device(ids)[0].clone()
+    for b in range(2):
+        want = model.forward_last_logits_device(ids[b:b + 1])[0]
+        assert rel_err(got[b].cpu().numpy(), want[0].cpu().numpy()) < 1e-5, b
