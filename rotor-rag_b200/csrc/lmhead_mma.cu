@@ -19,6 +19,7 @@
 // stages): 8 rows of d 2560 305 -> 131 us = 5.0 TB/s, 64 rows of d 8192 920 -> 404 us = 5.2 TB/s.  Loads of 128 rows
 // instead of 16 gave 10 %, evicting the table's lines first up to 10 % more; two 64-column panels a stage nothing.
 // Outputs: logits (optional) and one (max, argmax) partial per CTA and token row, merged by argmax_final_kernel.
+// (The file, its entry points and ROTOR_B200_NO_LMHEAD_MMA keep the name of the mma.sync kernel that stood here before.)
 #include <cuda_bf16.h>
 
 #include <cstdlib>
@@ -323,7 +324,7 @@ int launch_lmhead_mma(const __nv_bfloat16* embed, const float* x, __nv_bfloat16*
     p.part_val = part_val;
     p.part_idx = part_idx;
     // The token tile: all rows up to 128 in one pass over the table; a vocabulary of fewer shares than SMs takes narrower
-    // tiles while the grid still fits one CTA to an SM (its table is small and comes from L2).
+    // tiles while the grid still fits one CTA to an SM (its table is small and comes from L2: 200 rows of 512 x 512 19.1 -> 9.1 us).
     int nt = rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128;
     while (nt > 16 && lmhead_mma_parts(vocab) * ((rows + nt / 2 - 1) / (nt / 2)) <= fused_sm_count()) nt /= 2;
     switch (nt) {

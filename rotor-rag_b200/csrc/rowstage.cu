@@ -384,8 +384,11 @@ static int launch_one(const VecStageParams& p, int rows, cudaStream_t st) {
             return launch_status();
         }
     }
-    row_stage_kernel<V, RESID, TH, false><<<rows, TH, 0, st>>>(p, rows);
-    return launch_status();
+    if constexpr (TH == 256) return ROTOR_B200_ERR_SHAPE;  // float rows of at most 28 KB always have room to be staged
+    else {
+        row_stage_kernel<V, RESID, TH, false><<<rows, TH, 0, st>>>(p, rows);
+        return launch_status();
+    }
 }
 
 // One CTA per row (a single wave).
@@ -408,6 +411,7 @@ static int launch_few(const VecStageParams& p, int rows, cudaStream_t st) {
     return launch_status();
 }
 
+// Rows of up to 4096 elements.
 template <bool RESID>
 static int launch_row_stage_v(const VecStageParams& p, int rows, int v, cudaStream_t st) {
     if constexpr (RESID) {
@@ -417,12 +421,7 @@ static int launch_row_stage_v(const VecStageParams& p, int rows, int v, cudaStre
             return launch_one<5, true, RS_THREADS, true>(p, rows, st);
     }
     if (v <= 5) return launch_one<5, RESID, RS_THREADS>(p, rows, st);
-    if (v <= 8) return launch_one<8, RESID, RS_THREADS>(p, rows, st);
-    if constexpr (!RESID) {
-        if (v <= 14) return launch_one<14, RESID, RS_THREADS>(p, rows, st);
-        return launch_one<16, RESID, RS_THREADS>(p, rows, st);
-    }
-    return ROTOR_B200_ERR_SHAPE;  // wider rows with a residual take the 512-thread kernel (launch_row_stage)
+    return launch_one<8, RESID, RS_THREADS>(p, rows, st);
 }
 
 int launch_row_stage(const VecStageParams& p, int rows, cudaStream_t st) {
