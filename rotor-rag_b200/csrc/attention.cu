@@ -832,17 +832,21 @@ static bool attn_decode_stream_ok(const AttnParams& p, int rows) {
     return G >= 1 && G <= AC_MAX_GROUP;
 }
 
-// Fewer sequences than fill the GPU: cut each into runs (a power of two, at most max_nsplit), about 512 CTAs for any
-// length, so that every SM has work, and up to 2048 while a run keeps 64 of the cache's positions: three CTAs share an SM,
-// and with one CTA too many for a whole round the SMs that end first would idle.
+// Fewer sequences than fill the GPU: cut each into runs (a power of two, at most max_nsplit), about 512 CTAs, so that every
+// SM has work.  Where that leaves whole sequences, up to 2048 CTAs while the cache's capacity leaves a run 64 positions (the
+// host does not know the present lengths): a few CTAs share an SM, and with one too many for a whole round the SMs that end
+// first would idle.  Step of the XL shape (4 layers, 64 sequences, capacity 2100), whole / four runs: context 30 656 / 709 us,
+// 500 919 / 910, 2000 1591 / 1438; where 512 CTAs make runs already, more of them lose at every length (2B shape, 8 layers, 24
+// sequences: 4 / 16 runs 630 / 690 us at 30, 962 / 1029 at 2000).
 int attn_stream_splits(int rows, int n_heads, int n_kv_heads, int head_dim, int max_nsplit, int max_seq) {
     if (n_kv_heads < 1 || n_heads % n_kv_heads || (head_dim != 64 && head_dim != 128)) return 0;
     const int G = n_heads / n_kv_heads;
     if (G < 1 || G > AC_MAX_GROUP) return 0;
     int s = 1;
-    while (2 * s <= max_nsplit && ((long)rows * n_kv_heads * 2 * s <= 512 ||
-                                   ((long)rows * n_kv_heads * 2 * s <= 2048 && max_seq / (2 * s) >= 64)))
-        s *= 2;
+    const long ctas = (long)rows * n_kv_heads;
+    while (2 * s <= max_nsplit && ctas * 2 * s <= 512) s *= 2;
+    if (s == 1)
+        while (2 * s <= max_nsplit && ctas * 2 * s <= 2048 && max_seq / (2 * s) >= 64) s *= 2;
     return s;
 }
 
