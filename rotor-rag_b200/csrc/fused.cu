@@ -22,7 +22,7 @@ RB_TRACE_DEFINE(rotor_b200_trace_read_fused)
 
 namespace rb {
 
-template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, int KIND>
+template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, bool TP, bool ALONE = false>
 __global__ void __launch_bounds__(FG_THREADS, DEEP ? 1 : 2) fused_gemv_kernel(const __grid_constant__ FusedGemvParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_sx[8];
@@ -41,21 +41,21 @@ __global__ void __launch_bounds__(FG_THREADS, DEEP ? 1 : 2) fused_gemv_kernel(co
     pdl_wait();     // the weights above are constants; everything below depends on earlier kernels
     pdl_trigger();  // after the wait: see the rule in common.cuh
     RB_STAMP(tr, 2);
-    product_run<USE_MMA, NCOL, WIDE, DEEP, KIND>(p, c, wv, s_sx, s_xsum, tr);
+    product_run<USE_MMA, NCOL, WIDE, DEEP, TP, ALONE>(p, c, wv, s_sx, s_xsum, tr);
     RB_STAMP(tr, 5);
     RB_TRACE_COMMIT(tr, p.st.mode * 10 + p.halves);
 }
 
-template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, int KIND>
+template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP, bool TP, bool ALONE = false>
 static int launch_fused_kind(const FusedGemvParams& p, int grid, cudaStream_t st) {
     static PerDevice<bool> once;  // each variant raises its own shared-memory limit once per device
     bool& configured = once.here();
     if (!configured) {
-        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, KIND>,
+        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, TP, ALONE>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         // the largest shared-memory split for every variant: kernels of a step share SMs, and a CTA
         // whose request does not fit the split left by its neighbour waits for the SM to drain
-        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, KIND>,
+        RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, TP, ALONE>,
                                      cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         configured = true;
     }
@@ -70,8 +70,8 @@ static int launch_fused_kind(const FusedGemvParams& p, int grid, cudaStream_t st
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_use_pdl && KIND != FG_ALONE ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, KIND>, p) != cudaSuccess) {
+    cfg.numAttrs = g_use_pdl && !ALONE ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, fused_gemv_kernel<USE_MMA, NCOL, WIDE, DEEP, TP, ALONE>, p) != cudaSuccess) {
         ++g_launch_count;
         return ROTOR_B200_ERR_CUDA;
     }
@@ -80,22 +80,22 @@ static int launch_fused_kind(const FusedGemvParams& p, int grid, cudaStream_t st
 
 template <bool USE_MMA, int NCOL, bool WIDE, bool DEEP>
 static int launch_fused(const FusedGemvParams& p, int grid, cudaStream_t st, bool alone) {
-    if (alone) return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, FG_ALONE>(p, grid, st);
-    if (p.xs.size || p.part) return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, FG_SHARDED>(p, grid, st);
-    return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, FG_STEP>(p, grid, st);
+    if (alone) return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, false, true>(p, grid, st);
+    if (p.xs.size || p.part) return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, true>(p, grid, st);
+    return launch_fused_kind<USE_MMA, NCOL, WIDE, DEEP, false>(p, grid, st);
 }
 
 int configure_fused_gemv() {
     const int big = 200 * 1024;
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, false, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, false, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, false, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, true, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, true, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, true, true, FG_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 1, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<false, 2, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    RB_CUDA(cudaFuncSetAttribute(fused_gemv_kernel<true, 1, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     fused_sm_count();
     return ROTOR_B200_OK;
 }
@@ -186,9 +186,9 @@ int launch_staged_acc(const void* tiles, size_t out, size_t in, const int8_t* xq
     p.acc_out = acc;
     if (grid > p.units) grid = p.units;
     const bool mma = variant == ROTOR_B200_VARIANT_MMA || ncols > 2;
-    if (mma) return launch_fused_kind<true, 1, false, false, FG_STEP>(p, grid, st);
-    if (ncols == 1) return launch_fused_kind<false, 1, false, false, FG_STEP>(p, grid, st);
-    return launch_fused_kind<false, 2, false, false, FG_STEP>(p, grid, st);
+    if (mma) return launch_fused_kind<true, 1, false, false, false>(p, grid, st);
+    if (ncols == 1) return launch_fused_kind<false, 1, false, false, false>(p, grid, st);
+    return launch_fused_kind<false, 2, false, false, false>(p, grid, st);
 }
 
 }  // namespace rb

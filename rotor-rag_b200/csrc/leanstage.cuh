@@ -198,13 +198,17 @@ __device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& ls
         q2 = rintf(__fdiv_rn(v.z, s));
         q3 = rintf(__fdiv_rn(v.w, s));
     }
-    if (RESIDUAL || CLAMP) {
+    if constexpr (CLAMP && !RESIDUAL) {
         q0 = fminf(fmaxf(q0, -128.f), 127.f);
         q1 = fminf(fmaxf(q1, -128.f), 127.f);
         q2 = fminf(fmaxf(q2, -128.f), 127.f);
         q3 = fminf(fmaxf(q3, -128.f), 127.f);
     }
     if (RESIDUAL) {
+        q0 = fminf(fmaxf(q0, -128.f), 127.f);
+        q1 = fminf(fmaxf(q1, -128.f), 127.f);
+        q2 = fminf(fmaxf(q2, -128.f), 127.f);
+        q3 = fminf(fmaxf(q3, -128.f), 127.f);
         v.x = __fsub_rn(v.x, __fmul_rn(q0, s));
         v.y = __fsub_rn(v.y, __fmul_rn(q1, s));
         v.z = __fsub_rn(v.z, __fmul_rn(q2, s));

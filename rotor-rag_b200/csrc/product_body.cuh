@@ -22,11 +22,6 @@ constexpr int FG_L2_AHEAD = 32;  // deep variant: further tiles per warp pulled 
 constexpr size_t FG_STAGE_MAX = 96 * 1024;  // shallow variant: most tile bytes a CTA stages
 constexpr int FG_V = 4;        // float4 groups per thread in the register prologue: input width <= 8192
 constexpr int FG_V_NARROW = 2; // shallow variant, stages that hold four arrays per group: width <= 4096
-// What the product is part of: a generation step; the same with tensor-parallel hooks (scalar exchanges in the prologue,
-// int32 partial output); a stand-alone layer call (LM_PLAIN; an ordinary launch, because its weights may be the work of the
-// kernel before it).
-enum { FG_STEP = 0, FG_SHARDED = 1, FG_ALONE = 2 };
-
 struct FusedGemvParams {
     const uint4* tiles;   // tiles of the (stacked) matrix
     int nkt;              // K tiles per row tile
@@ -196,12 +191,13 @@ __device__ __forceinline__ void product_prefetch(const FusedGemvParams& p, const
 // (large matrices): the loop requests the following batch of tiles before multiplying the
 // current one and tracks its position by counting; the shallow loop (a few tiles per warp, the
 // latency-bound small matrices) keeps the shortest code path.
-// KIND: what only one caller needs is compiled for that one alone (a flag that every quantiser tested cost the generation
-// step of one sequence 0.3 %: 2B shape 890.9 against 888.5 us).
-template <bool USE_MMA, int NCOL, bool WIDE = false, bool DEEP = false, int KIND = FG_STEP>
+// TP: tensor-parallel hooks compiled in (scalar exchanges in the prologue, int32 partial output).  ALONE: a stand-alone layer
+// call (LM_PLAIN; an ordinary launch, because its weights may be the work of the kernel before it).  What only it needs is
+// compiled for it alone, and the step's text stays apart: with a flag that every quantiser tested a 2B step of one sequence took
+// 890.9 us, with one `kind` argument for all three 888.5, so 884.4.
+template <bool USE_MMA, int NCOL, bool WIDE = false, bool DEEP = false, bool TP = false, bool ALONE = false>
 __device__ __forceinline__ void product_run(const FusedGemvParams& p, const ProductCtx& c, uint4 (&wv)[FG_U],
                                             float* s_sx, int* s_xsum, TraceRec& tr) {
-    constexpr bool TP = KIND == FG_SHARDED, ALONE = KIND == FG_ALONE;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     int8_t* xs = c.xs;
     int* merge = c.merge;
@@ -324,8 +320,10 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
                                       s_sx + m * terms, s_xsum + m * terms, rk, m, writer, x);
             }
         };
-        if constexpr (DEEP || ALONE) {
-            rows(std::integral_constant<int, FG_V>(), std::bool_constant<ALONE>());
+        if constexpr (ALONE) {
+            rows(std::integral_constant<int, FG_V>(), std::true_type());
+        } else if constexpr (DEEP) {
+            rows(std::integral_constant<int, FG_V>(), std::false_type());
         } else {
             if (p.st.mode == LM_PLAIN)
                 rows(std::integral_constant<int, FG_V>(), std::true_type());
@@ -506,9 +504,10 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
             const int slot = DEEP ? lu * p.halves + half : half * (u1 - u0) + lu;
             const int* src = merge + slot * 128 + rl * 8 + m * T;
             float f = 0.f;
-            for (int tt = 0; tt < T; ++tt) {
-                const float q = (float)(src[tt] - s_xsum[m * T + tt]), sc = s_sx[m * T + tt];
-                f = ALONE ? __fadd_rn(f, __fmul_rn(q, sc)) : f + q * sc;  // (as dequant_kernel rounds: one result for any row count)
+            if constexpr (ALONE) {  // as dequant_kernel rounds: one result for any row count
+                for (int tt = 0; tt < T; ++tt) f = __fadd_rn(f, __fmul_rn((float)(src[tt] - s_xsum[m * T + tt]), s_sx[m * T + tt]));
+            } else {
+                for (int tt = 0; tt < T; ++tt) f += (float)(src[tt] - s_xsum[m * T + tt]) * s_sx[m * T + tt];
             }
             return f;
         };
