@@ -243,11 +243,7 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnParams p) {
     }
 }
 
-static bool attn_decode_stream_ok(const AttnParams& p, int rows);
-static int launch_attn_decode_stream(const AttnParams& p, int rows, cudaStream_t st);
-
 int launch_attention(const AttnParams& p, int rows, cudaStream_t st) {
-    if (attn_decode_stream_ok(p, rows)) return launch_attn_decode_stream(p, rows, st);  // batched generation steps
     if (attn_prefill_t5_supported(p, rows)) return launch_attn_prefill_t5(p, rows, st);  // head_dim 128 prompts
     if (attn_prefill_supported(p, rows)) return launch_attn_prefill_tc(p, rows, st);
     dim3 grid(p.n_heads, rows);
@@ -646,21 +642,25 @@ __global__ void __launch_bounds__(AC_MAX_THREADS) attn_decode_cluster_kernel(con
 }
 
 // ---------------------------------------------------------------------------------------
-// One-token attention for many sequences at once (batched generation steps): grid
-// (n_kv_heads, batch, runs), the H query heads of a group together.  q is finished (rotated), the new
-// k / v row is in the cache already.  One run: whole sequences, finished attention rows.  Several runs:
-// every run writes its un-normalised output with its (max, sum), merged by the stage that quantises the
-// attention rows.
+// One-token attention for several sequences at once (batched generation steps): grid
+// (runs, n_kv_heads, batch), the H query heads of a group together, a sequence's cache cut into `runs` equal parts, one CTA
+// of a cluster each.  From the q/k/v product's sums to finished attention rows in one launch: every warp dequantises and
+// rotates its queries, the last CTA of a cluster the new k / v row, which it appends; the runs meet through distributed
+// shared memory as in the kernel above.
 //
 // Bound by the cache's stream as long as issue slots keep up, so the rows go straight to registers (a
 // row of D floats is one load of the warp, read once for all H heads) and a warp takes four keys at a time: 4 H
 // partial dot products per lane are folded over the lanes by halving (a lane hands over half of its values and keeps the
 // sums of the other half: 31 shuffles for 32 products, after which a lane holds one finished score), so that exponentials
 // are one instruction per 32 scores; the weights return through a line of shared memory.  The warps of a CTA take every
-// fourth group of four keys and merge at the end.  The next four keys are requested before the present ones are used.
-// 64 sequences of 1025 positions, 64 / 8 heads of 128: 167 us through shared memory with two heads a warp, 126 us here
-// (4.3 TB/s of cache); 8 sequences of 518, 20 / 5 heads: 11.7 -> 10.7 us with its wait for the kernel before.
-constexpr int AS_WARPS = 4, AS_KEYS = 4;
+// W-th group of four keys and merge at the end.  The next four keys are requested before the present ones are used, the
+// first before the launch wait (cached rows are older than the kernel before this one).
+// A step of the 2B shape (12 layers) behind 517 positions, with a finish kernel before and the stage behind merging the runs /
+// here: 5 sequences 694 / 633 us, 8 709 / 651, 16 941 / 879, 64 1732 / 1659; XL shape (4 layers) 8 912 / 863, 64 1477 / 1461.
+constexpr int AS_KEYS = 4, AS_MAX_RUNS = 8;
+
+// Outputs that each of `runs` CTAs merges (the last one the rest).
+__device__ __forceinline__ int as_share(int outputs, int runs) { return (outputs / 4 + runs - 1) / runs * 4; }
 
 template <int E>
 __device__ __forceinline__ void as_load(const float* src, bool live, float (&v)[E]) {
@@ -673,21 +673,67 @@ __device__ __forceinline__ void as_load(const float* src, bool live, float (&v)[
     }
 }
 
-template <int D, int H>
-__global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_stream_kernel(const __grid_constant__ AttnParams p) {
+// This lane's elements of N pieces of token row b of the q/k/v product (first columns col[], E consecutive ones a lane).
+template <int E, int N>
+__device__ __forceinline__ void as_product(const AttnDecodeParams& p, int b, const int (&col)[N], const float (&ws)[N], float (&v)[N][E]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[i][e] = 0.f;
+    for (int t = 0; t < p.terms; ++t) {
+        int a[N][E] = {};
+        const int32_t* row = p.acc.acc + ((size_t)b * p.terms + t) * p.acc.out;
+        for (int pl = 0; pl < p.acc.planes; ++pl, row += p.acc.plane_stride)
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                if constexpr (E == 4) {
+                    const int4 r = __ldcg(reinterpret_cast<const int4*>(row + col[i]));
+                    a[i][0] += r.x, a[i][1] += r.y, a[i][2] += r.z, a[i][3] += r.w;
+                } else {
+                    const int2 r = __ldcg(reinterpret_cast<const int2*>(row + col[i]));
+                    a[i][0] += r.x, a[i][1] += r.y;
+                }
+            }
+        const float sx = __ldcg(&p.sx[(size_t)b * p.terms + t]);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+#pragma unroll
+            for (int e = 0; e < E; ++e) v[i][e] += (float)a[i][e] * sx;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[i][e] *= ws[i];
+}
+
+// Rotation of a row that the warp's lanes hold E elements each: element i pairs with element i + D/2, sixteen lanes on.
+template <int E>
+__device__ __forceinline__ void as_rotate(float (&v)[E], const float2 (&cs)[E], int lane) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const float o = __shfl_xor_sync(0xffffffffu, v[e], 16);
+        v[e] = lane < 16 ? v[e] * cs[e].x - o * cs[e].y : v[e] * cs[e].x + o * cs[e].y;
+    }
+}
+
+template <int D, int H, int W>
+__global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_decode_stream_kernel(const __grid_constant__ AttnDecodeParams p) {
     constexpr int E = D / 32, HP = H > 4 ? 8 : H > 2 ? 4 : H;      // heads, rounded up to a power of two for the folding
     constexpr int N = HP * AS_KEYS, SH = N == 32 ? 0 : N == 16 ? 1 : N == 8 ? 2 : 3;  // lane >> SH: value 4 h + key
-    __shared__ __align__(16) float s_w[AS_WARPS][2][N];            // weights of a group of keys
-    __shared__ float s_a[AS_WARPS][HP];                            // rescaling factors
-    __shared__ float s_m[AS_WARPS][HP], s_l[AS_WARPS][HP];
-    __shared__ __align__(16) float s_o[AS_WARPS][H][D];
+    __shared__ __align__(16) float s_w[W][2][N];                   // weights of a group of keys
+    __shared__ float s_a[W][HP];                                   // rescaling factors
+    __shared__ float s_m[W][HP], s_l[W][HP];
+    __shared__ __align__(16) float s_o[W][H][D];
+    __shared__ __align__(16) float s_ro[H * D + 4 * AS_MAX_RUNS];  // [runs][share] the runs' outputs that this CTA merges
+    __shared__ float s_rm[AS_MAX_RUNS][H], s_rl[AS_MAX_RUNS][H];   // (max, sum) of every run and head
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int hk = blockIdx.x, b = blockIdx.y, dq = p.n_heads * D;
-    const int T = min(p.past_len[b] + 1, p.max_seq);
+    const int run = blockIdx.x, nrun = (int)gridDim.x, hk = blockIdx.y, b = blockIdx.z;
+    const int dq = p.n_heads * D, dkv = p.n_kv_heads * D;
+    // every CTA of the cluster has started (its shared memory may be written) once this phase completes
+    if (nrun > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    const int pos = __ldcg(p.past_len + b), T = min(pos, p.max_seq);  // rows in the cache already
     const size_t head0 = ((size_t)b * p.n_kv_heads + hk) * p.max_seq * D + E * lane;
-    const float *kc = p.k_cache + head0, *vc = p.v_cache + head0;
-    // this CTA's run of the sequence: all of it, or one of gridDim.z equal parts
-    const int nrun = (int)gridDim.z, run = (int)blockIdx.z;
+    float *kc = p.k_cache + head0, *vc = p.v_cache + head0;
     const int rlen = (T + nrun - 1) / nrun, k0 = run * rlen, k1 = min(T, k0 + rlen);
 
     float ka[AS_KEYS][E], va[AS_KEYS][E], kb[AS_KEYS][E], vb[AS_KEYS][E];
@@ -698,19 +744,36 @@ __global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_str
         for (int u = 0; u < AS_KEYS; ++u) as_load<E>(vc + (size_t)(t + u) * D, t + u < k1, v[u]);
     };
     int t = k0 + AS_KEYS * warp;
-    // rows behind the new one are older than the kernel before this one (see the rule in common.cuh)
-    const bool early = t < k1 && min(t + AS_KEYS, k1) < T;
-    if (early) fetch(t, ka, va);
+    if (t < k1) fetch(t, ka, va);
+    float2 cs[E] = {};
+    if (p.rope) {  // (a constant table)
+        const float2* r = p.rope + (size_t)min(pos, p.max_seq - 1) * (D / 2) + ((E * lane) & (D / 2 - 1));
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+            const float4 c = __ldg(reinterpret_cast<const float4*>(r + e));
+            cs[e] = make_float2(c.x, c.y);
+            cs[e + 1] = make_float2(c.z, c.w);
+        }
+    }
     pdl_wait();
     pdl_trigger();
-    if (t < k1 && !early) fetch(t, ka, va);
     float q[H][E];
-    const float scale = 1.0f / sqrtf((float)D);
+    {
+        int col[H];
+        float ws[H];
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-        as_load<E>(p.q + (size_t)b * dq + (size_t)(hk * H + h) * D + E * lane, true, q[h]);
+        for (int h = 0; h < H; ++h) {
+            col[h] = (hk * H + h) * D + E * lane;
+            ws[h] = p.sq;
+        }
+        as_product<E, H>(p, b, col, ws, q);
+        const float scale = 1.0f / sqrtf((float)D);
 #pragma unroll
-        for (int e = 0; e < E; ++e) q[h][e] *= scale;
+        for (int h = 0; h < H; ++h) {
+            if (p.rope) as_rotate<E>(q[h], cs, lane);
+#pragma unroll
+            for (int e = 0; e < E; ++e) q[h][e] *= scale;
+        }
     }
     float m_run = -INFINITY, l_run = 0.f;  // of this lane's head; l_run: of this lane's keys alone
     float o[H][E];
@@ -720,7 +783,7 @@ __global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_str
         for (int e = 0; e < E; ++e) o[h][e] = 0.f;
     const int mine = lane >> SH, my_key = mine & 3, my_head = mine >> 2;
     int flip = 0;
-    auto step = [&](int t0, const float (&k)[AS_KEYS][E], const float (&v)[AS_KEYS][E]) {
+    auto step = [&](int left, const float (&k)[AS_KEYS][E], const float (&v)[AS_KEYS][E]) {
         float s[N];
 #pragma unroll
         for (int h = 0; h < HP; ++h)
@@ -748,7 +811,7 @@ __global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_str
                 s[0] += __shfl_xor_sync(0xffffffffu, s[0], w);
             }
         }
-        const bool live = t0 + my_key < k1;
+        const bool live = my_key < left;
         float top = live ? s[0] : -INFINITY;
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1 << SH));
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2 << SH));
@@ -779,14 +842,38 @@ __global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_str
         }
         flip ^= 1;
     };
-    constexpr int STRIDE = AS_KEYS * AS_WARPS;
+    // ---- the new row: the last run's last warp makes it, appends it and weighs it by itself
+    if (run == nrun - 1 && warp == W - 1 && pos < p.max_seq) {
+        float kv[2][E];
+        const int col[2] = {dq + hk * D + E * lane, dq + dkv + hk * D + E * lane};
+        const float ws[2] = {p.sk, p.sv};
+        as_product<E, 2>(p, b, col, ws, kv);
+        if (p.rope) as_rotate<E>(kv[0], cs, lane);
+#pragma unroll
+        for (int u = 0; u < AS_KEYS; ++u)
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                kb[u][e] = u ? 0.f : kv[0][e];
+                vb[u][e] = u ? 0.f : kv[1][e];
+            }
+        const size_t at = (size_t)pos * D;
+        if constexpr (E == 4) {
+            *reinterpret_cast<float4*>(kc + at) = make_float4(kv[0][0], kv[0][1], kv[0][2], kv[0][3]);
+            *reinterpret_cast<float4*>(vc + at) = make_float4(kv[1][0], kv[1][1], kv[1][2], kv[1][3]);
+        } else {
+            *reinterpret_cast<float2*>(kc + at) = make_float2(kv[0][0], kv[0][1]);
+            *reinterpret_cast<float2*>(vc + at) = make_float2(kv[1][0], kv[1][1]);
+        }
+        step(1, kb, vb);
+    }
+    constexpr int STRIDE = AS_KEYS * W;
     while (t < k1) {
         if (t + STRIDE < k1) fetch(t + STRIDE, kb, vb);
-        step(t, ka, va);
+        step(k1 - t, ka, va);
         t += STRIDE;
         if (t >= k1) break;
         if (t + STRIDE < k1) fetch(t + STRIDE, ka, va);
-        step(t, kb, vb);
+        step(k1 - t, kb, vb);
         t += STRIDE;
     }
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1 << SH);
@@ -798,76 +885,124 @@ __global__ void __launch_bounds__(32 * AS_WARPS, H >= 5 ? 3 : 4) attn_decode_str
 #pragma unroll
         for (int e = 0; e < E; ++e) s_o[warp][h][E * lane + e] = o[h][e];
     __syncthreads();
-    // ---- merge of the warps: thread = output element
-#pragma unroll
-    for (int i = threadIdx.x; i < H * D; i += 32 * AS_WARPS) {
+    // ---- merge of the warps, four outputs a thread; several runs: pushed to the CTA that merges these outputs
+    const int share = as_share(H * D, nrun);
+    if (nrun > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // (phase opened at the top of the kernel)
+    for (int i = 4 * threadIdx.x; i < H * D; i += 128 * W) {
         const int h = i / D, d = i - h * D;
         float M = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < AS_WARPS; ++w) M = fmaxf(M, s_m[w][h]);
-        float acc = 0.f, L = 0.f;
+        for (int w = 0; w < W; ++w) M = fmaxf(M, s_m[w][h]);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        float L = 0.f;
 #pragma unroll
-        for (int w = 0; w < AS_WARPS; ++w) {
+        for (int w = 0; w < W; ++w) {
             const float f = s_m[w][h] == -INFINITY ? 0.f : __expf(s_m[w][h] - M);
-            acc += f * s_o[w][h][d];
+            const float4 v = *reinterpret_cast<const float4*>(&s_o[w][h][d]);
+            acc.x += f * v.x, acc.y += f * v.y, acc.z += f * v.z, acc.w += f * v.w;
             L += f * s_l[w][h];
         }
-        if (nrun > 1) {  // partial results of this run: merged by the stage that follows
-            const size_t slot = ((size_t)b * p.n_heads + (hk * H + h)) * nrun + run;
-            p.part_o[slot * D + d] = acc;
-            if (d == 0) {
-                p.part_m[slot] = M;
-                p.part_l[slot] = L;
+        if (nrun > 1) {
+            const int dst = i / share, off = i - dst * share;
+            st_cluster_v4(cluster_addr(&s_ro[run * share + off], (unsigned)dst), acc);
+            if (d < 4 * nrun) {  // the head's first threads tell one CTA each
+                st_cluster_f32(cluster_addr(&s_rm[run][h], (unsigned)(d >> 2)), M);
+                st_cluster_f32(cluster_addr(&s_rl[run][h], (unsigned)(d >> 2)), L);
             }
         } else {
-            p.out[(size_t)b * dq + (size_t)(hk * H + h) * D + d] = acc * (1.0f / L);
+            const float inv = 1.0f / L;
+            *reinterpret_cast<float4*>(p.attn_out + (size_t)b * dq + (size_t)hk * H * D + i) =
+                make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
         }
+    }
+    if (nrun == 1) return;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = threadIdx.x; i < share && run * share + i < H * D; i += 32 * W) {
+        const int g = run * share + i, h = g / D;
+        float M = -INFINITY;
+        for (int r = 0; r < nrun; ++r) M = fmaxf(M, s_rm[r][h]);
+        float acc = 0.f, L = 0.f;
+        for (int r = 0; r < nrun; ++r) {
+            const float f = s_rm[r][h] == -INFINITY ? 0.f : __expf(s_rm[r][h] - M);
+            acc += f * s_ro[r * share + i];
+            L += f * s_rl[r][h];
+        }
+        p.attn_out[(size_t)b * dq + (size_t)hk * H * D + g] = acc * (1.0f / L);
     }
 }
 
-static bool attn_decode_stream_ok(const AttnParams& p, int rows) {
-    if (p.seq != 1 || (p.head_dim != 64 && p.head_dim != 128)) return false;
-    if (rows < 16 && !(p.nsplit > 1 && p.part_o && p.part_m && p.part_l)) return false;
-    const int G = p.n_heads / p.n_kv_heads;
-    return G >= 1 && G <= AC_MAX_GROUP;
+// Whether a one-token step of this shape takes the streaming kernel.
+bool attn_decode_stream_ok(int n_heads, int n_kv_heads, int head_dim) {
+    if (n_kv_heads < 1 || n_heads % n_kv_heads || (head_dim != 64 && head_dim != 128)) return false;
+    return n_heads / n_kv_heads <= AC_MAX_GROUP;
 }
 
-// Fewer sequences than fill the GPU: cut each into runs (a power of two, at most max_nsplit), about 512 CTAs, so that every
-// SM has work.  Where that leaves whole sequences, up to 2048 CTAs while the cache's capacity leaves a run 64 positions (the
-// host does not know the present lengths): a few CTAs share an SM, and with one too many for a whole round the SMs that end
-// first would idle.  Step of the XL shape (4 layers, 64 sequences, capacity 2100), whole / four runs: context 30 656 / 709 us,
-// 500 919 / 910, 2000 1591 / 1438; where 512 CTAs make runs already, more of them lose at every length (2B shape, 8 layers, 24
-// sequences: 4 / 16 runs 630 / 690 us at 30, 962 / 1029 at 2000).
-int attn_stream_splits(int rows, int n_heads, int n_kv_heads, int head_dim, int max_nsplit, int max_seq) {
-    if (n_kv_heads < 1 || n_heads % n_kv_heads || (head_dim != 64 && head_dim != 128)) return 0;
-    const int G = n_heads / n_kv_heads;
-    if (G < 1 || G > AC_MAX_GROUP) return 0;
+// Runs per sequence.  Every CTA of the launch should be resident at once (three an SM above four heads, else four), with a tenth
+// of the places left because a cluster needs its places in one GPC: a CTA more than fit costs a second round.  Eight where
+// few sequences leave room for them, else at most six (clusters of seven and eight spread worse).  us a step behind
+// 1900 positions with 1 / 2 / 3 / 4 / 5 / 6 / 8 runs: 2B shape, four layers, 5 sequences 534 / 415 / 358 / 349 / 341 / 333 / 324,
+// 8 sequences 542 / 420 / 381 / 362 / 353 / 350 / 367, 16 sequences 564 / 493 / 461 / 490 / 473 / 462 / 513, 24 sequences 672 /
+// 570 / 605 / 570 / 646 / 624 / 592; XL shape, two layers, 5 sequences 838 / 727 / 705 / 671 / 657 / 646 / 624, 16 sequences
+// 1151 / 969 / 896 / 976 / 934 / 906 / 932.
+// Where only whole sequences fit, long caches (the host does not know the present lengths) are cut all the same: 2B shape, 64
+// sequences, one / three runs 993 / 942 behind 1900 positions, 527 / 548 behind 70; XL shape, 40 sequences, one / two 1033 / 1019,
+// 767 / 784.  More sequences than fit: up to 2048 CTAs while the cache's capacity leaves a run 64 positions, so that the last
+// round is short.
+static int attn_stream_runs(int batch, int n_kv_heads, int group, int max_seq) {
+    const long n = (long)batch * n_kv_heads, sms = fused_sm_count(), places = sms * (group >= 5 ? 3 : 4) * 9 / 10;
+    if (n * 8 <= (group >= 5 ? places : 2 * sms)) return 8;
+    for (int s = 6; s > 1; --s)
+        if (n * s <= places) return s;
+    if (n <= places) return max_seq < 1024 ? 1 : group >= 5 ? 2 : 3;
     int s = 1;
-    const long ctas = (long)rows * n_kv_heads;
-    while (2 * s <= max_nsplit && ctas * 2 * s <= 512) s *= 2;
-    if (s == 1)
-        while (2 * s <= max_nsplit && ctas * 2 * s <= 2048 && max_seq / (2 * s) >= 64) s *= 2;
+    while (2 * s <= AS_MAX_RUNS && n * 2 * s <= 2048 && max_seq / (2 * s) >= 64) s *= 2;
     return s;
 }
 
+template <int D, int H, int W>
+static int launch_attn_decode_stream_k(const AttnDecodeParams& p, int batch, int runs, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(runs, p.n_kv_heads, batch);
+    cfg.blockDim = dim3(32 * W);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = runs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl ? 2 : 1;
+    if (cudaLaunchKernelEx(&cfg, attn_decode_stream_kernel<D, H, W>, p) != cudaSuccess) {
+        ++g_launch_count;
+        return ROTOR_B200_ERR_CUDA;
+    }
+    return launch_status();
+}
+
 template <int D>
-static int launch_attn_decode_stream_d(const AttnParams& p, int rows, cudaStream_t st) {
-    const dim3 grid(p.n_kv_heads, rows, p.nsplit > 1 ? p.nsplit : 1);
-    switch (p.n_heads / p.n_kv_heads) {
-        case 1: return launch_dependent(attn_decode_stream_kernel<D, 1>, grid, 32 * AS_WARPS, 0, p, st);
-        case 2: return launch_dependent(attn_decode_stream_kernel<D, 2>, grid, 32 * AS_WARPS, 0, p, st);
-        case 3: return launch_dependent(attn_decode_stream_kernel<D, 3>, grid, 32 * AS_WARPS, 0, p, st);
-        case 4: return launch_dependent(attn_decode_stream_kernel<D, 4>, grid, 32 * AS_WARPS, 0, p, st);
-        case 5: return launch_dependent(attn_decode_stream_kernel<D, 5>, grid, 32 * AS_WARPS, 0, p, st);
-        case 6: return launch_dependent(attn_decode_stream_kernel<D, 6>, grid, 32 * AS_WARPS, 0, p, st);
-        case 7: return launch_dependent(attn_decode_stream_kernel<D, 7>, grid, 32 * AS_WARPS, 0, p, st);
-        case 8: return launch_dependent(attn_decode_stream_kernel<D, 8>, grid, 32 * AS_WARPS, 0, p, st);
+static int launch_attn_decode_stream_d(const AttnDecodeParams& p, int batch, cudaStream_t st) {
+    const int G = p.n_heads / p.n_kv_heads, runs = attn_stream_runs(batch, p.n_kv_heads, G, p.max_seq);
+    // eight warps a CTA where two CTAs an SM hold the launch: 8 sequences of the 2B shape (12 layers) behind 70 / 517 / 1000 / 1990
+    // positions 615 / 651 / 701 / 777 us a step, with four warps 616 / 675 / 749 / 887
+    const bool wide = (long)runs * p.n_kv_heads * batch <= 2 * fused_sm_count();
+    switch (G) {
+        case 1: return launch_attn_decode_stream_k<D, 1, 4>(p, batch, runs, st);
+        case 2: return launch_attn_decode_stream_k<D, 2, 4>(p, batch, runs, st);
+        case 3: return launch_attn_decode_stream_k<D, 3, 4>(p, batch, runs, st);
+        case 4: return wide ? launch_attn_decode_stream_k<D, 4, 8>(p, batch, runs, st) : launch_attn_decode_stream_k<D, 4, 4>(p, batch, runs, st);
+        case 5: return launch_attn_decode_stream_k<D, 5, 4>(p, batch, runs, st);
+        case 6: return launch_attn_decode_stream_k<D, 6, 4>(p, batch, runs, st);
+        case 7: return launch_attn_decode_stream_k<D, 7, 4>(p, batch, runs, st);
+        case 8: return launch_attn_decode_stream_k<D, 8, 4>(p, batch, runs, st);
     }
     return ROTOR_B200_ERR_SHAPE;
 }
 
-static int launch_attn_decode_stream(const AttnParams& p, int rows, cudaStream_t st) {
-    return p.head_dim == 64 ? launch_attn_decode_stream_d<64>(p, rows, st) : launch_attn_decode_stream_d<128>(p, rows, st);
+int launch_attn_decode_stream(const AttnDecodeParams& p, int batch, cudaStream_t st) {
+    if (!p.acc.acc || !p.attn_out || !attn_decode_stream_ok(p.n_heads, p.n_kv_heads, p.head_dim)) return ROTOR_B200_ERR_ARG;
+    return p.head_dim == 64 ? launch_attn_decode_stream_d<64>(p, batch, st) : launch_attn_decode_stream_d<128>(p, batch, st);
 }
 
 static size_t attn_cluster_smem(int G, int D, int lcmax, int ns) {

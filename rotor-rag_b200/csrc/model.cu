@@ -212,6 +212,20 @@ static void quant_sink(const Ctx& c, VecStageParams& p, int slot, int n) {
     p.kpad = (int)kpad_of(n);
 }
 
+// Quantises the finished attention rows and multiplies them by the output projection.
+static int o_product(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView* vo, cudaStream_t st) {
+    const int cols = rows * c.terms;
+    VecStageParams qa = {};
+    qa.mode = VS_PLAIN;
+    qa.n = c.dq;
+    qa.src = c.attn;
+    qa.eps = c.eps;
+    quant_sink(c, qa, 1, c.dq);
+    clear_for(c, qa, c.d, c.dq, cols, c.accB);
+    RB_TRY(launch_vec_stage(qa, rows, st));
+    return gemv(c, L.o_tiles, c.d, c.dq, cols, 1, c.accB, vo, st);
+}
+
 // Attention half of a block.  In: quantised pre-normed rows in xq/sx[0]/xsum[0].
 // Out: accumulators of the output projection (view *vo), activation scales in sx[1].
 static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, int seq, AccView* vo,
@@ -221,12 +235,10 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
     const bool fuse_qkv = qkv_finishes(c, seq, cols);
     AccView va = {};
     if (!fuse_qkv) RB_TRY(gemv(c, L.qkv_tiles, qkv_out, c.d, cols, 0, c.accA, &va, st));
-    // five and more sequences: the streaming kernel reads each sequence's cache once per group of heads, cut into runs
-    // (attn_stream_splits) whose partial results the stage that quantises the attention rows merges
-    const int runs = (seq == 1 && batch >= 5 && batch <= c.max_batch)
-                         ? attn_stream_splits(batch, c.n_heads, c.n_kv_heads, c.head_dim, c.nsplit, c.max_seq) : 0;
-    if (seq == 1 && batch <= c.max_batch && batch < 16 && runs <= 1) {
-        // generation step: dequantise, rotate, append to the cache, attend, merge and quantise in one launch
+    // several sequences: dequantise, rotate, append to the cache and attend in one launch, each sequence's cache read once
+    // per group of heads
+    const bool stream = seq == 1 && batch >= 5 && attn_decode_stream_ok(c.n_heads, c.n_kv_heads, c.head_dim);
+    if (stream || (seq == 1 && batch <= c.max_batch && batch < 16)) {
         AttnDecodeParams dp = {};
         dp.acc = va;
         dp.sx = c.sx[0];
@@ -246,6 +258,12 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
         dp.part_o = c.part_o;
         dp.part_m = c.part_m;
         dp.part_l = c.part_l;
+        if (stream) {
+            dp.attn_out = c.attn;
+            RB_TRY(launch_attn_decode_stream(dp, batch, st));
+            return o_product(c, L, rows, vo, st);
+        }
+        // ... or merge and quantise in that launch too
         dp.counter = c.counters + 8;
         dp.xq = c.xq;
         dp.sx_out = c.sx[1];
@@ -290,28 +308,8 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
     ap.causal = c.causal;
     ap.kv_split = seq >= 16 ? c.kvsplit : nullptr;  // a key tile shared by several query tiles is split once
     ap.split_plane = c.kvsplit_plane;
-    if (runs > 1) {
-        ap.nsplit = runs;
-        ap.part_o = c.part_o;
-        ap.part_m = c.part_m;
-        ap.part_l = c.part_l;
-    }
     RB_TRY(launch_attention(ap, rows, st));
-    VecStageParams qa = {};
-    qa.mode = runs > 1 ? VS_ATTN : VS_PLAIN;
-    qa.n = c.dq;
-    qa.src = c.attn;
-    qa.part_o = c.part_o;
-    qa.part_m = c.part_m;
-    qa.part_l = c.part_l;
-    qa.nsplit = runs;
-    qa.n_heads = c.n_heads;
-    qa.head_dim = c.head_dim;
-    qa.eps = c.eps;
-    quant_sink(c, qa, 1, c.dq);
-    clear_for(c, qa, c.d, c.dq, cols, c.accB);
-    RB_TRY(launch_vec_stage(qa, rows, st));
-    return gemv(c, L.o_tiles, c.d, c.dq, cols, 1, c.accB, vo, st);
+    return o_product(c, L, rows, vo, st);
 }
 
 // FFN half of a block.  In: quantised pre-normed rows in xq/sx[0]/xsum[0].
@@ -593,7 +591,8 @@ static int run_blocks_tp(Model& m, int l0, int l1, const float* next_norm, bool 
         AccView va, vb;
         // ---- attention on this rank's heads
         RB_TRY(acc1(c, L.qkv_tiles, qkv_out, d, cols, 0, c.accA, &va, st));
-        if (seq == 1 && batch <= c.max_batch && batch < 16) {
+        const bool stream = seq == 1 && batch >= 16 && attn_decode_stream_ok(c.n_heads, c.n_kv_heads, c.head_dim);
+        if (stream || (seq == 1 && batch <= c.max_batch && batch < 16)) {
             AttnDecodeParams dp = {};
             dp.acc = va;
             dp.sx = c.sx[0];
@@ -615,7 +614,7 @@ static int run_blocks_tp(Model& m, int l0, int l1, const float* next_norm, bool 
             dp.part_l = c.part_l;
             dp.counter = c.counters + 8;
             dp.attn_out = c.attn;  // merged rows as float; quantised below with the global maximum
-            RB_TRY(launch_attn_decode(dp, batch, st));
+            RB_TRY(stream ? launch_attn_decode_stream(dp, batch, st) : launch_attn_decode(dp, batch, st));
         } else {
             QkvFinishParams qf = {};
             qf.acc = va;

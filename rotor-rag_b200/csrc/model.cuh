@@ -16,7 +16,7 @@ struct AccView {
     int out;
 };
 
-enum VecStageMode { VS_EMBED = 0, VS_PLAIN = 1, VS_OPROJ = 2, VS_FFN = 3, VS_DOWN = 4, VS_DEQ = 5, VS_ATTN = 6 };
+enum VecStageMode { VS_EMBED = 0, VS_PLAIN = 1, VS_OPROJ = 2, VS_FFN = 3, VS_DOWN = 4, VS_DEQ = 5 };
 
 struct VecStageParams {
     int mode;
@@ -33,11 +33,6 @@ struct VecStageParams {
     const float* norm0;          // VS_OPROJ: sub-norm weight
     float* h;                    // residual stream [rows][n] (read)
     float* h_out;                // where the updated stream goes (null = in place, h)
-    // VS_ATTN: merge the decode-attention partials of row m into the row
-    const float* part_o;         // [rows][n_heads][nsplit][head_dim]
-    const float* part_m;         // [rows][n_heads][nsplit]
-    const float* part_l;
-    int nsplit, n_heads, head_dim;
     // sinks
     const float* norm1;          // optional pre-norm weight applied before the sinks
     float eps;
@@ -168,6 +163,9 @@ int launch_attn_decode(const AttnDecodeParams& p, int batch, cudaStream_t st);
 // Cluster variant: finished attention rows in p.attn_out (needs p.qkv_f); see attention.cu.
 bool attn_decode_cluster_ok(int n_heads, int n_kv_heads, int head_dim, int max_seq, int nsplit);
 int launch_attn_decode_cluster(const AttnDecodeParams& p, int batch, cudaStream_t st);
+// Several sequences at once, from the product's sums (p.acc) to finished attention rows in p.attn_out and the appended cache.
+bool attn_decode_stream_ok(int n_heads, int n_kv_heads, int head_dim);
+int launch_attn_decode_stream(const AttnDecodeParams& p, int batch, cudaStream_t st);
 int attn_decode_nsplit(int max_seq);
 int attn_decode_nsplit_for(int n_heads, int n_kv_heads, int head_dim, int max_seq);
 size_t attn_decode_part_floats(int batch, int n_heads, int head_dim, int max_seq);
@@ -185,17 +183,8 @@ struct AttnParams {
     int causal;
     __nv_bfloat16* kv_split;  // optional scratch: K hi, K lo, V hi, V lo planes of the cache rows in use
     size_t split_plane;       // elements per plane (batch capacity * n_kv_heads * max_seq * head_dim)
-    // one-token steps of a few sequences: nsplit > 1 cuts every sequence's cache into nsplit runs, one CTA
-    // each, which write un-normalised partial outputs with their (max, sum) instead of `out`
-    int nsplit;
-    float* part_o;        // [rows][n_heads][nsplit][head_dim]
-    float* part_m;        // [rows][n_heads][nsplit]
-    float* part_l;
 };
 int launch_attention(const AttnParams& p, int rows, cudaStream_t st);
-// Runs for a one-token step of `rows` sequences handled by the streaming kernel (1 = whole sequences,
-// finished rows in `out`); 0 if that kernel does not take the shape.
-int attn_stream_splits(int rows, int n_heads, int n_kv_heads, int head_dim, int max_nsplit, int max_seq);
 bool attn_prefill_supported(const AttnParams& p, int rows);
 int launch_attn_prefill_tc(const AttnParams& p, int rows, cudaStream_t st);
 // head_dim 128 on tcgen05 / tensor memory (attn_prefill_t5.cu); needs the split planes sized for

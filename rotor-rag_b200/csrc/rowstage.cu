@@ -26,16 +26,13 @@ constexpr int RS_WIDE_THREADS = 512;
 // each load: the duration is the length of that chain, so a row takes as many threads as leave one or two groups to
 // each (512, or 1024 above 4096 elements) and the widest rows 1024 with seven.  These stages are launched as dependent
 // kernels and clear the accumulators of the product behind them, so that no memset stands between two kernels of a
-// generation step.  One step of 8 sequences of the 2B model: 2.71 -> 1.62 ms (with the partial rows of the decode
-// attention merged here, RS_RUN_BATCH loads at a time, instead of in the shared-memory stage: 16.5 -> 6 us a layer).
+// generation step.
 constexpr int RS_FEW_ROWS = 296;
 // Six CTAs an SM leave a thread 80 registers instead of 96: a row takes longer, so they are taken where the rows then need
 // fewer rounds over the SMs, while the shared memory of six fits.  Rows of 2560, one term, five / six: 1200 rows (two rounds
 // either way) 12.6 / 12.8 us, 1500 (three, two) 17.8 / 14.0, 2700 (four) 25.9 / 26.6, 4096 37.1 / 34.0, 16384 132.6 / 123.1;
 // three terms (40 KB: five fit) 1500 32.0 / 35.8.
 constexpr size_t RS_SIX_BYTES = 36 * 1024;
-constexpr int RS_MAX_RUNS = 32;        // VS_ATTN: runs of a sequence, one per lane
-constexpr int RS_RUN_BATCH = 8;        // ... whose partial rows a thread requests together
 
 __device__ __forceinline__ float4 rs_deq(const VecStageParams& p, size_t col0, int off, int g, const float (&sxv)[3],
                                          float wscale) {
@@ -98,8 +95,7 @@ __device__ __forceinline__ float4 rs_deq_staged(const int4* stage, int n4, int h
 // one.  Every thread stages exactly the 16-byte pieces it will read itself, so the staging area
 // needs no barrier: cp.async.wait_group by the owner is enough, and the next fetch may start
 // as soon as the owner has the pieces in registers.  Accumulator modes only.
-// MERGE: VS_ATTN, the row is merged from the partial results of the decode attention's runs.
-template <int V, bool RESID, int TH, bool PF, bool MERGE = false, bool SIX = false>
+template <int V, bool RESID, int TH, bool PF, bool SIX = false>
 __global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1) : TH > 128 ? 4 : V > 8 ? 4 : SIX ? 6 : 5)
     row_stage_kernel(const __grid_constant__ VecStageParams p, int rows) {
     __shared__ float scratch[64];
@@ -166,42 +162,6 @@ __global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1)
 
     // ---- build the row: every load of the stage in flight together
     float4 v[V], aux[RESID ? V : 1];
-    if constexpr (MERGE) {
-        // weights exp(m_s - M) / L of every (head, run) into shared memory, one warp per head, lane = run
-        const int D = p.head_dim, ns = p.nsplit, lane = tid & 31;
-        float* wf = reinterpret_cast<float*>(rs_stage);
-        const size_t hb = (size_t)m * p.n_heads * ns;
-        for (int h = tid >> 5; h < p.n_heads; h += TH / 32) {
-            const float ms = lane < ns ? __ldcg(p.part_m + hb + h * ns + lane) : -INFINITY;
-            const float ls = lane < ns ? __ldcg(p.part_l + hb + h * ns + lane) : 0.f;
-            const float M = warp_max(ms), f = ms == -INFINITY ? 0.f : __expf(ms - M), L = warp_sum(ls * f);
-            if (lane < ns) wf[h * ns + lane] = f * (1.0f / L);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < V; ++j) {
-            const int g = tid + j * TH;
-            v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (g >= n4) continue;
-            const int h = 4 * g / D;
-            const float* po = p.part_o + (hb + (size_t)h * ns) * D + (4 * g - h * D);
-            for (int s0 = 0; s0 < ns; s0 += RS_RUN_BATCH) {
-                float4 pv[RS_RUN_BATCH];
-#pragma unroll
-                for (int u = 0; u < RS_RUN_BATCH; ++u)
-                    pv[u] = s0 + u < ns ? ldcg4(po + (size_t)(s0 + u) * D) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int u = 0; u < RS_RUN_BATCH; ++u) {
-                    const float f = s0 + u < ns ? wf[h * ns + s0 + u] : 0.f;
-                    v[j].x += pv[u].x * f;
-                    v[j].y += pv[u].y * f;
-                    v[j].z += pv[u].z * f;
-                    v[j].w += pv[u].w * f;
-                }
-            }
-        }
-    }
-    if constexpr (!MERGE) {
 #pragma unroll
     for (int j = 0; j < V; ++j) {
         const int g = tid + j * TH;
@@ -240,7 +200,6 @@ __global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1)
             v[j] = a;
             if (RESID) aux[RESID ? j : 0] = ldcg4(p.h + ro + 4 * g);
         }
-    }
     }
     if (PF && m + (int)gridDim.x < rows) fetch(m + gridDim.x);  // the staged pieces are in registers now
     if constexpr (RESID) {
@@ -339,10 +298,7 @@ bool row_stage_supported(const VecStageParams& p, int rows) {
     static const bool off = getenv("ROTOR_B200_NO_ROWSTAGE") != nullptr;  // comparison aid
     if (off || rows < RS_MIN_ROWS) return false;
     if (p.mode != VS_EMBED && p.mode != VS_PLAIN && p.mode != VS_OPROJ && p.mode != VS_FFN && p.mode != VS_DOWN &&
-        p.mode != VS_DEQ && p.mode != VS_ATTN)
-        return false;
-    if (p.mode == VS_ATTN && (rows > RS_FEW_ROWS || p.nsplit > RS_MAX_RUNS || p.head_dim % 4 ||
-                              (size_t)p.n_heads * p.nsplit * sizeof(float) > 40 * 1024))
+        p.mode != VS_DEQ)
         return false;
     const bool from_acc = p.mode == VS_OPROJ || p.mode == VS_FFN || p.mode == VS_DOWN || p.mode == VS_DEQ;
     if (from_acc && (p.acc.planes != 1 || p.acc.out % 4 || p.terms < 1 || p.terms > 3)) return false;
@@ -362,7 +318,7 @@ static int launch_one(const VecStageParams& p, int rows, cudaStream_t st) {
     const size_t pieces = plain ? 1 : (size_t)p.terms * (p.mode == VS_FFN ? 2 : 1) + (RESID ? 1 : 0);
     const size_t smem = pieces * (size_t)p.n * sizeof(int);
     if ((from_acc || plain) && smem <= 200 * 1024) {
-        auto* k = row_stage_kernel<V, RESID, TH, true, false, SIX>;
+        auto* k = row_stage_kernel<V, RESID, TH, true, SIX>;
         static PerDevice<size_t> once;  // per instantiation and device
         static PerDevice<int> sm_counts;
         size_t& configured = once.here();
@@ -392,19 +348,18 @@ static int launch_one(const VecStageParams& p, int rows, cudaStream_t st) {
 }
 
 // One CTA per row (a single wave).
-template <int V, bool RESID, int TH, bool MERGE = false>
+template <int V, bool RESID, int TH>
 static int launch_few(const VecStageParams& p, int rows, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows);
     cfg.blockDim = dim3(TH);
-    cfg.dynamicSmemBytes = MERGE ? (size_t)p.n_heads * p.nsplit * sizeof(float) : 0;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_use_pdl ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, row_stage_kernel<V, RESID, TH, false, MERGE>, p, rows) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, row_stage_kernel<V, RESID, TH, false>, p, rows) != cudaSuccess) {
         ++g_launch_count;
         return ROTOR_B200_ERR_CUDA;
     }
@@ -428,9 +383,6 @@ int launch_row_stage(const VecStageParams& p, int rows, cudaStream_t st) {
     const int width = p.xq && p.kpad > p.n ? p.kpad : p.n;   // the quantiser also writes the zero padding
     if (rows <= RS_FEW_ROWS) {
         const bool resid = p.mode == VS_OPROJ || p.mode == VS_DOWN;
-        if (p.mode == VS_ATTN)
-            return width <= 4096 ? launch_few<2, false, 512, true>(p, rows, st) : width <= 8192 ? launch_few<2, false, 1024, true>(p, rows, st)
-                                                                                : launch_few<7, false, 1024, true>(p, rows, st);
         if (width <= 2048) return resid ? launch_few<1, true, 512>(p, rows, st) : launch_few<1, false, 512>(p, rows, st);
         if (width <= 4096) return resid ? launch_few<2, true, 512>(p, rows, st) : launch_few<2, false, 512>(p, rows, st);
         if (width <= 8192) return resid ? launch_few<2, true, 1024>(p, rows, st) : launch_few<2, false, 1024>(p, rows, st);

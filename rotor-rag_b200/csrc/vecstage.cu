@@ -29,8 +29,7 @@ int configure_vec_stage() {
 
 int launch_vec_stage(const VecStageParams& p, int rows, cudaStream_t st) {
     if (row_stage_supported(p, rows)) return launch_row_stage(p, rows, st);  // many rows: register-resident kernel
-    const size_t smem = 64 * 4 + (size_t)p.n * 4 +
-                        (p.mode == VS_ATTN ? 2 * (size_t)p.n_heads * p.nsplit * 4 : 0);  // merge weights behind the row
+    const size_t smem = 64 * 4 + (size_t)p.n * 4;
     static PerDevice<size_t> once;
     size_t& configured = once.here();
     if (smem > 48 * 1024 && smem > configured) {

@@ -136,57 +136,6 @@ __device__ __forceinline__ void vec_stage_row(const VecStageParams& p, int m, fl
                                               bool writer = true, const QuantSink* sink = nullptr) {
     const int n = p.n;
     float* hdst = p.h_out ? p.h_out : p.h;
-    if (p.mode == VS_ATTN) {
-        // weights of every (head, slice): f = exp(m_s - M) / L, then the weighted sum of partials
-        const int D = p.head_dim, ns = p.nsplit, nh = p.n_heads;
-        float* wf = row + n;  // [n_heads][nsplit] x2, directly behind the row
-        float* wl = wf + nh * ns;
-        const size_t hb = (size_t)m * nh * ns;
-        for (int e = threadIdx.x; e < nh * ns; e += blockDim.x) {
-            wf[e] = __ldcg(p.part_m + hb + e);
-            wl[e] = __ldcg(p.part_l + hb + e);
-        }
-        __syncthreads();
-        for (int h = threadIdx.x; h < nh; h += blockDim.x) {
-            float M = -INFINITY;
-            for (int s2 = 0; s2 < ns; ++s2) M = fmaxf(M, wf[h * ns + s2]);
-            float L = 0.f;
-            for (int s2 = 0; s2 < ns; ++s2) {
-                const float ms = wf[h * ns + s2];
-                const float f = ms == -INFINITY ? 0.f : __expf(ms - M);
-                L += wl[h * ns + s2] * f;
-                wf[h * ns + s2] = f;
-            }
-            const float inv = 1.0f / L;
-            for (int s2 = 0; s2 < ns; ++s2) wf[h * ns + s2] *= inv;
-        }
-        __syncthreads();
-        constexpr int MU = 4;
-        for (int i0 = threadIdx.x; i0 < n; i0 += MU * blockDim.x) {
-            float o[MU];
-#pragma unroll
-            for (int u = 0; u < MU; ++u) o[u] = 0.f;
-            for (int s2 = 0; s2 < ns; ++s2) {
-                float pv[MU];
-#pragma unroll
-                for (int u = 0; u < MU; ++u) {
-                    const int idx = i0 + u * blockDim.x;
-                    pv[u] = idx < n ? __ldcg(p.part_o + (hb + (size_t)(idx / D) * ns + s2) * D + idx % D) : 0.f;
-                }
-#pragma unroll
-                for (int u = 0; u < MU; ++u) {
-                    const int idx = i0 + u * blockDim.x;
-                    if (idx < n) o[u] += pv[u] * wf[(idx / D) * ns + s2];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < MU; ++u) {
-                const int idx = i0 + u * blockDim.x;
-                if (idx < n) row[idx] = o[u];
-            }
-        }
-        __syncthreads();
-    }
     const int bd = blockDim.x;
     const bool from_acc = p.mode == VS_OPROJ || p.mode == VS_FFN || p.mode == VS_DOWN || p.mode == VS_DEQ;
     float sxv[4] = {0.f, 0.f, 0.f, 0.f};
@@ -194,7 +143,7 @@ __device__ __forceinline__ void vec_stage_row(const VecStageParams& p, int m, fl
     if (from_acc)
         for (int t = 0; t < p.terms; ++t) sxv[t] = __ldcg(&p.sx_in[col0 + t]);
 
-    for (int i0 = threadIdx.x; i0 < n && p.mode != VS_ATTN; i0 += VS_U * bd) {
+    for (int i0 = threadIdx.x; i0 < n; i0 += VS_U * bd) {
         float v[VS_U], w[VS_U];
         if (p.mode == VS_EMBED) {
             const long long id = p.ids[m];

@@ -587,6 +587,36 @@ def test_batched_steps_equal_single_sequences(rb, shape, batch, context):
         assert rel_err(got[b].cpu().numpy(), steps([b])[0].cpu().numpy()) < 2e-4, b   # about 60 float32 sums of up to 9216 in a row
 
 
+@pytest.mark.parametrize("heads,kv,batch,context,capacity", [(4, 1, 5, 0, 4), (4, 1, 7, 3, 5), (8, 2, 20, 37, 39), (12, 4, 16, 41, 43),
+                                                            (8, 1, 17, 26, 28), (20, 5, 8, 47, 49), (20, 5, 8, 6, 700), (20, 5, 24, 9, 11),
+                                                            (16, 2, 64, 21, 23), (8, 8, 40, 19, 1500), (16, 8, 90, 11, 300)])
+def test_runs_of_batched_steps(rb, heads, kv, batch, context, capacity):
+    """Steps whose sequences are cut into every number of runs that the rule gives (one to six, eight), with empty runs, runs that
+    are no multiple of a warp's keys and outputs that do not divide by the runs, against each sequence alone.  Two steps: the
+    second reads the row that the first appended.  Three activation terms: float32 rounding is all that may differ."""
+    import torch
+    cfg = dict(vocab_size=512, d_model=heads * 64 if heads != 20 else 2560, n_layers=1, n_heads=heads, n_kv_heads=kv, d_ff=512)
+    model = rb.synth.random_model_on_device(cfg, seed=batch, semantics=rb.sem.REFERENCE, max_seq=capacity, max_batch=batch, max_rows=batch)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(heads + batch)
+    held = [torch.randn((batch, kv, context, cfg["d_model"] // heads), generator=g, device="cuda") for _ in range(2)]
+    ids = np.random.default_rng(batch).integers(0, 512, size=(2, batch, 1))
+
+    def steps(rows):
+        at = model.layers[0].attention
+        for cache, t in zip(at.ensure_cache(batch, capacity), held):
+            cache[:len(rows), :, :context] = t[rows]
+        caches, out = [rb.tr.KVCache(at, context, len(rows))], []
+        for i in range(2):
+            logits, caches = model.forward_last_logits_device(ids[i][rows], caches)
+            out.append(logits.clone())
+        return torch.stack(out, 1)
+
+    got = steps(list(range(batch)))
+    for b in (0, batch - 1):
+        assert rel_err(got[b].cpu().numpy(), steps([b])[0].cpu().numpy()) < 2e-4, b
+
+
 @pytest.mark.parametrize("heads,kv", [(4, 2), (8, 1), (3, 3)])
 @pytest.mark.parametrize("batch,context,hidden", [(5, 300, 4), (5, 300, 45), (5, 300, 300), (16, 30, 17), (33, 129, 128), (18, 5, 5)])
 def test_infinite_scores_weigh_nothing(rb, heads, kv, batch, context, hidden):
