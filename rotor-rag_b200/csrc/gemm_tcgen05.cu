@@ -16,9 +16,9 @@
 // the read-back subtracts the token's activation sum.  After the last stage the decoder warps read
 // the accumulators back (tcgen05.ld 32 lanes x 32 columns: a lane holds 32 consecutive outputs of
 // one token) and pass them through a per-warp shared-memory block so that they leave as whole
-// 128-byte rows.  Read-back variants: plain int32 sums; GATED (gate/up product: activation and
-// product in the read-back, float32 out); QKV (dequantise, rotary, cache append).  When 256-row tiles
-// do not cover the GPU the K range is split over blockIdx.z and the partial sums are added with
+// 128-byte rows.  Prompts whose tiles give every pair of SMs work take gemm_pair_kernel below, with further read-backs:
+// PAIR_GATED (gate/up product: activation and product, float32 out) and PAIR_QKV (dequantise, rotary, cache append).  When
+// 256-row tiles do not cover the GPU the K range is split over blockIdx.z and the partial sums are added with
 // integer atomics (64-row tiles remain for products too short to split).
 // Every wait is bounded by a cycle count; a wait that runs out records a code in the library status
 // word, the CTA stops issuing work, lets its copies land, frees its tensor memory and returns.
@@ -66,15 +66,16 @@ struct Tc5Params {
     unsigned* status;
     int out, nrt, nkt, ncols;
     int kt_per_split;   // > 0: CTA z takes K steps [z kt_per_split, +kt_per_split) and ADDS its sums into zeroed acc
-    // gated epilogue (GATED kernel): `tiles` holds the gate matrix followed by the up matrix (ff rows
-    // each); a CTA takes 128 gate rows and the matching 128 up rows, and writes
+    int mt, nt;         // pairs: tiles of 256 tokens, of 256 weight rows (128 channels when gated)
+    // PAIR_GATED: `tiles` holds the gate matrix followed by the up matrix (ff rows
+    // each); a tile takes 128 gate rows and the matching 128 up rows, and the read-back writes
     // gated[token][channel] = act(gate * sx[token] * sg) * (up * sx[token] * su) as float32 instead
     // of two int32 accumulators per channel
     float* gated;       // [ncols][ff]
     const float* sx;    // [ncols] activation scales (one term per token)
     float sg, su;
     int ff, ffn_act;
-    // q/k/v epilogue (QKV kernel, head_dim 128): `tiles` is the stacked [q; k; v] matrix; the read-back
+    // PAIR_QKV (head_dim 128): `tiles` is the stacked [q; k; v] matrix; the read-back
     // dequantises (sx[token] * sq / sk / sv), rotates q and k (half-split pairs i, i + 64) and writes q rows
     // and the K / V cache rows of the token's position; no int32 accumulator leaves the kernel
     int dq, dkv, seq, max_seq;
@@ -86,7 +87,7 @@ struct Tc5Params {
     float sq, sk, sv;
 };
 
-template <int ROWS, int T5_TOK = 256, bool GATED = false, bool QKV = false>
+template <int ROWS, int T5_TOK = 256>
 __global__ void __launch_bounds__(T5Cfg<ROWS, T5_TOK>::THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ Tc5Params p) {
     using Cfg = T5Cfg<ROWS, T5_TOK>;
@@ -138,12 +139,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
         auto fetch = [&](int kt, uint4 (&dst)[TPW]) {
 #pragma unroll
             for (int u = 0; u < TPW; ++u) {
-                int rt = rt0 + warp * TPW + u;
-                if constexpr (GATED) {
-                    // operand rows 0-127: gate row tiles 8 blockIdx.y ..; rows 128-255: the same channels of the up matrix
-                    const int i = warp * TPW + u, ch_rt = (int)blockIdx.y * 8 + (i & 7), ff_rt = p.ff / TILE_ROWS;
-                    rt = ch_rt < ff_rt ? (i < 8 ? ch_rt : ff_rt + ch_rt) : p.nrt;  // past the last channel: zero weights
-                }
+                const int rt = rt0 + warp * TPW + u;
                 dst[u] = (rt < p.nrt && kt < nk)
                              ? ld_stream_v4(p.tiles + ((size_t)rt * p.nkt + ktb + kt) * 32 + lane)
                              : make_uint4(0x55555555u, 0x55555555u, 0x55555555u, 0x55555555u);
@@ -222,105 +218,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
             // groups of four split the (token half, 32-row chunk) pairs between them
             constexpr int NCH = T5_ROWS / 32, GROUPS = NDW / 4;
             const int wq = warp & 3, grp = warp >> 2;
-            if constexpr (QKV) {
-                // lane = token; per item one head of the tile (0 / 1) and one pair of 32-row chunks (pp, pp + 2):
-                // rows 32 pp + [0, 32) of the head rotate with rows 64 + 32 pp + [0, 32)
-#pragma unroll 1
-                for (int item = grp; item < nhalf * 4; item += GROUPS) {
-                    const int half = item >> 2, hh = (item >> 1) & 1, pp = item & 1;
-                    const int R0 = row0 + hh * 128;  // first row of the head in the stacked matrix
-                    if (R0 >= p.out) continue;       // warp-uniform
-                    const int tok_base = tok0 + half * 128 + wq * 32;
-                    const int token = tok_base + lane;
-                    uint32_t gv[32], uv[32];
-                    const uint32_t taddr = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(half * ROWS + hh * 128 + pp * 32);
-                    t5_ld32(taddr, gv);
-                    t5_ld32(taddr + 64u, uv);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    const int kind = R0 < p.dq ? 0 : (R0 < p.dq + p.dkv ? 1 : 2);  // q, k, v
-                    const int head = (kind == 0 ? R0 : (kind == 1 ? R0 - p.dq : R0 - p.dq - p.dkv)) >> 7;
-                    const float sc = kind == 0 ? p.sq : (kind == 1 ? p.sk : p.sv);
-                    const bool live = token < p.ncols;
-                    const int bb = live ? token / p.seq : 0;
-                    const int pos = live ? __ldg(p.past_len + bb) + (token - bb * p.seq) : 0;
-                    const float sxv = live ? __ldg(p.sx + token) : 0.f;
-                    const int32_t xs = live ? __ldg(p.xsum + token) : 0;
-                    const bool rot = kind != 2 && p.rope != nullptr && live && pos < p.max_seq;
-                    const float4* cs4 = reinterpret_cast<const float4*>(p.rope + (size_t)(rot ? pos : 0) * 64 + 32 * pp);
-#pragma unroll
-                    for (int q = 0; q < 32; q += 2) {
-                        float a0 = ((float)((int32_t)gv[q] - xs) * sxv) * sc, a1 = ((float)((int32_t)gv[q + 1] - xs) * sxv) * sc;
-                        float c0 = ((float)((int32_t)uv[q] - xs) * sxv) * sc, c1 = ((float)((int32_t)uv[q + 1] - xs) * sxv) * sc;
-                        if (rot) {
-                            const float4 cs = __ldg(cs4 + (q >> 1));  // (cos, sin) of pairs q and q + 1
-                            const float r0 = a0 * cs.x - c0 * cs.y, r1 = a1 * cs.z - c1 * cs.w;
-                            c0 = c0 * cs.x + a0 * cs.y;
-                            c1 = c1 * cs.z + a1 * cs.w;
-                            a0 = r0;
-                            a1 = r1;
-                        }
-                        gv[q] = __float_as_uint(a0);
-                        gv[q + 1] = __float_as_uint(a1);
-                        uv[q] = __float_as_uint(c0);
-                        uv[q + 1] = __float_as_uint(c1);
-                    }
-                    // destination of token tok_base + tl: its q row, or its position's row of the head's cache
-                    auto dst_of = [&](int tl, int col) -> void* {
-                        const int t2 = tok_base + tl;
-                        if (t2 >= p.ncols) return nullptr;
-                        if (kind == 0) return p.qout + (size_t)t2 * p.dq + (size_t)head * 128 + col;
-                        const int b2 = t2 / p.seq, pos2 = __ldg(p.past_len + b2) + (t2 - b2 * p.seq);
-                        if (pos2 >= p.max_seq) return nullptr;
-                        float* cache = kind == 1 ? p.k_cache : p.v_cache;
-                        return cache + (((size_t)b2 * (p.dkv >> 7) + head) * p.max_seq + pos2) * 128 + col;
-                    };
-                    const uint32_t stage = ring + (uint32_t)warp * T5_XPOSE_BYTES;
-                    t5_store_rows_to(stage, gv, lane, [&](int tl) { return dst_of(tl, 32 * pp); });
-                    t5_store_rows_to(stage, uv, lane, [&](int tl) { return dst_of(tl, 64 + 32 * pp); });
-                }
-            } else if constexpr (GATED) {
-                // lane = token; per item 32 channels: gate accumulators in columns [32 ch, +32), up in [128 + 32 ch, +32)
-#pragma unroll 1
-                for (int item = grp; item < nhalf * (NCH / 2); item += GROUPS) {
-                    const int half = item / (NCH / 2), ch = item - half * (NCH / 2);
-                    const int token = tok0 + half * 128 + wq * 32 + lane;
-                    uint32_t gv[32], uv[32];
-                    const uint32_t taddr = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(half * ROWS + ch * 32);
-                    t5_ld32(taddr, gv);
-                    t5_ld32(taddr + 128u, uv);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    const int c0 = (int)blockIdx.y * 128 + ch * 32;
-                    if (c0 < p.ff) {  // warp-uniform
-                        const int tok_base = tok0 + half * 128 + wq * 32;
-                        const bool live = token < p.ncols;
-                        const float sxv = live ? __ldg(p.sx + token) : 0.f;
-                        const int32_t xs = live ? __ldg(p.xsum + token) : 0;
-                        // the gated values replace the gate accumulators in place (bit patterns of float32)
-#pragma unroll
-                        for (int q = 0; q < 32; ++q) {
-                            const float g = ((float)((int32_t)gv[q] - xs) * sxv) * p.sg, u = ((float)((int32_t)uv[q] - xs) * sxv) * p.su;
-                            float r;
-                            if (p.ffn_act == ROTOR_B200_FFN_RELU2) {
-                                const float a = fmaxf(g, 0.f);
-                                r = a * a * u;
-                            } else {
-                                const float c = fminf(fmaxf(u, -20.f), 20.f);
-                                r = g * (c / (1.f + expf(-c)));
-                            }
-                            gv[q] = __float_as_uint(r);
-                        }
-                        if (c0 + 32 <= p.ff && (p.ff & 3) == 0) {
-                            t5_store_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, gv, p.gated + (size_t)tok_base * p.ff + c0,
-                                          (size_t)p.ff * sizeof(float), tok_base, p.ncols, lane);
-                        } else if (live) {
-                            float* dst = p.gated + (size_t)token * p.ff + c0;
-#pragma unroll
-                            for (int q = 0; q < 32; ++q)
-                                if (c0 + q < p.ff) dst[q] = __uint_as_float(gv[q]);
-                        }
-                    }
-                }
-            } else
 #pragma unroll 1
             for (int item = grp; item < nhalf * NCH; item += GROUPS) {
                 const int half = item / NCH, ch = item - half * NCH;
@@ -478,6 +375,398 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// Products whose 256 x 256 tiles give every pair of SMs work (prompts): a pair of CTAs per tile, tcgen05.mma.cta_group::2
+// (M = 256 tokens, N = 256 weight rows, K = 32).  Each CTA holds 128 tokens and decodes 128 weight rows; the tensor cores of
+// both SMs read both halves of the weights.  A CTA's accumulator is then 128 lanes x 256 columns, so that two fit tensor memory
+// and the read-back of one tile runs beside the MMAs of the next, and a K step of the pair moves through each SM's shared
+// memory 16 KB of tokens and 16 KB of decoded weights for 128 x 256 outputs (a CTA by itself: 32 + 32 KB for twice the
+// outputs, and the read-back outside the K loop).  Persistent: one pair per two SMs walks the tiles.
+// 16384 tokens, us with a CTA per 256 x 256 tile / now: gate/up 2 x 6912 x 2560 523 / 353, o 2560 x 2560 105 / 78, down
+// 2560 x 6912 220 / 171, q/k/v 3840 x 2560 233 / 140; 1500 tokens: gate/up 63 / 45, q/k/v 35 / 29.
+// Per CTA: warps 0-3 decode the even and 4-7 the odd K steps, two 16-row tiles each, 8-15 read back, 16 loads tokens (TMA), 17 issues MMAs (rank 0).
+// Barriers: full (of rank 0: both CTAs' copies and decoder warps), empty (one per CTA, a commit to both), accumulator full (the
+// same) and empty (of rank 0: both CTAs' read-back warps).
+enum { PAIR_SUMS = 0, PAIR_GATED = 1, PAIR_QKV = 2 };
+constexpr int PR_DEC = 8, PR_EPI = 8, PR_THREADS = (PR_DEC + PR_EPI + 2) * 32;
+constexpr int PR_STAGES = 5, PR_HALF = 128 * TILE_K, PR_STAGE = 2 * PR_HALF, PR_AHEAD = 4;  // PR_AHEAD: steps of a decoder warp
+constexpr int PR_SMEM = PR_STAGES * PR_STAGE + PR_EPI * (int)T5_XPOSE_BYTES + 1024;
+
+// An mbarrier of CTA 0 of the pair.
+__device__ __forceinline__ uint32_t pr_lead(uint32_t bar) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(bar));
+    return r;
+}
+__device__ __forceinline__ void pr_arrive(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void pr_commit(uint32_t bar) {  // to the same barrier of both CTAs
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+        : "memory");
+}
+__device__ __forceinline__ void pr_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ Tc5Params p) {
+    extern __shared__ unsigned char t5_raw[];
+    __shared__ __align__(8) unsigned long long s_full[PR_STAGES], s_empty[PR_STAGES], s_accf[2], s_acce[2];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort;
+    const uint32_t ring = (smem_u32(t5_raw) + 1023u) & ~1023u, xpose = ring + PR_STAGES * PR_STAGE;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = blockIdx.x & 1;
+    const int nk = p.nkt, ntiles = p.mt * p.nt, pair0 = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    volatile int* abort_flag = &s_abort;
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < PR_STAGES; ++s) {
+            t5_bar_init(smem_u32(&s_full[s]), PR_DEC + 1);  // half of each CTA's decoders, the copies
+            t5_bar_init(smem_u32(&s_empty[s]), 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            t5_bar_init(smem_u32(&s_accf[s]), 1);
+            t5_bar_init(smem_u32(&s_acce[s]), 2 * PR_EPI);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == PR_DEC + PR_EPI) {  // all columns of both SMs (one CTA per SM)
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    pr_sync();  // both CTAs' barriers are initialised
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+
+    // tiles in blocks of 16 token tiles, token tiles fastest: the pairs of a wave share weight tiles
+    auto place = [&](int t, int& m, int& n) {
+        const int block = t / (16 * p.nt), bm = min(16, p.mt - block * 16), r = t - block * 16 * p.nt;
+        n = r / bm;
+        m = block * 16 + (r - n * bm);
+    };
+
+    if (warp < PR_DEC) {
+        // ---------------- weight decoders: a warp turns row tiles 2 w and 2 w + 1 of this CTA's half of every other K step into
+        // operand bytes (one chain of wait, decode, fence and arrival per two steps and two tiles: with a tile of every step a
+        // warp the 13824 x 2560 product of 16384 tokens took 439 us, so 353)
+        const int g = lane >> 2, t4 = lane & 3, w = warp & 3, odd = warp >> 2;
+        const uint4 none = make_uint4(0x55555555u, 0x55555555u, 0x55555555u, 0x55555555u);  // zero weights
+        auto row_of = [&](int t, int u) -> const uint4* {
+            int m, n;
+            place(t, m, n);
+            int rt = n * 16 + rank * 8 + 2 * w + u;
+            if constexpr (EPI == PAIR_GATED) {  // rank 0: 128 gate rows; rank 1: the same channels of the up matrix
+                const int ch = n * 8 + 2 * w + u, ff_rt = p.ff / TILE_ROWS;
+                rt = ch < ff_rt ? rank * ff_rt + ch : p.nrt;
+            }
+            return rt < p.nrt ? p.tiles + (size_t)rt * nk * 32 + lane : nullptr;
+        };
+        // requested PR_AHEAD of its steps before their decode, across tiles
+        int ft = pair0, fk = 0;
+        const uint4 *fp0 = nullptr, *fp1 = nullptr;
+        auto enter = [&] {
+            if (ft < ntiles) {
+                fp0 = row_of(ft, 0);
+                fp1 = row_of(ft, 1);
+            }
+        };
+        auto skip = [&](int steps) {
+            fk += steps;
+            if (fk < nk) return;
+            do {
+                fk -= nk;
+                ft += pairs;
+            } while (fk >= nk);
+            enter();
+        };
+        auto fetch = [&](uint4 (&dst)[2]) {
+            if (ft >= ntiles) return;
+            dst[0] = fp0 ? ld_stream_v4(fp0 + (size_t)fk * 32) : none;
+            dst[1] = fp1 ? ld_stream_v4(fp1 + (size_t)fk * 32) : none;
+            skip(2);
+        };
+        enter();
+        skip(odd);
+        uint4 wv[PR_AHEAD][2];
+#pragma unroll
+        for (int u = 0; u < PR_AHEAD; ++u) fetch(wv[u]);
+        const int total = pair0 < ntiles ? ((ntiles - pair0 + pairs - 1) / pairs) * nk : 0;
+        int s = odd;
+        uint32_t parity = 1;
+        bool ok = true;
+        for (int it0 = odd; it0 < total && ok; it0 += 2 * PR_AHEAD) {
+#pragma unroll
+            for (int u = 0; u < PR_AHEAD; ++u) {
+                if (it0 + 2 * u >= total) break;
+                ok = t5_wait(smem_u32(&s_empty[s]), parity, abort_flag, p.status, 0x7c000011u);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
+                }
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const uint32_t base = ring + s * PR_STAGE + PR_HALF + (uint32_t)(2 * w + v) * 2048u + (uint32_t)g * 128u;
+                    const uint32_t pw[4] = {wv[u][v].x, wv[u][v].y, wv[u][v].z, wv[u][v].w};
+#pragma unroll
+                    for (int rh = 0; rh < 2; ++rh) {
+                        const uint32_t lo = pw[rh], hi = pw[rh + 2];
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {  // 16-byte chunk 2 t4 + c holds bit pairs 2 c and 2 c + 1
+                            const uint32_t a0 = (lo >> (4 * c)) & 0x03030303u, a1 = (hi >> (4 * c)) & 0x03030303u;
+                            const uint32_t a2 = (lo >> (4 * c + 2)) & 0x03030303u, a3 = (hi >> (4 * c + 2)) & 0x03030303u;
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(base + rh * 1024u + (uint32_t)(((2 * t4 + c) ^ g) << 4)),
+                                         "r"(a0), "r"(a1), "r"(a2), "r"(a3)
+                                         : "memory");
+                        }
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
+                __syncwarp();
+                if (lane == 0) pr_arrive(pr_lead(smem_u32(&s_full[s])));
+                fetch(wv[u]);
+                s += 2;
+                if (s >= PR_STAGES) {
+                    s -= PR_STAGES;
+                    parity ^= 1u;
+                }
+            }
+        }
+    } else if (warp < PR_DEC + PR_EPI) {
+        // ---------------- read-back: lane = token, 32 columns (weight rows) per load; the two warps of a lane quarter alternate
+        const int wq = warp & 3, grp = (warp - PR_DEC) >> 2;
+        const uint32_t stage = xpose + (uint32_t)(warp - PR_DEC) * T5_XPOSE_BYTES;
+        int lt = 0;
+        for (int t = pair0; t < ntiles; t += pairs, ++lt) {
+            int m, n;
+            place(t, m, n);
+            const int buf = lt & 1, tok_base = m * 256 + rank * 128 + wq * 32, token = tok_base + lane;
+            const bool good = t5_wait(smem_u32(&s_accf[buf]), (lt >> 1) & 1, abort_flag, p.status, 0x7c000012u);
+            if (!__all_sync(0xffffffffu, good)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)buf * 256u;
+            const bool live = token < p.ncols;
+            const int32_t xs = live ? __ldg(p.xsum + token) : 0;
+            // the accumulator is free again once every warp has its last columns in registers
+            auto release = [&] {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) pr_arrive(pr_lead(smem_u32(&s_acce[buf])));
+            };
+            if constexpr (EPI == PAIR_QKV) {
+                // per item a head of the tile (0 / 1) and 16 pairs of its rows, 16 pc + i with 64 + 16 pc + i.  They are rotated on
+                // their way out, where four lanes share a token and read its angles as whole sectors (a lane per token read 32
+                // lines an instruction, and the read-back took 17 us a tile)
+                const int bb = live ? token / p.seq : 0;
+                const int pos = live ? __ldg(p.past_len + bb) + (token - bb * p.seq) : 0;
+                const float sxv = live ? __ldg(p.sx + token) : 0.f;
+#pragma unroll 1
+                for (int item = grp; item < 8; item += 2) {
+                    const int hh = item >> 2, pc = item & 3;
+                    const int R0 = n * 256 + hh * 128;  // first row of the head in the stacked matrix
+                    uint32_t gv[32], uv[32];
+                    t5_ld16(acc + (uint32_t)(hh * 128 + pc * 16), gv);
+                    t5_ld16(acc + (uint32_t)(hh * 128 + pc * 16 + 64), uv);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (item + 2 >= 8) release();
+                    if (R0 >= p.out) continue;  // warp-uniform
+                    const int kind = R0 < p.dq ? 0 : (R0 < p.dq + p.dkv ? 1 : 2);  // q, k, v
+                    const int head = (kind == 0 ? R0 : (kind == 1 ? R0 - p.dq : R0 - p.dq - p.dkv)) >> 7;
+                    const float sc = kind == 0 ? p.sq : (kind == 1 ? p.sk : p.sv);
+                    float* cache = kind == 1 ? p.k_cache : p.v_cache;
+#pragma unroll
+                    for (int q = 0; q < 16; q += 4) {
+                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)lane * 144u + 4u * q),
+                                     "f"(((float)((int32_t)gv[q] - xs) * sxv) * sc), "f"(((float)((int32_t)gv[q + 1] - xs) * sxv) * sc),
+                                     "f"(((float)((int32_t)gv[q + 2] - xs) * sxv) * sc), "f"(((float)((int32_t)gv[q + 3] - xs) * sxv) * sc)
+                                     : "memory");
+                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)lane * 144u + 64u + 4u * q),
+                                     "f"(((float)((int32_t)uv[q] - xs) * sxv) * sc), "f"(((float)((int32_t)uv[q + 1] - xs) * sxv) * sc),
+                                     "f"(((float)((int32_t)uv[q + 2] - xs) * sxv) * sc), "f"(((float)((int32_t)uv[q + 3] - xs) * sxv) * sc)
+                                     : "memory");
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int tl = 8 * i + (lane >> 2), at = 16 * pc + 4 * (lane & 3), t2 = tok_base + tl;
+                        const int pos2 = __shfl_sync(0xffffffffu, pos, tl), b2 = __shfl_sync(0xffffffffu, bb, tl);
+                        float4 a, c;
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+                                     : "r"(stage + (uint32_t)tl * 144u + 16u * (lane & 3)));
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(c.x), "=f"(c.y), "=f"(c.z), "=f"(c.w)
+                                     : "r"(stage + (uint32_t)tl * 144u + 64u + 16u * (lane & 3)));
+                        if (t2 >= p.ncols) continue;
+                        if (kind != 2 && p.rope != nullptr && pos2 < p.max_seq) {
+                            const float4* cs4 = reinterpret_cast<const float4*>(p.rope + (size_t)pos2 * 64 + at);
+                            const float4 s0 = __ldg(cs4), s1 = __ldg(cs4 + 1);  // (cos, sin) of four pairs
+                            const float4 r = make_float4(a.x * s0.x - c.x * s0.y, a.y * s0.z - c.y * s0.w, a.z * s1.x - c.z * s1.y,
+                                                         a.w * s1.z - c.w * s1.w);
+                            c = make_float4(c.x * s0.x + a.x * s0.y, c.y * s0.z + a.y * s0.w, c.z * s1.x + a.z * s1.y, c.w * s1.z + a.w * s1.w);
+                            a = r;
+                        }
+                        float* dst;  // the token's q row, or its position's row of the head's cache
+                        if (kind == 0)
+                            dst = p.qout + (size_t)t2 * p.dq + (size_t)head * 128;
+                        else if (pos2 < p.max_seq)
+                            dst = cache + (((size_t)b2 * (p.dkv >> 7) + head) * p.max_seq + pos2) * 128;
+                        else
+                            continue;
+                        *reinterpret_cast<float4*>(dst + at) = a;
+                        *reinterpret_cast<float4*>(dst + 64 + at) = c;
+                    }
+                    __syncwarp();  // the block is rewritten by the next item
+                }
+            } else if constexpr (EPI == PAIR_GATED) {
+                // per item 32 channels: gate sums in columns [32 ch, +32), up in [128 + 32 ch, +32)
+                const float sxv = live ? __ldg(p.sx + token) : 0.f;
+#pragma unroll 1
+                for (int ch = grp; ch < 4; ch += 2) {
+                    uint32_t gv[32], uv[32];
+                    t5_ld32(acc + (uint32_t)(ch * 32), gv);
+                    t5_ld32(acc + (uint32_t)(ch * 32 + 128), uv);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (ch + 2 >= 4) release();
+                    const int c0 = n * 128 + ch * 32;
+                    if (c0 >= p.ff) continue;  // warp-uniform
+                    // the gated values replace the gate sums in place (bit patterns of float32)
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) {
+                        const float g = ((float)((int32_t)gv[q] - xs) * sxv) * p.sg, u = ((float)((int32_t)uv[q] - xs) * sxv) * p.su;
+                        float r;
+                        if (p.ffn_act == ROTOR_B200_FFN_RELU2) {
+                            const float a = fmaxf(g, 0.f);
+                            r = a * a * u;
+                        } else {
+                            const float c = fminf(fmaxf(u, -20.f), 20.f);
+                            r = g * (c / (1.f + expf(-c)));
+                        }
+                        gv[q] = __float_as_uint(r);
+                    }
+                    if (c0 + 32 <= p.ff && (p.ff & 3) == 0) {
+                        t5_store_rows(stage, gv, p.gated + (size_t)tok_base * p.ff + c0, (size_t)p.ff * sizeof(float), tok_base, p.ncols, lane);
+                    } else if (live) {
+                        float* dst = p.gated + (size_t)token * p.ff + c0;
+#pragma unroll
+                        for (int q = 0; q < 32; ++q)
+                            if (c0 + q < p.ff) dst[q] = __uint_as_float(gv[q]);
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int ch = grp; ch < 8; ch += 2) {
+                    uint32_t v[32];
+                    t5_ld32(acc + (uint32_t)(ch * 32), v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (ch + 2 >= 8) release();
+                    const int rbase = n * 256 + ch * 32;
+                    if (rbase >= p.out) continue;  // warp-uniform
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) v[q] -= (uint32_t)xs;
+                    if (rbase + 32 <= p.out && (p.out & 3) == 0) {
+                        t5_store_rows(stage, v, p.acc + (size_t)tok_base * p.out + rbase, (size_t)p.out * sizeof(int32_t), tok_base, p.ncols, lane);
+                    } else if (live) {
+                        int32_t* dst = p.acc + (size_t)token * p.out + rbase;
+#pragma unroll
+                        for (int q = 0; q < 32; ++q)
+                            if (rbase + q < p.out) dst[q] = (int32_t)v[q];
+                    }
+                }
+            }
+        }
+    } else if (warp == PR_DEC + PR_EPI) {
+        // ---------------- token operand by TMA: this CTA's 128 tokens, counted by rank 0's barrier
+        if (elect_lane()) {
+            int s = 0;
+            uint32_t parity = 1;
+            bool ok = true;
+            for (int t = pair0; t < ntiles && ok; t += pairs) {
+                int m, n;
+                place(t, m, n);
+                for (int kt = 0; kt < nk; ++kt) {
+                    ok = t5_wait(smem_u32(&s_empty[s]), parity, abort_flag, p.status, 0x7c000013u);
+                    if (!ok) break;
+                    const uint32_t bar = smem_u32(&s_full[s]);
+                    if (rank == 0) t5_bar_expect(bar, 2 * PR_HALF);
+                    asm volatile(
+                        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+                        "[%0], [%1, {%2, %3}], [%4];" ::"r"(ring + s * PR_STAGE),
+                        "l"(&tmap), "r"(kt * TILE_K), "r"(m * 256 + rank * 128), "r"(pr_lead(bar))
+                        : "memory");
+                    if (++s == PR_STAGES) {
+                        s = 0;
+                        parity ^= 1u;
+                    }
+                }
+            }
+            for (int i = 0; i < PR_STAGES && ok; ++i) {  // the last commits to this CTA's barriers have landed
+                ok = t5_wait(smem_u32(&s_empty[s]), parity, abort_flag, p.status, 0x7c000016u);
+                if (++s == PR_STAGES) {
+                    s = 0;
+                    parity ^= 1u;
+                }
+            }
+        }
+    } else if (rank == 0) {
+        // ---------------- MMA issue for both SMs
+        if (elect_lane()) {
+            // kind::i8, S32 accumulate, signed tokens (A) x unsigned weight codes (B), both K-major, M = 256, N = 256
+            constexpr uint32_t idesc = (2u << 4) | (1u << 7) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
+            int s = 0, lt = 0;
+            uint32_t parity = 0;
+            bool ok = true;
+            for (int t = pair0; t < ntiles && ok; t += pairs, ++lt) {
+                const int buf = lt & 1;
+                ok = t5_wait(smem_u32(&s_acce[buf]), ((lt >> 1) & 1) ^ 1, abort_flag, p.status, 0x7c000014u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int kt = 0; kt < nk; ++kt) {
+                    ok = t5_wait(smem_u32(&s_full[s]), parity, abort_flag, p.status, 0x7c000015u);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t da = t5_desc(ring + s * PR_STAGE), db = t5_desc(ring + s * PR_STAGE + PR_HALF);
+#pragma unroll
+                    for (int k4 = 0; k4 < TILE_K / 32; ++k4)
+                        asm volatile(
+                            "{\n\t"
+                            ".reg .pred p;\n\t"
+                            "setp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t"
+                            "}\n" ::"r"(tmem + (uint32_t)buf * 256u),
+                            "l"(da + 2 * k4), "l"(db + 2 * k4), "r"(idesc), "r"((uint32_t)(kt > 0 || k4 > 0)), "r"(0u)
+                            : "memory");
+                    pr_commit(smem_u32(&s_empty[s]));
+                    if (++s == PR_STAGES) {
+                        s = 0;
+                        parity ^= 1u;
+                    }
+                }
+                if (ok) pr_commit(smem_u32(&s_accf[buf]));
+            }
+        }
+    }
+
+    // ---------------- common exit: nothing of either CTA may still be in flight when one returns
+    __syncwarp();
+    if (*abort_flag && threadIdx.x == 0) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000LL) {
+        }  // about a millisecond for copies already issued to land
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    pr_sync();
+    if (warp == PR_DEC + PR_EPI) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+    }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -502,12 +791,21 @@ int configure_gemm_tcgen05() {
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<256>::SMEM));
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<256, 128>::SMEM));
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<64>::SMEM));
-    RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 T5Cfg<256>::SMEM));
-    RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256, 256, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 T5Cfg<256>::SMEM));
+    RB_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<PAIR_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM));
+    RB_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<PAIR_GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM));
+    RB_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<PAIR_QKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM));
     g_tc5_ready.here() = true;
     return ROTOR_B200_OK;
+}
+
+// The token operand: int8 rows of kpad bytes, boxes of 128 tokens x 128 bytes; rows past the last token read zeros.
+static bool encode_tokens(CUtensorMap* tmap, const void* xq, size_t kpad, int ncols) {
+    const cuuint64_t gdim[2] = {(cuuint64_t)kpad, (cuuint64_t)ncols};
+    const cuuint64_t gstride[1] = {(cuuint64_t)kpad};  // bytes between token rows
+    const cuuint32_t box[2] = {(cuuint32_t)TILE_K, 128u};
+    const cuuint32_t estride[2] = {1u, 1u};
+    return g_encode(tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(xq), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // fewer 256-row tiles than SMs: split the K range so that the grid covers the GPU (a K step of a
@@ -521,6 +819,16 @@ int gemm_tcgen05_splits(size_t out, size_t in, int ncols) {
     if (splits < 2) return 1;
     const int per = (nkt + splits - 1) / splits;
     return (nkt + per - 1) / per;
+}
+
+// n: weight rows (or pairs of gate and up rows, two each) that the tiles of 256 cover.
+template <int EPI>
+static int launch_pair(const CUtensorMap& tmap, Tc5Params& p, int n, cudaStream_t st) {
+    p.mt = (p.ncols + 255) / 256;
+    p.nt = (n + 255) / 256;
+    const int tiles = p.mt * p.nt, pairs = fused_sm_count() / 2;
+    gemm_pair_kernel<EPI><<<2 * (tiles < pairs ? tiles : pairs), PR_THREADS, PR_SMEM, st>>>(tmap, p);
+    return launch_status();
 }
 
 int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
@@ -537,19 +845,12 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
     p.nkt = (int)(kpad_of(in) / TILE_K);
     p.ncols = ncols;
     if (!p.status) return ROTOR_B200_ERR_CUDA;
-    const size_t kpad = kpad_of(in);
     CUtensorMap tmap;
-    const cuuint64_t gdim[2] = {(cuuint64_t)kpad, (cuuint64_t)ncols};
-    const cuuint64_t gstride[1] = {(cuuint64_t)kpad};  // bytes between token rows
-    const cuuint32_t box[2] = {(cuuint32_t)TILE_K, 128u};
-    const cuuint32_t estride[2] = {1u, 1u};
-    if (g_encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)xq, gdim, gstride, box, estride,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return ROTOR_B200_ERR_CUDA;
+    if (!encode_tokens(&tmap, xq, kpad_of(in), ncols)) return ROTOR_B200_ERR_CUDA;
     const int tok_tiles = (ncols + 255) / 256, rows = p.nrt * TILE_ROWS;
     const int sms = fused_sm_count(), tiles256 = tok_tiles * ((rows + 255) / 256);
     int splits = gemm_tcgen05_splits(out, in, ncols);
+    if (ncols > 128 && 2 * tiles256 >= sms) return launch_pair<PAIR_SUMS>(tmap, p, rows, st);
     auto launch256 = [&](dim3 grid) {
         // (64 tokens, 57344 x 8192: 78.3 -> 66.9 us, 8192 x 28672: 44.7 -> 38.7; runs of fewer steps end before the
         // deeper look-ahead is filled and take the variant with less code)
@@ -600,19 +901,9 @@ int launch_gemm_tcgen05_gated(const void* tiles, size_t ff, size_t in, const int
     p.ff = (int)ff;
     p.ffn_act = ffn_act;
     if (!p.status) return ROTOR_B200_ERR_CUDA;
-    const size_t kpad = kpad_of(in);
     CUtensorMap tmap;
-    const cuuint64_t gdim[2] = {(cuuint64_t)kpad, (cuuint64_t)ncols};
-    const cuuint64_t gstride[1] = {(cuuint64_t)kpad};
-    const cuuint32_t box[2] = {(cuuint32_t)TILE_K, 128u};
-    const cuuint32_t estride[2] = {1u, 1u};
-    if (g_encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)xq, gdim, gstride, box, estride,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return ROTOR_B200_ERR_CUDA;
-    dim3 grid((ncols + 255) / 256, (unsigned)((ff + 127) / 128));
-    gemm_tcgen05_kernel<256, 256, true><<<grid, T5Cfg<256>::THREADS, T5Cfg<256>::SMEM, st>>>(tmap, p);
-    return launch_status();
+    if (!encode_tokens(&tmap, xq, kpad_of(in), ncols)) return ROTOR_B200_ERR_CUDA;
+    return launch_pair<PAIR_GATED>(tmap, p, (int)(2 * ((ff + 127) / 128 * 128)), st);
 }
 
 // q/k/v product with dequantisation, rotary and the cache append in its read-back: head_dim 128, one
@@ -650,19 +941,9 @@ int launch_gemm_tcgen05_qkv(const void* tiles, size_t in, const int8_t* xq, cons
     p.sk = f.sk;
     p.sv = f.sv;
     if (!p.status) return ROTOR_B200_ERR_CUDA;
-    const size_t kpad = kpad_of(in);
     CUtensorMap tmap;
-    const cuuint64_t gdim[2] = {(cuuint64_t)kpad, (cuuint64_t)ncols};
-    const cuuint64_t gstride[1] = {(cuuint64_t)kpad};
-    const cuuint32_t box[2] = {(cuuint32_t)TILE_K, 128u};
-    const cuuint32_t estride[2] = {1u, 1u};
-    if (g_encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)xq, gdim, gstride, box, estride,
-                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return ROTOR_B200_ERR_CUDA;
-    dim3 grid((ncols + 255) / 256, (unsigned)((p.nrt * TILE_ROWS + 255) / 256));
-    gemm_tcgen05_kernel<256, 256, false, true><<<grid, T5Cfg<256>::THREADS, T5Cfg<256>::SMEM, st>>>(tmap, p);
-    return launch_status();
+    if (!encode_tokens(&tmap, xq, kpad_of(in), ncols)) return ROTOR_B200_ERR_CUDA;
+    return launch_pair<PAIR_QKV>(tmap, p, p.nrt * TILE_ROWS, st);
 }
 
 }  // namespace rb

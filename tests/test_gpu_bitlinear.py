@@ -101,6 +101,22 @@ def test_many_column_product_bit_exact(ops, abi, shape):
     assert np.array_equal(acc2, want)
 
 
+@pytest.mark.parametrize("shape", [(18939, 100, 129), (9473, 260, 300), (6403, 384, 700), (2560, 6912, 4100), (19000, 1024, 255), (37888, 128, 130)])
+def test_tiles_of_cta_pairs_bit_exact(ops, abi, shape):
+    """Products with a 256 x 256 tile for every pair of SMs: one to 54 K steps a tile (fewer than the decoders look ahead),
+    a second half of a tile without tokens, rows and tokens that fill no tile, several tiles a pair."""
+    import torch
+    out, inn, ncols = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(out + ncols)
+    w = torch.randint(-1, 2, (out, inn), generator=g, device="cuda", dtype=torch.int8)
+    q = torch.zeros((ncols, abi.lib.rotor_b200_in_padded(inn)), device="cuda", dtype=torch.int8)
+    q[:, :inn] = torch.randint(-128, 128, (ncols, inn), generator=g, device="cuda", dtype=torch.int8)
+    acc = ops.bitlinear_acc(ops.int8_to_tiles(w), out, inn, q, q.sum(1, dtype=torch.int32), abi.VARIANT_AUTO)
+    assert torch.equal(acc.double(), q[:, :inn].double() @ w.double().T)
+    abi.device_status()
+
+
 @pytest.mark.parametrize("terms", [1, 2, 3])
 @pytest.mark.parametrize("shape", [(1, 4), (17, 132), (3001, 1924), (2560, 8192), (640, 9220), (8192, 2048)])
 @pytest.mark.parametrize("rows", [1, 2, 4, 5])
