@@ -10,60 +10,52 @@
 // accumulators in tensor memory, every operand split into hi + lo bf16 terms
 // (hi*hi + hi*lo + lo*hi: 16 operand mantissa bits), which holds the 1e-3-of-RMS bound of the
 // float32 reference.
-//   S = Q K^T : A = Q hi / lo from shared memory (staged and split once per CTA), B = K hi / lo
-//               tiles [64 keys][128] by TMA; accumulator 128 lanes x 64 columns, double buffered.
-//   O_j = P V : A = P hi / lo from TENSOR MEMORY (written by the softmax warps over the S buffer
-//               they have just read), B = V^T hi / lo tiles [128][64 keys] by TMA (the split
-//               kernel stores V transposed per key tile so that this operand is K-major too);
-//               accumulator 128 lanes x 128 columns, fresh for every key tile, double buffered.
-// Warps 0-7: two threads per query row (warps 0-3 take the first 32 keys of a tile and output
-// columns 0-63, warps 4-7 the other halves; a warp reaches the tensor-memory lanes of its quarter
-// warp % 4) -- row maximum (halves exchanged through shared memory), exponentials (base 2, log2 e
-// folded into the scale of Q), split of P, and the running output O = O * alpha + O_j in
-// registers.  Two warps per scheduler hide each other's latencies; one row per thread left the
-// tensor pipe waiting on a single dependent instruction stream.  The output update of tile j runs
-// after the softmax of tile j + 1, so that P V of tile j overlaps it.
+//   S = Q K^T : A = Q hi / lo from TENSOR MEMORY (scaled, split and written once per CTA), B = K hi / lo tiles
+//               [64 keys][128] by TMA; accumulator 128 lanes x 64 columns.
+//   O += P V  : A = P hi / lo from tensor memory (written by the softmax warps over the S buffer they have just
+//               read), B = V^T hi / lo tiles [128][64 keys] by TMA (the split kernel stores V transposed per key
+//               tile so that this operand is K-major too); accumulator 128 lanes x 128 columns.
+// Two groups of four warps, a thread per query row: group 0 takes the even key tiles, group 1 the odd ones, each with
+// an S buffer, a reference maximum, a sum and an accumulator of its own, so that one group's softmax runs while the tensor
+// pipe works for the other and no barrier joins them before the end, where a row's two results are weighed against each
+// other.  The accumulator stays in tensor memory: it is rescaled only when a tile's maximum passes the reference by more
+// than 2^8 (weights up to 2^8 lose nothing in float32), and then the tile's S being complete means that the products
+// before it are too.  With the shared-memory Q of before a 64-column S product read more shared memory (6 KB per
+// instruction of 32 clocks) than its port gives; all columns of tensor memory are used now (S 2 x 64, O 2 x 128, Q 2 x 64).
+// Persistent: one CTA per SM walks the query tiles, longest first, back and forth over the CTAs so that their sums agree.  The
+// next tile's Q arrives while the present one is worked on; when its products are done the Q goes to tensor memory first, so that
+// the next scores run beside the present tile's outputs (a CTA per tile spent 16 us before and behind its first key tile).
+// 2B shape, 8 x 2048 causal, a layer: 692 us with one stream of eight warps that met at two barriers a tile and added each
+// product to registers, 599 as above with a CTA per tile, 443 now.
 // Warps 8 and 9: TMA producers of the K and the V^T tiles -- separate two-deep rings, because a K
-// tile is free again as soon as its S product has run (one tile ahead of the softmax) while a V^T
-// tile stays until P V; with one ring the next K load would wait for P V and the tensor pipe for
-// that load.  Warp 10: MMA issue, one key tile ahead with S.
+// tile is free again as soon as its S product has run, while a V^T tile stays until P V.  Warp 10: MMA issue.  Warp 11: Q rows.
 // Every wait is bounded; a wait that runs out records a code in the library status word, the CTA
 // stops issuing work, frees its tensor memory and returns.  No multicast, this GPU's memory only.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "model.cuh"
-
-RB_TRACE_DEFINE(rotor_b200_trace_read_attn5)
+#include "tc5.cuh"
 
 namespace rb {
 
-// Phase timing of the softmax loop (compiled in with -DRB_TRACE): thread 0 of CTA (0, 0, 0) adds up
-// the time between the marks of every key tile and commits the sums once.
-#ifdef RB_TRACE
-#define A5_MARK(i)                                                                     \
-    do {                                                                               \
-        if (a5_traced) {                                                               \
-            const unsigned long long now_ = gtime();                                   \
-            tr.t[i] += now_ - a5_last;                                                 \
-            a5_last = now_;                                                            \
-        }                                                                              \
-    } while (0)
-#else
-#define A5_MARK(i) do {} while (0)
-#endif
-
 constexpr int A5_BM = 128, A5_BN = 64, A5_D = 128;
-constexpr int A5_THREADS = 352;  // 8 softmax / output warps, two TMA warps, MMA warp
+constexpr int A5_THREADS = 384;  // 8 softmax / output warps, two TMA warps, MMA warp, Q warp
 constexpr int A5_SOFT = 256;     // threads of the softmax warps
-constexpr int A5_Q_BYTES = 4 * 16384;     // Q hi panel 0, 1; Q lo panel 0, 1 (128 rows x 128 bytes each)
+constexpr int A5_Q_ROW = 132;             // floats per staged query row (padding: rows start in different banks)
+constexpr int A5_Q_BYTES = A5_BM * A5_Q_ROW * 4;
 constexpr int A5_K_BYTES = 32768;         // one K tile: hi panel 0, 1; lo panel 0, 1 (64 rows x 128 bytes each)
 constexpr int A5_V_BYTES = 32768;         // one V^T tile: hi, lo (128 rows x 128 bytes each)
 constexpr int A5_STAGES = 2;              // depth of the K ring and of the V^T ring
-constexpr int A5_SMEM = A5_Q_BYTES + A5_STAGES * (A5_K_BYTES + A5_V_BYTES) + 1024;
-constexpr int A5_TMEM_COLS = 512;         // S0 [0,64)  S1 [64,128)  O_j even [128,256)  O_j odd [256,384)
+constexpr int A5_OUT_ROW = 80;            // bytes per staged output row of 16 columns
+constexpr int A5_OUT_BYTES = 8 * 32 * A5_OUT_ROW;
+constexpr int A5_SMEM = A5_Q_BYTES + A5_OUT_BYTES + A5_STAGES * (A5_K_BYTES + A5_V_BYTES) + 1024;
+constexpr int A5_TMEM_COLS = 512;         // S0 [0,64)  S1 [64,128)  O0 [128,256)  O1 [256,384)  Q hi [384,448)  Q lo [448,512)
+constexpr uint32_t A5_O = 128, A5_QT = 384;
+constexpr float A5_SLACK = 8.f;           // log2 of the largest weight before the reference maximum moves
 constexpr long long A5_SPIN_CYCLES = 400000000LL;  // about 0.2 s
 
 struct A5Params {
@@ -73,6 +65,7 @@ struct A5Params {
     unsigned* status;
     int n_heads, n_kv_heads, seq, max_seq, causal;
     int split_seq;         // rows per (sequence, KV head) in the K planes (max_seq rounded up to 64)
+    int batch, nqt;        // sequences, query tiles of each (sequence, KV head)
 };
 
 __device__ __forceinline__ uint32_t a5_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -105,17 +98,6 @@ __device__ __forceinline__ uint64_t a5_desc(uint32_t smem_addr) {
 }
 
 // ACC == 0: the accumulator is overwritten (first MMA of a tile), 1: accumulated into.
-template <int ACC>
-__device__ __forceinline__ void a5_mma_ss(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t"
-        "}\n" ::"r"(d_tmem),
-        "l"(da), "l"(db), "r"(idesc), "n"(ACC), "r"(0u)
-        : "memory");
-}
 template <int ACC>
 __device__ __forceinline__ void a5_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc) {
     asm volatile(
@@ -233,40 +215,57 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                        const __grid_constant__ A5Params p) {
     extern __shared__ unsigned char a5_raw[];
     __shared__ __align__(8) unsigned long long s_kfull[A5_STAGES], s_kempty[A5_STAGES], s_vfull[A5_STAGES],
-        s_vempty[A5_STAGES], s_sfull[2], s_pfull[2], s_ofull[2], s_oempty[2], s_qready;
+        s_vempty[A5_STAGES], s_sfull[2], s_pfull[2], s_ofull, s_qready, s_qfull, s_qempty, s_oread;
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
-    __shared__ float s_xch[2][A5_BM];  // row maxima / sums exchanged between the two threads of a row
-    __shared__ int s_go;               // the softmax warps' common decision to go on (taken between two barriers)
-    const uint32_t base = (a5_smem(a5_raw) + 1023u) & ~1023u;
-    const uint32_t q_hi = base, q_lo = base + 32768, kring = base + A5_Q_BYTES, vring = kring + A5_STAGES * A5_K_BYTES;
+    __shared__ float s_m[2][2][A5_BM], s_l[2][2][A5_BM];  // by tile parity: each group's reference maximum and sum of a row
+    const uint32_t kring = (a5_smem(a5_raw) + 1023u) & ~1023u, vring = kring + A5_STAGES * A5_K_BYTES;
+    const uint32_t qstage = vring + A5_STAGES * A5_V_BYTES, ostage = qstage + A5_Q_BYTES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int G = p.n_heads / p.n_kv_heads, QT = A5_BM / G;
-    const int qt = gridDim.x - 1 - blockIdx.x;  // late query tiles see the most keys: start them first
-    const int hk = blockIdx.y, b = blockIdx.z;
-    const int s0 = qt * QT;
-    const int past = p.past_len[b];
+    const int G = p.n_heads / p.n_kv_heads, lg = 31 - __clz(G), QT = A5_BM >> lg;  // (G divides 128)
+    const int items = p.nqt * p.n_kv_heads * p.batch;
     volatile int* abort_flag = &s_abort;
 
-    int s_last = s0 + QT - 1;
-    if (s_last > p.seq - 1) s_last = p.seq - 1;
-    int t_all = p.causal ? past + s_last + 1 : past + p.seq;
-    if (t_all > p.max_seq) t_all = p.max_seq;
-    const int ntiles = (t_all + A5_BN - 1) / A5_BN;
+    // The k-th query tile of this CTA; n: its key tiles (0: there is none).
+    struct Item {
+        int s0, hk, b, past, last, t_all, n;
+    };
+    auto item = [&](int k) {
+        Item o = {};
+        const int i = k * (int)gridDim.x + ((k & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+        if (i >= items) return o;
+        const int per = p.n_kv_heads * p.batch, qt = p.nqt - 1 - i / per, e = i % per;
+        o.hk = e % p.n_kv_heads;
+        o.b = e / p.n_kv_heads;
+        o.s0 = qt * QT;
+        o.past = __ldg(p.past_len + o.b);
+        o.last = min(o.s0 + QT, p.seq) - 1;
+        o.t_all = min(o.past + (p.causal ? o.last + 1 : p.seq), p.max_seq);
+        o.n = (o.t_all + A5_BN - 1) / A5_BN;
+        return o;
+    };
+    const int rounds = (items + (int)gridDim.x - 1) / (int)gridDim.x;  // (the last may hold no tile for this CTA)
 
     if (threadIdx.x == 0) {
         s_abort = 0;
+        auto init = [](unsigned long long* bar, int count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(bar)), "r"(count));
+        };
         for (int s = 0; s < A5_STAGES; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_kfull[s])), "r"(1));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_kempty[s])), "r"(1));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_vfull[s])), "r"(1));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_vempty[s])), "r"(1));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_sfull[s])), "r"(1));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_pfull[s])), "r"(A5_SOFT));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_ofull[s])), "r"(1));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_oempty[s])), "r"(A5_SOFT));
+            init(&s_kfull[s], 1);
+            init(&s_kempty[s], 1);
+            init(&s_vfull[s], 1);
+            init(&s_vempty[s], 1);
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(&s_qready)), "r"(A5_SOFT));
+        for (int s = 0; s < 2; ++s) {
+            init(&s_sfull[s], 1);
+            init(&s_pfull[s], 4);   // one arrival per warp of the group
+        }
+        init(&s_ofull, 1);
+        init(&s_qready, 8);
+        init(&s_qfull, 1);
+        init(&s_qempty, 8);
+        init(&s_oread, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 8) {
@@ -279,241 +278,224 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
 
-#ifdef RB_TRACE
-    TraceRec tr2 = {};
-    RB_STAMP(tr2, 0);
-#endif
     if (warp < 8) {
-        // ---------------- Q tile: scaled, split into hi / lo bf16, K-major panels of 64 columns, 128-byte swizzle
-        {
-            const float scale = 1.4426950408889634f / sqrtf((float)A5_D);  // scores come out in units of log2: p = 2^(s - m)
-            // all sixteen loads of a thread are issued before the first conversion (one round trip to memory
-            // instead of sixteen: the MMA warp waits for this tile before it can start)
-            constexpr int QN = A5_BM * (A5_D / 4) / A5_SOFT;
-            float4 qv[QN];
-#pragma unroll
-            for (int u = 0; u < QN; ++u) {
-                const int idx = threadIdx.x + u * A5_SOFT;
-                const int r = idx / (A5_D / 4), c4 = idx - r * (A5_D / 4);
-                const int s = s0 + r / G, gi = r - (r / G) * G;
-                qv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (s < p.seq)
-                    qv[u] = __ldg(reinterpret_cast<const float4*>(p.q + ((size_t)b * p.seq + s) * p.n_heads * A5_D +
-                                                                  (size_t)(hk * G + gi) * A5_D + 4 * c4));
-            }
-#ifdef RB_TRACE
-#pragma unroll
-            for (int u = 0; u < QN; ++u) asm volatile("" ::"f"(qv[u].w));
-            RB_STAMP(tr2, 4);
-#endif
-#pragma unroll
-            for (int u = 0; u < QN; ++u) {
-                const int idx = threadIdx.x + u * A5_SOFT;
-                const int r = idx / (A5_D / 4), c4 = idx - r * (A5_D / 4);
-                const float4 v = qv[u];
-                uint32_t h0, l0, h1, l1;
-                a5_split2(v.x * scale, v.y * scale, h0, l0);
-                a5_split2(v.z * scale, v.w * scale, h1, l1);
-                // column 4 c4: panel (4 c4) / 64, byte (4 c4 % 64) * 2 of the 128-byte row: chunk c4 / 2 % 8, half c4 & 1
-                const int panel = c4 >> 4, chunk = (c4 >> 1) & 7;
-                const uint32_t off = (uint32_t)panel * 16384u + (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u +
-                                     (uint32_t)((chunk ^ (r & 7)) << 4) + (uint32_t)(c4 & 1) * 8u;
-                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(q_hi + off), "r"(h0), "r"(h1) : "memory");
-                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(q_lo + off), "r"(l0), "r"(l1) : "memory");
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_qready)) : "memory");
-        }
-#ifdef RB_TRACE
-        RB_STAMP(tr2, 1);
-#endif
-        // ---------------- softmax and output: this thread owns keys [32 half, 32 half + 32) of a tile and output
-        // columns [64 half, 64 half + 64) of query row r
         const int half = warp >> 2, wq = warp & 3;
-        const int r = wq * 32 + lane;
-        const int srow = s0 + r / G, gi = r - (r / G) * G;
-        int lim = p.causal ? past + (srow < p.seq ? srow : s_last) + 1 : past + p.seq;
-        if (lim > t_all) lim = t_all;
+        const int r = wq * 32 + lane;  // this thread's query row
         const uint32_t lane_base = tmem + ((uint32_t)(wq * 32) << 16);
-        float m_run = -INFINITY, l_run = 0.f, alpha_prev = 1.f;
-        float o[A5_D / 2];
-#pragma unroll
-        for (int i = 0; i < A5_D / 2; ++i) o[i] = 0.f;
+        const uint32_t sbuf = lane_base + 64u * half, obuf = lane_base + A5_O + 128u * half;
+        const uint32_t blk = ostage + (uint32_t)warp * (32u * A5_OUT_ROW);
         bool ok = true;
-#ifdef RB_TRACE
-        TraceRec tr = {};
-        const bool a5_traced = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0;
-        unsigned long long a5_last = gtime();
-#endif
-        // O = O * alpha + P V of key tile j (its accumulator buffer j & 1), this thread's 64 columns
-        auto accumulate = [&](int j, float alpha) {
-            bool good = a5_wait(a5_smem(&s_ofull[j & 1]), (uint32_t)(j >> 1) & 1u, abort_flag, p.status, 0x7b000002u);
-            if (!__all_sync(0xffffffffu, good)) return false;
-            A5_MARK(5);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t ov0[32], ov1[32];
-            const uint32_t ob = lane_base + 128u + (uint32_t)(j & 1) * 128u + (uint32_t)half * 64u;
-            a5_ld32(ob, ov0);
-            a5_ld32(ob + 32u, ov1);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        int tiles = 0;          // of this group, over all query tiles: phases of its barriers
+        Item prev = {};         // the tile whose products are done and whose outputs are still in tensor memory
+        float w0 = 0.f, w1 = 0.f;
+        // (after a failed wait every further one returns at once; the warps still meet at each barrier)
+        for (int k = 0; k <= rounds; ++k) {
+            const Item it = k < rounds ? item(k) : Item{};
+            if (it.n) {
+                // ---------------- Q: rows out of shared memory, scaled and split into tensor memory
+                const float scale = 1.4426950408889634f / sqrtf((float)A5_D);  // scores come out in units of log2: p = 2^(s - m)
+                ok = ok && a5_wait(a5_smem(&s_qfull), (uint32_t)k & 1u, abort_flag, p.status, 0x7b00000bu);
+                uint32_t qh[32], ql[32];  // columns [64 half, +64) of the row
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                o[i] = o[i] * alpha + __uint_as_float(ov0[i]);
-                o[32 + i] = o[32 + i] * alpha + __uint_as_float(ov1[i]);
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_oempty[j & 1])) : "memory");
-            A5_MARK(6);
-            return true;
-        };
-        // (the eight warps leave this loop together: whether to go on is decided by one thread between the
-        // two barriers of an iteration, so that no warp is left alone at a barrier after a failed wait)
-        for (int j = 0; j < ntiles; ++j) {
-            const uint32_t sbuf = lane_base + (uint32_t)(j & 1) * 64u;
-            ok = ok && a5_wait(a5_smem(&s_sfull[j & 1]), (uint32_t)(j >> 1) & 1u, abort_flag, p.status, 0x7b000001u);
-            ok = __all_sync(0xffffffffu, ok);
-            A5_MARK(0);
-            uint32_t sa[32];
-            float tmax = -INFINITY;
-            if (ok) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                a5_ld32(sbuf + (uint32_t)half * 32u, sa);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const int kb = j * A5_BN + half * 32;
-                if (kb + 32 > lim) {  // only the last tiles of a row need the mask
-#pragma unroll
-                    for (int c = 0; c < 32; ++c)
-                        if (kb + c >= lim) sa[c] = 0xff800000u;  // -inf
+                for (int i = 0; i < 16; ++i) {
+                    float4 v;
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                                 : "r"(qstage + (uint32_t)(r * A5_Q_ROW + 64 * half + 4 * i) * 4u));
+                    a5_split2(v.x * scale, v.y * scale, qh[2 * i], ql[2 * i]);
+                    a5_split2(v.z * scale, v.w * scale, qh[2 * i + 1], ql[2 * i + 1]);
                 }
-#pragma unroll
-                for (int c = 0; c < 32; ++c) tmax = fmaxf(tmax, __uint_as_float(sa[c]));
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_qempty)) : "memory");
+                a5_st32(lane_base + A5_QT + 32u * half, qh);
+                a5_st32(lane_base + A5_QT + 64u + 32u * half, ql);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_qready)) : "memory");
             }
-            // the two threads of a row exchange their maxima; past this barrier both have finished reading
-            // the S buffer, which the P stores below overwrite (every softmax warp takes part, also after a
-            // failed wait, so that the barrier count stays whole)
-            A5_MARK(1);
-            s_xch[half][r] = tmax;
+            if (prev.n && __all_sync(0xffffffffu, ok)) {
+                // ---------------- outputs of the tile before, columns [64 half, +64) of both accumulators.  A lane holds
+                // consecutive outputs of ONE row, so a 16-byte store instruction of the warp would touch 32 different lines:
+                // the rows cross a per-warp block and leave as 64-byte pieces, eight rows per instruction.
+#pragma unroll 1
+                for (uint32_t c = 0; c < 64u; c += 16u) {
+                    uint32_t o0[32], o1[32];
+                    t5_ld16(lane_base + A5_O + 64u * half + c, o0);
+                    if (prev.n > 1) t5_ld16(lane_base + A5_O + 128u + 64u * half + c, o1);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float o[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        o[i] = __uint_as_float(o0[i]) * w0;
+                        if (prev.n > 1) o[i] += __uint_as_float(o1[i]) * w1;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4)
+                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(blk + (uint32_t)lane * A5_OUT_ROW + 4u * i),
+                                     "f"(o[i]), "f"(o[i + 1]), "f"(o[i + 2]), "f"(o[i + 3])
+                                     : "memory");
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int rr = 8 * i + (lane >> 2), chunk = lane & 3;
+                        float4 w;
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(w.x), "=f"(w.y), "=f"(w.z), "=f"(w.w)
+                                     : "r"(blk + (uint32_t)rr * A5_OUT_ROW + 16u * chunk));
+                        const int r2 = wq * 32 + rr, srow = prev.s0 + (r2 >> lg), gi = r2 & (G - 1);
+                        if (srow < p.seq)
+                            *reinterpret_cast<float4*>(p.out + ((size_t)prev.b * p.seq + srow) * p.n_heads * A5_D +
+                                                       (size_t)(prev.hk * G + gi) * A5_D + half * 64 + c + 4 * chunk) = w;
+                    }
+                    __syncwarp();
+                }
+                // read by every warp before the next tile's first product: the groups read both accumulators
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) t5_bar_arrive(a5_smem(&s_oread));
+            }
+            prev = it;
+            if (!it.n) continue;
+            // ---------------- softmax of this group's key tiles
+            const int srow = it.s0 + (r >> lg);
+            int lim = p.causal ? it.past + (srow < p.seq ? srow : it.last) + 1 : it.past + p.seq;
+            if (lim > it.t_all) lim = it.t_all;
+            float m_ref = -INFINITY, l_run = 0.f;
+            for (int j = half; j < it.n; j += 2, ++tiles) {
+                ok = ok && a5_wait(a5_smem(&s_sfull[half]), (uint32_t)tiles & 1u, abort_flag, p.status, 0x7b000001u);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t sa[2][32];
+                a5_ld32(sbuf, sa[0]);
+                a5_ld32(sbuf + 32u, sa[1]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const int kb = j * A5_BN;
+                if (kb + A5_BN > lim) {  // only the last tiles of a row need the mask
+#pragma unroll
+                    for (int c = 0; c < 64; ++c)
+                        if (kb + c >= lim) sa[c >> 5][c & 31] = 0xff800000u;  // -inf
+                }
+                float t0 = -INFINITY, t1 = t0;
+#pragma unroll
+                for (int c = 0; c < 32; c += 2) {
+                    t0 = fmaxf(t0, fmaxf(__uint_as_float(sa[0][c]), __uint_as_float(sa[0][c + 1])));
+                    t1 = fmaxf(t1, fmaxf(__uint_as_float(sa[1][c]), __uint_as_float(sa[1][c + 1])));
+                }
+                const float tmax = fmaxf(t0, t1);
+                if (__any_sync(0xffffffffu, tmax > m_ref + A5_SLACK)) {  // the first tile, then rarely
+                    const float m_new = fmaxf(m_ref, tmax), alpha = m_ref == -INFINITY ? 0.f : a5_exp2(m_ref - m_new);
+                    m_ref = m_new;
+                    l_run *= alpha;
+                    if (j >= 2) {
+#pragma unroll 1
+                        for (uint32_t c = 0; c < 128u; c += 32u) {
+                            uint32_t ov[32];
+                            a5_ld32(obuf + c, ov);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+                            a5_st32(obuf + c, ov);
+                        }
+                    }
+                }
+                const float m_use = m_ref == -INFINITY ? 0.f : m_ref;  // (no visible key yet: every weight is 2^-inf)
+                float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t ph[16], pl[16];
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        const float e0 = a5_exp2(__uint_as_float(sa[h][2 * c]) - m_use), e1 = a5_exp2(__uint_as_float(sa[h][2 * c + 1]) - m_use);
+                        sum0 += e0;
+                        sum1 += e1;
+                        a5_split2(e0, e1, ph[c], pl[c]);  // keys 32 h + 2 c, + 1 -> column 16 h + c
+                    }
+                    a5_st16(sbuf + 16u * h, ph);        // P hi: 64 bf16 in columns [0, 32) of the S buffer
+                    a5_st16(sbuf + 32u + 16u * h, pl);  // P lo: columns [32, 64)
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_pfull[half])) : "memory");
+                l_run += sum0 + sum1;
+            }
+            // ---------------- the groups' results of a row, weighed against each other
+            float(*sm)[A5_BM] = s_m[k & 1], (*sl)[A5_BM] = s_l[k & 1];
+            sm[half][r] = m_ref;
+            sl[half][r] = l_run;
             asm volatile("bar.sync 1, %0;" ::"n"(A5_SOFT) : "memory");
-            tmax = fmaxf(tmax, s_xch[half ^ 1][r]);
-            if (threadIdx.x == 0) s_go = !*abort_flag;  // every failed wait of this iteration set the flag before the barrier
-            asm volatile("bar.sync 1, %0;" ::"n"(A5_SOFT) : "memory");  // the exchange slots are free again
-            if (!s_go) {
-                ok = false;
-                break;
-            }
-            A5_MARK(2);
-            const float m_new = fmaxf(m_run, tmax);  // finite from the first tile on: key 0 is visible to every row
-            const float alpha = a5_exp2(m_run - m_new);
-            float sum = 0.f;
-            uint32_t ph[16], pl[16];
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                const float e0 = a5_exp2(__uint_as_float(sa[2 * c]) - m_new), e1 = a5_exp2(__uint_as_float(sa[2 * c + 1]) - m_new);
-                sum += e0 + e1;
-                a5_split2(e0, e1, ph[c], pl[c]);  // keys 32 half + 2 c, + 1 -> column 16 half + c
-            }
-            A5_MARK(3);
-            a5_st16(sbuf + (uint32_t)half * 16u, ph);        // P hi: 64 bf16 in columns [0, 32) of the S buffer
-            a5_st16(sbuf + 32u + (uint32_t)half * 16u, pl);  // P lo: columns [32, 64)
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_pfull[j & 1])) : "memory");
-            l_run = l_run * alpha + sum;
-            m_run = m_new;
-            A5_MARK(4);
-            // the previous tile's P V has been running meanwhile: fold it in now
-            if (j > 0) ok = accumulate(j - 1, alpha_prev);
-            alpha_prev = alpha;
-        }
-        if (ok && ntiles > 0) ok = accumulate(ntiles - 1, alpha_prev);
-#ifdef RB_TRACE
-        if (a5_traced) {
-            tr.t[7] = (unsigned long long)ntiles;
-            RB_TRACE_COMMIT(tr, 500);
-        }
-        RB_STAMP(tr2, 2);
-#endif
-        // the row's sum is the sum of its two halves (same running maximum in both)
-        s_xch[half][r] = l_run;
-        asm volatile("bar.sync 1, %0;" ::"n"(A5_SOFT) : "memory");
-        l_run += s_xch[half ^ 1][r];
-        if (__all_sync(0xffffffffu, ok)) {
-            // A lane holds 64 consecutive outputs of ONE row, so a 16-byte store instruction of the warp would
-            // touch 32 different lines.  The rows cross a per-warp block of the K ring (idle: every MMA has
-            // completed) and leave as 256-byte pieces, two rows per instruction.
-            const float inv = 1.0f / l_run;
-            const uint32_t blk = kring + (uint32_t)warp * (32u * 272u);
-#pragma unroll
-            for (int i = 0; i < A5_D / 2; i += 4)
-                asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(blk + (uint32_t)lane * 272u + 4u * i),
-                             "f"(o[i] * inv), "f"(o[i + 1] * inv), "f"(o[i + 2] * inv), "f"(o[i + 3] * inv)
-                             : "memory");
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const int rr = 2 * k + (lane >> 4), chunk = lane & 15;
-                float4 w;
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                             : "=f"(w.x), "=f"(w.y), "=f"(w.z), "=f"(w.w)
-                             : "r"(blk + (uint32_t)rr * 272u + 16u * chunk));
-                const int r2 = wq * 32 + rr, srow2 = s0 + r2 / G, gi2 = r2 - (r2 / G) * G;
-                if (srow2 < p.seq)
-                    *reinterpret_cast<float4*>(p.out + ((size_t)b * p.seq + srow2) * p.n_heads * A5_D +
-                                               (size_t)(hk * G + gi2) * A5_D + half * 64 + 4 * chunk) = w;
-            }
-        } else if (ok && srow < p.seq) {
-            const float inv = 1.0f / l_run;
-            float* op = p.out + ((size_t)b * p.seq + srow) * p.n_heads * A5_D + (size_t)(hk * G + gi) * A5_D + half * 64;
-#pragma unroll
-            for (int i = 0; i < A5_D / 2; i += 4)
-                *reinterpret_cast<float4*>(op + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
+            const float m0 = sm[0][r], m1 = sm[1][r], M = fmaxf(m0, m1);
+            w0 = m0 == -INFINITY ? 0.f : a5_exp2(m0 - M);
+            w1 = m1 == -INFINITY ? 0.f : a5_exp2(m1 - M);
+            const float inv = 1.0f / (sl[0][r] * w0 + sl[1][r] * w1);
+            w0 *= inv;
+            w1 *= inv;
+            ok = ok && a5_wait(a5_smem(&s_ofull), (uint32_t)k & 1u, abort_flag, p.status, 0x7b000002u);
+            ok = __all_sync(0xffffffffu, ok);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
     } else if (warp == 8) {
         // ---------------- K tiles by TMA
         if (elect_lane()) {
-            const int krow0 = ((b * p.n_kv_heads + hk) * p.split_seq);
-            for (int j = 0; j < ntiles; ++j) {
-                const int s = j & 1;
-                if (!a5_wait(a5_smem(&s_kempty[s]), ((uint32_t)(j >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000003u)) break;
-                const uint32_t bar = a5_smem(&s_kfull[s]);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(A5_K_BYTES) : "memory");
-                const uint32_t st = kring + (uint32_t)s * A5_K_BYTES;
-                const int krow = krow0 + j * A5_BN;
+            int t = 0;
+            bool ok = true;
+            for (int k = 0; k < rounds && ok; ++k) {
+                const Item it = item(k);
+                const int krow0 = (it.b * p.n_kv_heads + it.hk) * p.split_seq;
+                for (int j = 0; j < it.n; ++j, ++t) {
+                    const int s = t & 1;
+                    ok = a5_wait(a5_smem(&s_kempty[s]), ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000003u);
+                    if (!ok) break;
+                    const uint32_t bar = a5_smem(&s_kfull[s]), st = kring + (uint32_t)s * A5_K_BYTES;
+                    t5_bar_expect(bar, A5_K_BYTES);
 #pragma unroll
-                for (int pn = 0; pn < 2; ++pn) {
-                    asm volatile(
-                        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                            st + (uint32_t)pn * 8192u),
-                        "l"(&tm_kh), "r"(pn * 64), "r"(krow), "r"(bar)
-                        : "memory");
-                    asm volatile(
-                        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                            st + 16384u + (uint32_t)pn * 8192u),
-                        "l"(&tm_kl), "r"(pn * 64), "r"(krow), "r"(bar)
-                        : "memory");
+                    for (int pn = 0; pn < 2; ++pn) {
+                        t5_tma_2d(st + (uint32_t)pn * 8192u, &tm_kh, pn * 64, krow0 + j * A5_BN, bar);
+                        t5_tma_2d(st + 16384u + (uint32_t)pn * 8192u, &tm_kl, pn * 64, krow0 + j * A5_BN, bar);
+                    }
                 }
             }
         }
     } else if (warp == 9) {
         // ---------------- V^T tiles by TMA
         if (elect_lane()) {
-            const int vrow0 = ((b * p.n_kv_heads + hk) * (p.split_seq / A5_BN)) * A5_D;
-            for (int j = 0; j < ntiles; ++j) {
-                const int s = j & 1;
-                if (!a5_wait(a5_smem(&s_vempty[s]), ((uint32_t)(j >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000009u)) break;
-                const uint32_t bar = a5_smem(&s_vfull[s]);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(A5_V_BYTES) : "memory");
-                const uint32_t st = vring + (uint32_t)s * A5_V_BYTES;
-                const int vrow = vrow0 + j * A5_D;
-                asm volatile(
-                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(st),
-                    "l"(&tm_vh), "r"(0), "r"(vrow), "r"(bar)
-                    : "memory");
-                asm volatile(
-                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                        st + 16384u),
-                    "l"(&tm_vl), "r"(0), "r"(vrow), "r"(bar)
-                    : "memory");
+            int t = 0;
+            bool ok = true;
+            for (int k = 0; k < rounds && ok; ++k) {
+                const Item it = item(k);
+                const int vrow0 = (it.b * p.n_kv_heads + it.hk) * (p.split_seq / A5_BN) * A5_D;
+                for (int j = 0; j < it.n; ++j, ++t) {
+                    const int s = t & 1;
+                    ok = a5_wait(a5_smem(&s_vempty[s]), ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000009u);
+                    if (!ok) break;
+                    const uint32_t bar = a5_smem(&s_vfull[s]), st = vring + (uint32_t)s * A5_V_BYTES;
+                    t5_bar_expect(bar, A5_V_BYTES);
+                    t5_tma_2d(st, &tm_vh, 0, vrow0 + j * A5_D, bar);
+                    t5_tma_2d(st + 16384u, &tm_vl, 0, vrow0 + j * A5_D, bar);
+                }
+            }
+        }
+    } else if (warp == 11) {
+        // ---------------- Q rows of the next tile (rows past the sequence keep what lies there: nobody stores their outputs)
+        bool ok = true;
+        for (int k = 0; k < rounds && ok; ++k) {
+            const Item it = item(k);
+            if (!it.n) break;
+            ok = a5_wait(a5_smem(&s_qempty), ((uint32_t)k & 1u) ^ 1u, abort_flag, p.status, 0x7b00000cu);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const uint32_t bar = a5_smem(&s_qfull);
+            const int live = (it.last - it.s0 + 1) << lg;
+            if (lane == 0) t5_bar_expect(bar, (uint32_t)live * (A5_D * 4));
+            __syncwarp();
+            for (int rr = lane; rr < live; rr += 32) {
+                const float* src = p.q + ((size_t)it.b * p.seq + it.s0 + (rr >> lg)) * p.n_heads * A5_D + (size_t)(it.hk * G + (rr & (G - 1))) * A5_D;
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 qstage + (uint32_t)(rr * A5_Q_ROW) * 4u),
+                             "l"(src), "r"(A5_D * 4), "r"(bar)
+                             : "memory");
             }
         }
     } else {
@@ -525,75 +507,76 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
             // One thread issues every MMA of the CTA, so its instruction count per MMA bounds the tensor pipe:
             // the descriptors of a tile are its base descriptor plus compile-time constants (the address field
             // counts 16-byte units and no operand crosses the field's range), nothing is recomputed per MMA.
-            const uint64_t dq_hi = a5_desc(q_hi), dq_lo = a5_desc(q_lo);
-            auto issue_s = [&](int j) {
-                const uint64_t dk_hi = a5_desc(kring + (uint32_t)(j & 1) * A5_K_BYTES), dk_lo = dk_hi + (16384u >> 4);
+            // j: key tile of the query tile (its group's buffers); t: over all query tiles (ring slots)
+            auto issue_s = [&](int j, int t) {
+                const uint64_t dk_hi = a5_desc(kring + (uint32_t)(t & 1) * A5_K_BYTES), dk_lo = dk_hi + (16384u >> 4);
                 const uint32_t d = tmem + (uint32_t)(j & 1) * 64u;
 #pragma unroll
                 for (int term = 0; term < 3; ++term)
 #pragma unroll
                     for (int k16 = 0; k16 < A5_D / 16; ++k16) {
-                        const uint64_t qo = (uint64_t)(((k16 >> 2) * 16384 + (k16 & 3) * 32) >> 4);
                         const uint64_t ko = (uint64_t)(((k16 >> 2) * 8192 + (k16 & 3) * 32) >> 4);
-                        const uint64_t da = (term == 2 ? dq_lo : dq_hi) + qo, db = (term == 1 ? dk_lo : dk_hi) + ko;
+                        const uint32_t qa = tmem + A5_QT + (term == 2 ? 64u : 0u) + (uint32_t)k16 * 8u;
+                        const uint64_t db = (term == 1 ? dk_lo : dk_hi) + ko;
                         if (term == 0 && k16 == 0)
-                            a5_mma_ss<0>(d, da, db, idesc_s);
+                            a5_mma_ts<0>(d, qa, db, idesc_s);
                         else
-                            a5_mma_ss<1>(d, da, db, idesc_s);
+                            a5_mma_ts<1>(d, qa, db, idesc_s);
                     }
+                a5_commit(a5_smem(&s_sfull[j & 1]));
+                a5_commit(a5_smem(&s_kempty[t & 1]));
             };
-            auto issue_pv = [&](int j) {
-                const uint64_t dv_hi = a5_desc(vring + (uint32_t)(j & 1) * A5_V_BYTES), dv_lo = dv_hi + (16384u >> 4);
-                const uint32_t pbase = tmem + (uint32_t)(j & 1) * 64u, d = tmem + 128u + (uint32_t)(j & 1) * 128u;
+            auto issue_pv = [&](int j, int t, auto first) {
+                const uint64_t dv_hi = a5_desc(vring + (uint32_t)(t & 1) * A5_V_BYTES), dv_lo = dv_hi + (16384u >> 4);
+                const uint32_t pbase = tmem + (uint32_t)(j & 1) * 64u, d = tmem + A5_O + (uint32_t)(j & 1) * 128u;
 #pragma unroll
                 for (int term = 0; term < 3; ++term)
 #pragma unroll
                     for (int k16 = 0; k16 < A5_BN / 16; ++k16) {
                         const uint32_t pa = pbase + (term == 2 ? 32u : 0u) + (uint32_t)k16 * 8u;
                         const uint64_t db = (term == 1 ? dv_lo : dv_hi) + (uint64_t)((k16 * 32) >> 4);
-                        if (term == 0 && k16 == 0)
+                        if (decltype(first)::value && term == 0 && k16 == 0)
                             a5_mma_ts<0>(d, pa, db, idesc_o);
                         else
                             a5_mma_ts<1>(d, pa, db, idesc_o);
                     }
+                a5_commit(a5_smem(&s_vempty[t & 1]));
             };
-            bool ok = a5_wait(a5_smem(&s_qready), 0, abort_flag, p.status, 0x7b000004u);
-            if (ok && ntiles > 0) {
-                ok = a5_wait(a5_smem(&s_kfull[0]), 0, abort_flag, p.status, 0x7b000005u);
-                if (ok) {
+            bool ok = true;
+            int base = 0;                // key tiles of the query tiles before
+            uint32_t phases = 0;         // of the groups' weights, a bit each
+            for (int k = 0; k < rounds && ok; ++k) {
+                const Item it = item(k);
+                if (!it.n) break;
+                ok = a5_wait(a5_smem(&s_qready), (uint32_t)k & 1u, abort_flag, p.status, 0x7b000004u);
+                auto scores = [&](int j) {
+                    const int t = base + j;
+                    ok = ok && a5_wait(a5_smem(&s_kfull[t & 1]), (uint32_t)(t >> 1) & 1u, abort_flag, p.status, 0x7b000005u);
+                    if (!ok) return;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    issue_s(0);
-                    a5_commit(a5_smem(&s_sfull[0]));
-                    a5_commit(a5_smem(&s_kempty[0]));
-                }
-            }
-            for (int j = 0; j < ntiles && ok; ++j) {
-                if (j + 1 < ntiles) {
-                    ok = a5_wait(a5_smem(&s_kfull[(j + 1) & 1]), (uint32_t)((j + 1) >> 1) & 1u, abort_flag, p.status, 0x7b000006u);
+                    issue_s(j, t);
+                };
+                for (int j = 0; j < 2 && j < it.n; ++j) scores(j);
+                for (int j = 0; j < it.n && ok; ++j) {
+                    const int t = base + j;
+                    ok = a5_wait(a5_smem(&s_pfull[j & 1]), (phases >> (j & 1)) & 1u, abort_flag, p.status, 0x7b000007u);
+                    phases ^= 1u << (j & 1);
+                    if (ok && j == 0 && k > 0) ok = a5_wait(a5_smem(&s_oread), (uint32_t)(k - 1) & 1u, abort_flag, p.status, 0x7b00000du);
+                    if (ok) ok = a5_wait(a5_smem(&s_vfull[t & 1]), (uint32_t)(t >> 1) & 1u, abort_flag, p.status, 0x7b00000au);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    issue_s(j + 1);
-                    a5_commit(a5_smem(&s_sfull[(j + 1) & 1]));
-                    a5_commit(a5_smem(&s_kempty[(j + 1) & 1]));
+                    if (j < 2)
+                        issue_pv(j, t, std::true_type());
+                    else
+                        issue_pv(j, t, std::false_type());
+                    if (j + 2 < it.n) scores(j + 2);  // (over the P that this product has read)
                 }
-                ok = a5_wait(a5_smem(&s_pfull[j & 1]), (uint32_t)(j >> 1) & 1u, abort_flag, p.status, 0x7b000007u);
-                if (ok) ok = a5_wait(a5_smem(&s_oempty[j & 1]), ((uint32_t)(j >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000008u);
-                if (ok) ok = a5_wait(a5_smem(&s_vfull[j & 1]), (uint32_t)(j >> 1) & 1u, abort_flag, p.status, 0x7b00000au);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                issue_pv(j);
-                a5_commit(a5_smem(&s_ofull[j & 1]));
-                a5_commit(a5_smem(&s_vempty[j & 1]));
+                if (ok) a5_commit(a5_smem(&s_ofull));
+                base += it.n;
             }
         }
     }
 
-#ifdef RB_TRACE
-    if (warp < 8) {
-        RB_STAMP(tr2, 3);
-        RB_TRACE_COMMIT(tr2, 501);
-    }
-#endif
     // ---------------- common exit: nothing of this CTA may still be in flight when it returns
     if (*abort_flag && threadIdx.x == 0) {
         const long long t0 = clock64();
@@ -679,8 +662,10 @@ int launch_attn_prefill_t5(const AttnParams& p, int rows, cudaStream_t st) {
     a.causal = p.causal;
     a.split_seq = split_seq;
     if (!a.status) return ROTOR_B200_ERR_CUDA;
-    dim3 grid((p.seq + QT - 1) / QT, p.n_kv_heads, batch);
-    attn_prefill_t5_kernel<<<grid, A5_THREADS, A5_SMEM, st>>>(tm[0], tm[1], tm[2], tm[3], a);
+    a.batch = batch;
+    a.nqt = (p.seq + QT - 1) / QT;
+    const int items = a.nqt * p.n_kv_heads * batch, sms = fused_sm_count();
+    attn_prefill_t5_kernel<<<items < sms ? items : sms, A5_THREADS, A5_SMEM, st>>>(tm[0], tm[1], tm[2], tm[3], a);
     return launch_status();
 }
 

@@ -644,6 +644,80 @@ def test_infinite_scores_weigh_nothing(rb, heads, kv, batch, context, hidden):
     assert np.array_equal(*got)
 
 
+def _attention_layer(rb, d, heads, kv, seed, **kw):
+    """An attention layer with random weights, and the weights (times their scales) in float64."""
+    import torch
+    at = rb.tr.MultiHeadAttention(d, heads, kv, **kw)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    mats = []
+    for p in (at.q_proj, at.k_proj, at.v_proj, at.o_proj):
+        w = torch.randint(-1, 2, (p.out_features, p.in_features), generator=g, device="cuda", dtype=torch.int8)
+        p.load_from_int8(w, 0.04)
+        mats.append(w.double() * float(np.float32(0.04)))
+    return at, mats
+
+
+@pytest.mark.parametrize("heads,kv,batch,seq", [(3, 1, 3, 100), (4, 1, 2, 131), (5, 5, 1, 300)])
+def test_qkv_rows_of_a_prompt(rb, heads, kv, batch, seq):
+    """256 rows and more of one activation term: the q/k/v product finishes its rows in its read-back (an odd number of heads, tiles
+    across sequences, a cache that holds something already).  The cache against the one that portions below 16 tokens
+    leave (float32 rounding), the outputs within what a quantiser's ties explain."""
+    sem = rb.sem.BASELINE
+    at, _ = _attention_layer(rb, 128 * heads, heads, kv, heads + seq, semantics=sem, max_seq=seq + 7, max_batch=batch)
+    x = np.random.default_rng(seq).standard_normal((batch, seq + 7, 128 * heads)).astype(np.float32)
+
+    def run(cuts):
+        out, cache = [], None
+        for a, b in zip(cuts, cuts[1:]):
+            y, cache = at.forward(x[:, a:b], kv_cache=cache, use_cache=True)
+            out.append(y)
+        return np.concatenate(out, 1), cache["k"], cache["v"]
+
+    whole, k, v = run([0, 7, seq + 7])
+    parts, k2, v2 = run(list(range(0, seq + 7, 15)) + [seq + 7])
+    assert rel_err(k, k2) < 1e-6 and rel_err(v, v2) < 1e-6
+    assert np.linalg.norm(whole - parts) < 2e-2 * np.linalg.norm(parts)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("heads,kv,batch,past,seq", [(1, 1, 1, 0, 16), (2, 1, 1, 0, 65), (4, 1, 3, 300, 33), (8, 1, 2, 64, 47), (5, 5, 2, 10, 300),
+                                                     (16, 4, 9, 0, 200), (3, 3, 5, 130, 1300)])
+def test_prompt_attention_against_float64(rb, heads, kv, batch, past, seq, causal):
+    """Prompts behind cached rows whose scores rise and fall by far more than the weights' reference follows without moving, more
+    query tiles than SMs (each CTA several, of unequal length), tiles of one and two key tiles, rows that see nothing of a
+    tile, a last tile without whole rows.  Three activation terms."""
+    import dataclasses
+    import torch
+    d = 128 * heads
+    sem = dataclasses.replace(rb.sem.REFERENCE, causal=causal)
+    at, (wq, wk, wv, wo) = _attention_layer(rb, d, heads, kv, heads + seq + past, semantics=sem, max_seq=past + seq, max_batch=batch)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seq)
+    x = torch.randn((batch, seq, d), generator=g, device="cuda")
+    k, v = at.ensure_cache()
+    if past:
+        k[:, :, :past] = torch.randn(k[:, :, :past].shape, generator=g, device="cuda") * (torch.arange(past, device="cuda") % 97 / 8.0)[:, None]
+        v[:, :, :past] = torch.randn(v[:, :, :past].shape, generator=g, device="cuda")
+    held = [t[:, :, :past].double() for t in (k, v)]
+    cache = rb.tr.KVCache(at, past, batch) if past else None
+    got = torch.as_tensor(at.forward(x.cpu().numpy(), kv_cache=cache)[0]).cuda().double()
+    rows = x.double()
+    q, kn, vn = ((rows @ w.T).reshape(batch, seq, -1, 128).transpose(1, 2) for w in (wq, wk, wv))
+    kk, vv = (torch.cat(t, 2).repeat_interleave(heads // kv, 1) for t in zip(held, (kn, vn)))
+    want, top = torch.empty_like(rows), 0.0
+    for b in range(batch):
+        s = q[b] @ kk[b].transpose(-1, -2) * 128 ** -0.5
+        top = max(top, float(s.abs().max()))
+        if causal:
+            at_, key = torch.arange(seq, device="cuda")[:, None] + past, torch.arange(past + seq, device="cuda")[None]
+            s = s.masked_fill(key > at_, -np.inf)
+        want[b] = (s.softmax(-1) @ vv[b]).transpose(0, 1).reshape(seq, d) @ wo.T
+    want = want / (want.square().mean(-1, keepdim=True) + sem.eps).sqrt()
+    # an operand keeps 16 bits: a score of size s is off by up to 2^-16 s, its weight by as much of itself
+    assert (got - want).norm() < (3e-5 + top * 2.0 ** -16) * want.norm(), float((got - want).norm() / want.norm())
+
+
 @pytest.mark.parametrize("rows", [2, 4, 5, 9])
 @pytest.mark.parametrize("ff", [10880, 10944])
 def test_ffn_sums_cleared_by_stage_or_memset(rb, ff, rows):
