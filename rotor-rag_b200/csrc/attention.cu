@@ -159,7 +159,7 @@ static int launch_dependent(void (*kernel)(P), dim3 grid, int threads, size_t sm
 }
 
 int launch_qkv_finish(const QkvFinishParams& p, int rows, cudaStream_t st) {
-    if (rows >= 5 && p.acc.planes == 1 && p.acc.out % 4 == 0 && p.head_dim % 8 == 0 && p.terms >= 1 && p.terms <= 3)
+    if (rows >= 2 && p.acc.planes == 1 && p.acc.out % 4 == 0 && p.head_dim % 8 == 0 && p.terms >= 1 && p.terms <= 3)
         return launch_dependent(qkv_finish_vec_kernel, dim3(rows), 256, 0, p, st);
     else
         qkv_finish_kernel<<<rows, 256, 0, st>>>(p);

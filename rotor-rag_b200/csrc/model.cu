@@ -153,11 +153,11 @@ static int derive(Model& m) {
 static int gemv(Ctx& c, const void* tiles, size_t out, size_t in, int ncols, int xs, int32_t* acc, AccView* view,
                 cudaStream_t st) {
     GemvPlan plan = plan_gemv(out, in, ncols < 8 ? ncols : 8);
-    // five and more columns: the K splits add into one plane, so that the register-resident row stages
-    // (complete sums in one plane) can follow; fewer columns keep one plane per split, which the
+    // two and more columns: the K splits add into one plane, so that the register-resident row stages
+    // (complete sums in one plane) can follow; one column keeps one plane per split, which the
     // generation-step stages add while they dequantise
     const bool gemm = ncols >= GEMM_MIN_COLS && c.variant == ROTOR_B200_VARIANT_AUTO;
-    const bool one_plane = gemm || ncols >= 5;
+    const bool one_plane = gemm || ncols >= 2;
     const size_t plane_stride = one_plane ? 0 : (size_t)ncols * out;
     view->acc = acc;
     view->plane_stride = plane_stride;
@@ -174,7 +174,7 @@ static int gemv(Ctx& c, const void* tiles, size_t out, size_t in, int ncols, int
 constexpr size_t CLEAR_ROW_MAX = 256 * 1024;
 static void clear_for(Ctx& c, VecStageParams& p, size_t out, size_t in, int ncols, int32_t* acc) {
     c.zeroed = nullptr;
-    if (ncols < 5 || (size_t)c.terms * out * sizeof(int32_t) > CLEAR_ROW_MAX || !gemv_adds(out, in, ncols, c.xq, c.variant)) return;
+    if (ncols < 2 || (size_t)c.terms * out * sizeof(int32_t) > CLEAR_ROW_MAX || !gemv_adds(out, in, ncols, c.xq, c.variant)) return;
     p.zero = acc;
     p.zero_n = (size_t)ncols * out;
     c.zeroed = acc;
@@ -237,7 +237,7 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
     if (!fuse_qkv) RB_TRY(gemv(c, L.qkv_tiles, qkv_out, c.d, cols, 0, c.accA, &va, st));
     // several sequences: dequantise, rotate, append to the cache and attend in one launch, each sequence's cache read once
     // per group of heads
-    const bool stream = seq == 1 && batch >= 5 && attn_decode_stream_ok(c.n_heads, c.n_kv_heads, c.head_dim);
+    const bool stream = seq == 1 && batch >= 2 && attn_decode_stream_ok(c.n_heads, c.n_kv_heads, c.head_dim);
     if (stream || (seq == 1 && batch <= c.max_batch && batch < 16)) {
         AttnDecodeParams dp = {};
         dp.acc = va;
@@ -416,7 +416,11 @@ static bool fused_step_ok(const Model& m, int batch, int seq) {
     static const bool off = getenv("ROTOR_B200_NO_FUSED_STEP") != nullptr;  // measurement aid
     const size_t qkv_out = (size_t)c.dq + 2 * c.dkv;
     const bool tp_ok = c.tp_size <= 1 || (c.terms == 1 && tp_fused_ready(c.tp) && (size_t)batch * c.d <= (size_t)XCH_CAP);
-    const bool shape_ok = !off && tp_ok && seq == 1 && batch <= FUSED_MAX_ROWS && batch <= c.max_batch &&
+    // (several sequences: every CTA of a fused product makes each row again, one after the other; a step of the 2B shape, 12
+    // layers, 517 positions, fused / in stages: 2 sequences 680 / 585 us, 3 814 / 667, 4 971 / 694, 2 with three terms 898 / 739;
+    // tensor parallel keeps it, its exchanges ride in the products)
+    const int most = c.tp_size > 1 ? FUSED_MAX_ROWS : 1;
+    const bool shape_ok = !off && tp_ok && seq == 1 && batch <= most && batch <= c.max_batch &&
                           c.terms <= 3 && batch * c.terms <= 8 && c.ff % 16 == 0;
     const bool q = fused_gemv_supported(qkv_out, c.d, batch, c.terms, 1, 0);
     const bool o = fused_gemv_supported(c.d, c.dq, batch, c.terms, 1, c.n_heads * c.nsplit);

@@ -20,7 +20,7 @@
 namespace rb {
 
 constexpr int RS_THREADS = 128;
-constexpr int RS_MIN_ROWS = 5;         // (fewer rows: the generation-step kernels or the shared-memory stage)
+constexpr int RS_MIN_ROWS = 2;         // (one row: the generation-step kernels or the shared-memory stage)
 constexpr int RS_WIDE_THREADS = 512;
 // With fewer rows than two per SM every CTA runs its code once, from a cold instruction cache, and waits once for
 // each load: the duration is the length of that chain, so a row takes as many threads as leave one or two groups to
