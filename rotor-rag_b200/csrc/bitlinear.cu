@@ -64,9 +64,9 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar) {
 
 // Sums that the product adds to are cleared by the quantiser, a share per row, so that no memset stands between the two, up to
 // this many bytes a row: 8192 -> 28672, 8 rows (115 KB) 27.1 / 27.5 us, 5 rows of two terms (229 KB) 43.4 / 41.9, of three
-// (344 KB) 56.8 / 53.1.  The product starts early where it is one launch (4096 -> 11008, 8 rows: 10.6 against 12.6 us); several
-// launches of eight columns get in each other's way then (2560 -> 6912: 16 rows 12.4 / 11.4, 31 rows 19.9 / 17.6).
+// (344 KB) 56.8 / 53.1.  The product starts early where it is one launch (4096 -> 11008, 8 rows: 10.6 against 12.6 us).
 constexpr size_t LINEAR_CLEAR_MAX = 128 * 1024;
+constexpr int ACC_MMA_COLS = 32;   // columns of one launch of the MMA variant
 constexpr size_t LINEAR_FUSED_ROWS = 4, LINEAR_FUSED_COLS = 6;  // a stand-alone layer call in one launch: see its rule
 
 struct AccParams {
@@ -83,7 +83,10 @@ struct AccParams {
     size_t plane_stride;   // != 0: K split s stores its partial sums to acc + s*plane_stride instead
 };
 
-template <int WARPS, int UMAX, bool USE_MMA, int NCOL>
+// NT: groups of eight columns of the MMA variant.  A weight word is loaded and masked once for all of them, so that more columns
+// cost shared-memory reads and MMAs but no further pass over the matrix.  A step of the 2B shape (12 layers), a launch for every eight
+// columns / one for all: 12 sequences 843 / 734 us, 16 876 / 750, 24 1090 / 921; three terms 5 sequences 952 / 829, 8 1132 / 940.
+template <int WARPS, int UMAX, bool USE_MMA, int NCOL, int NT>
 __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_constant__ AccParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -95,19 +98,21 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
     const int kbase = kt0 * TILE_K;
 
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
-    int* red = reinterpret_cast<int*>(smem_raw + 16);            // [WARPS][128]
-    int8_t* xs = reinterpret_cast<int8_t*>(smem_raw + 16 + WARPS * 128 * 4);
+    int* red = reinterpret_cast<int*>(smem_raw + 16);            // [WARPS][NT][128]
+    int8_t* xs = reinterpret_cast<int8_t*>(smem_raw + 16 + WARPS * NT * 128 * 4);
 
     stage_init(bar);
 
     const uint4* trow = p.tiles + ((size_t)rt * p.nkt) * 32 + lane;
 
-    int accm[4][4];          // MMA: [bit pair j][fragment register]
+    int accm[NT][4][4];      // MMA: [bit pair j][fragment register]
     int accd[2][4][NCOL];    // DP4A: [row half][bit pair j][column]
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) accm[j][r] = 0;
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) accm[n][j][r] = 0;
 #pragma unroll
         for (int c = 0; c < NCOL; ++c) accd[0][j][c] = accd[1][j][c] = 0;
     }
@@ -131,7 +136,9 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
             if (kt < kt1) {
                 const uint32_t pw[4] = {wv[u].x, wv[u].y, wv[u].z, wv[u].w};
                 const int koff = kt * TILE_K - kbase + 32 * t;
-                tile_mac<USE_MMA, NCOL>(pw, xs, xs_stride, koff, g, p.ncols, accm, accd);
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+                    tile_mac<USE_MMA, NCOL>(pw, xs + (size_t)8 * n * xs_stride, xs_stride, koff, g, p.ncols - 8 * n, accm[n], accd);
             }
         }
         base += UMAX * WARPS;
@@ -141,14 +148,16 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
     }
 
     // exact rescale of the per-bit-pair partial sums, then reduce across the CTA
-    int* myred = red + warp * 128;
+    int* myred = red + warp * NT * 128;
     if constexpr (USE_MMA) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int v = accm[0][r] + (accm[1][r] >> 2) + (accm[2][r] >> 4) + (accm[3][r] >> 6);
-            const int row_l = g + 8 * (r >> 1), col = 2 * t + (r & 1);
-            myred[row_l * 8 + col] = v;
-        }
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int v = accm[n][0][r] + (accm[n][1][r] >> 2) + (accm[n][2][r] >> 4) + (accm[n][3][r] >> 6);
+                const int row_l = g + 8 * (r >> 1), col = 2 * t + (r & 1);
+                myred[n * 128 + row_l * 8 + col] = v;
+            }
     } else {
 #pragma unroll
         for (int rh = 0; rh < 2; ++rh)
@@ -161,22 +170,25 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
             }
     }
     __syncthreads();
-    if (threadIdx.x < 128) {
-        const int row_l = threadIdx.x >> 3, col = threadIdx.x & 7;
-        const int row = rt * TILE_ROWS + row_l;
-        if (col < p.ncols && row < p.out) {
-            int s = 0;
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) s += red[w * 128 + threadIdx.x];
-            if (blockIdx.y == 0) s -= p.xsum[col];
-            int32_t* dst = p.acc + (size_t)blockIdx.y * p.plane_stride + (size_t)col * p.out + row;
-            if (p.atomic)
-                atomicAdd(dst, s);
-            else
-                *dst = s;
+    for (int n = 0; n < NT; ++n) {
+        for (int e = threadIdx.x; e < 128; e += WARPS * 32) {
+            // several groups: a warp's sums of one column lie in consecutive rows (a quarter of a line an instruction)
+            const int row_l = NT > 1 ? e & 15 : e >> 3, col_l = NT > 1 ? e >> 4 : e & 7, col = 8 * n + col_l;
+            const int row = rt * TILE_ROWS + row_l;
+            if (col < p.ncols && row < p.out) {
+                int s = 0;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) s += red[(w * NT + n) * 128 + row_l * 8 + col_l];
+                if (blockIdx.y == 0) s -= p.xsum[col];
+                int32_t* dst = p.acc + (size_t)blockIdx.y * p.plane_stride + (size_t)col * p.out + row;
+                if (p.atomic)
+                    atomicAdd(dst, s);
+                else
+                    *dst = s;
+            }
         }
     }
-
 }
 
 __global__ void dequant_kernel(const int32_t* __restrict__ acc, const float* __restrict__ sx, int m, int terms,
@@ -193,10 +205,10 @@ __global__ void dequant_kernel(const int32_t* __restrict__ acc, const float* __r
     }
 }
 
-template <int WARPS, int UMAX, bool USE_MMA, int NCOL>
+template <int WARPS, int UMAX, bool USE_MMA, int NCOL, int NT = 1>
 static int launch_acc(const AccParams& p, int nrt, int ksplit, cudaStream_t st) {
-    auto kern = bitlinear_acc_kernel<WARPS, UMAX, USE_MMA, NCOL>;
-    const size_t smem = 16 + WARPS * 128 * 4 + (size_t)p.ncols * (p.kt_per_split * TILE_K + XS_PAD);
+    auto kern = bitlinear_acc_kernel<WARPS, UMAX, USE_MMA, NCOL, NT>;
+    const size_t smem = 16 + WARPS * NT * 128 * 4 + (size_t)p.ncols * (p.kt_per_split * TILE_K + XS_PAD);
     if (smem > 200 * 1024) return ROTOR_B200_ERR_SHAPE;
     if (smem > 48 * 1024) {
         static PerDevice<size_t> once;  // per instantiation and device
@@ -240,7 +252,15 @@ static int choose_ksplit(int nrt, int nkt, int ncols, int warps) {
 
 static int dispatch_acc(const AccParams& p, int nrt, int ksplit, int variant, cudaStream_t st) {
     constexpr int WARPS = 4, UMAX = 8;
-    if (variant == ROTOR_B200_VARIANT_MMA) return launch_acc<WARPS, UMAX, true, 1>(p, nrt, ksplit, st);
+    if (variant == ROTOR_B200_VARIANT_MMA) {
+        switch ((p.ncols + 7) / 8) {
+            case 1: return launch_acc<WARPS, UMAX, true, 1>(p, nrt, ksplit, st);
+            case 2: return launch_acc<WARPS, UMAX, true, 1, 2>(p, nrt, ksplit, st);
+            case 3: return launch_acc<WARPS, UMAX, true, 1, 3>(p, nrt, ksplit, st);
+            case 4: return launch_acc<WARPS, UMAX, true, 1, 4>(p, nrt, ksplit, st);
+        }
+        return ROTOR_B200_ERR_ARG;
+    }
     switch (p.ncols) {
         case 1: return launch_acc<WARPS, UMAX, false, 1>(p, nrt, ksplit, st);
         case 2: return launch_acc<WARPS, UMAX, false, 2>(p, nrt, ksplit, st);
@@ -250,9 +270,9 @@ static int dispatch_acc(const AccParams& p, int nrt, int ksplit, int variant, cu
     return ROTOR_B200_ERR_ARG;
 }
 
-template <bool USE_MMA, int NCOL>
+template <bool USE_MMA, int NCOL, int NT = 1>
 static int configure_one() {
-    RB_CUDA(cudaFuncSetAttribute(bitlinear_acc_kernel<4, 8, USE_MMA, NCOL>,
+    RB_CUDA(cudaFuncSetAttribute(bitlinear_acc_kernel<4, 8, USE_MMA, NCOL, NT>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     return ROTOR_B200_OK;
 }
@@ -261,7 +281,9 @@ static int configure_one() {
 int configure_gemv_kernels() {
     int rc = (library_status_word() ? ROTOR_B200_OK : ROTOR_B200_ERR_CUDA);
     if (rc) return rc;
-    if ((rc = configure_one<true, 1>())) return rc;
+    if ((rc = configure_one<true, 1>()) || (rc = configure_one<true, 1, 2>()) || (rc = configure_one<true, 1, 3>()) ||
+        (rc = configure_one<true, 1, 4>()))
+        return rc;
     if ((rc = configure_one<false, 1>())) return rc;
     if ((rc = configure_one<false, 2>())) return rc;
     if ((rc = configure_one<false, 3>())) return rc;
@@ -274,12 +296,12 @@ static int pick_variant(int variant, int ncols) {
 }
 
 int gemv_cols_per_launch(int variant, int ncols) {
-    return pick_variant(variant, ncols < 8 ? ncols : 8) == ROTOR_B200_VARIANT_MMA ? 8 : 4;
+    return pick_variant(variant, ncols < 8 ? ncols : 8) == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
 }
 
 GemvPlan plan_gemv(size_t out, size_t in, int ncols) {
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
-    const int per_pass = ncols < 8 ? ncols : 8;
+    const int per_pass = ncols < ACC_MMA_COLS ? ncols : ACC_MMA_COLS;
     int ks = choose_ksplit(nrt, nkt, per_pass, 4);
     GemvPlan g;
     g.kt_per_split = (nkt + ks - 1) / ks;
@@ -305,7 +327,7 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
     const size_t kpad = kpad_of(in);
     variant = pick_variant(variant, ncols);
-    const int chunk = variant == ROTOR_B200_VARIANT_MMA ? 8 : 4;
+    const int chunk = variant == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
     for (int c0 = 0; c0 < ncols; c0 += chunk) {
         AccParams p;
         p.tiles = (const uint4*)tiles;
@@ -351,7 +373,7 @@ static int run_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, c
     if (ncols <= 8 && staged_acc_supported(out, in, (int)ncols, variant))
         return launch_staged_acc(tiles, out, in, xq, xsum, (int)ncols, acc, variant, st);
     variant = pick_variant(variant, (int)(ncols < 8 ? ncols : 8));
-    const size_t chunk = variant == ROTOR_B200_VARIANT_MMA ? 8 : 4;
+    const size_t chunk = variant == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
     for (size_t c0 = 0; c0 < ncols; c0 += chunk) {
         const int nc = (int)((ncols - c0) < chunk ? (ncols - c0) : chunk);
         const int ksplit = choose_ksplit(nrt, nkt, nc, 4);
@@ -380,7 +402,7 @@ static bool acc_adds(size_t out, size_t in, size_t ncols, const int8_t* xq, int 
     if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO)
         return gemm_tcgen05_supported(out, in, (int)ncols, xq) && gemm_tcgen05_splits(out, in, (int)ncols) >= 2;
     if (ncols <= 8 && staged_acc_supported(out, in, (int)ncols, variant)) return false;
-    const size_t chunk = pick_variant(variant, (int)(ncols < 8 ? ncols : 8)) == ROTOR_B200_VARIANT_MMA ? 8 : 4;
+    const size_t chunk = pick_variant(variant, (int)(ncols < 8 ? ncols : 8)) == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS), rest = (int)(ncols % chunk);
     return (ncols >= chunk && choose_ksplit(nrt, nkt, (int)chunk, 4) > 1) || (rest && choose_ksplit(nrt, nkt, rest, 4) > 1);
 }
@@ -455,7 +477,7 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
     w += al256(nc * 4);
     int32_t* acc = (int32_t*)w;
     const bool adds = out < (1u << 30) && in <= 49152 && nc * out * sizeof(int32_t) <= m * LINEAR_CLEAR_MAX && acc_adds(out, in, nc, xq, variant);
-    int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, nc <= 8, as_stream(stream));
+    int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, nc < GEMM_MIN_COLS, as_stream(stream));
     if (rc) return rc;
     rc = run_acc(tiles, out, in, xq, xsum, nc, acc, variant, as_stream(stream), adds);
     if (rc) return rc;
@@ -542,7 +564,7 @@ int rotor_b200_bitlinear_forward_static(const void* tiles, size_t out, size_t in
     if (rc) return rc;
     const int nkt = (int)(kpad / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
     variant = pick_variant(variant, (int)(nc < 8 ? nc : 8));
-    const size_t chunk = variant == ROTOR_B200_VARIANT_MMA ? 8 : 4;
+    const size_t chunk = variant == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
     for (size_t c0 = 0; c0 < nc; c0 += chunk) {
         const int ncols = (int)((nc - c0) < chunk ? (nc - c0) : chunk);
         const int ksplit = choose_ksplit(nrt, nkt, ncols, 4);

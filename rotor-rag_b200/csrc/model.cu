@@ -152,7 +152,7 @@ static int derive(Model& m) {
 // One BitLinear product into partial planes, activations taken from xq/xsum[xs].
 static int gemv(Ctx& c, const void* tiles, size_t out, size_t in, int ncols, int xs, int32_t* acc, AccView* view,
                 cudaStream_t st) {
-    GemvPlan plan = plan_gemv(out, in, ncols < 8 ? ncols : 8);
+    GemvPlan plan = plan_gemv(out, in, ncols);
     // two and more columns: the K splits add into one plane, so that the register-resident row stages
     // (complete sums in one plane) can follow; one column keeps one plane per split, which the
     // generation-step stages add while they dequantise
