@@ -10,13 +10,13 @@
 
 namespace rb {
 
-constexpr int LM_WARPS = 8;
+constexpr int LM_WARPS = 8, LM_MOST_WARPS = 16;  // (sixteen where four rows leave an SM room for one CTA)
 constexpr int LM_PARTS = 148 * 4;  // CTAs = argmax partials per token row
 
 int lmhead_parts() { return LM_PARTS; }
 
 template <int NROWS>
-__global__ void __launch_bounds__(LM_WARPS * 32) lmhead_kernel(const __grid_constant__ LmHeadParams p, int row0) {
+__global__ void __launch_bounds__((NROWS > 3 ? LM_MOST_WARPS : LM_WARPS) * 32) lmhead_kernel(const __grid_constant__ LmHeadParams p, int row0) {
     extern __shared__ __align__(16) float xs[];  // [NROWS][d]
     pdl_wait();
     pdl_trigger();
@@ -78,7 +78,7 @@ static int launch_lm(const LmHeadParams& p, int row0, cudaStream_t st) {
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(LM_PARTS);
-    cfg.blockDim = dim3(LM_WARPS * 32);
+    cfg.blockDim = dim3((NROWS > 3 && smem > 100 * 1024 ? LM_MOST_WARPS : LM_WARPS) * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
