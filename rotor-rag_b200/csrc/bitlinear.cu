@@ -321,7 +321,7 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
     if (rc) return rc;
     if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO) {
         // compute-bound regime: the tiled GEMM writes complete sums into plane 0 (callers use one plane)
-        if (gemm_tcgen05_supported(out, in, ncols, xq)) return launch_gemm_tcgen05(tiles, out, in, xq, xsum, ncols, acc, st, zeroed);
+        if (gemm_tcgen05_supported(out, in, ncols, xq)) return launch_gemm_tcgen05(tiles, out, in, xq, xsum, ncols, acc, st, zeroed, true);
         return launch_gemm_mma(tiles, out, in, xq, xsum, ncols, acc, st);
     }
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
@@ -353,8 +353,9 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
 
 using namespace rb;
 
+// dependent: the kernel before is this call's own (its weights are older).
 static int run_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, size_t ncols,
-                   int32_t* acc, int variant, cudaStream_t st, bool zeroed) {
+                   int32_t* acc, int variant, cudaStream_t st, bool zeroed, bool dependent) {
     RB_REQUIRE(tiles && xq && xsum && acc && out > 0 && in > 0 && ncols > 0);
     RB_REQUIRE(out < (1u << 30) && in < (1u << 30));
     RB_REQUIRE(((uintptr_t)tiles & 15) == 0 && ((uintptr_t)xq & 15) == 0);
@@ -365,7 +366,7 @@ static int run_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, c
     const size_t kpad = kpad_of(in);
     if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO) {
         if (gemm_tcgen05_supported(out, in, (int)ncols, xq))
-            return launch_gemm_tcgen05(tiles, out, in, xq, xsum, (int)ncols, acc, st, zeroed);
+            return launch_gemm_tcgen05(tiles, out, in, xq, xsum, (int)ncols, acc, st, zeroed, dependent);
         return launch_gemm_mma(tiles, out, in, xq, xsum, (int)ncols, acc, st);
     }
     // small matrices, up to eight columns: the staged kernel (every CTA's share of the tiles sits in shared
@@ -411,7 +412,7 @@ extern "C" {
 
 int rotor_b200_bitlinear_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum,
                              size_t ncols, int32_t* acc, int variant, void* stream) {
-    return run_acc(tiles, out, in, xq, xsum, ncols, acc, variant, as_stream(stream), false);
+    return run_acc(tiles, out, in, xq, xsum, ncols, acc, variant, as_stream(stream), false, false);
 }
 
 int rotor_b200_bitlinear_dequant(const int32_t* acc, const float* sx, size_t m, int terms, size_t out,
@@ -479,7 +480,7 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
     const bool adds = out < (1u << 30) && in <= 49152 && nc * out * sizeof(int32_t) <= m * LINEAR_CLEAR_MAX && acc_adds(out, in, nc, xq, variant);
     int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, nc < GEMM_MIN_COLS, as_stream(stream));
     if (rc) return rc;
-    rc = run_acc(tiles, out, in, xq, xsum, nc, acc, variant, as_stream(stream), adds);
+    rc = run_acc(tiles, out, in, xq, xsum, nc, acc, variant, as_stream(stream), adds, true);
     if (rc) return rc;
     return rotor_b200_bitlinear_dequant(acc, sx, m, terms, out, wscale, wscale_vec, y, stream);
 }

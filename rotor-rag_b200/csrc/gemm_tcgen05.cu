@@ -50,12 +50,16 @@ struct T5Cfg {
     // ring depth and decoder look-ahead: with 64-row tiles a stage is only four short MMAs, so the
     // copy and weight-load latencies need more stages in flight to stay hidden
     static constexpr int STAGES = TOK == 128 ? 4 : (ROWS >= 256 ? 3 : 5);
-    static constexpr int PREFETCH = ROWS < 256 ? 6 : TOK == 128 ? 4 : 2;           // K steps of weight tiles requested ahead
+    // decoder warps take every GROUPS-th K step with GROUPS times the tiles: one chain of wait, decode, fence and arrival per
+    // GROUPS steps (with this, an arrival per warp and dependent launches a step of 64 sequences of the 2B shape, 12 layers, went
+    // from 1653 to 1546 us, of 32 from 1316 to 1162, of 64 of the XL shape, 4 layers, from 1464 to 1408)
+    static constexpr int GROUPS = ROWS >= 256 ? 2 : 1;
+    static constexpr int PREFETCH = ROWS < 256 ? 6 : TOK == 128 ? 4 : 2;           // of its K steps that a warp requests ahead
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024;       // + slack to align the ring to 1024 bytes
     static constexpr int TMEM_COLS = (TOK / 128) * ROWS < 32 ? 32 : (TOK / 128) * ROWS;  // one accumulator of ROWS columns per token half
     static constexpr int DECODERS = ROWS >= 256 ? 8 : 4;           // decoder warps
     static constexpr int THREADS = (DECODERS + 2) * 32;
-    static constexpr int TILES_PER_WARP = ROWS / TILE_ROWS / DECODERS;  // row tiles each decoder warp handles
+    static constexpr int TILES_PER_WARP = ROWS / TILE_ROWS * GROUPS / DECODERS;  // row tiles a decoder warp handles a step
 };
 constexpr int T5_SCATTER_COLS = 48;  // columns up to which a split product's sums are added by a lane per token
 constexpr int T5_DEEP_STEPS = 12;  // K steps of a CTA from which the 128-token variant is taken
@@ -93,7 +97,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     using Cfg = T5Cfg<ROWS, T5_TOK>;
     constexpr int T5_A_BYTES = Cfg::A_BYTES, A_HALF = 128 * TILE_K;
     constexpr int T5_ROWS = ROWS, T5_STAGE_BYTES = Cfg::STAGE_BYTES, TPW = Cfg::TILES_PER_WARP;
-    constexpr int T5_STAGES = Cfg::STAGES, PF = Cfg::PREFETCH, NDW = Cfg::DECODERS;
+    constexpr int T5_STAGES = Cfg::STAGES, PF = Cfg::PREFETCH, NDW = Cfg::DECODERS, GR = Cfg::GROUPS;
 #ifdef RB_TRACE
     const unsigned long long t_entry = gtime();
 #endif
@@ -114,7 +118,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int s = 0; s < T5_STAGES; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[s])), "r"(NDW * 32 + 1));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_full[s])), "r"(NDW / GR + 1));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_empty[s])), "r"(1));
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&s_accf)), "r"(1));
@@ -131,35 +135,36 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     const uint32_t tmem = s_tmem;
 
     if (warp < NDW) {
-        // ---------------- weight decoders: warp w owns row tiles TPW w .. TPW w + TPW - 1 of the CTA's
-        const int g = lane >> 2, t = lane & 3;
-        // weight tiles are requested PF K steps ahead of their decode, so that the L2 / HBM latency
-        // hides behind the decode of the step in between and the wait for a free stage
+        // ---------------- weight decoders: warp w of a group owns row tiles TPW w .. TPW w + TPW - 1 of the CTA's
+        const int g = lane >> 2, t = lane & 3, w = warp % (NDW / GR), grp0 = warp / (NDW / GR);
+        // weight tiles (constants) are requested PF of the warp's steps ahead of their decode, the first before the launch wait
         uint4 wv[PF][TPW];
         auto fetch = [&](int kt, uint4 (&dst)[TPW]) {
 #pragma unroll
             for (int u = 0; u < TPW; ++u) {
-                const int rt = rt0 + warp * TPW + u;
+                const int rt = rt0 + w * TPW + u;
                 dst[u] = (rt < p.nrt && kt < nk)
                              ? ld_stream_v4(p.tiles + ((size_t)rt * p.nkt + ktb + kt) * 32 + lane)
                              : make_uint4(0x55555555u, 0x55555555u, 0x55555555u, 0x55555555u);
             }
         };
 #pragma unroll
-        for (int par = 0; par < PF; ++par) fetch(par, wv[par]);
+        for (int par = 0; par < PF; ++par) fetch(GR * par + grp0, wv[par]);
 #ifdef RB_TRACE
         TraceRec trd = {};
         const bool tracedd = blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
         unsigned long long tld = gtime(), t0d = tld;
 #endif
-        for (int kt2 = 0; kt2 < nk; kt2 += PF) {
+        bool going = true;
+        for (int kt2 = grp0; kt2 < nk && going; kt2 += GR * PF) {
 #pragma unroll
           for (int par = 0; par < PF; ++par) {
-            const int kt = kt2 + par;
+            const int kt = kt2 + GR * par;
             if (kt >= nk) break;
             const int s = kt % T5_STAGES;
-            if (!t5_wait(smem_u32(&s_empty[s]), ((kt / T5_STAGES) & 1) ^ 1, abort_flag, p.status, 0x7c000001u)) {
-                kt2 = nk;  // leave both loops
+            going = t5_wait(smem_u32(&s_empty[s]), ((kt / T5_STAGES) & 1) ^ 1, abort_flag, p.status, 0x7c000001u);
+            if (!__all_sync(0xffffffffu, going)) {
+                going = false;
                 break;
             }
 #ifdef RB_TRACE
@@ -171,8 +176,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
                 const uint32_t pw[4] = {wv[par][u].x, wv[par][u].y, wv[par][u].z, wv[par][u].w};
 #pragma unroll
                 for (int rh = 0; rh < 2; ++rh) {
-                    // operand row R = 16 (TPW warp + u) + g + 8 rh; R % 8 == g; K bytes [32 t, 32 t + 32)
-                    const uint32_t row = bbase + (uint32_t)((warp * TPW + u) * 2 + rh) * 1024u + (uint32_t)g * 128u;
+                    // operand row R = 16 (TPW w + u) + g + 8 rh; R % 8 == g; K bytes [32 t, 32 t + 32)
+                    const uint32_t row = bbase + (uint32_t)((w * TPW + u) * 2 + rh) * 1024u + (uint32_t)g * 128u;
                     const uint32_t lo = pw[rh], hi = pw[rh + 2];
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {  // 16-byte chunk 2 t + c holds bit pairs 2 c and 2 c + 1
@@ -190,13 +195,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
                 }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
-            t5_bar_arrive(smem_u32(&s_full[s]));
-            fetch(kt + PF, wv[par]);
+            __syncwarp();
+            if (lane == 0) t5_bar_arrive(smem_u32(&s_full[s]));  // (an arrival a thread: 256 in turn on one word)
+            fetch(kt + GR * PF, wv[par]);
 #ifdef RB_TRACE
             if (tracedd) { const unsigned long long n_ = gtime(); trd.t[1] += n_ - tld; tld = n_; }
 #endif
           }
         }
+        pdl_wait();  // sums of the activations, and what is added to, belong to earlier kernels until here
+        pdl_trigger();
 #ifdef RB_TRACE
         if (tracedd) {
             trd.t[2] = gtime() - t0d;
@@ -285,6 +293,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
     } else if (warp == NDW) {
         // ---------------- token operand by TMA
         if (elect_lane()) {
+            pdl_wait();  // the tokens are the work of the kernel before
             for (int kt = 0; kt < nk; ++kt) {
                 const int s = kt % T5_STAGES;
                 if (!t5_wait(smem_u32(&s_empty[s]), ((kt / T5_STAGES) & 1) ^ 1, abort_flag, p.status, 0x7c000003u)) break;
@@ -821,6 +830,26 @@ int gemm_tcgen05_splits(size_t out, size_t in, int ncols) {
     return (nkt + per - 1) / per;
 }
 
+// dependent: the launch may start while the kernel before it ends (the weights are older than that kernel).
+template <int ROWS, int TOK>
+static int launch_t5(const CUtensorMap& tmap, const Tc5Params& p, dim3 grid, bool dependent, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(T5Cfg<ROWS, TOK>::THREADS);
+    cfg.dynamicSmemBytes = T5Cfg<ROWS, TOK>::SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl && dependent ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<ROWS, TOK>, tmap, p) != cudaSuccess) {
+        ++g_launch_count;
+        return ROTOR_B200_ERR_CUDA;
+    }
+    return launch_status();
+}
+
 // n: weight rows (or pairs of gate and up rows, two each) that the tiles of 256 cover.
 template <int EPI>
 static int launch_pair(const CUtensorMap& tmap, Tc5Params& p, int n, cudaStream_t st) {
@@ -832,7 +861,7 @@ static int launch_pair(const CUtensorMap& tmap, Tc5Params& p, int n, cudaStream_
 }
 
 int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
-                        int32_t* acc, cudaStream_t st, bool zeroed) {
+                        int32_t* acc, cudaStream_t st, bool zeroed, bool dependent) {
     int rc = configure_gemm_tcgen05();
     if (rc) return rc;
     Tc5Params p = {};
@@ -854,23 +883,17 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
     auto launch256 = [&](dim3 grid) {
         // (64 tokens, 57344 x 8192: 78.3 -> 66.9 us, 8192 x 28672: 44.7 -> 38.7; runs of fewer steps end before the
         // deeper look-ahead is filled and take the variant with less code)
-        if (ncols <= 128 && (p.kt_per_split ? p.kt_per_split : p.nkt) >= T5_DEEP_STEPS)
-            gemm_tcgen05_kernel<256, 128><<<grid, T5Cfg<256, 128>::THREADS, T5Cfg<256, 128>::SMEM, st>>>(tmap, p);
-        else
-            gemm_tcgen05_kernel<256><<<grid, T5Cfg<256>::THREADS, T5Cfg<256>::SMEM, st>>>(tmap, p);
+        if (ncols <= 128 && (p.kt_per_split ? p.kt_per_split : p.nkt) >= T5_DEEP_STEPS) return launch_t5<256, 128>(tmap, p, grid, dependent, st);
+        return launch_t5<256, 256>(tmap, p, grid, dependent, st);
     };
     if (splits >= 2) {
         p.kt_per_split = (p.nkt + splits - 1) / splits;
         if (!zeroed) RB_CUDA(cudaMemsetAsync(acc, 0, (size_t)ncols * out * sizeof(int32_t), st));
-        dim3 grid(tok_tiles, (rows + 255) / 256, splits);
-        launch256(grid);
+        return launch256(dim3(tok_tiles, (rows + 255) / 256, splits));
     } else if (tiles256 < sms) {  // 256-row tiles would leave SMs idle
-        dim3 grid(tok_tiles, (rows + 63) / 64);
-        gemm_tcgen05_kernel<64><<<grid, T5Cfg<64>::THREADS, T5Cfg<64>::SMEM, st>>>(tmap, p);
-    } else {
-        launch256(dim3(tok_tiles, (rows + 255) / 256));
+        return launch_t5<64, 256>(tmap, p, dim3(tok_tiles, (rows + 63) / 64), dependent, st);
     }
-    return launch_status();
+    return launch256(dim3(tok_tiles, (rows + 255) / 256));
 }
 
 // Gate/up product with the gating in the epilogue: `tiles` holds the gate matrix followed by the up

@@ -77,7 +77,7 @@ int gemv_cols_per_launch(int variant, int ncols);
 constexpr int GEMM_MIN_COLS = 32;
 bool gemm_tcgen05_supported(size_t out, size_t in, int ncols, const void* xq);
 int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
-                        int32_t* acc, cudaStream_t st, bool zeroed = false);
+                        int32_t* acc, cudaStream_t st, bool zeroed, bool dependent);
 int gemm_tcgen05_splits(size_t out, size_t in, int ncols);
 int configure_gemm_tcgen05();
 // gate/up product with the gating in its epilogue (float32 gated rows out, one activation term per token)
