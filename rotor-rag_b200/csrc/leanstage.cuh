@@ -226,8 +226,9 @@ __device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& ls
 // (shared memory, zero padded to kpad), its scale and sum to sx[t] / xsum[t] (shared).
 // Same results as quantize_row_from_smem.  Requires kpad <= 4 * LEAN_V * blockDim.x; sx / xsum are
 // complete after the next CTA barrier.  ONE_TERM: p.terms is 1 (the loop and the residual drop out).
-// given_absmax: optional max|row| of term 0 supplied by the caller (sharded rows).  CLAMP: see quant4_pack.
-template <int LEAN_V, bool ONE_TERM = false, bool CLAMP = false>
+// given_absmax: optional max|row| of term 0 supplied by the caller (sharded rows).  CLAMP: see quant4_pack.  RAGGED: the row ends
+// inside its last group, at p.norm_n, and what lies behind stays zero in every term (also behind an infinity).
+template <int LEAN_V, bool ONE_TERM = false, bool CLAMP = false, bool RAGGED = false>
 __device__ __forceinline__ void lean_quantize(const LeanStage& p, float4 (&v)[LEAN_V], float* scratch, int8_t* xq,
                                               size_t tstride, float* sx, int* xsum, int& rk, int m = 0,
                                               bool writer = false, const XchScalarDev* x = nullptr,
@@ -235,6 +236,17 @@ __device__ __forceinline__ void lean_quantize(const LeanStage& p, float4 (&v)[LE
     const int n4 = p.n >> 2, k4 = p.kpad >> 2, bd = blockDim.x;
     const int terms = ONE_TERM ? 1 : p.terms;
     for (int t = 0; t < terms; ++t) {
+        if constexpr (RAGGED) {
+            if (t > 0) {
+#pragma unroll
+                for (int j = 0; j < LEAN_V; ++j) {
+                    const int i = 4 * (threadIdx.x + j * bd);
+                    if (i + 1 >= p.norm_n) v[j].y = 0.f;
+                    if (i + 2 >= p.norm_n) v[j].z = 0.f;
+                    if (i + 3 >= p.norm_n) v[j].w = 0.f;
+                }
+            }
+        }
         float mx = 0.f;
 #pragma unroll
         for (int j = 0; j < LEAN_V; ++j) mx = fmaxf(mx, amax4(v[j]));

@@ -1136,14 +1136,17 @@ size_t rotor_b200_block_workspace_bytes(const rotor_b200_model_config* cfg, int 
     return cv.off;
 }
 
+// attention: the counters and the rotary table that only it reads are made too.
 static int block_ctx(Ctx& c, const rotor_b200_model_config* cfg, int rows, void* workspace, size_t workspace_bytes,
-                     cudaStream_t st) {
+                     cudaStream_t st, bool attention) {
     int rc = block_derive(c, cfg);
     if (rc) return rc;
     Carve cv{(unsigned char*)workspace, 0};
     carve_ctx(c, cv, (size_t)rows);
     if (cv.off > workspace_bytes) return ROTOR_B200_ERR_WORKSPACE;
-    if ((rc = configure_gemv_kernels()) || (rc = configure_vec_stage()) || (rc = configure_attention())) return rc;
+    if ((rc = configure_gemv_kernels()) || (rc = configure_vec_stage())) return rc;
+    if (!attention) return ROTOR_B200_OK;
+    if ((rc = configure_attention())) return rc;
     return init_ctx(c, st);
 }
 
@@ -1193,7 +1196,7 @@ int rotor_b200_ffn_forward(const rotor_b200_model_config* cfg, const rotor_b200_
             return launch_fused_gemv(layer->down_tiles, c.d, c.ff, 1, rows, ls, y, sd, c.d, c.d, 0, st);
         }
     }
-    RB_TRY(block_ctx(c, cfg, rows, workspace, workspace_bytes, st));
+    RB_TRY(block_ctx(c, cfg, rows, workspace, workspace_bytes, st, false));
     VecStageParams e = {};
     e.mode = VS_PLAIN;
     e.n = c.d;
@@ -1232,7 +1235,7 @@ int rotor_b200_attention_forward(const rotor_b200_model_config* cfg, const rotor
     const int rows = batch * seq;
     Ctx c;
     cudaStream_t st = as_stream(stream);
-    RB_TRY(block_ctx(c, cfg, rows, workspace, workspace_bytes, st));
+    RB_TRY(block_ctx(c, cfg, rows, workspace, workspace_bytes, st, true));
     RB_TRY(launch_set_pos(c.d_pos, c.max_batch, past_len, nullptr, st));
     VecStageParams e = {};
     e.mode = VS_PLAIN;
