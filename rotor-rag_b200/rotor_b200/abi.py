@@ -200,15 +200,22 @@ def ptr(t):
 
 
 def stream():
-    import torch
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, as the address that the C ABI takes."""
+    torch = require_cuda()
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+_torch = None  # (the module, once a device has been found: the search costs 2 us a call)
 
 
 def require_cuda():
-    import torch
-    if not torch.cuda.is_available():
-        raise RotorB200Error("no CUDA device: the rotor_b200 path runs on a B200 only (no CPU fallback)")
-    return torch
+    global _torch
+    if _torch is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RotorB200Error("no CUDA device: the rotor_b200 path runs on a B200 only (no CPU fallback)")
+        _torch = torch
+    return _torch
 
 
 def set_pdl(enable: bool) -> bool:

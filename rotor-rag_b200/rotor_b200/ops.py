@@ -18,6 +18,8 @@ def to_device(a, dtype=None):
     torch = _torch()
     if isinstance(a, np.ndarray):
         a = torch.from_numpy(np.ascontiguousarray(a))
+    elif a.dtype is dtype and a.is_contiguous() and a.get_device() == torch.cuda.current_device():
+        return a             # (what the three conversions below come to; each costs about a microsecond)
     if dtype is not None:
         a = a.to(dtype)
     return a.contiguous().cuda()
@@ -138,14 +140,20 @@ def bitlinear_forward(tiles, out, inn, x, terms, wscale=1.0, wscale_vec=None, va
     """y float32 [M, out] = BitLinear(x float32 [M, in])."""
     torch = _torch()
     x = to_device(x, torch.float32)
-    m = x.shape[0]
-    need = lib.rotor_b200_bitlinear_workspace_bytes(out, inn, m, terms)
+    need = lib.rotor_b200_bitlinear_workspace_bytes(out, inn, x.shape[0], terms)
     if workspace is None or workspace.numel() < need:
         workspace = torch.empty(need, dtype=torch.uint8, device="cuda")
-    y = torch.empty((m, out), dtype=torch.float32, device="cuda")
-    check(lib.rotor_b200_bitlinear_forward(ptr(tiles), out, inn, ptr(x), m, terms, float(wscale),
-                                           ptr(wscale_vec), ptr(y), ptr(workspace), workspace.numel(),
-                                           variant, abi.stream()), "bitlinear_forward")
+    return bitlinear_into(tiles, out, inn, x, terms, float(wscale), ptr(wscale_vec), variant, workspace)
+
+
+def bitlinear_into(tiles, out, inn, x, terms, wscale, wscale_vec, variant, workspace):
+    """The call itself: x on the current device, float32 and contiguous, a workspace that is large enough."""
+    m = x.shape[0]
+    y = x.new_empty((m, out))
+    status = lib.rotor_b200_bitlinear_forward(ptr(tiles), out, inn, x.data_ptr(), m, terms, wscale, wscale_vec, y.data_ptr(),
+                                              workspace.data_ptr(), workspace.numel(), variant, abi.stream())
+    if status:
+        check(status, "bitlinear_forward")
     return y
 
 

@@ -90,6 +90,7 @@ class TernaryLinear:
         self._loaded = False
         self._cache = None
         self._workspace = None
+        self._need = (None, 0)        # scratch bytes of the last call's shape
 
     # -- loading ---------------------------------------------------------------------------
     def _tile_buffer(self):
@@ -141,15 +142,17 @@ class TernaryLinear:
     # -- compute ---------------------------------------------------------------------------
     def forward_device(self, x):
         """x: CUDA float32 [M, in] -> CUDA float32 [M, out]."""
-        torch = abi.require_cuda()
-        m = x.shape[0]
-        need = lib.rotor_b200_bitlinear_workspace_bytes(self.out_features, self.in_features, m,
-                                                        self.semantics.act_terms)
-        if self._workspace is None or self._workspace.numel() < need:
-            self._workspace = torch.empty(need, dtype=torch.uint8, device="cuda")
-        return ops.bitlinear_forward(self.tiles, self.out_features, self.in_features, x,
-                                     self.semantics.act_terms, self.scale,
-                                     variant=self.semantics.gemv_variant, workspace=self._workspace)
+        # (a call of one row is bound by the host: what Python does per call is kept to the call itself)
+        torch, sem = abi.require_cuda(), self.semantics
+        x = ops.to_device(x, torch.float32)
+        out, inn, terms = self.out_features, self.in_features, sem.act_terms
+        shape = (x.shape[0], out, inn, terms)
+        need, workspace = self._need, self._workspace
+        if need[0] != shape:
+            self._need = need = (shape, lib.rotor_b200_bitlinear_workspace_bytes(out, inn, shape[0], terms))
+        if workspace is None or workspace.numel() < need[1]:
+            self._workspace = workspace = torch.empty(need[1], dtype=torch.uint8, device="cuda")
+        return ops.bitlinear_into(self.tiles, out, inn, x, terms, float(self.scale), None, sem.gemv_variant, workspace)
 
     def forward(self, x: np.ndarray) -> np.ndarray:
         torch = abi.require_cuda()
@@ -194,9 +197,10 @@ class _BlockBase:
                                max_batch=max_batch, max_seq=max_seq, max_rows=rows,
                                gemv_variant=sem.gemv_variant)
 
-    def _workspace_for(self, cfg, rows):
+    def _workspace_for(self, cfg, rows, need=None):
         torch = abi.require_cuda()
-        need = lib.rotor_b200_block_workspace_bytes(C.byref(cfg), rows)
+        if need is None:
+            need = lib.rotor_b200_block_workspace_bytes(C.byref(cfg), rows)
         if need == 0:
             raise RotorB200Error("shape not supported by the GPU path (head_dim must be 32/64/128, "
                                  "projection widths multiples of 16)")
@@ -332,6 +336,7 @@ class GatedFFN(_BlockBase):
         self.up_proj = TernaryLinear(d_model, d_ff, semantics=semantics, _tiles=self.gate_up_tiles[n:])
         self.down_proj = TernaryLinear(d_ff, d_model, semantics=semantics, _tiles=self.down_tiles)
         self.ffn_norm = RMSNorm(d_ff, eps=semantics.eps)
+        self._call = (None, None, 0)
 
     def fill_layer_struct(self, lw: abi.LayerWeights):
         for p in (self.gate_proj, self.up_proj, self.down_proj):
@@ -345,11 +350,16 @@ class GatedFFN(_BlockBase):
         torch = abi.require_cuda()
         rows = xd.shape[0]
         sem = self.semantics
-        cfg = self._cfg_struct(sem, 1, 1, rows)
+        shape = (rows, sem, self.d_model, self.n_heads, self.n_kv_heads, self.d_ff)
+        call = self._call
+        if call[0] != shape:   # (the description of a call depends on these alone)
+            cfg = self._cfg_struct(sem, 1, 1, rows)
+            self._call = call = (shape, cfg, lib.rotor_b200_block_workspace_bytes(C.byref(cfg), rows))
+        _, cfg, need = call
         lw = abi.LayerWeights()
         self.fill_layer_struct(lw)
         y = torch.empty_like(xd)
-        ws = self._workspace_for(cfg, rows)
+        ws = self._workspace_for(cfg, rows, need)
         check(lib.rotor_b200_ffn_forward(C.byref(cfg), C.byref(lw),
                                          ptr(pre_norm.device_weight()) if pre_norm is not None else None,
                                          ptr(xd), rows, ptr(y), ptr(ws), ws.numel(), abi.stream()), "ffn_forward")
