@@ -74,10 +74,17 @@ int launch_quantize_rows(const float* x, size_t m, size_t k, int terms, int8_t* 
         }
     }
     const size_t kpad = kpad_of(k);
-    const auto lean = kpad <= 4 * 128 ? quantize_rows_lean_kernel<1, 128> : kpad <= 4 * 512 ? quantize_rows_lean_kernel<1, 512>
-                      : kpad <= 8 * 512 ? quantize_rows_lean_kernel<2, 512> : quantize_rows_lean_kernel<2, 1024>;
     if (kpad <= 8 * 1024) {
-        lean<<<(unsigned)m, kpad <= 4 * 128 ? 128 : kpad <= 8 * 512 ? 512 : 1024, 0, st>>>(x, (int)k, (int)kpad, terms, xq, sx, xsum, zero, zero_n, early);
+        const unsigned rows = (unsigned)m;
+        const int ki = (int)k, kp = (int)kpad;
+        if (kpad <= 4 * 128)
+            quantize_rows_lean_kernel<1, 128><<<rows, 128, 0, st>>>(x, ki, kp, terms, xq, sx, xsum, zero, zero_n, early);
+        else if (kpad <= 4 * 512)
+            quantize_rows_lean_kernel<1, 512><<<rows, 512, 0, st>>>(x, ki, kp, terms, xq, sx, xsum, zero, zero_n, early);
+        else if (kpad <= 8 * 512)
+            quantize_rows_lean_kernel<2, 512><<<rows, 512, 0, st>>>(x, ki, kp, terms, xq, sx, xsum, zero, zero_n, early);
+        else
+            quantize_rows_lean_kernel<2, 1024><<<rows, 1024, 0, st>>>(x, ki, kp, terms, xq, sx, xsum, zero, zero_n, early);
         return launch_status();
     }
     const int threads = k >= 4096 ? 1024 : (k >= 1024 ? 512 : 128);
