@@ -66,7 +66,20 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar) {
 // this many bytes a row: 8192 -> 28672, 8 rows (115 KB) 27.1 / 27.5 us, 5 rows of two terms (229 KB) 43.4 / 41.9, of three
 // (344 KB) 56.8 / 53.1.  The product starts early where it is one launch (4096 -> 11008, 8 rows: 10.6 against 12.6 us).
 constexpr size_t LINEAR_CLEAR_MAX = 128 * 1024;
-constexpr int ACC_MMA_COLS = 32;   // columns of one launch of the MMA variant
+constexpr int ACC_MMA_COLS = 40;   // columns of one launch of the MMA variant
+// Columns up to which the MMA variant is faster than the tiled tensor-core kernel, which takes the same time for any number up to
+// 128 but sixteen rows at a time reads its columns over and over in a large matrix.  us, MMA variant / tiled: 2560 x 2560 40 columns 6.5 /
+// 12.5, 48 9.1 / 14.1; 13824 x 2560 40 14.1 / 17.7, 48 21.9 / 20.1; 2560 x 6912 40 12.4 / 15.7, 48 19.0 / 16.9; 8192 x 8192 24 15.9 /
+// 17, 32 25.9 / 17.4; 10240 x 8192 24 18.5 / 20, 32 29.0 / 20.7; 8192 x 28672 16 30.4 / 34, 24 43.4 / 34; 57344 x 8192 16 56.1 / 62,
+// 24 77.5 / 62.
+static int acc_most_cols(size_t out, size_t in) {
+    const size_t weights = out * in;
+    return weights <= ((size_t)48 << 20) ? ACC_MMA_COLS : weights <= ((size_t)128 << 20) ? 24 : ACC_FEW_COLS;
+}
+// Whether a product takes the tiled kernels.
+static bool takes_tiles(size_t out, size_t in, size_t ncols, int variant) {
+    return variant == ROTOR_B200_VARIANT_AUTO && ncols > (size_t)acc_most_cols(out, in);
+}
 constexpr size_t LINEAR_FUSED_ROWS = 4, LINEAR_FUSED_COLS = 6;  // a stand-alone layer call in one launch: see its rule
 
 struct AccParams {
@@ -77,20 +90,32 @@ struct AccParams {
     unsigned* status;      // device word, set to ROTOR_B200_ERR_TIMEOUT on a staging timeout
     int out;
     int nkt;               // k-tiles per row of tiles
+    int nrt;               // row tiles
+    int row_tiles;         // row tiles of a CTA, one after the other against the same staged columns
     int kt_per_split;
     int ncols;
     int atomic;            // gridDim.y > 1: accumulate with integer atomics into zeroed acc
     size_t plane_stride;   // != 0: K split s stores its partial sums to acc + s*plane_stride instead
+    // whole K ranges (one split): finished float rows [y_rows][out] instead of sums, y_terms columns each
+    float* y;
+    const float *y_sx, *y_scales;
+    float y_scale;
+    int y_rows, y_terms;
 };
 
 // NT: groups of eight columns of the MMA variant.  A weight word is loaded and masked once for all of them, so that more columns
 // cost shared-memory reads and MMAs but no further pass over the matrix.  A step of the 2B shape (12 layers), a launch for every eight
 // columns / one for all: 12 sequences 843 / 734 us, 16 876 / 750, 24 1090 / 921; three terms 5 sequences 952 / 829, 8 1132 / 940.
-template <int WARPS, int UMAX, bool USE_MMA, int NCOL, int NT>
-__global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_constant__ AccParams p) {
+// FORM: what a launch needs is compiled for it alone (2B step of two sequences, 12 layers, 579 us; with the loop of ACC_MANY compiled
+// into it 623, with the finished rows 585; two groups: 96 registers let five CTAs share an SM, at 99 only four, and a step of 16
+// sequences took 759 instead of 744).
+enum { ACC_ONE = 0, ACC_MANY = 1, ACC_FINISH = 2 };  // one row tile a CTA; several (acc_row_tiles); one, finished rows
+template <int WARPS, int UMAX, bool USE_MMA, int NCOL, int NT, int FORM>
+__global__ void __launch_bounds__(WARPS * 32, NT == 2 && FORM == ACC_ONE ? 5 : 0) bitlinear_acc_kernel(const __grid_constant__ AccParams p) {
+    constexpr bool MANY = FORM == ACC_MANY;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int rt = blockIdx.x;
+    const int rt0 = MANY ? blockIdx.x * p.row_tiles : blockIdx.x, rt1 = MANY ? min(p.nrt, rt0 + p.row_tiles) : rt0 + 1;
     const int kt0 = blockIdx.y * p.kt_per_split;
     const int kt1 = min(p.nkt, kt0 + p.kt_per_split);
     const int ks = (kt1 - kt0) * TILE_K;
@@ -98,97 +123,135 @@ __global__ void __launch_bounds__(WARPS * 32) bitlinear_acc_kernel(const __grid_
     const int kbase = kt0 * TILE_K;
 
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
-    int* red = reinterpret_cast<int*>(smem_raw + 16);            // [WARPS][NT][128]
-    int8_t* xs = reinterpret_cast<int8_t*>(smem_raw + 16 + WARPS * NT * 128 * 4);
+    int* red = reinterpret_cast<int*>(smem_raw + 16);            // [WARPS][NT][128]; MANY: two of them, in turn
+    int8_t* xs = reinterpret_cast<int8_t*>(smem_raw + 16 + (MANY ? 2 : 1) * WARPS * NT * 128 * 4);
 
     stage_init(bar);
 
-    const uint4* trow = p.tiles + ((size_t)rt * p.nkt) * 32 + lane;
-
-    int accm[NT][4][4];      // MMA: [bit pair j][fragment register]
-    int accd[2][4][NCOL];    // DP4A: [row half][bit pair j][column]
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) accm[n][j][r] = 0;
-#pragma unroll
-        for (int c = 0; c < NCOL; ++c) accd[0][j][c] = accd[1][j][c] = 0;
-    }
-
-    // First batch of weight tiles is requested before the activations are waited for.
+    const uint4* trow = p.tiles + ((size_t)rt0 * p.nkt) * 32 + lane;
+    // The first batch of a row tile's weights: of the CTA's first one before the activations are waited for, of the others
+    // before the sums of the one before are put together.
     uint4 wv[UMAX];
-    int base = kt0 + warp;
+    auto first = [&]() {
+        const int base = kt0 + warp;
 #pragma unroll
-    for (int u = 0; u < UMAX; ++u)
-        if (base + u * WARPS < kt1) wv[u] = ld_stream_v4(trow + (size_t)(base + u * WARPS) * 32);
+        for (int u = 0; u < UMAX; ++u)
+            if (base + u * WARPS < kt1) wv[u] = ld_stream_v4(trow + (size_t)(base + u * WARPS) * 32);
+    };
+    first();
     pdl_wait();     // weights above are constants; everything below depends on the producer kernel
     pdl_trigger();  // after the wait: see the rule in common.cuh
     stage_issue(bar, xs, xs_stride, p.xq + (size_t)kt0 * TILE_K, (size_t)p.nkt * TILE_K, p.ncols, (uint32_t)ks);
     __syncthreads();  // mbarrier initialised, bulk copies issued
     if (!stage_wait(bar) && threadIdx.x == 0) atomicMax(p.status, (unsigned)ROTOR_B200_ERR_TIMEOUT);
 
-    while (base < kt1) {
+    int rt = rt0;
+    do {
+        int accm[NT][4][4];      // MMA: [bit pair j][fragment register]
+        int accd[2][4][NCOL];    // DP4A: [row half][bit pair j][column]
 #pragma unroll
-        for (int u = 0; u < UMAX; ++u) {
-            const int kt = base + u * WARPS;
-            if (kt < kt1) {
-                const uint32_t pw[4] = {wv[u].x, wv[u].y, wv[u].z, wv[u].w};
-                const int koff = kt * TILE_K - kbase + 32 * t;
+        for (int j = 0; j < 4; ++j) {
 #pragma unroll
-                for (int n = 0; n < NT; ++n)
-                    tile_mac<USE_MMA, NCOL>(pw, xs + (size_t)8 * n * xs_stride, xs_stride, koff, g, p.ncols - 8 * n, accm[n], accd);
-            }
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) accm[n][j][r] = 0;
+#pragma unroll
+            for (int c = 0; c < NCOL; ++c) accd[0][j][c] = accd[1][j][c] = 0;
         }
-        base += UMAX * WARPS;
+        int base = kt0 + warp;
+        while (base < kt1) {
 #pragma unroll
-        for (int u = 0; u < UMAX; ++u)
-            if (base + u * WARPS < kt1) wv[u] = ld_stream_v4(trow + (size_t)(base + u * WARPS) * 32);
-    }
+            for (int u = 0; u < UMAX; ++u) {
+                const int kt = base + u * WARPS;
+                if (kt < kt1) {
+                    const uint32_t pw[4] = {wv[u].x, wv[u].y, wv[u].z, wv[u].w};
+                    const int koff = kt * TILE_K - kbase + 32 * t;
+#pragma unroll
+                    for (int n = 0; n < NT; ++n)
+                        tile_mac<USE_MMA, NCOL>(pw, xs + (size_t)8 * n * xs_stride, xs_stride, koff, g, p.ncols - 8 * n, accm[n], accd);
+                }
+            }
+            base += UMAX * WARPS;
+#pragma unroll
+            for (int u = 0; u < UMAX; ++u)
+                if (base + u * WARPS < kt1) wv[u] = ld_stream_v4(trow + (size_t)(base + u * WARPS) * 32);
+        }
+        if (MANY && rt + 1 < rt1) {
+            trow += (size_t)p.nkt * 32;
+            first();
+        }
 
-    // exact rescale of the per-bit-pair partial sums, then reduce across the CTA
-    int* myred = red + warp * NT * 128;
-    if constexpr (USE_MMA) {
+        // exact rescale of the per-bit-pair partial sums, then reduce across the CTA
+        int* cta_red = red + (MANY ? ((rt - rt0) & 1) * WARPS * NT * 128 : 0);
+        int* myred = cta_red + warp * NT * 128;
+        if constexpr (USE_MMA) {
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int v = accm[n][0][r] + (accm[n][1][r] >> 2) + (accm[n][2][r] >> 4) + (accm[n][3][r] >> 6);
-                const int row_l = g + 8 * (r >> 1), col = 2 * t + (r & 1);
-                myred[n * 128 + row_l * 8 + col] = v;
+                for (int r = 0; r < 4; ++r) {
+                    const int v = accm[n][0][r] + (accm[n][1][r] >> 2) + (accm[n][2][r] >> 4) + (accm[n][3][r] >> 6);
+                    const int row_l = g + 8 * (r >> 1), col = 2 * t + (r & 1);
+                    myred[n * 128 + row_l * 8 + col] = v;
+                }
+        } else {
+#pragma unroll
+            for (int rh = 0; rh < 2; ++rh)
+#pragma unroll
+                for (int c = 0; c < NCOL; ++c) {
+                    int v = accd[rh][0][c] + (accd[rh][1][c] >> 2) + (accd[rh][2][c] >> 4) + (accd[rh][3][c] >> 6);
+                    v += __shfl_xor_sync(0xffffffffu, v, 1);
+                    v += __shfl_xor_sync(0xffffffffu, v, 2);
+                    if (t == 0) myred[(g + 8 * rh) * 8 + c] = v;
+                }
+        }
+        __syncthreads();  // (the other half is written next: whoever still reads this one has passed the barrier before that)
+        if constexpr (FORM == ACC_FINISH) {  // whole sums: finished rows, rounded as dequant_kernel rounds
+            for (int e = threadIdx.x; e < 16 * p.y_rows; e += WARPS * 32) {
+                const int row_l = e & 15, m = e >> 4, row = rt * TILE_ROWS + row_l;
+                if (row >= p.out) continue;
+                float v = 0.f;
+                for (int tt = 0; tt < p.y_terms; ++tt) {
+                    const int col = m * p.y_terms + tt;
+                    int s = -__ldcg(p.xsum + col);
+#pragma unroll
+                    for (int w = 0; w < WARPS; ++w) s += cta_red[(w * NT + (col >> 3)) * 128 + row_l * 8 + (col & 7)];
+                    v = __fadd_rn(v, __fmul_rn((float)s, __ldcg(p.y_sx + col)));
+                }
+                p.y[(size_t)m * p.out + row] = __fmul_rn(v, p.y_scales ? __ldg(p.y_scales + row) : p.y_scale);
             }
-    } else {
+        } else
 #pragma unroll
-        for (int rh = 0; rh < 2; ++rh)
+        for (int n = 0; n < NT; ++n) {
+            for (int e = threadIdx.x; e < 128; e += WARPS * 32) {
+                // several groups: a warp's sums of one column lie in consecutive rows (a quarter of a line an instruction)
+                const int row_l = NT > 1 ? e & 15 : e >> 3, col_l = NT > 1 ? e >> 4 : e & 7, col = 8 * n + col_l;
+                const int row = rt * TILE_ROWS + row_l;
+                if (col < p.ncols && row < p.out) {
+                    int s = 0;
 #pragma unroll
-            for (int c = 0; c < NCOL; ++c) {
-                int v = accd[rh][0][c] + (accd[rh][1][c] >> 2) + (accd[rh][2][c] >> 4) + (accd[rh][3][c] >> 6);
-                v += __shfl_xor_sync(0xffffffffu, v, 1);
-                v += __shfl_xor_sync(0xffffffffu, v, 2);
-                if (t == 0) myred[(g + 8 * rh) * 8 + c] = v;
-            }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        for (int e = threadIdx.x; e < 128; e += WARPS * 32) {
-            // several groups: a warp's sums of one column lie in consecutive rows (a quarter of a line an instruction)
-            const int row_l = NT > 1 ? e & 15 : e >> 3, col_l = NT > 1 ? e >> 4 : e & 7, col = 8 * n + col_l;
-            const int row = rt * TILE_ROWS + row_l;
-            if (col < p.ncols && row < p.out) {
-                int s = 0;
-#pragma unroll
-                for (int w = 0; w < WARPS; ++w) s += red[(w * NT + n) * 128 + row_l * 8 + col_l];
-                if (blockIdx.y == 0) s -= p.xsum[col];
-                int32_t* dst = p.acc + (size_t)blockIdx.y * p.plane_stride + (size_t)col * p.out + row;
-                if (p.atomic)
-                    atomicAdd(dst, s);
-                else
-                    *dst = s;
+                    for (int w = 0; w < WARPS; ++w) s += cta_red[(w * NT + n) * 128 + row_l * 8 + col_l];
+                    if (blockIdx.y == 0) s -= p.xsum[col];
+                    int32_t* dst = p.acc + (size_t)blockIdx.y * p.plane_stride + (size_t)col * p.out + row;
+                    if (p.atomic)
+                        atomicAdd(dst, s);
+                    else
+                        *dst = s;
+                }
             }
         }
-    }
+    } while (MANY && ++rt < rt1);
+}
+
+// Row tiles of a CTA.  One after the other against the same staged columns: a CTA a row tile copies the columns of its K
+// range for every 16 rows, which from two groups of eight on is more than the weights.  Kept small enough that the grid covers
+// the GPU.  us with 1 / 2 / 4 row tiles: 8 columns 57344 x 8192 36.4 / 35.0 / 36.1; 16 columns 8192 x 8192 14.1 / 12.2 / 11.8, 57344 x 8192
+// 71.7 / 60.4 / 56.1; 24 columns 2560 x 6912 8.7 / 7.1 / 9.4, 57344 x 8192 107.9 / 85.3 / 77.5; 40 columns 13824 x 2560 19.7 / 15.9 / 14.1.
+static int acc_row_tiles(int nrt, int ksplit, int groups) {
+    if (groups == 1) return 1;
+    const int least = groups == 2 ? 1000 : 240;  // CTAs left
+    int r = 1;
+    while (r < 4 && nrt * ksplit >= 2 * r * least) r *= 2;
+    return r;
 }
 
 __global__ void dequant_kernel(const int32_t* __restrict__ acc, const float* __restrict__ sx, int m, int terms,
@@ -205,10 +268,11 @@ __global__ void dequant_kernel(const int32_t* __restrict__ acc, const float* __r
     }
 }
 
-template <int WARPS, int UMAX, bool USE_MMA, int NCOL, int NT = 1>
-static int launch_acc(const AccParams& p, int nrt, int ksplit, cudaStream_t st) {
-    auto kern = bitlinear_acc_kernel<WARPS, UMAX, USE_MMA, NCOL, NT>;
-    const size_t smem = 16 + WARPS * NT * 128 * 4 + (size_t)p.ncols * (p.kt_per_split * TILE_K + XS_PAD);
+template <int WARPS, int UMAX, bool USE_MMA, int NCOL, int NT, int FORM>
+static int launch_acc_kind(const AccParams& p, int nrt, int ksplit, cudaStream_t st) {
+    constexpr bool MANY = FORM == ACC_MANY;
+    auto kern = bitlinear_acc_kernel<WARPS, UMAX, USE_MMA, NCOL, NT, FORM>;
+    const size_t smem = 16 + (MANY ? 2 : 1) * WARPS * NT * 128 * 4 + (size_t)p.ncols * (p.kt_per_split * TILE_K + XS_PAD);
     if (smem > 200 * 1024) return ROTOR_B200_ERR_SHAPE;
     if (smem > 48 * 1024) {
         static PerDevice<size_t> once;  // per instantiation and device
@@ -219,7 +283,7 @@ static int launch_acc(const AccParams& p, int nrt, int ksplit, cudaStream_t st) 
         }
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nrt, ksplit);
+    cfg.gridDim = dim3(MANY ? (nrt + p.row_tiles - 1) / p.row_tiles : nrt, ksplit);
     cfg.blockDim = dim3(WARPS * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -233,6 +297,20 @@ static int launch_acc(const AccParams& p, int nrt, int ksplit, cudaStream_t st) 
         return ROTOR_B200_ERR_CUDA;
     }
     return launch_status();
+}
+
+template <int WARPS, int UMAX, bool USE_MMA, int NCOL, int NT = 1>
+static int launch_acc(const AccParams& pin, int nrt, int ksplit, cudaStream_t st) {
+    AccParams p = pin;
+    p.nrt = nrt;
+    if constexpr (USE_MMA) {
+        if (p.y) return launch_acc_kind<WARPS, UMAX, USE_MMA, NCOL, NT, ACC_FINISH>(p, nrt, ksplit, st);
+    }
+    p.row_tiles = acc_row_tiles(nrt, ksplit, NT);
+    if constexpr (NT > 1) {
+        if (p.row_tiles > 1) return launch_acc_kind<WARPS, UMAX, USE_MMA, NCOL, NT, ACC_MANY>(p, nrt, ksplit, st);
+    }
+    return launch_acc_kind<WARPS, UMAX, USE_MMA, NCOL, NT, ACC_ONE>(p, nrt, ksplit, st);
 }
 
 // Split the K range over gridDim.y so that the grid covers the GPU a few times and
@@ -258,6 +336,7 @@ static int dispatch_acc(const AccParams& p, int nrt, int ksplit, int variant, cu
             case 2: return launch_acc<WARPS, UMAX, true, 1, 2>(p, nrt, ksplit, st);
             case 3: return launch_acc<WARPS, UMAX, true, 1, 3>(p, nrt, ksplit, st);
             case 4: return launch_acc<WARPS, UMAX, true, 1, 4>(p, nrt, ksplit, st);
+            case 5: return launch_acc<WARPS, UMAX, true, 1, 5>(p, nrt, ksplit, st);
         }
         return ROTOR_B200_ERR_ARG;
     }
@@ -270,10 +349,14 @@ static int dispatch_acc(const AccParams& p, int nrt, int ksplit, int variant, cu
     return ROTOR_B200_ERR_ARG;
 }
 
-template <bool USE_MMA, int NCOL, int NT = 1>
+template <bool USE_MMA, int NCOL, int NT = 1, int FORM = ACC_ONE>
 static int configure_one() {
-    RB_CUDA(cudaFuncSetAttribute(bitlinear_acc_kernel<4, 8, USE_MMA, NCOL, NT>,
+    RB_CUDA(cudaFuncSetAttribute(bitlinear_acc_kernel<4, 8, USE_MMA, NCOL, NT, FORM>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    if constexpr (FORM == ACC_ONE && USE_MMA) {
+        if (int rc = configure_one<USE_MMA, NCOL, NT, ACC_FINISH>()) return rc;
+        if constexpr (NT > 1) return configure_one<USE_MMA, NCOL, NT, ACC_MANY>();
+    }
     return ROTOR_B200_OK;
 }
 
@@ -282,7 +365,7 @@ int configure_gemv_kernels() {
     int rc = (library_status_word() ? ROTOR_B200_OK : ROTOR_B200_ERR_CUDA);
     if (rc) return rc;
     if ((rc = configure_one<true, 1>()) || (rc = configure_one<true, 1, 2>()) || (rc = configure_one<true, 1, 3>()) ||
-        (rc = configure_one<true, 1, 4>()))
+        (rc = configure_one<true, 1, 4>()) || (rc = configure_one<true, 1, 5>()))
         return rc;
     if ((rc = configure_one<false, 1>())) return rc;
     if ((rc = configure_one<false, 2>())) return rc;
@@ -310,7 +393,7 @@ GemvPlan plan_gemv(size_t out, size_t in, int ncols) {
 }
 
 bool gemv_adds(size_t out, size_t in, int ncols, const void* xq, int variant) {
-    if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO)
+    if (takes_tiles(out, in, ncols, variant))
         return gemm_tcgen05_supported(out, in, ncols, xq) && gemm_tcgen05_splits(out, in, ncols) >= 2;
     return plan_gemv(out, in, ncols).ksplit > 1;
 }
@@ -319,7 +402,7 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
                        int32_t* acc, size_t plane_stride, const GemvPlan& plan, int variant, cudaStream_t st, bool zeroed) {
     int rc = (library_status_word() ? ROTOR_B200_OK : ROTOR_B200_ERR_CUDA);
     if (rc) return rc;
-    if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO) {
+    if (takes_tiles(out, in, ncols, variant)) {
         // compute-bound regime: the tiled GEMM writes complete sums into plane 0 (callers use one plane)
         if (gemm_tcgen05_supported(out, in, ncols, xq)) return launch_gemm_tcgen05(tiles, out, in, xq, xsum, ncols, acc, st, zeroed, true);
         return launch_gemm_mma(tiles, out, in, xq, xsum, ncols, acc, st);
@@ -329,7 +412,7 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
     variant = pick_variant(variant, ncols);
     const int chunk = variant == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
     for (int c0 = 0; c0 < ncols; c0 += chunk) {
-        AccParams p;
+        AccParams p = {};
         p.tiles = (const uint4*)tiles;
         p.xq = xq + (size_t)c0 * kpad;
         p.xsum = xsum + c0;
@@ -349,6 +432,37 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
     return ROTOR_B200_OK;
 }
 
+// Whether a product can finish its rows itself: one launch of whole K ranges, where the matrix has enough row tiles and few
+// enough K tiles for that (else the K range is split and the sums are put together in memory).
+bool acc_finish_supported(size_t out, size_t in, size_t ncols, int variant) {
+    if (variant != ROTOR_B200_VARIANT_AUTO || out >= (1u << 30) || in > 49152 || ncols < 3 || ncols > (size_t)ACC_MMA_COLS || takes_tiles(out, in, ncols, variant))
+        return false;
+    const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
+    const size_t staged = ncols * (nkt * TILE_K + XS_PAD);  // (16 columns of 6912 leave one CTA an SM: feed-forward of 16 rows 22.2 -> 23.0 us)
+    return choose_ksplit(nrt, nkt, (int)ncols, 4) == 1 || (nrt >= 128 && nkt <= 64 && staged <= (nkt <= 32 ? 96 : 64) * 1024);
+}
+
+// y[rows][out] from quantised rows of `terms` columns each.
+int launch_acc_finish(const void* tiles, size_t out, size_t in, const int8_t* xq, const float* sx, const int32_t* xsum, int rows, int terms,
+                      float wscale, const float* wscale_vec, float* y, cudaStream_t st) {
+    AccParams p = {};
+    p.tiles = (const uint4*)tiles;
+    p.xq = xq;
+    p.xsum = xsum;
+    p.status = library_status_word();
+    if (!p.status) return ROTOR_B200_ERR_CUDA;
+    p.out = (int)out;
+    p.nkt = p.kt_per_split = (int)(kpad_of(in) / TILE_K);
+    p.ncols = rows * terms;
+    p.y = y;
+    p.y_sx = sx;
+    p.y_scales = wscale_vec;
+    p.y_scale = wscale;
+    p.y_rows = rows;
+    p.y_terms = terms;
+    return dispatch_acc(p, (int)(opad_of(out) / TILE_ROWS), 1, ROTOR_B200_VARIANT_MMA, st);
+}
+
 }  // namespace rb
 
 using namespace rb;
@@ -364,7 +478,7 @@ static int run_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, c
     if (rc) return rc;
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
     const size_t kpad = kpad_of(in);
-    if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO) {
+    if (takes_tiles(out, in, ncols, variant)) {
         if (gemm_tcgen05_supported(out, in, (int)ncols, xq))
             return launch_gemm_tcgen05(tiles, out, in, xq, xsum, (int)ncols, acc, st, zeroed, dependent);
         return launch_gemm_mma(tiles, out, in, xq, xsum, (int)ncols, acc, st);
@@ -378,7 +492,7 @@ static int run_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, c
     for (size_t c0 = 0; c0 < ncols; c0 += chunk) {
         const int nc = (int)((ncols - c0) < chunk ? (ncols - c0) : chunk);
         const int ksplit = choose_ksplit(nrt, nkt, nc, 4);
-        AccParams p;
+        AccParams p = {};
         p.tiles = (const uint4*)tiles;
         p.xq = xq + c0 * kpad;
         p.xsum = xsum + c0;
@@ -400,7 +514,7 @@ static int run_acc(const void* tiles, size_t out, size_t in, const int8_t* xq, c
 
 // Whether run_acc adds to acc for any of its column chunks (it then clears acc first unless it is told `zeroed`).
 static bool acc_adds(size_t out, size_t in, size_t ncols, const int8_t* xq, int variant) {
-    if (ncols >= GEMM_MIN_COLS && variant == ROTOR_B200_VARIANT_AUTO)
+    if (takes_tiles(out, in, ncols, variant))
         return gemm_tcgen05_supported(out, in, (int)ncols, xq) && gemm_tcgen05_splits(out, in, (int)ncols) >= 2;
     if (ncols <= 8 && staged_acc_supported(out, in, (int)ncols, variant)) return false;
     const size_t chunk = pick_variant(variant, (int)(ncols < 8 ? ncols : 8)) == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
@@ -477,8 +591,14 @@ int rotor_b200_bitlinear_forward(const void* tiles, size_t out, size_t in, const
     int32_t* xsum = (int32_t*)w;
     w += al256(nc * 4);
     int32_t* acc = (int32_t*)w;
+    if (((uintptr_t)tiles & 15) == 0 && acc_finish_supported(out, in, nc, variant)) {
+        // the product leaves finished rows: no sums to clear before it, no launch behind it (13 rows of 1923 -> 3001, three terms:
+        // 14.3 us a call with both, 12.2 so)
+        const int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, nullptr, 0, true, as_stream(stream));
+        return rc ? rc : launch_acc_finish(tiles, out, in, xq, sx, xsum, (int)m, terms, wscale, wscale_vec, y, as_stream(stream));
+    }
     const bool adds = out < (1u << 30) && in <= 49152 && nc * out * sizeof(int32_t) <= m * LINEAR_CLEAR_MAX && acc_adds(out, in, nc, xq, variant);
-    int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, nc < GEMM_MIN_COLS, as_stream(stream));
+    int rc = launch_quantize_rows(x, m, in, terms, xq, sx, xsum, adds ? acc : nullptr, adds ? nc * out : 0, !takes_tiles(out, in, nc, variant), as_stream(stream));
     if (rc) return rc;
     rc = run_acc(tiles, out, in, xq, xsum, nc, acc, variant, as_stream(stream), adds, true);
     if (rc) return rc;
@@ -569,7 +689,7 @@ int rotor_b200_bitlinear_forward_static(const void* tiles, size_t out, size_t in
     for (size_t c0 = 0; c0 < nc; c0 += chunk) {
         const int ncols = (int)((nc - c0) < chunk ? (nc - c0) : chunk);
         const int ksplit = choose_ksplit(nrt, nkt, ncols, 4);
-        AccParams p;
+        AccParams p = {};
         p.tiles = (const uint4*)tiles;
         p.xq = xq + c0 * kpad;
         p.xsum = xsum + c0;

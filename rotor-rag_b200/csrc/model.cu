@@ -156,8 +156,7 @@ static int gemv(Ctx& c, const void* tiles, size_t out, size_t in, int ncols, int
     // two and more columns: the K splits add into one plane, so that the register-resident row stages
     // (complete sums in one plane) can follow; one column keeps one plane per split, which the
     // generation-step stages add while they dequantise
-    const bool gemm = ncols >= GEMM_MIN_COLS && c.variant == ROTOR_B200_VARIANT_AUTO;
-    const bool one_plane = gemm || ncols >= 2;
+    const bool one_plane = ncols >= 2;
     const size_t plane_stride = one_plane ? 0 : (size_t)ncols * out;
     view->acc = acc;
     view->plane_stride = plane_stride;
@@ -313,9 +312,16 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
 }
 
 // FFN half of a block.  In: quantised pre-normed rows in xq/sx[0]/xsum[0].
-// Out: accumulators of the down projection (view *vd), activation scales in sx[1].
-static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView* vd, cudaStream_t st) {
+// Out: accumulators of the down projection (view *vd), activation scales in sx[1]; or, where `y` is given and the product can,
+// the finished rows in y (vd->acc null).
+static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView* vd, cudaStream_t st, float* y = nullptr) {
     const int cols = rows * c.terms;
+    const bool finish = y && acc_finish_supported(c.d, c.ff, cols, c.variant);
+    auto down = [&]() -> int {
+        if (!finish) return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
+        vd->acc = nullptr;
+        return launch_acc_finish(L.down_tiles, c.d, c.ff, c.xq, c.sx[1], c.xsum[1], rows, c.terms, L.down_scale, nullptr, y, st);
+    };
     if (gate_up_gates(c, cols)) {
         // prompt-sized row counts, one activation term: the gate/up product applies the gating in its epilogue and
         // writes float32 gated rows (into the accumulator area: a quarter of the bytes of the two int32 halves);
@@ -330,9 +336,9 @@ static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView
         gp.norm1 = L.ffn_sub_norm;
         gp.eps = c.eps;
         quant_sink(c, gp, 1, c.ff);
-        clear_for(c, gp, c.d, c.ff, cols, c.accB);
+        if (!finish) clear_for(c, gp, c.d, c.ff, cols, c.accB);
         RB_TRY(launch_vec_stage(gp, rows, st));
-        return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
+        return down();
     }
     AccView va;
     RB_TRY(gemv(c, L.gate_up_tiles, 2 * (size_t)c.ff, c.d, cols, 0, c.accA, &va, st));
@@ -348,9 +354,9 @@ static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView
     fp.norm1 = L.ffn_sub_norm;
     fp.eps = c.eps;
     quant_sink(c, fp, 1, c.ff);
-    clear_for(c, fp, c.d, c.ff, cols, c.accB);
+    if (!finish) clear_for(c, fp, c.d, c.ff, cols, c.accB);
     RB_TRY(launch_vec_stage(fp, rows, st));
-    return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
+    return down();
 }
 
 // Blocks [l0, l1) on the residual stream c.h, whose pre-normed quantised copy is already in
@@ -1207,7 +1213,8 @@ int rotor_b200_ffn_forward(const rotor_b200_model_config* cfg, const rotor_b200_
     clear_for_gate_up(c, e, rows * c.terms);
     RB_TRY(launch_vec_stage(e, rows, st));
     AccView vd;
-    RB_TRY(ffn_part(c, *layer, rows, &vd, st));
+    RB_TRY(ffn_part(c, *layer, rows, &vd, st, y));
+    if (!vd.acc) return ROTOR_B200_OK;
     VecStageParams o = {};
     o.mode = VS_DEQ;
     o.n = c.d;

@@ -72,9 +72,13 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
                        int32_t* acc, size_t plane_stride, const GemvPlan& plan, int variant, cudaStream_t st,
                        bool zeroed = false);
 int gemv_cols_per_launch(int variant, int ncols);
+// Products that leave finished float rows.
+bool acc_finish_supported(size_t out, size_t in, size_t ncols, int variant);
+int launch_acc_finish(const void* tiles, size_t out, size_t in, const int8_t* xq, const float* sx, const int32_t* xsum, int rows, int terms,
+                      float wscale, const float* wscale_vec, float* y, cudaStream_t st);
 
+constexpr int ACC_FEW_COLS = 16;  // columns up to which no product takes the tiled kernels
 // Many-column product (gemm_mma.cu): complete int32 sums into acc[ncols][out].
-constexpr int GEMM_MIN_COLS = 32;
 bool gemm_tcgen05_supported(size_t out, size_t in, int ncols, const void* xq);
 int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
                         int32_t* acc, cudaStream_t st, bool zeroed, bool dependent);
