@@ -785,9 +785,8 @@ static PerDevice<bool> g_tc5_ready;
 // Shapes this kernel takes: enough tokens to be worth its tile, 16-byte aligned operands.
 bool gemm_tcgen05_supported(size_t out, size_t in, int ncols, const void* xq) {
     static const bool off = getenv("ROTOR_B200_NO_TCGEN05") != nullptr;  // measurement aid: legacy mma.sync path
-    // from 32 tokens on: with fewer than 256 the tile is partly empty, but the product is then bound by
-    // the weight stream, which this kernel moves faster than the mma.sync kernel does
-    return !off && ncols >= 32 && out >= 16 && in >= 4 && ((uintptr_t)xq & 15) == 0;
+    // with fewer than 256 tokens the tile is partly empty, but the product is then bound by the weight stream
+    return !off && ncols > ACC_FEW_COLS && out >= 16 && in >= 4 && ((uintptr_t)xq & 15) == 0;
 }
 
 int configure_gemm_tcgen05() {
@@ -817,13 +816,20 @@ static bool encode_tokens(CUtensorMap* tmap, const void* xq, size_t kpad, int nc
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Whether a product goes to pairs of CTAs: tiles for every pair, or, above 128 columns, K ranges so short that splitting them
+// only adds read-backs (prompt of 200 tokens, 2B shape, 12 layers: 1851 -> 1587 us, of 300 1959 -> 1886), or a pair for every
+// fourth tile (700 tokens 2220 -> 2181; fewer tiles of long ranges are faster split: 140 tokens 1457, all paired 1532).
+static bool takes_pairs(int ncols, int nkt, int tiles256) {
+    return ncols > 128 && (2 * tiles256 >= fused_sm_count() || nkt <= 24 || tiles256 >= 20);
+}
+
 // fewer 256-row tiles than SMs: split the K range so that the grid covers the GPU (a K step of a
 // 256-row tile costs a decoder less per weight than four steps of 64-row tiles); at least four K
 // steps per CTA, partial sums added into the zeroed accumulators
 int gemm_tcgen05_splits(size_t out, size_t in, int ncols) {
     const int nkt = (int)(kpad_of(in) / TILE_K), rows = (int)opad_of(out);
     const int tiles256 = (ncols + 255) / 256 * ((rows + 255) / 256), sms = fused_sm_count();
-    int splits = tiles256 < sms ? sms / tiles256 : 1;
+    int splits = tiles256 < sms && !takes_pairs(ncols, nkt, tiles256) ? sms / tiles256 : 1;
     if (splits > nkt / 4) splits = nkt / 4;
     if (splits < 2) return 1;
     const int per = (nkt + splits - 1) / splits;
@@ -879,7 +885,7 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
     const int tok_tiles = (ncols + 255) / 256, rows = p.nrt * TILE_ROWS;
     const int sms = fused_sm_count(), tiles256 = tok_tiles * ((rows + 255) / 256);
     int splits = gemm_tcgen05_splits(out, in, ncols);
-    if (ncols > 128 && 2 * tiles256 >= sms) return launch_pair<PAIR_SUMS>(tmap, p, rows, st);
+    if (takes_pairs(ncols, p.nkt, tiles256)) return launch_pair<PAIR_SUMS>(tmap, p, rows, st);
     auto launch256 = [&](dim3 grid) {
         // (64 tokens, 57344 x 8192: 78.3 -> 66.9 us, 8192 x 28672: 44.7 -> 38.7; runs of fewer steps end before the
         // deeper look-ahead is filled and take the variant with less code)
@@ -900,7 +906,7 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
 // matrix (ff rows each, ff a multiple of 16), one activation term per token.  Writes
 // gated[token][channel] as float32; no int32 accumulator leaves the kernel.
 bool gemm_tcgen05_gated_supported(size_t ff, size_t in, int ncols, const void* xq) {
-    return ff % TILE_ROWS == 0 && ncols >= 256 && gemm_tcgen05_supported(2 * ff, in, ncols, xq);
+    return ff % TILE_ROWS == 0 && ncols > 128 && gemm_tcgen05_supported(2 * ff, in, ncols, xq);
 }
 
 int launch_gemm_tcgen05_gated(const void* tiles, size_t ff, size_t in, const int8_t* xq, const float* sx,
@@ -932,7 +938,7 @@ int launch_gemm_tcgen05_gated(const void* tiles, size_t ff, size_t in, const int
 // q/k/v product with dequantisation, rotary and the cache append in its read-back: head_dim 128, one
 // activation term per token, enough tokens for 256-row tiles to cover the GPU.
 bool gemm_tcgen05_qkv_supported(size_t dq, size_t dkv, size_t in, int head_dim, int ncols, const void* xq) {
-    return head_dim == 128 && dq % 128 == 0 && dkv % 128 == 0 && ncols >= 256 &&
+    return head_dim == 128 && dq % 128 == 0 && dkv % 128 == 0 && ncols > 128 &&
            gemm_tcgen05_supported(dq + 2 * dkv, in, ncols, xq);
 }
 
