@@ -127,6 +127,20 @@ __device__ __forceinline__ float block_max_alt(float v, float* scratch, int& k) 
     return warp_max(r);
 }
 
+// Sum of s and maximum of m (not negative, not NaN) over the CTA in one such reduction, through places of their own behind the 64
+// floats of the others: scratch holds BLOCK_SCRATCH floats.
+constexpr int BLOCK_SCRATCH = 64 + 2 * 64;
+__device__ __forceinline__ float2 block_sum_max_alt(float s, float m, float* scratch, int& k) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    float2* p = reinterpret_cast<float2*>(scratch + 64 + 64 * (k++ & 1));
+    s = warp_sum(s);
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    if (lane == 0) p[w] = make_float2(s, m);
+    __syncthreads();
+    const float2 r = lane < nw ? p[lane] : make_float2(0.f, 0.f);
+    return make_float2(warp_sum(r.x), __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(r.y))));
+}
+
 // One lane of a whole, converged warp.  The compiler knows that exactly one lane runs the guarded code and keeps the
 // operands of tcgen05 and TMA instructions in uniform registers; behind `lane == 0` every operand is moved there one by
 // one (an MMA then took about 60 cycles to issue, here 16).

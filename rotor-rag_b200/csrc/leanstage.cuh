@@ -55,10 +55,12 @@ __device__ __forceinline__ float amax4(const float4& v) {
 // running count of one-barrier reductions over it (block_sum_alt);
 // `aux`: shared floats for the attention merge weights (2 * n_heads * nsplit, LM_ATTN only).
 // All threads of the block must call.
-// PLAIN_ONLY: the caller guarantees p.mode == LM_PLAIN; the other modes' code (and registers) are left out.
-template <int LEAN_V, bool PLAIN_ONLY = false>
+// PLAIN_ONLY: the caller guarantees p.mode == LM_PLAIN; the other modes' code (and registers) are left out.  AMAX (no sharded
+// rows): a row under norm1 also gives its absolute maximum, from the reduction of its sum of squares (the norm scales every
+// element alike); else *amax is left as it was.  `scratch` then holds BLOCK_SCRATCH floats.
+template <int LEAN_V, bool PLAIN_ONLY = false, bool AMAX = false>
 __device__ __forceinline__ void lean_row(const LeanStage& p, int m, float4 (&v)[LEAN_V], float* scratch, float* aux,
-                                         bool writer, int& rk, const XchScalarDev* x = nullptr) {
+                                         bool writer, int& rk, const XchScalarDev* x = nullptr, float* amax = nullptr) {
     const int n4 = p.n >> 2, bd = blockDim.x;
     const size_t ro = (size_t)m * p.n;
 #pragma unroll
@@ -154,7 +156,20 @@ __device__ __forceinline__ void lean_row(const LeanStage& p, int m, float4 (&v)[
         const int g = threadIdx.x + j * bd;
         if (!PLAIN_ONLY && writer && p.h_out && g < n4) *reinterpret_cast<float4*>(p.h_out + ro + g * 4) = v[j];
     }
-    if (p.norm1) {
+    if (AMAX && p.norm1) {
+        float ss = 0.f, mx = 0.f;
+#pragma unroll
+        for (int j = 0; j < LEAN_V; ++j) {
+            ss += sq4(v[j]);
+            v[j] = make_float4(v[j].x * w1[j].x, v[j].y * w1[j].y, v[j].z * w1[j].z, v[j].w * w1[j].w);
+            mx = fmaxf(mx, amax4(v[j]));
+        }
+        const float2 r = block_sum_max_alt(ss, mx, scratch, rk);
+        const float inv = 1.0f / sqrtf(r.x / (float)p.n + p.eps);
+#pragma unroll
+        for (int j = 0; j < LEAN_V; ++j) v[j] = make_float4(v[j].x * inv, v[j].y * inv, v[j].z * inv, v[j].w * inv);
+        *amax = r.y * inv;
+    } else if (p.norm1) {
         float ss = 0.f;
 #pragma unroll
         for (int j = 0; j < LEAN_V; ++j) ss += sq4(v[j]);
@@ -228,7 +243,8 @@ __device__ __forceinline__ int quant4_pack(float4& v, float s, float rs, int& ls
 // complete after the next CTA barrier.  ONE_TERM: p.terms is 1 (the loop and the residual drop out).
 // given_absmax: optional max|row| of term 0 supplied by the caller (sharded rows).  CLAMP: see quant4_pack.  RAGGED: the row ends
 // inside its last group, at p.norm_n, and what lies behind stays zero in every term (also behind an infinity).
-template <int LEAN_V, bool ONE_TERM = false, bool CLAMP = false, bool RAGGED = false>
+// KNOWN: *given_absmax may hold the first term's maximum already (not negative); the caller has cleared xsum[0] before a CTA barrier.
+template <int LEAN_V, bool ONE_TERM = false, bool CLAMP = false, bool RAGGED = false, bool KNOWN = false>
 __device__ __forceinline__ void lean_quantize(const LeanStage& p, float4 (&v)[LEAN_V], float* scratch, int8_t* xq,
                                               size_t tstride, float* sx, int* xsum, int& rk, int m = 0,
                                               bool writer = false, const XchScalarDev* x = nullptr,
@@ -248,12 +264,16 @@ __device__ __forceinline__ void lean_quantize(const LeanStage& p, float4 (&v)[LE
             }
         }
         float mx = 0.f;
+        if (KNOWN && t == 0 && *given_absmax >= 0.f) {
+            mx = *given_absmax;
+        } else {
 #pragma unroll
-        for (int j = 0; j < LEAN_V; ++j) mx = fmaxf(mx, amax4(v[j]));
-        if (threadIdx.x == 0) xsum[t] = 0;  // ordered before the atomics below by the reduction's barrier
-        mx = block_max_alt(mx, scratch, rk);
+            for (int j = 0; j < LEAN_V; ++j) mx = fmaxf(mx, amax4(v[j]));
+            if (threadIdx.x == 0) xsum[t] = 0;  // ordered before the atomics below by the reduction's barrier
+            mx = block_max_alt(mx, scratch, rk);
+        }
         if (x && p.xi_max && t == 0) mx = xch_scalar(*x, p.xi_max - 1, m, mx, true, writer, scratch);
-        if (given_absmax && t == 0) mx = *given_absmax;  // the row is a slice: the whole row's maximum comes from outside
+        if (!KNOWN && given_absmax && t == 0) mx = *given_absmax;  // the row is a slice: the whole row's maximum comes from outside
         const float s = mx > 0.f ? __fdiv_rn(mx, 127.f) : 1.f;
         const float rs = __fdiv_rn(1.0f, s);
         int lsum = 0;

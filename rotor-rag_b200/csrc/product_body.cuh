@@ -68,7 +68,7 @@ inline size_t fused_smem(const FusedGemvParams& p, bool staged) {
     const size_t xs = round_up((size_t)p.cols * (p.nkt * TILE_K + XS_PAD), 16);
     const size_t aux = p.st.mode == LM_ATTN ? 2 * (size_t)p.st.n_heads * p.st.nsplit : 0;
     const size_t wide = fused_wide(p.st) ? (size_t)p.st.n : 0;
-    const size_t fixed = xs + (size_t)p.upc * p.halves * 512 + round_up((64 + aux + wide) * sizeof(float), 16);
+    const size_t fixed = xs + (size_t)p.upc * p.halves * 512 + round_up((BLOCK_SCRATCH + aux + wide) * sizeof(float), 16);
     return fixed + (staged ? fused_stage_bytes(p) : 0);
 }
 
@@ -123,12 +123,12 @@ __device__ __forceinline__ ProductCtx product_ctx(const FusedGemvParams& p, unsi
     c.slots = p.upc * p.halves;
     c.xs = reinterpret_cast<int8_t*>(smem_raw);                                      // [cols][xs_stride]
     c.merge = reinterpret_cast<int*>(smem_raw + round_up((size_t)p.cols * c.xs_stride, 16));  // [slots][128]
-    c.scratch = reinterpret_cast<float*>(c.merge + c.slots * 128);                   // [64]
-    c.aux = c.scratch + 64;                                                          // attention merge weights,
+    c.scratch = reinterpret_cast<float*>(c.merge + c.slots * 128);                   // [BLOCK_SCRATCH]
+    c.aux = c.scratch + BLOCK_SCRATCH;                                                          // attention merge weights,
                                                                                      // or the staged wide row
     const size_t auxn = p.st.mode == LM_ATTN ? 2 * (size_t)p.st.n_heads * p.st.nsplit : 0;
     c.wt = reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(c.scratch) +
-                                    round_up((64 + auxn) * sizeof(float), 16));
+                                    round_up((BLOCK_SCRATCH + auxn) * sizeof(float), 16));
     // units (row tiles / row-tile pairs) of this CTA, and the warp's share of their tiles
     // (32-bit arithmetic: units * gridDim.x stays far below 2^31)
     c.u0 = (int)((unsigned)p.units * blockIdx.x / gridDim.x);
@@ -314,10 +314,15 @@ __device__ __forceinline__ void product_run(const FusedGemvParams& p, const Prod
             const int nrows = ONE ? 1 : p.rows, terms = ONE ? 1 : p.st.terms;
             for (int m = 0; m < nrows; ++m) {
                 float4 v[V];
-                lean_row<V, PLAIN>(p.st, m, v, scratch, aux, writer, rk, x);
+                // (the norm's and the quantiser's reduction in one, where no exchange stands between them: 2B step of one sequence, 12
+                // layers, 472 -> 466 us; the row stages, which hold more of a row, spilled and took 5 % longer with the same)
+                constexpr bool JOIN = !TP && !ALONE;
+                float amax = -1.f;
+                if (JOIN && threadIdx.x == 0) s_xsum[m * terms] = 0;
+                lean_row<V, PLAIN, JOIN>(p.st, m, v, scratch, aux, writer, rk, x, &amax);
                 RB_STAMP(tr, 6);
-                lean_quantize<V, ONE, ALONE>(p.st, v, scratch, xs + (size_t)m * terms * xs_stride, (size_t)xs_stride,
-                                      s_sx + m * terms, s_xsum + m * terms, rk, m, writer, x);
+                lean_quantize<V, ONE, ALONE, false, JOIN>(p.st, v, scratch, xs + (size_t)m * terms * xs_stride, (size_t)xs_stride,
+                                                          s_sx + m * terms, s_xsum + m * terms, rk, m, writer, x, JOIN ? &amax : nullptr);
             }
         };
         if constexpr (ALONE) {
