@@ -70,6 +70,7 @@ struct Tc5Params {
     unsigned* status;
     int out, nrt, nkt, ncols;
     int kt_per_split;   // > 0: CTA z takes K steps [z kt_per_split, +kt_per_split) and ADDS its sums into zeroed acc
+    int box_rows;       // token rows of a copy
     int mt, nt;         // pairs: tiles of 256 tokens, of 256 weight rows (128 channels when gated)
     // PAIR_GATED: `tiles` holds the gate matrix followed by the up matrix (ff rows
     // each); a tile takes 128 gate rows and the matching 128 up rows, and the read-back writes
@@ -299,7 +300,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
                 if (!t5_wait(smem_u32(&s_empty[s]), ((kt / T5_STAGES) & 1) ^ 1, abort_flag, p.status, 0x7c000003u)) break;
                 const uint32_t bar = smem_u32(&s_full[s]);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                             "r"(nhalf * A_HALF)
+                             "r"(nhalf * p.box_rows * TILE_K)
                              : "memory");
                 for (int half = 0; half < nhalf; ++half) {
                     const uint32_t dst = ring + s * T5_STAGE_BYTES + half * A_HALF;
@@ -807,10 +808,11 @@ int configure_gemm_tcgen05() {
 }
 
 // The token operand: int8 rows of kpad bytes, boxes of 128 tokens x 128 bytes; rows past the last token read zeros.
-static bool encode_tokens(CUtensorMap* tmap, const void* xq, size_t kpad, int ncols) {
+// (rows: of a box, fewer where there are fewer tokens: what lies behind lands in accumulator lanes that nobody reads)
+static bool encode_tokens(CUtensorMap* tmap, const void* xq, size_t kpad, int ncols, int rows = 128) {
     const cuuint64_t gdim[2] = {(cuuint64_t)kpad, (cuuint64_t)ncols};
     const cuuint64_t gstride[1] = {(cuuint64_t)kpad};  // bytes between token rows
-    const cuuint32_t box[2] = {(cuuint32_t)TILE_K, 128u};
+    const cuuint32_t box[2] = {(cuuint32_t)TILE_K, (cuuint32_t)rows};
     const cuuint32_t estride[2] = {1u, 1u};
     return g_encode(tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(xq), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -881,7 +883,8 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
     p.ncols = ncols;
     if (!p.status) return ROTOR_B200_ERR_CUDA;
     CUtensorMap tmap;
-    if (!encode_tokens(&tmap, xq, kpad_of(in), ncols)) return ROTOR_B200_ERR_CUDA;
+    p.box_rows = ncols < 128 ? (ncols + 7) / 8 * 8 : 128;
+    if (!encode_tokens(&tmap, xq, kpad_of(in), ncols, p.box_rows)) return ROTOR_B200_ERR_CUDA;
     const int tok_tiles = (ncols + 255) / 256, rows = p.nrt * TILE_ROWS;
     const int sms = fused_sm_count(), tiles256 = tok_tiles * ((rows + 255) / 256);
     int splits = gemm_tcgen05_splits(out, in, ncols);
