@@ -7,7 +7,7 @@
 // Launch sequence of a forward, per layer run
 //   many rows:  stage (streams, norms) -> input product -> mixer -> o product -> feed-forward (with a stage in
 //               front where the sublayers follow one another)
-//   up to DENSE_FEW_ROWS rows: the stages ride in the input products' prologues
+//   up to DENSE_GEMV_ROWS rows (float32: DENSE_FEW_ROWS): the stages ride in the input products' prologues
 // Mixers, many rows / generation step
 //   bias:    [head finish ->] attention              / attention (normalises and appends its own row)
 //   latent:  [query latent norm, product (rotates) ->] finish -> expansion of the cached latents -> attention (prompts), or
@@ -249,7 +249,7 @@ struct DecoderPass {
     int expand = -1;       // latent attention: 0 absorbed, 1 expanded, -1 by what is at hand
 
     DecoderPass(Model& m_, DecoderStack& d_, int batch_, int seq_, cudaStream_t st_)
-        : m(m_), d(d_), batch(batch_), seq(seq_), rows(batch_ * seq_), f32(d_.cfg.f32), few(rows <= DENSE_FEW_ROWS && !m_.no_fused), st(st_), sg() {
+        : m(m_), d(d_), batch(batch_), seq(seq_), rows(batch_ * seq_), f32(d_.cfg.f32), few(rows <= (d_.cfg.f32 ? DENSE_FEW_ROWS : DENSE_GEMV_ROWS) && !m_.no_fused), st(st_), sg() {
         const rotor_b200_decoder_config& c = d.cfg;
         sg.streams = c.streams;
         sg.n = c.width;

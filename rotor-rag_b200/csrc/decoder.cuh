@@ -14,7 +14,11 @@
 namespace rb {
 
 constexpr int DENSE_LD = 64;       // row strides are multiples of this
-constexpr int DENSE_FEW_ROWS = 4;  // up to this many rows a product is a matrix-vector product with its stage fused in
+constexpr int DENSE_FEW_ROWS = 4;  // up to this many rows a product can be a matrix-vector product with its stage fused in
+// ... and in bf16 is, up to this many: with more rows each CTA makes every row again, and the tensor-core product of a small token
+// box is faster.  Step of 3 / 4 sequences, 6 layers, us: Likerax 825 / 926 as vectors, 738 / 731 so; Miborax 982 / 1180, 964 / 1038
+// (two take 580 / 730 as vectors, five 675 / 1046 in tiles).  float32 runs stay off the tensor cores and keep four.
+constexpr int DENSE_GEMV_ROWS = 2;
 constexpr int STREAMS_MAX = 16;
 
 inline int dense_ld(int n) { return (n + DENSE_LD - 1) / DENSE_LD * DENSE_LD; }

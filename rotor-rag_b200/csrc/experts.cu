@@ -1,6 +1,6 @@
 // Routing of many tokens to their experts: choice and weights, slots grouped by expert, the table of token
-// tiles the expert products walk, and the copy of the rows into their slots.  (Up to DENSE_FEW_ROWS tokens
-// need none of this: the matrix-vector products choose for themselves.)
+// tiles the expert products walk, and the copy of the rows into their slots.  (Up to DENSE_GEMV_ROWS tokens,
+// DENSE_FEW_ROWS in float32, need none of this: the matrix-vector products choose for themselves.)
 #include "decoder.cuh"
 
 namespace rb {
