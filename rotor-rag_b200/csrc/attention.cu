@@ -648,13 +648,16 @@ __global__ void __launch_bounds__(AC_MAX_THREADS) attn_decode_cluster_kernel(con
 // rotates its queries, the last CTA of a cluster the new k / v row, which it appends; the runs meet through distributed
 // shared memory as in the kernel above.
 //
-// Bound by the cache's stream as long as issue slots keep up, so the rows go straight to registers (a
-// row of D floats is one load of the warp, read once for all H heads) and a warp takes four keys at a time: 4 H
-// partial dot products per lane are folded over the lanes by halving (a lane hands over half of its values and keeps the
-// sums of the other half: 31 shuffles for 32 products, after which a lane holds one finished score), so that exponentials
-// are one instruction per 32 scores; the weights return through a line of shared memory.  The warps of a CTA take every
-// W-th group of four keys and merge at the end.  The next four keys are requested before the present ones are used, the
-// first before the launch wait (cached rows are older than the kernel before this one).
+// Bound by the cache's stream.  Every lane copies its D / 32 columns of a row into shared memory (cp.async) and reads back itself
+// what it copied, once for all H heads: no barrier, and a ring of stages keeps 4 to 8 KB a warp on their way at 128 registers a
+// thread, sixteen warps an SM.  (With the rows requested into registers, twelve warps and half of the bytes: 64 sequences of the XL
+// shape behind 1024 positions 151 us = 3.6 TB/s, now 117 us = 4.6 TB/s.)  Two stages up to four heads, three above: 2B shape, 12
+// layers, 8 / 16 sequences 628 / 723 us a step with two, 636 / 730 with three; XL shape, 4 layers, 64 behind 1990 positions 1809 /
+// 1781.  A warp takes four keys at a time: 4 H partial dot products per lane are folded over the lanes by halving (a lane hands over
+// half of its values and keeps the sums of the other half: 31 shuffles for 32 products, after which a lane holds one finished
+// score), so that exponentials are one instruction per 32 scores; the weights return through a line of shared memory.  The warps of
+// a CTA take every W-th group of four keys and merge at the end.  The first keys are requested before the launch wait (cached rows
+// are older than the kernel before this one).
 // A step of the 2B shape (12 layers) behind 517 positions, with a finish kernel before and the stage behind merging the runs /
 // here: 5 sequences 694 / 633 us, 8 709 / 651, 16 941 / 879, 64 1732 / 1659; XL shape (4 layers) 8 912 / 863, 64 1477 / 1461.
 constexpr int AS_KEYS = 4, AS_MAX_RUNS = 8;
@@ -662,15 +665,34 @@ constexpr int AS_KEYS = 4, AS_MAX_RUNS = 8;
 // Outputs that each of `runs` CTAs merges (the last one the rest).
 __device__ __forceinline__ int as_share(int outputs, int runs) { return (outputs / 4 + runs - 1) / runs * 4; }
 
+// E floats of a row into shared memory, zeros where the row is not one of the run's (nothing is read then).
 template <int E>
-__device__ __forceinline__ void as_load(const float* src, bool live, float (&v)[E]) {
+__device__ __forceinline__ void as_request(const float* dst, const float* src, bool live) {
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    const int bytes = live ? E * 4 : 0;
+    if constexpr (E == 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(to), "l"(src), "r"(bytes) : "memory");
+}
+
+template <int E>
+__device__ __forceinline__ void as_get(const float* src, float (&v)[E]) {
     if constexpr (E == 4) {
-        const float4 r = live ? __ldcg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 r = *reinterpret_cast<const float4*>(src);
         v[0] = r.x, v[1] = r.y, v[2] = r.z, v[3] = r.w;
     } else {
-        const float2 r = live ? __ldcg(reinterpret_cast<const float2*>(src)) : make_float2(0.f, 0.f);
+        const float2 r = *reinterpret_cast<const float2*>(src);
         v[0] = r.x, v[1] = r.y;
     }
+}
+
+template <int E>
+__device__ __forceinline__ void as_put(float* dst, const float (&v)[E]) {
+    if constexpr (E == 4)
+        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else
+        *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
 }
 
 // This lane's elements of N pieces of token row b of the q/k/v product (first columns col[], E consecutive ones a lane).
@@ -716,14 +738,20 @@ __device__ __forceinline__ void as_rotate(float (&v)[E], const float2 (&cs)[E], 
     }
 }
 
+template <int H>
+constexpr int AS_STAGES = H > 4 ? 3 : 2;
 template <int D, int H, int W>
-__global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_decode_stream_kernel(const __grid_constant__ AttnDecodeParams p) {
+constexpr int as_ring_bytes() { return W * AS_STAGES<H> * 2 * AS_KEYS * D * 4; }
+
+template <int D, int H, int W>
+__global__ void __launch_bounds__(32 * W, 16 / W) attn_decode_stream_kernel(const __grid_constant__ AttnDecodeParams p) {
     constexpr int E = D / 32, HP = H > 4 ? 8 : H > 2 ? 4 : H;      // heads, rounded up to a power of two for the folding
     constexpr int N = HP * AS_KEYS, SH = N == 32 ? 0 : N == 16 ? 1 : N == 8 ? 2 : 3;  // lane >> SH: value 4 h + key
     __shared__ __align__(16) float s_w[W][2][N];                   // weights of a group of keys
+    extern __shared__ __align__(16) float as_ring[];               // [W][STAGES][k, v][AS_KEYS][D]
+    constexpr int STAGE = 2 * AS_KEYS * D, STAGES = AS_STAGES<H>;
     __shared__ float s_a[W][HP];                                   // rescaling factors
     __shared__ float s_m[W][HP], s_l[W][HP];
-    __shared__ __align__(16) float s_o[W][H][D];
     __shared__ __align__(16) float s_q[H <= 4 ? H : 1][D];
     __shared__ __align__(16) float s_ro[H * D + 4 * AS_MAX_RUNS];  // [runs][share] the runs' outputs that this CTA merges
     __shared__ float s_rm[AS_MAX_RUNS][H], s_rl[AS_MAX_RUNS][H];   // (max, sum) of every run and head
@@ -737,15 +765,24 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_deco
     float *kc = p.k_cache + head0, *vc = p.v_cache + head0;
     const int rlen = (T + nrun - 1) / nrun, k0 = run * rlen, k1 = min(T, k0 + rlen);
 
-    float ka[AS_KEYS][E], va[AS_KEYS][E], kb[AS_KEYS][E], vb[AS_KEYS][E];
-    auto fetch = [&](int t, float (&k)[AS_KEYS][E], float (&v)[AS_KEYS][E]) {
+    // a lane reads back what it requested itself: no barrier between the two
+    float* const ring = as_ring + warp * STAGES * STAGE + E * lane;
+    constexpr int STRIDE = AS_KEYS * W;
+    auto fetch = [&](int t, int slot) {
+        if (t < k1) {
+            float* to = ring + slot * STAGE;
 #pragma unroll
-        for (int u = 0; u < AS_KEYS; ++u) as_load<E>(kc + (size_t)(t + u) * D, t + u < k1, k[u]);
-#pragma unroll
-        for (int u = 0; u < AS_KEYS; ++u) as_load<E>(vc + (size_t)(t + u) * D, t + u < k1, v[u]);
+            for (int u = 0; u < AS_KEYS; ++u) {
+                const size_t at = (size_t)min(t + u, k1 - 1) * D;
+                as_request<E>(to + u * D, kc + at, t + u < k1);
+                as_request<E>(to + (AS_KEYS + u) * D, vc + at, t + u < k1);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
     int t = k0 + AS_KEYS * warp;
-    if (t < k1) fetch(t, ka, va);
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) fetch(t + i * STRIDE, i);
     float2 cs[E] = {};
     if (p.rope) {  // (a constant table)
         const float2* r = p.rope + (size_t)min(pos, p.max_seq - 1) * (D / 2) + ((E * lane) & (D / 2 - 1));
@@ -801,19 +838,22 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_deco
         for (int e = 0; e < E; ++e) o[h][e] = 0.f;
     const int mine = lane >> SH, my_key = mine & 3, my_head = mine >> 2;
     int flip = 0;
-    auto step = [&](int left, const float (&k)[AS_KEYS][E], const float (&v)[AS_KEYS][E]) {
+    auto step = [&](int left, const float* kv) {
         float s[N];
 #pragma unroll
-        for (int h = 0; h < HP; ++h)
+        for (int u = 0; u < AS_KEYS; ++u) {
+            float k[E];
+            as_get<E>(kv + u * D, k);
 #pragma unroll
-            for (int u = 0; u < AS_KEYS; ++u) {
+            for (int h = 0; h < HP; ++h) {
                 float d = 0.f;
                 if (h < H) {
 #pragma unroll
-                    for (int e = 0; e < E; ++e) d += q[h < H ? h : 0][e] * k[u][e];
+                    for (int e = 0; e < E; ++e) d += q[h < H ? h : 0][e] * k[e];
                 }
                 s[4 * h + u] = d;
             }
+        }
 #pragma unroll
         for (int w = 16, n = N; w >= 1; w >>= 1) {
             if (n > 1) {
@@ -851,6 +891,9 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_deco
         }
         m_run = m_new;
         l_run += w;
+        float v[AS_KEYS][E];
+#pragma unroll
+        for (int u = 0; u < AS_KEYS; ++u) as_get<E>(kv + (AS_KEYS + u) * D, v[u]);
         __syncwarp();  // weights written; the other buffer's readers have passed the previous one
 #pragma unroll
         for (int h = 0; h < H; ++h) {
@@ -867,33 +910,26 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_deco
         const float ws[2] = {p.sk, p.sv};
         as_product<E, 2>(p, b, col, ws, kv);
         if (p.rope) as_rotate<E>(kv[0], cs, lane);
-#pragma unroll
-        for (int u = 0; u < AS_KEYS; ++u)
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                kb[u][e] = u ? 0.f : kv[0][e];
-                vb[u][e] = u ? 0.f : kv[1][e];
-            }
         const size_t at = (size_t)pos * D;
-        if constexpr (E == 4) {
-            *reinterpret_cast<float4*>(kc + at) = make_float4(kv[0][0], kv[0][1], kv[0][2], kv[0][3]);
-            *reinterpret_cast<float4*>(vc + at) = make_float4(kv[1][0], kv[1][1], kv[1][2], kv[1][3]);
-        } else {
-            *reinterpret_cast<float2*>(kc + at) = make_float2(kv[0][0], kv[0][1]);
-            *reinterpret_cast<float2*>(vc + at) = make_float2(kv[1][0], kv[1][1]);
+        as_put<E>(kc + at, kv[0]);
+        as_put<E>(vc + at, kv[1]);
+        float* to = ring + (STAGES - 1) * STAGE;  // (the stage that the loop requests first)
+        const float zero[E] = {};
+#pragma unroll
+        for (int u = 0; u < AS_KEYS; ++u) {
+            if (u) as_put<E>(to + u * D, zero), as_put<E>(to + (AS_KEYS + u) * D, zero);
         }
-        step(1, kb, vb);
+        as_put<E>(to, kv[0]);
+        as_put<E>(to + AS_KEYS * D, kv[1]);
+        step(1, to);
     }
-    constexpr int STRIDE = AS_KEYS * W;
-    while (t < k1) {
-        if (t + STRIDE < k1) fetch(t + STRIDE, kb, vb);
-        step(k1 - t, ka, va);
-        t += STRIDE;
-        if (t >= k1) break;
-        if (t + STRIDE < k1) fetch(t + STRIDE, ka, va);
-        step(k1 - t, kb, vb);
-        t += STRIDE;
+    for (int slot = 0; t < k1; t += STRIDE) {
+        fetch(t + (STAGES - 1) * STRIDE, slot ? slot - 1 : STAGES - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+        step(k1 - t, ring + slot * STAGE);
+        slot = slot == STAGES - 1 ? 0 : slot + 1;
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");  // (the groups behind the last are empty)
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1 << SH);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2 << SH);
     s_m[warp][my_head] = m_run;
@@ -901,7 +937,7 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_deco
 #pragma unroll
     for (int h = 0; h < H; ++h)
 #pragma unroll
-        for (int e = 0; e < E; ++e) s_o[warp][h][E * lane + e] = o[h][e];
+        for (int e = 0; e < E; ++e) ring[h * D + e] = o[h][e];
     __syncthreads();
     // ---- merge of the warps, four outputs a thread; several runs: pushed to the CTA that merges these outputs
     const int share = as_share(H * D, nrun);
@@ -916,7 +952,7 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : H >= 5 ? 3 : 4) attn_deco
 #pragma unroll
         for (int w = 0; w < W; ++w) {
             const float f = s_m[w][h] == -INFINITY ? 0.f : __expf(s_m[w][h] - M);
-            const float4 v = *reinterpret_cast<const float4*>(&s_o[w][h][d]);
+            const float4 v = *reinterpret_cast<const float4*>(as_ring + w * STAGES * STAGE + h * D + d);
             acc.x += f * v.x, acc.y += f * v.y, acc.z += f * v.z, acc.w += f * v.w;
             L += f * s_l[w][h];
         }
@@ -955,26 +991,29 @@ bool attn_decode_stream_ok(int n_heads, int n_kv_heads, int head_dim) {
     return n_heads / n_kv_heads <= AC_MAX_GROUP;
 }
 
-// Runs per sequence.  Every CTA of the launch should be resident at once (three an SM above four heads, else four), with a tenth
-// of the places left because a cluster needs its places in one GPC: a CTA more than fit costs a second round.  Eight where
-// few sequences leave room for them, else at most six (clusters of seven and eight spread worse).  us a step behind
-// 1900 positions with 1 / 2 / 3 / 4 / 5 / 6 / 8 runs: 2B shape, four layers, 5 sequences 534 / 415 / 358 / 349 / 341 / 333 / 324,
-// 8 sequences 542 / 420 / 381 / 362 / 353 / 350 / 367, 16 sequences 564 / 493 / 461 / 490 / 473 / 462 / 513, 24 sequences 672 /
-// 570 / 605 / 570 / 646 / 624 / 592; XL shape, two layers, 5 sequences 838 / 727 / 705 / 671 / 657 / 646 / 624, 16 sequences
-// 1151 / 969 / 896 / 976 / 934 / 906 / 932.
-// Where only whole sequences fit, long caches (the host does not know the present lengths) are cut all the same: 2B shape, 64
-// sequences, one / three runs 993 / 942 behind 1900 positions, 527 / 548 behind 70; XL shape, 40 sequences, one / two 1033 / 1019,
-// 767 / 784.  More sequences than fit: up to 2048 CTAs while the cache's capacity leaves a run 64 positions, so that the last
-// round is short.
-static int attn_stream_runs(int batch, int n_kv_heads, int group, int max_seq) {
-    const long n = (long)batch * n_kv_heads, sms = fused_sm_count(), places = sms * (group >= 5 ? 3 : 4) * 9 / 10;
-    if (n * 8 <= (group >= 5 ? places : 2 * sms)) return 8;
-    for (int s = 6; s > 1; --s)
-        if (n * s <= places) return s;
-    if (n <= places) return max_seq < 1024 ? 1 : group >= 5 ? 2 : 3;
-    int s = 1;
-    while (2 * s <= AS_MAX_RUNS && n * 2 * s <= 2048 && max_seq / (2 * s) >= 64) s *= 2;
-    return s;
+// Runs per sequence and warps per CTA: one round of CTAs, sixteen warps an SM.  Two CTAs of eight warps an SM where the launch
+// fits so, cut into up to eight runs (above two runs a tenth of the places stays free, because a cluster needs its places in one
+// GPC).  us a step behind 1900 positions, four warps a CTA with the best number of runs / eight warps so: 2B shape, four layers, 10
+// sequences 380 / 359, 20 456 / 447, 40 663 / 636, 56 822 / 788; XL shape, two layers, 3 724 / 703, 16 750 / 746, 32 858 / 852.
+// Else four CTAs of four warps.  Where only whole sequences fit, long caches (the host does not know the present lengths) are cut
+// all the same: 2B shape, 64 sequences, one / three runs 919 / 862 behind 1900 positions, 470 / 488 behind 70; XL shape, 40
+// sequences, one / two 1060 / 954 behind 1900, 802 / 788 behind 500, 722 / 735 behind 70; 64 sequences 1091 / 1069, 834 / 849.  More sequences than fit: up to 2048 CTAs while the cache's capacity leaves a run 64
+// positions, so that the last round is short.
+struct AsPlan {
+    int runs;
+    bool wide;  // eight warps a CTA
+};
+
+static AsPlan attn_stream_plan(int batch, int n_kv_heads, int group, int max_seq) {
+    const long n = (long)batch * n_kv_heads, two = 2L * fused_sm_count();
+    int s = AS_MAX_RUNS;
+    if (n <= two) {
+        while (s > 1 && n * s > (s > 2 ? two * 9 / 10 : two)) --s;
+        return {s, true};
+    }
+    if (n <= 2 * two) return group >= 5 ? AsPlan{max_seq < (2 * n <= 3 * two ? 512 : 1024) ? 1 : 2, false} : AsPlan{max_seq < 1024 ? 1 : 3, false};
+    for (s = 1; 2 * s <= AS_MAX_RUNS && n * 2 * s <= 2048 && max_seq / (2 * s) >= 64;) s *= 2;
+    return {s, false};
 }
 
 template <int D, int H, int W>
@@ -982,6 +1021,7 @@ static int launch_attn_decode_stream_k(const AttnDecodeParams& p, int batch, int
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(runs, p.n_kv_heads, batch);
     cfg.blockDim = dim3(32 * W);
+    cfg.dynamicSmemBytes = as_ring_bytes<D, H, W>();
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -999,28 +1039,28 @@ static int launch_attn_decode_stream_k(const AttnDecodeParams& p, int batch, int
     return launch_status();
 }
 
-template <int D>
+template <int D, int H>
+static int configure_attn_stream() {
+    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<D, H, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (as_ring_bytes<D, H, 4>())));
+    RB_CUDA(cudaFuncSetAttribute(attn_decode_stream_kernel<D, H, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (as_ring_bytes<D, H, 8>())));
+    if constexpr (H < AC_MAX_GROUP) return configure_attn_stream<D, H + 1>();
+    return ROTOR_B200_OK;
+}
+
+template <int D, int H>
 static int launch_attn_decode_stream_d(const AttnDecodeParams& p, int batch, cudaStream_t st) {
-    const int G = p.n_heads / p.n_kv_heads, runs = attn_stream_runs(batch, p.n_kv_heads, G, p.max_seq);
-    // eight warps a CTA where two CTAs an SM hold the launch: 8 sequences of the 2B shape (12 layers) behind 70 / 517 / 1000 / 1990
-    // positions 615 / 651 / 701 / 777 us a step, with four warps 616 / 675 / 749 / 887
-    const bool wide = (long)runs * p.n_kv_heads * batch <= 2 * fused_sm_count();
-    switch (G) {
-        case 1: return launch_attn_decode_stream_k<D, 1, 4>(p, batch, runs, st);
-        case 2: return launch_attn_decode_stream_k<D, 2, 4>(p, batch, runs, st);
-        case 3: return launch_attn_decode_stream_k<D, 3, 4>(p, batch, runs, st);
-        case 4: return wide ? launch_attn_decode_stream_k<D, 4, 8>(p, batch, runs, st) : launch_attn_decode_stream_k<D, 4, 4>(p, batch, runs, st);
-        case 5: return launch_attn_decode_stream_k<D, 5, 4>(p, batch, runs, st);
-        case 6: return launch_attn_decode_stream_k<D, 6, 4>(p, batch, runs, st);
-        case 7: return launch_attn_decode_stream_k<D, 7, 4>(p, batch, runs, st);
-        case 8: return launch_attn_decode_stream_k<D, 8, 4>(p, batch, runs, st);
+    const int G = p.n_heads / p.n_kv_heads;
+    if (G != H) {
+        if constexpr (H < AC_MAX_GROUP) return launch_attn_decode_stream_d<D, H + 1>(p, batch, st);
+        return ROTOR_B200_ERR_SHAPE;
     }
-    return ROTOR_B200_ERR_SHAPE;
+    const AsPlan plan = attn_stream_plan(batch, p.n_kv_heads, G, p.max_seq);
+    return plan.wide ? launch_attn_decode_stream_k<D, H, 8>(p, batch, plan.runs, st) : launch_attn_decode_stream_k<D, H, 4>(p, batch, plan.runs, st);
 }
 
 int launch_attn_decode_stream(const AttnDecodeParams& p, int batch, cudaStream_t st) {
     if (!p.acc.acc || !p.attn_out || !attn_decode_stream_ok(p.n_heads, p.n_kv_heads, p.head_dim)) return ROTOR_B200_ERR_ARG;
-    return p.head_dim == 64 ? launch_attn_decode_stream_d<64>(p, batch, st) : launch_attn_decode_stream_d<128>(p, batch, st);
+    return p.head_dim == 64 ? launch_attn_decode_stream_d<64, 1>(p, batch, st) : launch_attn_decode_stream_d<128, 1>(p, batch, st);
 }
 
 static size_t attn_cluster_smem(int G, int D, int lcmax, int ns) {
@@ -1191,6 +1231,8 @@ int configure_attention() {
                                  cudaSharedmemCarveoutMaxShared));
     RB_CUDA(cudaFuncSetAttribute(attn_decode_cluster_kernel<128, 16>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared));
+    if (int rc = configure_attn_stream<64, 1>()) return rc;
+    if (int rc = configure_attn_stream<128, 1>()) return rc;
     if (int rc = configure_attn_prefill_t5()) return rc;
     return configure_attn_prefill_tc();
 }

@@ -589,13 +589,14 @@ def test_batched_steps_equal_single_sequences(rb, shape, batch, context):
 
 @pytest.mark.parametrize("heads,kv,batch,context,capacity", [(4, 1, 5, 0, 4), (4, 1, 7, 3, 5), (8, 2, 20, 37, 39), (12, 4, 16, 41, 43),
                                                             (8, 1, 17, 26, 28), (20, 5, 8, 47, 49), (20, 5, 8, 6, 700), (20, 5, 24, 9, 11),
-                                                            (16, 2, 64, 21, 23), (8, 8, 40, 19, 1500), (16, 8, 90, 11, 300)])
+                                                            (16, 2, 64, 21, 23), (8, 8, 40, 19, 1500), (16, 8, 90, 11, 300),
+                                                            (32, 4, 8, 333, 335), (20, 4, 35, 150, 152), (8, 8, 37, 65, 67), (16, 2, 150, 97, 600)])
 def test_runs_of_batched_steps(rb, heads, kv, batch, context, capacity):
-    """Steps whose sequences are cut into every number of runs that the rule gives (one to six, eight), with empty runs, runs that
+    """Steps whose sequences are cut into every number of runs that the rule gives, with empty runs, rings that wrap, runs that
     are no multiple of a warp's keys and outputs that do not divide by the runs, against each sequence alone.  Two steps: the
     second reads the row that the first appended.  Three activation terms: float32 rounding is all that may differ."""
     import torch
-    cfg = dict(vocab_size=512, d_model=heads * 64 if heads != 20 else 2560, n_layers=1, n_heads=heads, n_kv_heads=kv, d_ff=512)
+    cfg = dict(vocab_size=512, d_model=heads * (128 if heads in (20, 32) else 64), n_layers=1, n_heads=heads, n_kv_heads=kv, d_ff=512)
     model = rb.synth.random_model_on_device(cfg, seed=batch, semantics=rb.sem.REFERENCE, max_seq=capacity, max_batch=batch, max_rows=batch)
     g = torch.Generator(device="cuda")
     g.manual_seed(heads + batch)
