@@ -16,6 +16,10 @@
 // the output columns): scale, distance bias and mask in float32, row maximum (halves exchanged through
 // shared memory), exponentials (base 2), the running output O = O * alpha + O_j in registers, one tile
 // behind the scores.  Warps 8 and 9: TMA of K and V; warp 10: MMA issue, one tile ahead with S.
+// Rows find their position and head by a multiplication, and a warp arrives at a barrier once (256 arrivals on one word are taken
+// in turn): 8 x 2048 positions of 20 heads of 128 over 5 KV heads in chunks of 1024, with divisions and an arrival a thread / so:
+// 248 / 231 us; 16 heads with 64 shared key columns 293 / 270.  Bound by the chain of a row tile (an item of one key tile takes 7 us,
+// every further tile 1.5, of which the tensor cores work 0.6); a CTA per SM that walks the items was no faster (253).
 // Waits are bounded; a wait that runs out records a code in the library status word, the CTA stops
 // issuing work, frees its tensor memory and returns.  No multicast, this GPU's memory only.
 #include <cstdlib>
@@ -72,6 +76,8 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
     const uint32_t qbase = (smem_u32(b5_raw) + 1023u) & ~1023u, kring = qbase + C::Q_BYTES, vring = kring + 2 * C::K_BYTES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.heads / p.kv_heads, QT = B5_BM / G;
+    const uint32_t per_row = (65536u + G - 1) / G;  // r / G = r per_row >> 16 for the 128 rows
+    auto position_of = [&](int r) { return (int)((uint32_t)r * per_row >> 16); };
     const int qt = gridDim.x - 1 - blockIdx.x;  // late query tiles tend to see more keys: start them first
     const int hk = blockIdx.y, b = blockIdx.z, s0 = qt * QT;
     const int past = cached_len(p.past_len, b, p.max_seq);
@@ -91,11 +97,11 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             t5_bar_init(smem_u32(&s_vfull[s]), 1);
             t5_bar_init(smem_u32(&s_vempty[s]), 1);
             t5_bar_init(smem_u32(&s_sfull[s]), 1);
-            t5_bar_init(smem_u32(&s_pfull[s]), B5_SOFT);
+            t5_bar_init(smem_u32(&s_pfull[s]), B5_SOFT / 32);
             t5_bar_init(smem_u32(&s_ofull[s]), 1);
-            t5_bar_init(smem_u32(&s_oempty[s]), B5_SOFT);
+            t5_bar_init(smem_u32(&s_oempty[s]), B5_SOFT / 32);
         }
-        t5_bar_init(smem_u32(&s_qready), B5_SOFT);
+        t5_bar_init(smem_u32(&s_qready), B5_SOFT / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 8) {
@@ -115,7 +121,7 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
 #pragma unroll
             for (int u = 0; u < QN; ++u) {
                 const int idx = threadIdx.x + u * B5_SOFT, r = idx / (DQ / 8), c8 = idx - r * (DQ / 8);
-                const int sp = r / G, s = s0 + sp, gi = r - sp * G;
+                const int sp = position_of(r), s = s0 + sp, gi = r - sp * G;
                 // own key columns, then the shared ones; what lies between in a panel is zero
                 const int col = c8 < DK / 8 ? c8 * 8 : p.kd + c8 * 8 - DK;
                 const bool on = c8 < DK / 8 ? col < p.kd : col < qd;
@@ -132,11 +138,12 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                              : "memory");
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> tensor-core reads
-            t5_bar_arrive(smem_u32(&s_qready));
+            __syncwarp();
+            if (lane == 0) t5_bar_arrive(smem_u32(&s_qready));
         }
         constexpr int DH = DV / 2;  // output columns of this thread
         const int half = warp >> 2, wq = warp & 3, r = wq * 32 + lane;
-        const int sp = min(r / G, QT - 1), gi = r - (r / G) * G;
+        const int sp = min(position_of(r), QT - 1), gi = r - position_of(r) * G;
         const int pos = past + min(s0 + sp, s_last);
         const int lo = first_visible(pos, p.chunk, p.window), hi = pos;  // visible keys [lo, hi]
         const float slope2 = p.slopes ? __ldg(p.slopes + hk * G + gi) * 1.4426950408889634f : 0.f;
@@ -160,7 +167,8 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 for (int i = 0; i < 32; ++i) o[c + i] = o[c + i] * alpha + __uint_as_float(v[i]);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            t5_bar_arrive(smem_u32(&s_oempty[j & 1]));
+            __syncwarp();
+            if (lane == 0) t5_bar_arrive(smem_u32(&s_oempty[j & 1]));
             return true;
         };
         // (the eight warps leave this loop together: whether to go on is decided by one thread between the
@@ -216,7 +224,8 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             t5_st32(sbuf + (uint32_t)half * 32u, pk);  // 128 bf16 weights in columns [0, 64) of the S buffer
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            t5_bar_arrive(smem_u32(&s_pfull[j & 1]));
+            __syncwarp();
+            if (lane == 0) t5_bar_arrive(smem_u32(&s_pfull[j & 1]));
             l_run = l_run * alpha + sum;
             m_run = m_new;
             if (j > 0) ok = accumulate(j - 1, alpha_prev);
@@ -237,7 +246,7 @@ attn_bias_t5_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             const uint32_t blk = kring + (uint32_t)warp * T5_XPOSE_BYTES;
             const int cpl = lane & (DV == 128 ? 7 : 3);  // 16-byte piece this lane stores
             auto dst_of = [&](int tl) -> void* {
-                const int r2 = wq * 32 + tl, sp2 = r2 / G, s2 = s0 + sp2, col = half * DH + cpl * 8;
+                const int r2 = wq * 32 + tl, sp2 = position_of(r2), s2 = s0 + sp2, col = half * DH + cpl * 8;
                 if (sp2 >= QT || s2 >= p.seq || col >= p.vdim) return nullptr;
                 return p.out + ((size_t)b * p.seq + s2) * p.ld_out + (size_t)(hk * G + r2 - sp2 * G) * p.vdim + half * DH;
             };
