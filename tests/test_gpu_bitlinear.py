@@ -200,6 +200,38 @@ def test_layer_call_equals_its_three_parts(ops, abi, out, inn, rows, terms):
     abi.device_status()
 
 
+@pytest.mark.parametrize("out,inn", [(3001, 1924), (600, 9216), (18432, 2560)])
+@pytest.mark.parametrize("cols", [8, 9, 16, 17, 24, 25, 31, 32, 40, 41])
+def test_products_of_a_few_dozen_columns(ops, abi, out, inn, cols):
+    """One row tile a CTA, several, and the tensor-core tiles, on either side of every column count where the rule changes:
+    the integers against a float64 product, in which they are exact; then the layer call, whose product may finish the rows,
+    against its three parts to the bit, with one scale and one per output, rows off a 16-byte boundary, a row of zeros and rows
+    with an infinity and a NaN."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(out + cols)
+    w = torch.randint(-1, 2, (out, inn), generator=g, device="cuda", dtype=torch.int8)
+    tiles = ops.int8_to_tiles(w)
+    q = torch.zeros((cols, abi.lib.rotor_b200_in_padded(inn)), dtype=torch.int8, device="cuda")
+    q[:, :inn] = torch.randint(-128, 128, (cols, inn), generator=g, device="cuda", dtype=torch.int8)
+    acc = ops.bitlinear_acc(tiles, out, inn, q, q.sum(1, dtype=torch.int32), abi.VARIANT_AUTO)
+    assert torch.equal(acc.double(), q[:, :inn].double() @ w.double().T)
+    x = torch.randn(cols * inn + 1, generator=g, device="cuda")[1:].view(cols, inn)
+    x[1], x[2, 5], x[3, inn - 1] = 0.0, float("inf"), float("nan")
+    vec = torch.rand(out, generator=g, device="cuda")
+    for terms in (1, 3):
+        rows = x[:max(1, cols // terms)]
+        xq, sx, xsum = ops.quantize_rows(rows.clone(), terms)
+        parts = ops.bitlinear_acc(tiles, out, inn, xq, xsum, abi.VARIANT_DP4A)
+        for scales in (None, vec):
+            want = torch.empty((len(rows), out), device="cuda")
+            abi.check(abi.lib.rotor_b200_bitlinear_dequant(abi.ptr(parts), abi.ptr(sx), len(rows), terms, out, 0.037,
+                                                           None if scales is None else abi.ptr(scales), abi.ptr(want), abi.stream()))
+            got = ops.bitlinear_forward(tiles, out, inn, rows, terms, 0.037, wscale_vec=scales)
+            assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0)), (terms, scales is None)
+    abi.device_status()
+
+
 def test_tcgen05_extreme_values(ops, abi):
     """-128 x -1 and 127 x +1 over K = 6912 on the tcgen05 path: sums stay exact in int32."""
     out, inn, ncols = 256, 6912, 256

@@ -276,6 +276,28 @@ def test_experts(n, top, ff, width, dtype):
         assert rel(y.cpu().numpy()[clear, :width], want[clear]) < (5e-6 if dtype == "float32" else 1.5e-2), rows
 
 
+@pytest.mark.parametrize("n,top", [(7, 1), (40, 8), (64, 6), (150, 32)])
+def test_routing_in_one_launch_and_in_several(n, top):
+    """Up to 32 rows are routed by one block, more by three launches: the same rows alone and with one more behind them, whose
+    tiles hold other slots (bf16 outputs of float32 sums of at most `top` experts: one rounding may differ)."""
+    import torch
+    from rotor_b200 import abi
+    g, width = np.random.default_rng(n), 232
+    m = M.make(M.config([M.window(4, mlp=M.experts(n, top, 40))], width=width, vocab=8), seed=1)
+    model = M.load(m, dtype="bfloat16", max_seq=33, max_rows=33)
+    cfg, layer = model._ensure_handle(1, 33, 33).cfg, model._layers[0]
+    need = abi.lib.rotor_b200_decoder_layer_workspace_bytes(C.byref(cfg), C.byref(layer))
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    h = dev(bf16(g.standard_normal((33, width))), "bfloat16", ld(width))
+    out = {}
+    for rows in (33, 32, 31, 5, 3, 32):
+        y = torch.zeros((rows, ld(width)), device="cuda")
+        abi.check(abi.lib.rotor_b200_experts(C.byref(cfg), C.byref(layer), abi.ptr(h), rows, abi.ptr(y), abi.ptr(ws), need, abi.stream()))
+        abi.device_status()
+        out[rows] = y.cpu().numpy()[:, :width]
+        assert rel(out[rows], out[33][:rows]) < 4e-3, rows
+
+
 # ------------------------------------------------------------------------------- whole models
 CONFIGS = {
     "mixed": lambda: M.config([M.window(24), M.window(17, kv_from=0, heads=2, dim=28, vdim=36), M.full(),
