@@ -6,7 +6,7 @@
 namespace rb {
 
 template <int TERMS, int PLANES>
-__device__ __forceinline__ float deq_acc_t(const AccView& a, const float* __restrict__ sx, int m, int o, float wscale) {
+__device__ __forceinline__ float deq_acc_t(const AccView& a, const float* sx, int m, int o, float wscale) {
     int s[TERMS];
     float f[TERMS];
 #pragma unroll
@@ -25,7 +25,7 @@ __device__ __forceinline__ float deq_acc_t(const AccView& a, const float* __rest
 
 // Dequantised element o of token row m.  The common (terms, planes) pairs are straight-line
 // code so that independent calls overlap their loads.
-__device__ __forceinline__ float deq_acc(const AccView& a, const float* __restrict__ sx, int m, int terms, int o,
+__device__ __forceinline__ float deq_acc(const AccView& a, const float* sx, int m, int terms, int o,
                                          float wscale) {
     if (a.planes == 1) {
         if (terms == 1) return deq_acc_t<1, 1>(a, sx, m, o, wscale);

@@ -254,17 +254,17 @@ static int acc_row_tiles(int nrt, int ksplit, int groups) {
     return r;
 }
 
-__global__ void dequant_kernel(const int32_t* __restrict__ acc, const float* __restrict__ sx, int m, int terms,
-                               int out, float wscale, const float* __restrict__ wscale_vec,
-                               float* __restrict__ y) {
+__global__ void dequant_kernel(const int32_t* acc, const float* sx, int m, int terms,
+                               int out, float wscale, const float* wscale_vec,
+                               float* y) {
     pdl_wait();
     const size_t total = (size_t)m * out;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int r = (int)(i / out), o = (int)(i % out);
         float v = 0.f;
         for (int tt = 0; tt < terms; ++tt)
-            v = __fadd_rn(v, __fmul_rn((float)acc[((size_t)r * terms + tt) * out + o], sx[r * terms + tt]));
-        y[i] = __fmul_rn(v, wscale_vec ? wscale_vec[o] : wscale);
+            v = __fadd_rn(v, __fmul_rn((float)__ldcg(acc + ((size_t)r * terms + tt) * out + o), __ldcg(sx + r * terms + tt)));
+        y[i] = __fmul_rn(v, wscale_vec ? __ldg(wscale_vec + o) : wscale);
     }
 }
 

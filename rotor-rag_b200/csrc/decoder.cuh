@@ -295,7 +295,7 @@ inline int launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
 #ifdef __CUDACC__
 // Cached length of sequence b, kept inside the cache whatever the word holds.
 __device__ __forceinline__ int cached_len(const int* past_len, int b, int max_seq) {
-    return min(max(__ldg(past_len + b), 0), max_seq - 1);
+    return min(max(__ldcg(past_len + b), 0), max_seq - 1);
 }
 // First position the query at `pos` sees.
 __device__ __forceinline__ int first_visible(int pos, int chunk, int window) {

@@ -89,7 +89,7 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     volatile int* abort_flag = &s_abort;
     const int nk = (p.k + 63) >> 6;
     if (p.table) pdl_wait();  // (the table is the work of the kernel before; without one only the weights are read ahead)
-    const int mt = p.table ? __ldg(p.table) : p.mt, per_group = mt * p.nt, ntiles = per_group * p.groups;
+    const int mt = p.table ? __ldcg(p.table) : p.mt, per_group = mt * p.nt, ntiles = per_group * p.groups;
 
     if (threadIdx.x == 0) {
         s_abort = 0;
@@ -122,9 +122,9 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         const int m = block * 16 + (r - o.n * bm);
         if (p.table) {
             const int* e = p.table + 1 + 3 * m;
-            o.group = __ldg(e);
-            o.x_row = o.row0 = __ldg(e + 1);
-            o.rows = __ldg(e + 2);
+            o.group = __ldcg(e);
+            o.x_row = o.row0 = __ldcg(e + 1);
+            o.rows = __ldcg(e + 2);
             o.x_col = o.y_col = 0;
         } else {
             o.x_row = o.group * p.gx_row + m * 128;
@@ -221,7 +221,7 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 }
             } else if constexpr (EPI == DENSE_HALF) {
                 float gate = 1.f;
-                if (p.head_gate && tok0 + lane < tok_end) gate = sigmoid(__ldg(p.head_gate + (size_t)(tok0 + lane) * p.ld_head_gate + at.group));
+                if (p.head_gate && tok0 + lane < tok_end) gate = sigmoid(__ldcg(p.head_gate + (size_t)(tok0 + lane) * p.ld_head_gate + at.group));
 #pragma unroll 1
                 for (int c = 0; c < BN / 32; ++c) {
                     const int col = n * TN + c * 32;

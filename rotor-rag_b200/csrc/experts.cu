@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(const __grid_constan
         auto fetch = [&](int c0) {
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (c0 + 32 * u + lane < pieces) v[u] = __ldg(src + c0 + 32 * u + lane);
+                if (c0 + 32 * u + lane < pieces) v[u] = __ldcg(src + c0 + 32 * u + lane);
         };
         fetch(0);
         int slot = 0;
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(ROUTE_TH) route_few_kernel(const __grid_consta
     for (int p = blockIdx.x; p < pairs; p += gridDim.x) {
         const int row = p / r.top, e = chosen[p], slot = first_of[e] + __popc(mask[e] & ((1u << row) - 1u));
         if (threadIdx.x == 0) r.slot_of[p] = slot;
-        for (int c = threadIdx.x; c < pieces; c += ROUTE_TH) permuted[(size_t)slot * pieces + c] = __ldg(x + (size_t)row * pieces + c);
+        for (int c = threadIdx.x; c < pieces; c += ROUTE_TH) permuted[(size_t)slot * pieces + c] = __ldcg(x + (size_t)row * pieces + c);
     }
 }
 

@@ -250,7 +250,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
                         const int tok_base = tok0 + half * 128 + wq * 32;
                         // remove the +1 of the codes: once per output, i.e. in the first K split only
                         const uint32_t xs =
-                            ((p.kt_per_split && blockIdx.z) || token >= p.ncols) ? 0u : (uint32_t)__ldg(p.xsum + token);
+                            ((p.kt_per_split && blockIdx.z) || token >= p.ncols) ? 0u : (uint32_t)__ldcg(p.xsum + token);
 #pragma unroll
                         for (int q = 0; q < 32; ++q) v[q] -= xs;
                         if (p.kt_per_split) {  // one of several partial sums: exact, in any order

@@ -42,3 +42,43 @@ def test_trigger_follows_wait(file, name):
         assert re.search(name + r"(<[^;()]*>)?<<<", text) and not re.search(r"cudaLaunchKernelEx\([^;]*\b" + name, text), name
     else:
         assert len(waits) >= len(triggers) and all(w < t for w, t in zip(waits, triggers)), name
+
+
+#: What no kernel of a call writes: weights and their scales, norms, tables, biases.  (r, rope, cs: (cos, sin) pairs.)
+CONSTANTS = {"p.embed", "p.norm", "p.norm0", "p.norm1", "p.pro_norm", "p.st.norm1", "a.st.norm", "s.norm", "norm", "w", "b", "p.rope", "rope", "r",
+             "cs", "cs4", "p.slopes", "p.sinks", "r.bias", "p.y_scales", "wscale_vec"}
+
+
+def read_only(text):
+    """Arguments of the non-coherent loads of a piece of source: the pointer that each starts from."""
+    for m in re.finditer(r"\b__ldg\(", text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[i], 0)
+            i += 1
+        yield re.sub(r"^[&(]+", "", re.sub(r"reinterpret_cast<[^<>]*>\s*\(", "", text[m.end():i - 1])).lstrip("(& ")
+
+
+def pointer(argument):
+    return re.match(r"[\w.]+", argument).group(0)
+
+
+@pytest.mark.parametrize("file,name", [(f, n) for f, n, b, _ in FOUND if "pdl_wait()" in b])
+def test_dependent_kernels_read_what_others_write_with_coherent_loads(file, name):
+    """A dependent kernel starts before the one in front of it has ended, so what that one writes is not read-only for the
+    kernel's life, which a non-coherent load (__ldg, or a const __restrict__ parameter) takes for granted: it could be moved over
+    the wait."""
+    path = os.path.join(CSRC, file)
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    body = next(b for f, n, b, _ in FOUND if (f, n) == (file, name))
+    head = re.search(r"\b" + name + r"\s*\(((?:[^()]|\([^()]*\))*)\)\s*\{", text).group(1)
+    assert not re.search(r"const[^,]*__restrict__", head), head
+    assert {pointer(a) for a in read_only(body)} <= CONSTANTS, name
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*.cuh"))), ids=os.path.basename)
+def test_shared_device_code_reads_only_constants_with_non_coherent_loads(path):
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    assert {pointer(a) for a in read_only(text)} <= CONSTANTS | {"p"}   # (p: ldg4, whose calls are below)
+    for m in re.finditer(r"\bldg4\(([\w.]+)", text):
+        assert m.group(1) in CONSTANTS | {"const"}, m.group(0)
