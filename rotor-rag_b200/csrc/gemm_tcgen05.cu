@@ -408,8 +408,15 @@ __device__ __forceinline__ uint32_t pr_lead(uint32_t bar) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(bar));
     return r;
 }
+// Release at cluster scope: what this CTA's decoders wrote to its shared memory is read by an MMA that a thread of the other CTA
+// issues (which waits with an acquire of that scope).  Restricted to shared memory: the unrestricted form also waits for the
+// weights that the warp has requested ahead (13824 x 2560, 16384 tokens, int32 sums: 742 us, so 400; one thread of CTA 1 that
+// passes its warps' arrivals on 867).
 __device__ __forceinline__ void pr_arrive(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+    asm volatile(
+        "fence.release.sync_restrict::shared::cta.cluster;\n\t"
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar)
+        : "memory");
 }
 __device__ __forceinline__ void pr_commit(uint32_t bar) {  // to the same barrier of both CTAs
     asm volatile(
@@ -555,7 +562,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
             int m, n;
             place(t, m, n);
             const int buf = lt & 1, tok_base = m * 256 + rank * 128 + wq * 32, token = tok_base + lane;
-            const bool good = t5_wait(smem_u32(&s_accf[buf]), (lt >> 1) & 1, abort_flag, p.status, 0x7c000012u);
+            const bool good = t5_wait<true>(smem_u32(&s_accf[buf]), (lt >> 1) & 1, abort_flag, p.status, 0x7c000012u);
             if (!__all_sync(0xffffffffu, good)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)buf * 256u;
@@ -732,11 +739,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
             bool ok = true;
             for (int t = pair0; t < ntiles && ok; t += pairs, ++lt) {
                 const int buf = lt & 1;
-                ok = t5_wait(smem_u32(&s_acce[buf]), ((lt >> 1) & 1) ^ 1, abort_flag, p.status, 0x7c000014u);
+                ok = t5_wait<true>(smem_u32(&s_acce[buf]), ((lt >> 1) & 1) ^ 1, abort_flag, p.status, 0x7c000014u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int kt = 0; kt < nk; ++kt) {
-                    ok = t5_wait(smem_u32(&s_full[s]), parity, abort_flag, p.status, 0x7c000015u);
+                    ok = t5_wait<true>(smem_u32(&s_full[s]), parity, abort_flag, p.status, 0x7c000015u);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t da = t5_desc(ring + s * PR_STAGE), db = t5_desc(ring + s * PR_STAGE + PR_HALF);

@@ -11,16 +11,26 @@ namespace rb {
 
 constexpr long long T5_SPIN_CYCLES = 400000000LL;  // about 0.2 s
 
+// PEER: the barrier counts arrivals of another CTA of the cluster, whose writes to shared memory before them are seen once the wait
+// returns (the unqualified forms of arrive and wait order memory within one CTA only).
+template <bool PEER = false>
 __device__ __forceinline__ bool t5_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status,
                                         unsigned code) {
     long long t0 = 0;
     for (int it = 0;; ++it) {
         uint32_t ok;
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
+        if constexpr (PEER)
+            asm volatile(
+                "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                : "=r"(ok)
+                : "r"(bar), "r"(parity)
+                : "memory");
+        else
+            asm volatile(
+                "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                : "=r"(ok)
+                : "r"(bar), "r"(parity)
+                : "memory");
         if (ok) return true;
         if (*abort_flag) return false;
         if (it == 0) t0 = clock64();

@@ -82,3 +82,22 @@ def test_shared_device_code_reads_only_constants_with_non_coherent_loads(path):
     assert {pointer(a) for a in read_only(text)} <= CONSTANTS | {"p"}   # (p: ldg4, whose calls are below)
     for m in re.finditer(r"\bldg4\(([\w.]+)", text):
         assert m.group(1) in CONSTANTS | {"const"}, m.group(0)
+
+
+def test_arrivals_at_another_ctas_barrier_release_at_cluster_scope():
+    """An arrival without a scope orders memory within one CTA only: what a CTA writes for the other one of a pair needs the release
+    of the whole cluster, and the waits that count such arrivals the acquire."""
+    found = 0
+    for path in glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"asm volatile\(((?:[^()\"]|\"[^\"]*\"|\([^()]*\))*)\)", text):
+            arrive = re.search(r"mbarrier\.arrive([.\w:]*)\.shared::cluster", m.group(1))
+            if not arrive or "tcgen05.commit" in m.group(1):
+                continue
+            found += 1
+            fence = re.search(r"fence\.release\.sync_restrict::shared::cta\.cluster;", m.group(1)[:arrive.start()])
+            assert ".release.cluster" in arrive.group(1) or (fence and ".relaxed.cluster" in arrive.group(1)), m.group(1)
+    assert found
+    body = next(b for _, n, b, _ in FOUND if n == "gemm_pair_kernel")
+    waits = re.findall(r"t5_wait(<true>)?\(smem_u32\(&(s_full|s_acce|s_accf)\[", body)
+    assert {bar for _, bar in waits} == {"s_full", "s_acce", "s_accf"} and all(peer for peer, _ in waits)
