@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(TH, TH > 512 ? 1 : TH > 256 ? (V <= 4 ? 2 : 1)
     }  // rows of this CTA
 }
 
-// Whether the register-resident kernel takes this stage: enough rows, complete accumulators in
-// one plane, 16-byte aligned rows, no sharded-row statistics.
+// Whether the register-resident kernel takes this stage: enough rows, complete accumulators in one plane, rows and norm
+// weights on 16-byte boundaries.
 bool row_stage_supported(const VecStageParams& p, int rows) {
     static const bool off = getenv("ROTOR_B200_NO_ROWSTAGE") != nullptr;  // comparison aid
     if (off || rows < RS_MIN_ROWS) return false;
@@ -302,6 +302,9 @@ bool row_stage_supported(const VecStageParams& p, int rows) {
         return false;
     const bool from_acc = p.mode == VS_OPROJ || p.mode == VS_FFN || p.mode == VS_DOWN || p.mode == VS_DEQ;
     if (from_acc && (p.acc.planes != 1 || p.acc.out % 4 || p.terms < 1 || p.terms > 3)) return false;
+    // the kernel reads and writes groups of four elements; what callers hand over may start at any of them
+    const uintptr_t floats = (uintptr_t)p.src | (uintptr_t)p.norm0 | (uintptr_t)p.norm1 | (uintptr_t)p.h | (uintptr_t)p.h_out | (uintptr_t)p.y_out;
+    if ((floats | (uintptr_t)p.acc.acc) & 15 || (uintptr_t)p.embed & 7 || (uintptr_t)p.xq & 3) return false;
     const bool resid = p.mode == VS_OPROJ || p.mode == VS_DOWN;
     const int widest = resid ? 4 * 16 * RS_THREADS : 4 * 14 * RS_WIDE_THREADS;  // 8192, or 28672 without a residual row
     if (p.n % 4 || p.n > widest) return false;

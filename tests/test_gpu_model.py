@@ -747,3 +747,72 @@ def test_prompt_rows_of_many_equal_few(rb, d):
     for b in range(2):
         want = model.forward_last_logits_device(ids[b:b + 1])[0]
         assert rel_err(got[b].cpu().numpy(), want[0].cpu().numpy()) < 1e-5, b
+
+
+def _off(t):
+    """The same values, four bytes behind a 16-byte boundary."""
+    import torch
+    return torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 300])
+def test_rmsnorm_off_a_16_byte_boundary(rb, rows):
+    """Rows, weights and results that start at any float: the register stage moves four at a time and leaves these to the other."""
+    import torch
+    abi, n = rb.tr.abi, 2560
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    x, w = torch.randn((rows, n), generator=g, device="cuda"), torch.rand(n, generator=g, device="cuda")
+    want = x.double() / (x.double().square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double()
+    for which in range(8):
+        a, b, y = (_off(t) if which >> i & 1 else t.clone() for i, t in enumerate((x, w, torch.empty_like(x))))
+        abi.check(abi.lib.rotor_b200_rmsnorm(abi.ptr(a), rows, n, abi.ptr(b), 1e-6, abi.ptr(y), abi.stream()))
+        abi.device_status()
+        assert (y.double() - want).norm() < 1e-6 * want.norm(), which   # a few float32 roundings
+
+
+@pytest.mark.parametrize("batch,seq", [(1, 1), (2, 1), (4, 1), (1, 3), (5, 1), (1, 300)])
+def test_attention_rows_off_a_16_byte_boundary(rb, batch, seq):
+    """Rows in, rows out and the sub-norm's weights at any float, against the same rows on a boundary.  Three activation terms: other
+    stages round float32 sums of 256 in another order, and a term's quantiser moves by that."""
+    import ctypes as C
+    import torch
+    abi, d = rb.tr.abi, 256
+    at, _ = _attention_layer(rb, d, 4, 2, batch + seq, semantics=rb.sem.REFERENCE, max_seq=seq, max_batch=batch)
+    at.attn_norm.weight = (1 + 0.1 * np.random.default_rng(seq).standard_normal(d)).astype(np.float32)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seq)
+    x = torch.randn((batch * seq, d), generator=g, device="cuda")
+    cfg, lw = at._cfg_struct(at.semantics, batch, seq, batch * seq), abi.LayerWeights()
+    at.fill_layer_struct(lw)
+    ws, norm, out = at._workspace_for(cfg, batch * seq), at.attn_norm.device_weight(), []
+    for place in (torch.clone, _off):
+        a, w, y = place(x), place(norm), place(torch.empty_like(x))
+        lw.attn_sub_norm = abi.ptr(w)
+        abi.check(abi.lib.rotor_b200_attention_forward(C.byref(cfg), C.byref(lw), abi.ptr(a), batch, seq, 0, abi.ptr(y), abi.ptr(ws), ws.numel(),
+                                                       abi.stream()))
+        abi.device_status()
+        out.append(y.double())
+    assert (out[1] - out[0]).norm() < 1e-5 * out[0].norm()
+
+
+@pytest.mark.parametrize("rows", [3, 4, 5, 9, 300])
+def test_ffn_rows_off_a_16_byte_boundary(rb, rows):
+    """The same of the feed-forward, whose row norm and sub-norm may start anywhere too."""
+    import torch
+    d, ff = 512, 1536
+    ffn, pre = rb.tr.GatedFFN(d, ff, semantics=rb.sem.REFERENCE), rb.tr.RMSNorm(d)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(rows)
+    for p in (ffn.gate_proj, ffn.up_proj, ffn.down_proj):
+        p.load_from_int8(torch.randint(-1, 2, (p.out_features, p.in_features), generator=g, device="cuda", dtype=torch.int8), 0.02)
+    norms = [torch.rand(n, generator=g, device="cuda") + 0.5 for n in (d, ff)]
+    x = torch.randn((rows, d), generator=g, device="cuda")
+    out = []
+    for place in (torch.clone, _off):
+        for norm, w in zip((pre, ffn.ffn_norm), norms):
+            held = place(w)
+            norm.device_weight = lambda held=held: held
+        out.append(ffn.forward_device(place(x), pre_norm=pre).double())
+        rb.tr.abi.device_status()
+    assert (out[1] - out[0]).norm() < 1e-5 * out[0].norm()
