@@ -1170,10 +1170,11 @@ int rotor_b200_ffn_forward(const rotor_b200_model_config* cfg, const rotor_b200_
     Ctx c;
     cudaStream_t st = as_stream(stream);
     {
-        // a few token rows: two launches, the vector stages ride in the products' prologues
+        // a few token rows: two launches, the vector stages ride in the products' prologues (which read four floats at a time)
         RB_TRY(block_derive(c, cfg));
         static const bool off = getenv("ROTOR_B200_NO_FUSED_STEP") != nullptr;
-        if (!off && rows <= FUSED_MAX_ROWS && c.terms <= 3 && rows * c.terms <= 8 && c.ff % 16 == 0 &&
+        const bool aligned = (((uintptr_t)x | (uintptr_t)pre_norm | (uintptr_t)layer->ffn_sub_norm) & 15) == 0;
+        if (!off && aligned && rows <= FUSED_MAX_ROWS && c.terms <= 3 && rows * c.terms <= 8 && c.ff % 16 == 0 &&
             fused_gemv_supported(c.ff, c.d, rows, c.terms, 2, 0) && fused_gemv_supported(c.d, c.ff, rows, c.terms, 1, 0)) {
             Carve cv{(unsigned char*)workspace, 0};
             carve_ctx(c, cv, (size_t)rows);
