@@ -267,8 +267,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
                                         if (rbase + q < p.out) atomicAdd(dst + q, (int32_t)v[q]);
                                 }
                             } else {
-                                t5_add_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
-                                            (size_t)p.out, p.out - rbase, tok_base, p.ncols, lane);
+                                t5_put_rows<true>(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
+                                                  (size_t)p.out, p.out - rbase, tok_base, p.ncols, lane);
                             }
                         } else if (rbase + 32 <= p.out && (p.out & 3) == 0) {
                             t5_store_rows(ring + (uint32_t)warp * T5_XPOSE_BYTES, v, p.acc + (size_t)tok_base * p.out + rbase,
@@ -687,11 +687,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
                     for (int q = 0; q < 32; ++q) v[q] -= (uint32_t)xs;
                     if (rbase + 32 <= p.out && (p.out & 3) == 0) {
                         t5_store_rows(stage, v, p.acc + (size_t)tok_base * p.out + rbase, (size_t)p.out * sizeof(int32_t), tok_base, p.ncols, lane);
-                    } else if (live) {
-                        int32_t* dst = p.acc + (size_t)token * p.out + rbase;
-#pragma unroll
-                        for (int q = 0; q < 32; ++q)
-                            if (rbase + q < p.out) dst[q] = (int32_t)v[q];
+                    } else {
+                        t5_put_rows<false>(stage, v, p.acc + (size_t)tok_base * p.out + rbase, (size_t)p.out, p.out - rbase, tok_base, p.ncols, lane);
                     }
                 }
             }
@@ -826,10 +823,20 @@ static bool encode_tokens(CUtensorMap* tmap, const void* xq, size_t kpad, int nc
 }
 
 // Whether a product goes to pairs of CTAs: tiles for every pair, or, above 128 columns, K ranges so short that splitting them
-// only adds read-backs (prompt of 200 tokens, 2B shape, 12 layers: 1851 -> 1587 us, of 300 1959 -> 1886), or a pair for every
-// fourth tile (700 tokens 2220 -> 2181; fewer tiles of long ranges are faster split: 140 tokens 1457, all paired 1532).
-static bool takes_pairs(int ncols, int nkt, int tiles256) {
-    return ncols > 128 && (2 * tiles256 >= fused_sm_count() || nkt <= 24 || tiles256 >= 20);
+// only adds read-backs, or a pair for every fourth tile whose K range is not too long for the pairs that are left idle.  us of a layer
+// call, split / paired: 3840 x 2560 129 columns 24.9 / 22.8, 1500 65.8 / 55.6; 1000 x 1000 256 29.1 / 18.8; 4096 x 4096 (16 tiles) 129
+// 25.0 / 26.9, (32) 257 37.3 / 29.1; 8192 x 8192 (32) 129 35.2 / 39.4, 144 39.1 / 41.3, 168 43.4 / 41.5, (64) 257 55.7 / 45.4; 2560 x
+// 6912 (10) 256 33.2 / 35.1, (20) 300 37.3 / 36.9, (40) 903 53.7 / 47.4; 4096 x 11008 (16) 256 43.7 / 49.8, (32) 257 49.6 / 51.0, (64) 903
+// 92.5 / 81.7; 8192 x 28672 (32) 129 66.0 / 95.4, 256 83.3 / 104.0, (64) 257 112.8 / 102.7.  A whole tile a CTA / paired, 57344 x
+// 8192: 129 145.7 / 151.9, 257 242.0 / 253.5, 512 328 / 306, 1500 824 / 761.  Rows of sums off a 16-byte boundary leave
+// a value at a time and take longer: 3001 x 1923 129 23.2 / 26.9, 168 31.2 / 28.5; 8001 x 8190 (32) 256 47.5 / 51.8, (64) 257 55.9 /
+// 52.8; 2562 x 6912 (33) 700 47.5 / 49.5, (44) 903 53.7 / 53.1; 999 x 8000 (24) 1500 53.4 / 59.7; too short a K range to be split
+// (5003 x 777) 192 25.0 / 29.0, 300 33.0 / 29.0.
+static bool takes_pairs(size_t out, int ncols, int nkt, int tiles256) {
+    const bool ragged = out & 3;
+    if (ncols <= 128 || 2 * tiles256 >= fused_sm_count()) return ncols > 128;
+    if (nkt <= 24) return !ragged || ncols > (nkt < 8 ? 256 : 144);
+    return tiles256 >= (ragged ? 40 : 20) && nkt <= 4 * tiles256 && ncols > 144;
 }
 
 // fewer 256-row tiles than SMs: split the K range so that the grid covers the GPU (a K step of a
@@ -838,7 +845,7 @@ static bool takes_pairs(int ncols, int nkt, int tiles256) {
 int gemm_tcgen05_splits(size_t out, size_t in, int ncols) {
     const int nkt = (int)(kpad_of(in) / TILE_K), rows = (int)opad_of(out);
     const int tiles256 = (ncols + 255) / 256 * ((rows + 255) / 256), sms = fused_sm_count();
-    int splits = tiles256 < sms && !takes_pairs(ncols, nkt, tiles256) ? sms / tiles256 : 1;
+    int splits = tiles256 < sms && !takes_pairs(out, ncols, nkt, tiles256) ? sms / tiles256 : 1;
     if (splits > nkt / 4) splits = nkt / 4;
     if (splits < 2) return 1;
     const int per = (nkt + splits - 1) / splits;
@@ -895,7 +902,7 @@ int launch_gemm_tcgen05(const void* tiles, size_t out, size_t in, const int8_t* 
     const int tok_tiles = (ncols + 255) / 256, rows = p.nrt * TILE_ROWS;
     const int sms = fused_sm_count(), tiles256 = tok_tiles * ((rows + 255) / 256);
     int splits = gemm_tcgen05_splits(out, in, ncols);
-    if (takes_pairs(ncols, p.nkt, tiles256)) return launch_pair<PAIR_SUMS>(tmap, p, rows, st);
+    if (takes_pairs(out, ncols, p.nkt, tiles256)) return launch_pair<PAIR_SUMS>(tmap, p, rows, st);
     auto launch256 = [&](dim3 grid) {
         // (64 tokens, 57344 x 8192: 78.3 -> 66.9 us, 8192 x 28672: 44.7 -> 38.7; runs of fewer steps end before the
         // deeper look-ahead is filled and take the variant with less code)

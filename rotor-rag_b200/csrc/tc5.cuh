@@ -96,8 +96,9 @@ __device__ __forceinline__ void t5_store_rows(uint32_t stage, const uint32_t (&v
     __syncwarp();  // the block is rewritten by the warp's next item
 }
 
-// The same block of int32 sums, added to what is there: a token's 32 values are one line per instruction.
-__device__ __forceinline__ void t5_add_rows(uint32_t stage, const uint32_t (&v)[32], int32_t* dst0, size_t row_ints, int n,
+// The same block of int32 sums, n of the 32 at any address, a token's values one instruction: stored, or (ADD) added to what is there.
+template <bool ADD>
+__device__ __forceinline__ void t5_put_rows(uint32_t stage, const uint32_t (&v)[32], int32_t* dst0, size_t row_ints, int n,
                                             int tok_base, int ntok, int lane) {
 #pragma unroll
     for (int q = 0; q < 8; ++q)
@@ -110,7 +111,13 @@ __device__ __forceinline__ void t5_add_rows(uint32_t stage, const uint32_t (&v)[
         uint32_t w;
         asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(stage + (uint32_t)tl * 144u + 4u * lane));
         if (tok_base + tl >= ntok) break;  // warp-uniform
-        if (lane < n) atomicAdd(dst0 + (size_t)tl * row_ints + lane, (int32_t)w);
+        if (lane < n) {
+            int32_t* dst = dst0 + (size_t)tl * row_ints + lane;
+            if constexpr (ADD)
+                atomicAdd(dst, (int32_t)w);
+            else
+                *dst = (int32_t)w;
+        }
     }
     __syncwarp();
 }
