@@ -96,7 +96,7 @@ def test_dense_linear_more_tiles_than_sms(rows, n, k, gated):
     _dense(rows, n, k, gated, "bfloat16")
 
 
-@pytest.mark.parametrize("rows", [3, 31, 32, 33])
+@pytest.mark.parametrize("rows", [3, 5, 25, 26, 31, 32, 33])
 @pytest.mark.parametrize("n,k,gated", [(200, 136, 1), (10000, 776, 0), (40, 5000, 0), (5000, 200, 1)])
 def test_dense_linear_around_the_small_token_box(rows, n, k, gated):
     _dense(rows, n, k, gated, "bfloat16")
