@@ -249,7 +249,7 @@ struct DecoderPass {
     int expand = -1;       // latent attention: 0 absorbed, 1 expanded, -1 by what is at hand
 
     DecoderPass(Model& m_, DecoderStack& d_, int batch_, int seq_, cudaStream_t st_)
-        : m(m_), d(d_), batch(batch_), seq(seq_), rows(batch_ * seq_), f32(d_.cfg.f32), few(rows <= (d_.cfg.f32 ? DENSE_FEW_ROWS : DENSE_GEMV_ROWS) && !m_.no_fused), st(st_), sg() {
+        : m(m_), d(d_), batch(batch_), seq(seq_), rows(batch_ * seq_), f32(d_.cfg.f32), few(rows <= dense_gemv_rows(d_.cfg.f32) && !m_.no_fused), st(st_), sg() {
         const rotor_b200_decoder_config& c = d.cfg;
         sg.streams = c.streams;
         sg.n = c.width;
@@ -790,7 +790,8 @@ int rotor_b200_dense_linear(const void* w, int n, int k, const void* x, int rows
     }
     RB_TRY(configure_dense());
     cudaStream_t st = as_stream(stream);
-    if (dense_gemv_supported(p, rows)) return launch_dense_gemv(p, rows, st);
+    const bool few = rows <= dense_gemv_rows(f32) || (!f32 && !dense_gemm_t5_supported(p, rows));
+    if (few && dense_gemv_supported(p, rows)) return launch_dense_gemv(p, rows, st);
     return f32 ? launch_dense_gemm_f32(p, rows, scratch, st) : launch_dense_gemm_t5(p, rows, st);
 }
 

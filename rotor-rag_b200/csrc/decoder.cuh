@@ -19,6 +19,7 @@ constexpr int DENSE_FEW_ROWS = 4;  // up to this many rows a product can be a ma
 // box is faster.  Step of 3 / 4 sequences, 6 layers, us: Likerax 825 / 926 as vectors, 738 / 731 so; Miborax 982 / 1180, 964 / 1038
 // (two take 580 / 730 as vectors, five 675 / 1046 in tiles).  float32 runs stay off the tensor cores and keep four.
 constexpr int DENSE_GEMV_ROWS = 2;
+inline int dense_gemv_rows(bool f32) { return f32 ? DENSE_FEW_ROWS : DENSE_GEMV_ROWS; }
 constexpr int STREAMS_MAX = 16;
 
 inline int dense_ld(int n) { return (n + DENSE_LD - 1) / DENSE_LD * DENSE_LD; }
