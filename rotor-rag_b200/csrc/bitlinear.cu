@@ -433,13 +433,19 @@ int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* x
 }
 
 // Whether a product can finish its rows itself: one launch of whole K ranges, where the matrix has enough row tiles and few
-// enough K tiles for that (else the K range is split and the sums are put together in memory).
+// enough K tiles for that (else the K range is split and the sums are put together in memory).  The staged columns have to leave an SM
+// room for three CTAs, or, where one round of two an SM takes all row tiles, for two.  us of a layer call, sums in memory / finished:
+// 1000 x 1000 5-40 columns 10.5 / 8.2-9; 2560 x 2560 8 10.7 / 8.1, 32 11.4 / 10.7; 13824 x 2560 8 12.5 / 8.9, 17 14.8 / 14.7, 24 14.8 /
+// 16.2; 4096 x 4096 16 10.9 / 8.7, 20 12.5 / 10.7; 6144 x 4096 16 13.5 / 10.4, 20 12.7 / 16.6; 16384 x 4096 13 20.4 / 18.6, 17 20.9 /
+// 23.0, 20 20.9 / 27.0; 22016 x 4096 16 23.0 / 20.9, 20 27.1 / 32.9; 2560 x 6912 9 10.9 / 10.7, 17 12.7 / 18.8; 8192 x 8192 6 13.0 /
+// 12.2, 8 14.0 / 14.5, 16 18.6 / 26.8; 4096 x 11008 6 16.8 / 14.5, 12 18.9 / 21.7.
 bool acc_finish_supported(size_t out, size_t in, size_t ncols, int variant) {
     if (variant != ROTOR_B200_VARIANT_AUTO || out >= (1u << 30) || in > 49152 || ncols < 3 || ncols > (size_t)ACC_MMA_COLS || takes_tiles(out, in, ncols, variant))
         return false;
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
     const size_t staged = ncols * (nkt * TILE_K + XS_PAD);  // (16 columns of 6912 leave one CTA an SM: feed-forward of 16 rows 22.2 -> 23.0 us)
-    return choose_ksplit(nrt, nkt, (int)ncols, 4) == 1 || (nrt >= 128 && nkt <= 64 && staged <= (nkt <= 32 ? 96 : 64) * 1024);
+    const size_t most = nkt > 32 ? 64 : nrt <= 2 * fused_sm_count() ? 96 : 68;  // KB
+    return choose_ksplit(nrt, nkt, (int)ncols, 4) == 1 || (nrt >= 128 && nkt <= 64 && staged <= most * 1024);
 }
 
 // y[rows][out] from quantised rows of `terms` columns each.
