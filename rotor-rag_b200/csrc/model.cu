@@ -316,12 +316,6 @@ static int attention_part(Ctx& c, const rotor_b200_layer_weights& L, int batch, 
 // the finished rows in y (vd->acc null).
 static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView* vd, cudaStream_t st, float* y = nullptr) {
     const int cols = rows * c.terms;
-    const bool finish = y && acc_finish_supported(c.d, c.ff, cols, c.variant);
-    auto down = [&]() -> int {
-        if (!finish) return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
-        vd->acc = nullptr;
-        return launch_acc_finish(L.down_tiles, c.d, c.ff, c.xq, c.sx[1], c.xsum[1], rows, c.terms, L.down_scale, nullptr, y, st);
-    };
     if (gate_up_gates(c, cols)) {
         // prompt-sized row counts, one activation term: the gate/up product applies the gating in its epilogue and
         // writes float32 gated rows (into the accumulator area: a quarter of the bytes of the two int32 halves);
@@ -336,9 +330,9 @@ static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView
         gp.norm1 = L.ffn_sub_norm;
         gp.eps = c.eps;
         quant_sink(c, gp, 1, c.ff);
-        if (!finish) clear_for(c, gp, c.d, c.ff, cols, c.accB);
+        clear_for(c, gp, c.d, c.ff, cols, c.accB);
         RB_TRY(launch_vec_stage(gp, rows, st));
-        return down();
+        return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
     }
     AccView va;
     RB_TRY(gemv(c, L.gate_up_tiles, 2 * (size_t)c.ff, c.d, cols, 0, c.accA, &va, st));
@@ -354,9 +348,12 @@ static int ffn_part(Ctx& c, const rotor_b200_layer_weights& L, int rows, AccView
     fp.norm1 = L.ffn_sub_norm;
     fp.eps = c.eps;
     quant_sink(c, fp, 1, c.ff);
+    const bool finish = y && acc_finish_supported(c.d, c.ff, cols, c.variant);
     if (!finish) clear_for(c, fp, c.d, c.ff, cols, c.accB);
     RB_TRY(launch_vec_stage(fp, rows, st));
-    return down();
+    if (!finish) return gemv(c, L.down_tiles, c.d, c.ff, cols, 1, c.accB, vd, st);
+    vd->acc = nullptr;
+    return launch_acc_finish(L.down_tiles, c.d, c.ff, c.xq, c.sx[1], c.xsum[1], rows, c.terms, L.down_scale, nullptr, y, st);
 }
 
 // Blocks [l0, l1) on the residual stream c.h, whose pre-normed quantised copy is already in

@@ -458,8 +458,8 @@ def test_empty_and_single_element_inputs(rb):
 
 @pytest.mark.parametrize("batch", [2, 9, 17])
 def test_batched_decode_step(rb, batch):
-    """One-token steps for several sequences at once against the oracle run sequence by sequence.
-    Sixteen sequences and more take the tiled attention kernel instead of the split decode kernel."""
+    """One-token steps for several sequences at once against the oracle run sequence by sequence: two and more go through the
+    attention that takes several sequences in one launch."""
     om, prompt, model = _tiny(rb, "hd128", rb.sem.REFERENCE, max_batch=batch)
     rng = np.random.default_rng(40 + batch)
     vocab = om["cfg"]["vocab_size"]
@@ -554,7 +554,7 @@ def test_batched_greedy_generation_ragged(rb, lens):
 
 @pytest.mark.parametrize("shape", [(1024, 8, 2, 1536), (2560, 20, 5, 6912), (8192, 64, 8, 9216), (512, 8, 8, 512), (512, 4, 2, 512),
                                    (768, 12, 4, 512), (1280, 20, 4, 512), (768, 6, 1, 512), (1792, 14, 2, 512), (1024, 16, 2, 512)])
-@pytest.mark.parametrize("batch,context", [(5, 300), (16, 30), (33, 129)])
+@pytest.mark.parametrize("batch,context", [(2, 129), (3, 30), (4, 300), (5, 300), (16, 30), (33, 129)])
 def test_batched_steps_equal_single_sequences(rb, shape, batch, context):
     """Two steps of several sequences (row stages with few rows, merged runs of the decode attention, sums cleared ahead
     of split products) against the same steps of each sequence alone: widths of every thread count, contexts with and
@@ -733,6 +733,34 @@ def test_ffn_sums_cleared_by_stage_or_memset(rb, ff, rows):
     x = torch.randn((rows, 512), generator=g, device="cuda")
     got, want = ffn.forward_device(x), torch.cat([ffn.forward_device(x[i:i + 1].contiguous()) for i in range(rows)])
     assert (got - want).norm() < 2e-5 * want.norm()
+
+
+@pytest.mark.parametrize("terms,few,many", [(1, (5, 8, 9), (10, 16)), (3, (3,), (4, 5))])
+def test_ffn_rows_that_the_down_product_finishes(rb, terms, few, many):
+    """Up to nine columns of 6912 the down product leaves finished rows, one launch less than with its sums in memory.  The same stages
+    and the same integer sums: one term's rows are equal to the bit, three terms' sums may be rounded once more each."""
+    import torch
+    lib, sem = rb.tr.abi.lib, {1: rb.sem.BASELINE, 3: rb.sem.REFERENCE}[terms]
+    ffn = rb.tr.GatedFFN(2560, 6912, semantics=sem)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(terms)
+    for p in (ffn.gate_proj, ffn.up_proj, ffn.down_proj):
+        p.load_from_int8(torch.randint(-1, 2, (p.out_features, p.in_features), generator=g, device="cuda", dtype=torch.int8), 0.02)
+    x = torch.randn((max(many), 2560), generator=g, device="cuda")
+
+    def run(rows):
+        before = lib.rotor_b200_launch_count()
+        y = ffn.forward_device(x[:rows])
+        return y, lib.rotor_b200_launch_count() - before
+
+    sums = [run(rows) for rows in many]
+    for rows in few:
+        y, launches = run(rows)
+        assert launches == sums[0][1] - 1, rows
+        for want, _ in sums:
+            n = min(rows, len(want))
+            assert torch.equal(y[:n], want[:n]) if terms == 1 else (y[:n] - want[:n]).norm() < 1e-6 * want[:n].norm(), rows
+    rb.tr.abi.device_status()
 
 
 @pytest.mark.parametrize("d", [512, 1536, 2560])
