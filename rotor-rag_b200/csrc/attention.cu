@@ -1130,10 +1130,6 @@ int attn_decode_nsplit(int max_seq) {
     return n < 8 ? 8 : (n > 32 ? 32 : n);
 }
 
-size_t attn_decode_part_floats(int batch, int n_heads, int head_dim, int max_seq) {
-    return (size_t)batch * n_heads * attn_decode_nsplit(max_seq) * (head_dim + 2);
-}
-
 // Whether the current device can place one 16-CTA cluster of the cluster kernel with this much shared
 // memory per CTA (asked of the occupancy calculator; nothing is launched).
 template <int D>

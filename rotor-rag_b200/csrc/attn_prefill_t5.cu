@@ -56,7 +56,6 @@ constexpr int A5_SMEM = A5_Q_BYTES + A5_OUT_BYTES + A5_STAGES * (A5_K_BYTES + A5
 constexpr int A5_TMEM_COLS = 512;         // S0 [0,64)  S1 [64,128)  O0 [128,256)  O1 [256,384)  Q hi [384,448)  Q lo [448,512)
 constexpr uint32_t A5_O = 128, A5_QT = 384;
 constexpr float A5_SLACK = 8.f;           // log2 of the largest weight before the reference maximum moves
-constexpr long long A5_SPIN_CYCLES = 400000000LL;  // about 0.2 s
 
 struct A5Params {
     const float* q;        // [rows][n_heads * 128]
@@ -67,35 +66,6 @@ struct A5Params {
     int split_seq;         // rows per (sequence, KV head) in the K planes (max_seq rounded up to 64)
     int batch, nqt;        // sequences, query tiles of each (sequence, KV head)
 };
-
-__device__ __forceinline__ uint32_t a5_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ bool a5_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status,
-                                        unsigned code) {
-    long long t0 = 0;
-    for (int it = 0;; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
-        if (it == 0) t0 = clock64();
-        if (clock64() - t0 > A5_SPIN_CYCLES) {
-            *abort_flag = 1;
-            atomicExch(status, code);
-            return false;
-        }
-    }
-}
-
-// Shared-memory matrix descriptor, K-major, 128-byte swizzle: 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t a5_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr >> 4) & 0x3fffu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
-}
 
 // ACC == 0: the accumulator is overwritten (first MMA of a tile), 1: accumulated into.
 template <int ACC>
@@ -109,32 +79,6 @@ __device__ __forceinline__ void a5_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint
         "r"(a_tmem), "l"(db), "r"(idesc), "n"(ACC), "r"(0u)
         : "memory");
 }
-__device__ __forceinline__ void a5_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void a5_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void a5_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
-        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
-        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-}
-
 __device__ __forceinline__ void a5_st16(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -219,7 +163,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     __shared__ float s_m[2][2][A5_BM], s_l[2][2][A5_BM];  // by tile parity: each group's reference maximum and sum of a row
-    const uint32_t kring = (a5_smem(a5_raw) + 1023u) & ~1023u, vring = kring + A5_STAGES * A5_K_BYTES;
+    const uint32_t kring = (smem_u32(a5_raw) + 1023u) & ~1023u, vring = kring + A5_STAGES * A5_K_BYTES;
     const uint32_t qstage = vring + A5_STAGES * A5_V_BYTES, ostage = qstage + A5_Q_BYTES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.n_heads / p.n_kv_heads, lg = 31 - __clz(G), QT = A5_BM >> lg;  // (G divides 128)
@@ -248,9 +192,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
 
     if (threadIdx.x == 0) {
         s_abort = 0;
-        auto init = [](unsigned long long* bar, int count) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a5_smem(bar)), "r"(count));
-        };
+        auto init = [](unsigned long long* bar, int count) { t5_bar_init(smem_u32(bar), count); };
         for (int s = 0; s < A5_STAGES; ++s) {
             init(&s_kfull[s], 1);
             init(&s_kempty[s], 1);
@@ -269,7 +211,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 8) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(a5_smem(&s_tmem)),
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
                      "r"(A5_TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
@@ -294,7 +236,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
             if (it.n) {
                 // ---------------- Q: rows out of shared memory, scaled and split into tensor memory
                 const float scale = 1.4426950408889634f / sqrtf((float)A5_D);  // scores come out in units of log2: p = 2^(s - m)
-                ok = ok && a5_wait(a5_smem(&s_qfull), (uint32_t)k & 1u, abort_flag, p.status, 0x7b00000bu);
+                ok = ok && t5_wait(smem_u32(&s_qfull), (uint32_t)k & 1u, abort_flag, p.status, 0x7b00000bu);
                 uint32_t qh[32], ql[32];  // columns [64 half, +64) of the row
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
@@ -306,13 +248,13 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                     a5_split2(v.z * scale, v.w * scale, qh[2 * i + 1], ql[2 * i + 1]);
                 }
                 __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_qempty)) : "memory");
-                a5_st32(lane_base + A5_QT + 32u * half, qh);
-                a5_st32(lane_base + A5_QT + 64u + 32u * half, ql);
+                if (lane == 0) t5_bar_arrive(smem_u32(&s_qempty));
+                t5_st32(lane_base + A5_QT + 32u * half, qh);
+                t5_st32(lane_base + A5_QT + 64u + 32u * half, ql);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_qready)) : "memory");
+                if (lane == 0) t5_bar_arrive(smem_u32(&s_qready));
             }
             if (prev.n && __all_sync(0xffffffffu, ok)) {
                 // ---------------- outputs of the tile before, columns [64 half, +64) of both accumulators.  A lane holds
@@ -353,7 +295,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                 // read by every warp before the next tile's first product: the groups read both accumulators
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) t5_bar_arrive(a5_smem(&s_oread));
+                if (lane == 0) t5_bar_arrive(smem_u32(&s_oread));
             }
             prev = it;
             if (!it.n) continue;
@@ -363,13 +305,13 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
             if (lim > it.t_all) lim = it.t_all;
             float m_ref = -INFINITY, l_run = 0.f;
             for (int j = half; j < it.n; j += 2, ++tiles) {
-                ok = ok && a5_wait(a5_smem(&s_sfull[half]), (uint32_t)tiles & 1u, abort_flag, p.status, 0x7b000001u);
+                ok = ok && t5_wait(smem_u32(&s_sfull[half]), (uint32_t)tiles & 1u, abort_flag, p.status, 0x7b000001u);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t sa[2][32];
-                a5_ld32(sbuf, sa[0]);
-                a5_ld32(sbuf + 32u, sa[1]);
+                t5_ld32(sbuf, sa[0]);
+                t5_ld32(sbuf + 32u, sa[1]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 const int kb = j * A5_BN;
                 if (kb + A5_BN > lim) {  // only the last tiles of a row need the mask
@@ -392,11 +334,11 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
 #pragma unroll 1
                         for (uint32_t c = 0; c < 128u; c += 32u) {
                             uint32_t ov[32];
-                            a5_ld32(obuf + c, ov);
+                            t5_ld32(obuf + c, ov);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                             for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-                            a5_st32(obuf + c, ov);
+                            t5_st32(obuf + c, ov);
                         }
                     }
                 }
@@ -418,7 +360,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a5_smem(&s_pfull[half])) : "memory");
+                if (lane == 0) t5_bar_arrive(smem_u32(&s_pfull[half]));
                 l_run += sum0 + sum1;
             }
             // ---------------- the groups' results of a row, weighed against each other
@@ -432,7 +374,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
             const float inv = 1.0f / (sl[0][r] * w0 + sl[1][r] * w1);
             w0 *= inv;
             w1 *= inv;
-            ok = ok && a5_wait(a5_smem(&s_ofull), (uint32_t)k & 1u, abort_flag, p.status, 0x7b000002u);
+            ok = ok && t5_wait(smem_u32(&s_ofull), (uint32_t)k & 1u, abort_flag, p.status, 0x7b000002u);
             ok = __all_sync(0xffffffffu, ok);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
@@ -446,9 +388,9 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                 const int krow0 = (it.b * p.n_kv_heads + it.hk) * p.split_seq;
                 for (int j = 0; j < it.n; ++j, ++t) {
                     const int s = t & 1;
-                    ok = a5_wait(a5_smem(&s_kempty[s]), ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000003u);
+                    ok = t5_wait(smem_u32(&s_kempty[s]), ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000003u);
                     if (!ok) break;
-                    const uint32_t bar = a5_smem(&s_kfull[s]), st = kring + (uint32_t)s * A5_K_BYTES;
+                    const uint32_t bar = smem_u32(&s_kfull[s]), st = kring + (uint32_t)s * A5_K_BYTES;
                     t5_bar_expect(bar, A5_K_BYTES);
 #pragma unroll
                     for (int pn = 0; pn < 2; ++pn) {
@@ -468,9 +410,9 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                 const int vrow0 = (it.b * p.n_kv_heads + it.hk) * (p.split_seq / A5_BN) * A5_D;
                 for (int j = 0; j < it.n; ++j, ++t) {
                     const int s = t & 1;
-                    ok = a5_wait(a5_smem(&s_vempty[s]), ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000009u);
+                    ok = t5_wait(smem_u32(&s_vempty[s]), ((uint32_t)(t >> 1) & 1u) ^ 1u, abort_flag, p.status, 0x7b000009u);
                     if (!ok) break;
-                    const uint32_t bar = a5_smem(&s_vfull[s]), st = vring + (uint32_t)s * A5_V_BYTES;
+                    const uint32_t bar = smem_u32(&s_vfull[s]), st = vring + (uint32_t)s * A5_V_BYTES;
                     t5_bar_expect(bar, A5_V_BYTES);
                     t5_tma_2d(st, &tm_vh, 0, vrow0 + j * A5_D, bar);
                     t5_tma_2d(st + 16384u, &tm_vl, 0, vrow0 + j * A5_D, bar);
@@ -483,10 +425,10 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
         for (int k = 0; k < rounds && ok; ++k) {
             const Item it = item(k);
             if (!it.n) break;
-            ok = a5_wait(a5_smem(&s_qempty), ((uint32_t)k & 1u) ^ 1u, abort_flag, p.status, 0x7b00000cu);
+            ok = t5_wait(smem_u32(&s_qempty), ((uint32_t)k & 1u) ^ 1u, abort_flag, p.status, 0x7b00000cu);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
-            const uint32_t bar = a5_smem(&s_qfull);
+            const uint32_t bar = smem_u32(&s_qfull);
             const int live = (it.last - it.s0 + 1) << lg;
             if (lane == 0) t5_bar_expect(bar, (uint32_t)live * (A5_D * 4));
             __syncwarp();
@@ -509,7 +451,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
             // counts 16-byte units and no operand crosses the field's range), nothing is recomputed per MMA.
             // j: key tile of the query tile (its group's buffers); t: over all query tiles (ring slots)
             auto issue_s = [&](int j, int t) {
-                const uint64_t dk_hi = a5_desc(kring + (uint32_t)(t & 1) * A5_K_BYTES), dk_lo = dk_hi + (16384u >> 4);
+                const uint64_t dk_hi = t5_desc(kring + (uint32_t)(t & 1) * A5_K_BYTES), dk_lo = dk_hi + (16384u >> 4);
                 const uint32_t d = tmem + (uint32_t)(j & 1) * 64u;
 #pragma unroll
                 for (int term = 0; term < 3; ++term)
@@ -523,11 +465,11 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                         else
                             a5_mma_ts<1>(d, qa, db, idesc_s);
                     }
-                a5_commit(a5_smem(&s_sfull[j & 1]));
-                a5_commit(a5_smem(&s_kempty[t & 1]));
+                t5_commit(smem_u32(&s_sfull[j & 1]));
+                t5_commit(smem_u32(&s_kempty[t & 1]));
             };
             auto issue_pv = [&](int j, int t, auto first) {
-                const uint64_t dv_hi = a5_desc(vring + (uint32_t)(t & 1) * A5_V_BYTES), dv_lo = dv_hi + (16384u >> 4);
+                const uint64_t dv_hi = t5_desc(vring + (uint32_t)(t & 1) * A5_V_BYTES), dv_lo = dv_hi + (16384u >> 4);
                 const uint32_t pbase = tmem + (uint32_t)(j & 1) * 64u, d = tmem + A5_O + (uint32_t)(j & 1) * 128u;
 #pragma unroll
                 for (int term = 0; term < 3; ++term)
@@ -540,7 +482,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                         else
                             a5_mma_ts<1>(d, pa, db, idesc_o);
                     }
-                a5_commit(a5_smem(&s_vempty[t & 1]));
+                t5_commit(smem_u32(&s_vempty[t & 1]));
             };
             bool ok = true;
             int base = 0;                // key tiles of the query tiles before
@@ -548,10 +490,10 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
             for (int k = 0; k < rounds && ok; ++k) {
                 const Item it = item(k);
                 if (!it.n) break;
-                ok = a5_wait(a5_smem(&s_qready), (uint32_t)k & 1u, abort_flag, p.status, 0x7b000004u);
+                ok = t5_wait(smem_u32(&s_qready), (uint32_t)k & 1u, abort_flag, p.status, 0x7b000004u);
                 auto scores = [&](int j) {
                     const int t = base + j;
-                    ok = ok && a5_wait(a5_smem(&s_kfull[t & 1]), (uint32_t)(t >> 1) & 1u, abort_flag, p.status, 0x7b000005u);
+                    ok = ok && t5_wait(smem_u32(&s_kfull[t & 1]), (uint32_t)(t >> 1) & 1u, abort_flag, p.status, 0x7b000005u);
                     if (!ok) return;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     issue_s(j, t);
@@ -559,10 +501,10 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                 for (int j = 0; j < 2 && j < it.n; ++j) scores(j);
                 for (int j = 0; j < it.n && ok; ++j) {
                     const int t = base + j;
-                    ok = a5_wait(a5_smem(&s_pfull[j & 1]), (phases >> (j & 1)) & 1u, abort_flag, p.status, 0x7b000007u);
+                    ok = t5_wait(smem_u32(&s_pfull[j & 1]), (phases >> (j & 1)) & 1u, abort_flag, p.status, 0x7b000007u);
                     phases ^= 1u << (j & 1);
-                    if (ok && j == 0 && k > 0) ok = a5_wait(a5_smem(&s_oread), (uint32_t)(k - 1) & 1u, abort_flag, p.status, 0x7b00000du);
-                    if (ok) ok = a5_wait(a5_smem(&s_vfull[t & 1]), (uint32_t)(t >> 1) & 1u, abort_flag, p.status, 0x7b00000au);
+                    if (ok && j == 0 && k > 0) ok = t5_wait(smem_u32(&s_oread), (uint32_t)(k - 1) & 1u, abort_flag, p.status, 0x7b00000du);
+                    if (ok) ok = t5_wait(smem_u32(&s_vfull[t & 1]), (uint32_t)(t >> 1) & 1u, abort_flag, p.status, 0x7b00000au);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (j < 2)
@@ -571,7 +513,7 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                         issue_pv(j, t, std::false_type());
                     if (j + 2 < it.n) scores(j + 2);  // (over the P that this product has read)
                 }
-                if (ok) a5_commit(a5_smem(&s_ofull));
+                if (ok) t5_commit(smem_u32(&s_ofull));
                 base += it.n;
             }
         }
@@ -591,21 +533,10 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
     }
 }
 
-typedef CUresult (*A5EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static A5EncodeFn g_a5_encode = nullptr;
 static PerDevice<bool> g_a5_ready;
 
 int configure_attn_prefill_t5() {
     if (g_a5_ready.here()) return ROTOR_B200_OK;
-    if (!g_a5_encode) {
-        cudaDriverEntryPointQueryResult q;
-        void* fn = nullptr;
-        RB_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-        if (!fn || q != cudaDriverEntryPointSuccess) return ROTOR_B200_ERR_CUDA;
-        g_a5_encode = (A5EncodeFn)fn;
-    }
     RB_CUDA(cudaFuncSetAttribute(attn_prefill_t5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, A5_SMEM));
     g_a5_ready.here() = true;
     return ROTOR_B200_OK;
@@ -636,18 +567,10 @@ int launch_attn_prefill_t5(const AttnParams& p, int rows, cudaStream_t st) {
     if (rc) return rc;
     // ---- tensor maps: K planes [rows][128] in boxes of 64 columns x 64 rows, V^T planes [rows][64] in boxes of 64 x 128
     CUtensorMap tm[4];
-    const cuuint64_t krows = (cuuint64_t)batch * p.n_kv_heads * split_seq;
-    const cuuint64_t vrows = (cuuint64_t)batch * p.n_kv_heads * (split_seq / A5_BN) * A5_D;
-    const cuuint32_t estride[2] = {1u, 1u};
+    const size_t krows = (size_t)batch * p.n_kv_heads * split_seq, vrows = krows / A5_BN * A5_D;
     for (int i = 0; i < 4; ++i) {
-        const bool is_v = i >= 2;
-        const cuuint64_t gdim[2] = {(cuuint64_t)(is_v ? A5_BN : A5_D), is_v ? vrows : krows};
-        const cuuint64_t gstride[1] = {(cuuint64_t)(is_v ? A5_BN : A5_D) * 2};
-        const cuuint32_t box[2] = {64u, is_v ? 128u : 64u};
-        void* ptr = (void*)(p.kv_split + (size_t)i * p.split_plane);
-        if (g_a5_encode(&tm[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, gdim, gstride, box, estride,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        const __nv_bfloat16* plane = p.kv_split + (size_t)i * p.split_plane;
+        if (!(i < 2 ? t5_map_bf16(&tm[i], plane, krows, A5_D, A5_D, A5_BN) : t5_map_bf16(&tm[i], plane, vrows, A5_BN, A5_BN, A5_D)))
             return ROTOR_B200_ERR_CUDA;
     }
     A5Params a;

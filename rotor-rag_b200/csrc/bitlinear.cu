@@ -378,10 +378,6 @@ static int pick_variant(int variant, int ncols) {
     return ncols <= 2 ? ROTOR_B200_VARIANT_DP4A : ROTOR_B200_VARIANT_MMA;
 }
 
-int gemv_cols_per_launch(int variant, int ncols) {
-    return pick_variant(variant, ncols < 8 ? ncols : 8) == ROTOR_B200_VARIANT_MMA ? ACC_MMA_COLS : 4;
-}
-
 GemvPlan plan_gemv(size_t out, size_t in, int ncols) {
     const int nkt = (int)(kpad_of(in) / TILE_K), nrt = (int)(opad_of(out) / TILE_ROWS);
     const int per_pass = ncols < ACC_MMA_COLS ? ncols : ACC_MMA_COLS;

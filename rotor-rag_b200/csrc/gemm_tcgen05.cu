@@ -781,10 +781,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn g_encode = nullptr;
 static PerDevice<bool> g_tc5_ready;
 
 // Shapes this kernel takes: enough tokens to be worth its tile, 16-byte aligned operands.
@@ -796,11 +792,7 @@ bool gemm_tcgen05_supported(size_t out, size_t in, int ncols, const void* xq) {
 
 int configure_gemm_tcgen05() {
     if (g_tc5_ready.here()) return ROTOR_B200_OK;
-    cudaDriverEntryPointQueryResult q;
-    void* fn = nullptr;
-    RB_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-    if (!fn || q != cudaDriverEntryPointSuccess) return ROTOR_B200_ERR_CUDA;
-    g_encode = (EncodeTiledFn)fn;
+    if (!t5_encoder()) return ROTOR_B200_ERR_CUDA;
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<256>::SMEM));
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<256, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<256, 128>::SMEM));
     RB_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, T5Cfg<64>::SMEM));
@@ -818,7 +810,8 @@ static bool encode_tokens(CUtensorMap* tmap, const void* xq, size_t kpad, int nc
     const cuuint64_t gstride[1] = {(cuuint64_t)kpad};  // bytes between token rows
     const cuuint32_t box[2] = {(cuuint32_t)TILE_K, (cuuint32_t)rows};
     const cuuint32_t estride[2] = {1u, 1u};
-    return g_encode(tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(xq), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const T5EncodeFn encode = t5_encoder();
+    return encode && encode(tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(xq), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

@@ -71,7 +71,6 @@ bool gemv_adds(size_t out, size_t in, int ncols, const void* xq, int variant);
 int launch_gemv_planes(const void* tiles, size_t out, size_t in, const int8_t* xq, const int32_t* xsum, int ncols,
                        int32_t* acc, size_t plane_stride, const GemvPlan& plan, int variant, cudaStream_t st,
                        bool zeroed = false);
-int gemv_cols_per_launch(int variant, int ncols);
 // Products that leave finished float rows.
 bool acc_finish_supported(size_t out, size_t in, size_t ncols, int variant);
 int launch_acc_finish(const void* tiles, size_t out, size_t in, const int8_t* xq, const float* sx, const int32_t* xsum, int rows, int terms,
@@ -172,7 +171,6 @@ bool attn_decode_stream_ok(int n_heads, int n_kv_heads, int head_dim);
 int launch_attn_decode_stream(const AttnDecodeParams& p, int batch, cudaStream_t st);
 int attn_decode_nsplit(int max_seq);
 int attn_decode_nsplit_for(int n_heads, int n_kv_heads, int head_dim, int max_seq);
-size_t attn_decode_part_floats(int batch, int n_heads, int head_dim, int max_seq);
 int configure_attention();
 
 struct AttnParams {
