@@ -202,18 +202,25 @@ def ptr(t):
 def stream():
     """The current stream of the current device, as the address that the C ABI takes."""
     torch = require_cuda()
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return _current_stream(torch.cuda.current_device())
 
 
-_torch = None  # (the module, once a device has been found: the search costs 2 us a call)
+def _stream_lookup(torch):
+    """What gives a device's current stream as an address: torch's own short cut (a microsecond less per call) where this
+    version has it, else the public way."""
+    return getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+
+
+_torch = _current_stream = None  # (the module, once a device has been found: the search costs 2 us a call)
 
 
 def require_cuda():
-    global _torch
+    global _torch, _current_stream
     if _torch is None:
         import torch
         if not torch.cuda.is_available():
             raise RotorB200Error("no CUDA device: the rotor_b200 path runs on a B200 only (no CPU fallback)")
+        _current_stream = _stream_lookup(torch)
         _torch = torch
     return _torch
 

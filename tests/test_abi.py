@@ -83,3 +83,13 @@ print(f(1 << 20, out, inn, 1 << 21, rows, terms, 1.0, None, 1 << 22, 1 << 23, 1 
 """
     r = subprocess.run([sys.executable, "-c", code, LIB] + [str(v) for v in (out, inn, rows, terms, variant)], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.split() == ["1"], (r.returncode, r.stdout, r.stderr)
+
+
+def test_stream_without_the_short_cut():
+    """A torch without the private entry gives the same address through the public one."""
+    from types import SimpleNamespace
+    from rotor_b200 import abi
+    cuda = SimpleNamespace(current_stream=lambda device: SimpleNamespace(cuda_stream=100 + device))
+    assert abi._stream_lookup(SimpleNamespace(_C=SimpleNamespace(), cuda=cuda))(3) == 103
+    short = SimpleNamespace(_C=SimpleNamespace(_cuda_getCurrentRawStream=lambda device: 200 + device), cuda=cuda)
+    assert abi._stream_lookup(short)(3) == 203
