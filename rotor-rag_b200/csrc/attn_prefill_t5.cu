@@ -326,9 +326,11 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                     t1 = fmaxf(t1, fmaxf(__uint_as_float(sa[1][c]), __uint_as_float(sa[1][c + 1])));
                 }
                 const float tmax = fmaxf(t0, t1);
-                if (__any_sync(0xffffffffu, tmax > m_ref + A5_SLACK)) {  // the first tile, then rarely
-                    const float m_new = fmaxf(m_ref, tmax), alpha = m_ref == -INFINITY ? 0.f : a5_exp2(m_ref - m_new);
-                    m_ref = m_new;
+                // (each row for itself: what another row of the warp does, one past the sequence above all, changes nothing here)
+                const bool far = tmax > m_ref + A5_SLACK;
+                if (__any_sync(0xffffffffu, far)) {  // the first tile, then rarely
+                    const float alpha = !far ? 1.f : m_ref == -INFINITY ? 0.f : a5_exp2(m_ref - tmax);
+                    if (far) m_ref = tmax;
                     l_run *= alpha;
                     if (j >= 2) {
 #pragma unroll 1

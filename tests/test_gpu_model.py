@@ -845,3 +845,17 @@ def test_ffn_rows_off_a_16_byte_boundary(rb, rows):
         out.append(ffn.forward_device(place(x), pre_norm=pre).double())
         rb.tr.abi.device_status()
     assert (out[1] - out[0]).norm() < 1e-5 * out[0].norm()
+
+
+@pytest.mark.parametrize("seq", [33, 391, 700])
+def test_prompt_rows_do_not_depend_on_earlier_calls(rb, seq):
+    """A prompt whose last query tile has rows past its end, behind calls of other magnitudes: what shared memory still holds of those
+    lies in these rows, and must not change what the others round to."""
+    import dataclasses
+    at, _ = _attention_layer(rb, 512, 4, 1, 5, semantics=dataclasses.replace(rb.sem.REFERENCE, causal=True), max_seq=1024)
+    x = np.random.default_rng(seq).standard_normal((1, 1024, 512)).astype(np.float32)
+    got = []
+    for scale in (0.0, 0.01, 3.0, 30.0, 300.0):
+        at.forward(x * np.float32(scale))
+        got.append(at.forward(x[:, :seq])[0])
+    assert all(np.array_equal(got[0], y) for y in got[1:])
