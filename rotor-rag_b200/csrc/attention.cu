@@ -651,15 +651,14 @@ __global__ void __launch_bounds__(AC_MAX_THREADS) attn_decode_cluster_kernel(con
 // Bound by the cache's stream.  Every lane copies its D / 32 columns of a row into shared memory (cp.async) and reads back itself
 // what it copied, once for all H heads: no barrier, and a ring of stages keeps 4 to 8 KB a warp on their way at 128 registers a
 // thread, sixteen warps an SM.  (With the rows requested into registers, twelve warps and half of the bytes: 64 sequences of the XL
-// shape behind 1024 positions 151 us = 3.6 TB/s, now 117 us = 4.6 TB/s.)  Two stages up to four heads, three above: 2B shape, 12
-// layers, 8 / 16 sequences 628 / 723 us a step with two, 636 / 730 with three; XL shape, 4 layers, 64 behind 1990 positions 1809 /
-// 1781.  A warp takes four keys at a time: 4 H partial dot products per lane are folded over the lanes by halving (a lane hands over
+// shape behind 1024 positions 151 us = 3.6 TB/s, now 117 us = 4.6 TB/s.)  Two stages up to four heads (2B shape, 12 layers, 8 / 16
+// sequences 628 / 723 us a step with two, 636 / 730 with three), three above where eight warps a CTA leave the room.  A warp takes four keys at a time: 4 H partial dot products per lane are folded over the lanes by halving (a lane hands over
 // half of its values and keeps the sums of the other half: 31 shuffles for 32 products, after which a lane holds one finished
 // score), so that exponentials are one instruction per 32 scores; the weights return through a line of shared memory.  The warps of
 // a CTA take every W-th group of four keys and merge at the end.  The first keys are requested before the launch wait (cached rows
 // are older than the kernel before this one).
-// A step of the 2B shape (12 layers) behind 517 positions, with a finish kernel before and the stage behind merging the runs /
-// here: 5 sequences 694 / 633 us, 8 709 / 651, 16 941 / 879, 64 1732 / 1659; XL shape (4 layers) 8 912 / 863, 64 1477 / 1461.
+// A step behind 480 positions, with a finish kernel before, rows through registers and the stage behind merging the runs / here: 2B
+// shape (6 layers) 5 sequences 316 / 271 us, 8 326 / 289, 16 446 / 337, 64 826 / 682; XL shape (2 layers) 8 344 / 309, 64 612 / 531.
 constexpr int AS_KEYS = 4, AS_MAX_RUNS = 8;
 
 // Outputs that each of `runs` CTAs merges (the last one the rest).
@@ -738,18 +737,27 @@ __device__ __forceinline__ void as_rotate(float (&v)[E], const float2 (&cs)[E], 
     }
 }
 
-template <int H>
-constexpr int AS_STAGES = H > 4 ? 3 : 2;
+template <int H, int W>
+constexpr int AS_STAGES = H > 4 && W == 8 ? 3 : 2;
+// Where a warp's share is long, its outputs are summed AS_PART groups of keys at a time, the parts in shared memory: a sum of hundreds
+// of keys in a row rounds more than the shorter sums of more runs (attention layer of 64 sequences behind 1024 positions, error
+// against float64: XL shape 2.52e-7 with two runs, 2.41e-7 with four, 2.42e-7 so; 2B shape 2.62e-7 with one, 2.33e-7 with four, 2.35e-7
+// so).  The time is the same (2B shape, 64 sequences, 6 layers 849 / 845 us a step) where the ring has two stages anyway; XL shape, 2
+// layers, with three stages and no parts / so: 64 sequences behind 1024 positions 618 / 614, 1900 746 / 754, 40 sequences 544 / 547,
+// 641 / 656.  Eight warps a CTA of more than four heads need the room for their third stage.
+constexpr int AS_PART = 16;
+template <int H, int W>
+constexpr bool AS_PARTS = AS_STAGES<H, W> == 2;
 template <int D, int H, int W>
-constexpr int as_ring_bytes() { return W * AS_STAGES<H> * 2 * AS_KEYS * D * 4; }
+constexpr int as_ring_bytes() { return W * (AS_STAGES<H, W> * 2 * AS_KEYS + (AS_PARTS<H, W> ? H : 0)) * D * 4; }
 
 template <int D, int H, int W>
 __global__ void __launch_bounds__(32 * W, 16 / W) attn_decode_stream_kernel(const __grid_constant__ AttnDecodeParams p) {
     constexpr int E = D / 32, HP = H > 4 ? 8 : H > 2 ? 4 : H;      // heads, rounded up to a power of two for the folding
     constexpr int N = HP * AS_KEYS, SH = N == 32 ? 0 : N == 16 ? 1 : N == 8 ? 2 : 3;  // lane >> SH: value 4 h + key
     __shared__ __align__(16) float s_w[W][2][N];                   // weights of a group of keys
-    extern __shared__ __align__(16) float as_ring[];               // [W][STAGES][k, v][AS_KEYS][D]
-    constexpr int STAGE = 2 * AS_KEYS * D, STAGES = AS_STAGES<H>;
+    extern __shared__ __align__(16) float as_ring[];               // [W][STAGES][k, v][AS_KEYS][D], then [W][H][D] parts
+    constexpr int STAGE = 2 * AS_KEYS * D, STAGES = AS_STAGES<H, W>;
     __shared__ float s_a[W][HP];                                   // rescaling factors
     __shared__ float s_m[W][HP], s_l[W][HP];
     __shared__ __align__(16) float s_q[H <= 4 ? H : 1][D];
@@ -780,6 +788,8 @@ __global__ void __launch_bounds__(32 * W, 16 / W) attn_decode_stream_kernel(cons
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    float* const parts = as_ring + W * STAGES * STAGE + warp * H * D + E * lane;  // (of this lane alone, like the ring)
+    bool parted = false;
     int t = k0 + AS_KEYS * warp;
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) fetch(t + i * STRIDE, i);
@@ -887,6 +897,13 @@ __global__ void __launch_bounds__(32 * W, 16 / W) attn_decode_stream_kernel(cons
                 const float ah = s_a[warp][h];
 #pragma unroll
                 for (int e = 0; e < E; ++e) o[h][e] *= ah;
+                if (AS_PARTS<H, W> && parted) {
+                    float a[E];
+                    as_get<E>(parts + h * D, a);
+#pragma unroll
+                    for (int e = 0; e < E; ++e) a[e] *= ah;
+                    as_put<E>(parts + h * D, a);
+                }
             }
         }
         m_run = m_new;
@@ -923,11 +940,35 @@ __global__ void __launch_bounds__(32 * W, 16 / W) attn_decode_stream_kernel(cons
         as_put<E>(to + AS_KEYS * D, kv[1]);
         step(1, to);
     }
-    for (int slot = 0; t < k1; t += STRIDE) {
+    for (int slot = 0, since = 0; t < k1; t += STRIDE) {
         fetch(t + (STAGES - 1) * STRIDE, slot ? slot - 1 : STAGES - 1);
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
         step(k1 - t, ring + slot * STAGE);
         slot = slot == STAGES - 1 ? 0 : slot + 1;
+        if (AS_PARTS<H, W> && ++since == p.part) {
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                float a[E] = {};
+                if (parted) as_get<E>(parts + h * D, a);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    a[e] += o[h][e];
+                    o[h][e] = 0.f;
+                }
+                as_put<E>(parts + h * D, a);
+            }
+            parted = true;
+            since = 0;
+        }
+    }
+    if (AS_PARTS<H, W> && parted) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            float a[E];
+            as_get<E>(parts + h * D, a);
+#pragma unroll
+            for (int e = 0; e < E; ++e) o[h][e] += a[e];
+        }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");  // (the groups behind the last are empty)
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1 << SH);
@@ -996,28 +1037,36 @@ bool attn_decode_stream_ok(int n_heads, int n_kv_heads, int head_dim) {
 // GPC).  us a step behind 1900 positions, four warps a CTA with the best number of runs / eight warps so: 2B shape, four layers, 10
 // sequences 380 / 359, 20 456 / 447, 40 663 / 636, 56 822 / 788; XL shape, two layers, 3 724 / 703, 16 750 / 746, 32 858 / 852.
 // Else four CTAs of four warps.  Where only whole sequences fit, long caches (the host does not know the present lengths) are cut
-// all the same: 2B shape, 64 sequences, one / three runs 919 / 862 behind 1900 positions, 470 / 488 behind 70; XL shape, 40
-// sequences, one / two 1060 / 954 behind 1900, 802 / 788 behind 500, 722 / 735 behind 70; 64 sequences 1091 / 1069, 834 / 849.  More sequences than fit: up to 2048 CTAs while the cache's capacity leaves a run 64
-// positions, so that the last round is short.
+// all the same, behind 70 / 1024 / 1900 positions: 2B shape, six layers, 64 sequences one run 529 / 894 / 1222, two 555 / 946 / 1289,
+// three 555 / 845 / 1103, four 576 / 889 / 1167; XL shape, two layers, 40 sequences one run 409 / 603 / 767, two 423 / 555 / 661, four
+// 431 / 548 / 644, 64 sequences one 429 / 619 / 785, two 446 / 616 / 757, four 468 / 636 / 781.  More sequences than fit: up to 2048
+// CTAs while the cache's capacity leaves a run 64 positions, so that the last round is short.
 struct AsPlan {
     int runs;
-    bool wide;  // eight warps a CTA
+    bool wide;   // eight warps a CTA
+    bool parts;  // outputs summed in parts
 };
 
 static AsPlan attn_stream_plan(int batch, int n_kv_heads, int group, int max_seq) {
     const long n = (long)batch * n_kv_heads, two = 2L * fused_sm_count();
     int s = AS_MAX_RUNS;
-    if (n <= two) {
+    // (parts: where a sequence would otherwise be summed in fewer pieces than sixteen, or the eight of up to 256 CTAs; more than
+    // four heads have no room for them beside eight warps: 36 sequences of the XL shape behind 480 positions 438 us a step with eight
+    // warps and no parts, 449 so)
+    const bool few = n <= two * 7 / 8;
+    if (few || (group <= 4 && n <= two)) {
         while (s > 1 && n * s > (s > 2 ? two * 9 / 10 : two)) --s;
-        return {s, true};
+        return {s, true, !few};
     }
-    if (n <= 2 * two) return group >= 5 ? AsPlan{max_seq < (2 * n <= 3 * two ? 512 : 1024) ? 1 : 2, false} : AsPlan{max_seq < 1024 ? 1 : 3, false};
+    if (n <= 2 * two) return group >= 5 ? AsPlan{max_seq < (2 * n <= 3 * two ? 512 : 1024) ? 1 : 2, false, true} : AsPlan{max_seq < 1024 ? 1 : 3, false, true};
     for (s = 1; 2 * s <= AS_MAX_RUNS && n * 2 * s <= 2048 && max_seq / (2 * s) >= 64;) s *= 2;
-    return {s, false};
+    return {s, false, true};
 }
 
 template <int D, int H, int W>
-static int launch_attn_decode_stream_k(const AttnDecodeParams& p, int batch, int runs, cudaStream_t st) {
+static int launch_attn_decode_stream_k(AttnDecodeParams p, int batch, const AsPlan& plan, cudaStream_t st) {
+    const int runs = plan.runs;
+    p.part = plan.parts ? AS_PART : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(runs, p.n_kv_heads, batch);
     cfg.blockDim = dim3(32 * W);
@@ -1055,7 +1104,7 @@ static int launch_attn_decode_stream_d(const AttnDecodeParams& p, int batch, cud
         return ROTOR_B200_ERR_SHAPE;
     }
     const AsPlan plan = attn_stream_plan(batch, p.n_kv_heads, G, p.max_seq);
-    return plan.wide ? launch_attn_decode_stream_k<D, H, 8>(p, batch, plan.runs, st) : launch_attn_decode_stream_k<D, H, 4>(p, batch, plan.runs, st);
+    return plan.wide ? launch_attn_decode_stream_k<D, H, 8>(p, batch, plan, st) : launch_attn_decode_stream_k<D, H, 4>(p, batch, plan, st);
 }
 
 int launch_attn_decode_stream(const AttnDecodeParams& p, int batch, cudaStream_t st) {

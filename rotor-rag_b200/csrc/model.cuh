@@ -156,6 +156,7 @@ struct AttnDecodeParams {
     float* part_l;
     unsigned* counter;    // [batch], zero before the launch
     float* attn_out;      // optional float copy of the merged rows [batch][n_heads*head_dim]
+    int part;             // several sequences at once: groups of keys summed before they are added to the rest (0: all; set at launch)
     int8_t* xq;           // quantised merged rows for the output projection
     float* sx_out;
     int32_t* xsum_out;
