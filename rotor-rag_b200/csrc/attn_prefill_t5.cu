@@ -7,9 +7,12 @@
 //
 // CTA: 128 query rows of one KV head (128 / G positions x G heads of the group), keys walked 64
 // at a time.  Both products run as tcgen05.mma.kind::f16 with bf16 operands and float32
-// accumulators in tensor memory, every operand split into hi + lo bf16 terms
-// (hi*hi + hi*lo + lo*hi: 16 operand mantissa bits), which holds the 1e-3-of-RMS bound of the
-// float32 reference.
+// accumulators in tensor memory, every operand split into hi + lo bf16 terms (16 operand mantissa bits), which holds
+// the 1e-3-of-RMS bound of the float32 reference.  O takes lo*hi + hi*lo + hi*hi; S takes lo*lo too, and both add the small
+// products first: an accumulator that stays in tensor memory over a row's keys rounds more than tiles that are added in registers,
+// and the scores give it back (error of the attention layer against float64, three activation terms, 2 x 700 positions of the 2B
+// shape: 7.68e-6 with each tile added in registers, 7.94e-6 with three products in S, 6.53e-6 so; one prompt of 2048 8.07e-6, 8.46e-6,
+// 6.96e-6; 6 layers of 8 x 2048 11.08 / 11.30 ms with three / four).
 //   S = Q K^T : A = Q hi / lo from TENSOR MEMORY (scaled, split and written once per CTA), B = K hi / lo tiles
 //               [64 keys][128] by TMA; accumulator 128 lanes x 64 columns.
 //   O += P V  : A = P hi / lo from tensor memory (written by the softmax warps over the S buffer they have just
@@ -456,13 +459,13 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                 const uint64_t dk_hi = t5_desc(kring + (uint32_t)(t & 1) * A5_K_BYTES), dk_lo = dk_hi + (16384u >> 4);
                 const uint32_t d = tmem + (uint32_t)(j & 1) * 64u;
 #pragma unroll
-                for (int term = 0; term < 3; ++term)
+                for (int term = 3; term >= 0; --term)  // lo lo, lo hi, hi lo, hi hi
 #pragma unroll
                     for (int k16 = 0; k16 < A5_D / 16; ++k16) {
                         const uint64_t ko = (uint64_t)(((k16 >> 2) * 8192 + (k16 & 3) * 32) >> 4);
-                        const uint32_t qa = tmem + A5_QT + (term == 2 ? 64u : 0u) + (uint32_t)k16 * 8u;
-                        const uint64_t db = (term == 1 ? dk_lo : dk_hi) + ko;
-                        if (term == 0 && k16 == 0)
+                        const uint32_t qa = tmem + A5_QT + (term >= 2 ? 64u : 0u) + (uint32_t)k16 * 8u;
+                        const uint64_t db = ((term & 1) ? dk_lo : dk_hi) + ko;
+                        if (term == 3 && k16 == 0)
                             a5_mma_ts<0>(d, qa, db, idesc_s);
                         else
                             a5_mma_ts<1>(d, qa, db, idesc_s);
@@ -474,12 +477,12 @@ attn_prefill_t5_kernel(const __grid_constant__ CUtensorMap tm_kh, const __grid_c
                 const uint64_t dv_hi = t5_desc(vring + (uint32_t)(t & 1) * A5_V_BYTES), dv_lo = dv_hi + (16384u >> 4);
                 const uint32_t pbase = tmem + (uint32_t)(j & 1) * 64u, d = tmem + A5_O + (uint32_t)(j & 1) * 128u;
 #pragma unroll
-                for (int term = 0; term < 3; ++term)
+                for (int term = 2; term >= 0; --term)  // lo hi, hi lo, hi hi
 #pragma unroll
                     for (int k16 = 0; k16 < A5_BN / 16; ++k16) {
                         const uint32_t pa = pbase + (term == 2 ? 32u : 0u) + (uint32_t)k16 * 8u;
                         const uint64_t db = (term == 1 ? dv_lo : dv_hi) + (uint64_t)((k16 * 32) >> 4);
-                        if (decltype(first)::value && term == 0 && k16 == 0)
+                        if (decltype(first)::value && term == 2 && k16 == 0)
                             a5_mma_ts<0>(d, pa, db, idesc_o);
                         else
                             a5_mma_ts<1>(d, pa, db, idesc_o);
