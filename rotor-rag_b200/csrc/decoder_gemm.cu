@@ -213,10 +213,15 @@ dense_gemm_t5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 #pragma unroll 1
                 for (int c = 0; c < BN / 32; ++c) {
                     const int col = n * TN + c * 32;
-                    if (col >= p.ldy) break;  // (ldy is a multiple of 32; columns past n are zeros)
+                    if (col >= p.ldy) break;  // (ldy is a multiple of 32; columns past n are zeros ...
                     uint32_t v[32];
                     t5_ld32(tb + c * 32, v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (p.table && col + 32 > p.n) {  // ... but not where the next expert's weights follow
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (col + i >= p.n) v[i] = 0u;
+                    }
                     t5_store_rows(stage, v, p.y + (size_t)tok0 * p.ldy + col, (size_t)p.ldy * 4, tok0, tok_end, lane);
                 }
             } else if constexpr (EPI == DENSE_HALF) {

@@ -298,6 +298,35 @@ def test_routing_in_one_launch_and_in_several(n, top):
         assert rel(out[rows], out[33][:rows]) < 4e-3, rows
 
 
+@pytest.mark.parametrize("n,top,ff", [(7, 3, 40), (64, 6, 136), (5, 1, 1408)])
+def test_experts_of_a_few_tokens_add_up_in_float32(n, top, ff):
+    """Three and four tokens take the tensor-core products, whose rows stay float32 until they are weighted and added, as the sums
+    of the matrix-vector product of one and two tokens do: the same rows two at a time, up to a gated value that rounds to the
+    other bf16 (rows rounded to bf16 would differ by 1e-3).  Behind a call of many tokens, whose rows lie in bf16."""
+    import torch
+    from rotor_b200 import abi
+    g, width = np.random.default_rng(n), 232
+    m = M.make(M.config([M.window(4, mlp=M.experts(n, top, ff))], width=width, vocab=8), seed=1)
+    model = M.load(m, dtype="bfloat16", max_seq=9, max_rows=9)
+    cfg, layer = model._ensure_handle(1, 9, 9).cfg, model._layers[0]
+    need = abi.lib.rotor_b200_decoder_layer_workspace_bytes(C.byref(cfg), C.byref(layer))
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    h = dev(bf16(g.standard_normal((9, width))), "bfloat16", ld(width))
+
+    def run(a, b):
+        y = torch.zeros((b - a, ld(width)), device="cuda")
+        abi.check(abi.lib.rotor_b200_experts(C.byref(cfg), C.byref(layer), abi.ptr(h[a:b]), b - a, abi.ptr(y), abi.ptr(ws), need, abi.stream()))
+        abi.device_status()
+        return y.cpu().numpy()
+
+    want = np.concatenate([run(0, 2), run(2, 4)])
+    run(0, 9)
+    for rows in (3, 4):
+        got = run(0, rows)
+        assert not got[:, width:].any()
+        assert rel(got[:, :width], want[:rows, :width]) < 4e-4, rows
+
+
 # ------------------------------------------------------------------------------- whole models
 CONFIGS = {
     "mixed": lambda: M.config([M.window(24), M.window(17, kv_from=0, heads=2, dim=28, vdim=36), M.full(),
