@@ -53,8 +53,8 @@ enum {
 /* GEMV variant selector for rotor_b200_bitlinear_acc */
 enum {
     ROTOR_B200_VARIANT_AUTO = 0,
-    ROTOR_B200_VARIANT_DP4A = 1,   /* integer dot-product lanes, <= 4 columns per pass */
-    ROTOR_B200_VARIANT_MMA = 2     /* int8 tensor-core fragments, 8 columns per pass */
+    ROTOR_B200_VARIANT_DP4A = 1,   /* integer dot-product lanes, <= 4 columns a launch */
+    ROTOR_B200_VARIANT_MMA = 2     /* int8 tensor-core fragments, <= 40 columns a launch */
 };
 
 int rotor_b200_version(void);
@@ -124,7 +124,8 @@ int rotor_b200_quantize_rows(const float* x, size_t m, size_t k, int terms,
 /* ---------------------------------------------------------------- BitLinear (a5, a14)
  * Integer core of TernaryLinear.forward (src/rotor/transformer.py:147-150):
  * acc[c][o] = sum_k xq[c][k] * w[o][k], exact int32, acc is [ncols][out].
- * Any ncols >= 1; columns are processed 8 (MMA) or up to 4 (DP4A) per pass. */
+ * Any ncols >= 1; a launch takes up to 40 (MMA) or 4 (DP4A) columns, AUTO gives
+ * larger counts to the tiled kernels. */
 int rotor_b200_bitlinear_acc(const void* tiles, size_t out, size_t in,
                              const int8_t* xq, const int32_t* xsum, size_t ncols,
                              int32_t* acc, int variant, void* stream);

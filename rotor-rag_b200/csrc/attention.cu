@@ -652,13 +652,14 @@ __global__ void __launch_bounds__(AC_MAX_THREADS) attn_decode_cluster_kernel(con
 // what it copied, once for all H heads: no barrier, and a ring of stages keeps 4 to 8 KB a warp on their way at 128 registers a
 // thread, sixteen warps an SM.  (With the rows requested into registers, twelve warps and half of the bytes: 64 sequences of the XL
 // shape behind 1024 positions 151 us = 3.6 TB/s, now 117 us = 4.6 TB/s.)  Two stages up to four heads (2B shape, 12 layers, 8 / 16
-// sequences 628 / 723 us a step with two, 636 / 730 with three), three above where eight warps a CTA leave the room.  A warp takes four keys at a time: 4 H partial dot products per lane are folded over the lanes by halving (a lane hands over
+// sequences 628 / 723 us a step with two, 636 / 730 with three), three above where eight warps a CTA leave the room.
+// A warp takes four keys at a time: 4 H partial dot products per lane are folded over the lanes by halving (a lane hands over
 // half of its values and keeps the sums of the other half: 31 shuffles for 32 products, after which a lane holds one finished
 // score), so that exponentials are one instruction per 32 scores; the weights return through a line of shared memory.  The warps of
 // a CTA take every W-th group of four keys and merge at the end.  The first keys are requested before the launch wait (cached rows
 // are older than the kernel before this one).
-// A step behind 480 positions, with a finish kernel before, rows through registers and the stage behind merging the runs / here: 2B
-// shape (6 layers) 5 sequences 316 / 271 us, 8 326 / 289, 16 446 / 337, 64 826 / 682; XL shape (2 layers) 8 344 / 309, 64 612 / 531.
+// What one launch gave, both sides with rows through registers still: a step behind 480 positions with a finish kernel before and the
+// stage behind merging the runs / with both in here, 2B shape (6 layers) 5 sequences 316 / 271 us, 8 326 / 289, 16 446 / 337, 64 826 / 682; XL shape (2 layers) 8 344 / 309, 64 612 / 531.
 constexpr int AS_KEYS = 4, AS_MAX_RUNS = 8;
 
 // Outputs that each of `runs` CTAs merges (the last one the rest).

@@ -1,5 +1,4 @@
-// Device bodies of the decode-attention kernel, shared by the stand-alone kernel
-// (attention.cu) and the single-launch generation step (megastep.cu).
+// Device bodies of the decode-attention kernel in attention.cu.
 #pragma once
 #include "model.cuh"
 

@@ -8,11 +8,11 @@
 // of the code is removed by subtracting sum_k xq[c][k] (xsum).
 //
 // Two instruction mixes share the layout:
-//   DP4A : dp4a.u32.s32 lanes, up to 4 columns per pass (decode work is per weight,
+//   DP4A : dp4a.u32.s32 lanes, up to 4 columns a launch (decode work is per weight,
 //          multiply work per weight per column);
 //   MMA  : mma.sync m16n8k32 u8 x s8 -> s32; the tile IS the A fragment, 8 columns
-//          per pass at the cost of one, which also carries the residual terms of the
-//          multi-term activation quantiser.
+//          at the cost of one, which also carries the residual terms of the
+//          multi-term activation quantiser; up to 40 columns a launch.
 #include "gemv_core.cuh"
 #include "leanstage.cuh"
 #include "model.cuh"

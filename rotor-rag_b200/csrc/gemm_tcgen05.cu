@@ -16,7 +16,7 @@
 // the read-back subtracts the token's activation sum.  After the last stage the decoder warps read
 // the accumulators back (tcgen05.ld 32 lanes x 32 columns: a lane holds 32 consecutive outputs of
 // one token) and pass them through a per-warp shared-memory block so that they leave as whole
-// 128-byte rows.  Prompts whose tiles give every pair of SMs work take gemm_pair_kernel below, with further read-backs:
+// 128-byte rows.  Products of more than 128 tokens mostly take gemm_pair_kernel below (takes_pairs), with further read-backs:
 // PAIR_GATED (gate/up product: activation and product, float32 out) and PAIR_QKV (dequantise, rotary, cache append).  When
 // 256-row tiles do not cover the GPU the K range is split over blockIdx.z and the partial sums are added with
 // integer atomics (64-row tiles remain for products too short to split).
@@ -386,7 +386,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_const
 }
 
 // ---------------------------------------------------------------------------------------
-// Products whose 256 x 256 tiles give every pair of SMs work (prompts): a pair of CTAs per tile, tcgen05.mma.cta_group::2
+// Products of more than 128 tokens (takes_pairs; gate/up and q/k/v always): a pair of CTAs per tile, tcgen05.mma.cta_group::2
 // (M = 256 tokens, N = 256 weight rows, K = 32).  Each CTA holds 128 tokens and decodes 128 weight rows; the tensor cores of
 // both SMs read both halves of the weights.  A CTA's accumulator is then 128 lanes x 256 columns, so that two fit tensor memory
 // and the read-back of one tile runs beside the MMAs of the next, and a K step of the pair moves through each SM's shared
@@ -946,7 +946,7 @@ int launch_gemm_tcgen05_gated(const void* tiles, size_t ff, size_t in, const int
 }
 
 // q/k/v product with dequantisation, rotary and the cache append in its read-back: head_dim 128, one
-// activation term per token, enough tokens for 256-row tiles to cover the GPU.
+// activation term per token, more than 128 tokens.
 bool gemm_tcgen05_qkv_supported(size_t dq, size_t dkv, size_t in, int head_dim, int ncols, const void* xq) {
     return head_dim == 128 && dq % 128 == 0 && dkv % 128 == 0 && ncols > 128 &&
            gemm_tcgen05_supported(dq + 2 * dkv, in, ncols, xq);
